@@ -16,10 +16,11 @@
 // IFFT_xy(psi_x) (unnormalised, nx*ny times larger), which the next z pass
 // turns into ifftn(psi_x) with its 1/cells. A z pass that ends a step (no
 // plane pass follows) multiplies by nx*ny on the way out so the state is
-// again in the form a z pass reads. Both components of a cell travel together as one float4
-// (a.re, a.im, b.re, b.im), so every load and store is a 16-byte vector and
-// the nonlinear step sees both components in registers. The FFTs run in
-// shared memory (fft_smem.cuh); each pass reads and writes the state once.
+// again in the form a z pass reads. Both components of a cell travel together as one float4,
+// stored (a.re, b.re, a.im, b.im): the register passes operate on the two components as packed
+// pairs (fft_reg.cuh). Every load and store is a 16-byte vector and the nonlinear step sees both
+// components in registers; the kernels of this file reorder a cell to (a.re, a.im, b.re, b.im)
+// on its way in and back on its way out. The FFTs run in shared memory (fft_smem.cuh); each pass reads and writes the state once.
 #include "engine.h"
 #include "fft_smem.cuh"
 #include "reduce.cuh"
@@ -45,6 +46,9 @@ inline void ztile(const ClassGeom &c, int &tx, int &ty)
     if (ty > c.ny) ty = c.ny;
 }
 
+// (a.re, b.re, a.im, b.im) <-> (a.re, a.im, b.re, b.im)
+__device__ __forceinline__ float4 cell_swap(float4 v) { return make_float4(v.x, v.z, v.y, v.w); }
+
 // ---------------------------------------------------------------- init
 // initializeEnsembles (wigner_kernel.cu:295-317): x-space a = gs + Va eta_a / sqrt(dV),
 // b = Vb eta_b / sqrt(dV), eta = (n0 + i n1) / 2 from Philox or injected.
@@ -66,8 +70,8 @@ __global__ void k_init(float4 *state, int cells, int ne, GroupParamsF gp, const 
             eb = make_float2(0.5f * r[2], 0.5f * r[3]);
         }
         const double2 g = gs[i];
-        state[idx] = make_float4((float)g.x + gp.init_a * ea.x, (float)g.y + gp.init_a * ea.y,
-                                 gp.init_b * eb.x, gp.init_b * eb.y);
+        state[idx] = make_float4((float)g.x + gp.init_a * ea.x, gp.init_b * eb.x,
+                                 (float)g.y + gp.init_a * ea.y, gp.init_b * eb.y);
     }
 }
 
@@ -96,7 +100,7 @@ __global__ void k_init_batched(float4 *state, int cells, int n_traj, const int *
         const float2 ea = make_float2(0.5f * r[0], 0.5f * r[1]);
         const float2 eb = make_float2(0.5f * r[2], 0.5f * r[3]);
         const float2 g = gs_value(static_cast<const T *>(gs_ptrs[grp]), i);
-        state[idx] = make_float4(g.x + P.init_a * ea.x, g.y + P.init_a * ea.y, P.init_b * eb.x, P.init_b * eb.y);
+        state[idx] = make_float4(g.x + P.init_a * ea.x, P.init_b * eb.x, g.y + P.init_a * ea.y, P.init_b * eb.y);
     }
 }
 
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(kThreads) k_ppass(float4 *state, ClassGeom c, 
         const int y = (idx >> c.lx) & (c.ny - 1);
         const int p = idx >> (c.lx + c.ly);
         const int dst = brev_in ? (p * plane + brev_bits(y, c.ly) * c.nx + brev_bits(x, c.lx)) : idx;
-        buf[dst] = g[idx];
+        buf[dst] = cell_swap(g[idx]);
     }
     __syncthreads();
 
@@ -203,7 +207,7 @@ __global__ void __launch_bounds__(kThreads) k_ppass(float4 *state, ClassGeom c, 
         const int y = (idx >> c.lx) & (c.ny - 1);
         const int p = idx >> (c.lx + c.ly);
         const int src = brev_out ? (p * plane + brev_bits(y, c.ly) * c.nx + brev_bits(x, c.lx)) : idx;
-        g[idx] = buf[src];
+        g[idx] = cell_swap(buf[src]);
     }
 }
 
@@ -244,7 +248,8 @@ __global__ void __launch_bounds__(kThreads) k_zpass(float4 *state, ClassGeom c, 
         const int r = idx / tx;
         const int yl = r % ty;
         const int z = r / ty;
-        buf[(yl * tx + xl) * n + brev_bits(z, c.lz)] = g[(size_t)z * plane + (y0 + yl) * c.nx + x0 + xl];
+        buf[(yl * tx + xl) * n + brev_bits(z, c.lz)] =
+            cell_swap(g[(size_t)z * plane + (y0 + yl) * c.nx + x0 + xl]);
     }
     __syncthreads();
 
@@ -310,7 +315,8 @@ __global__ void __launch_bounds__(kThreads) k_zpass(float4 *state, ClassGeom c, 
         const int r = idx / tx;
         const int yl = r % ty;
         const int z = r / ty;
-        g[(size_t)z * plane + (y0 + yl) * c.nx + x0 + xl] = buf[(yl * tx + xl) * n + brev_bits(z, c.lz)];
+        g[(size_t)z * plane + (y0 + yl) * c.nx + x0 + xl] =
+            cell_swap(buf[(yl * tx + xl) * n + brev_bits(z, c.lz)]);
     }
 }
 
@@ -351,7 +357,7 @@ __global__ void k_state_sums(const float4 *__restrict__ state, int cells, int bl
     // plain FP64 sums over a thread's few dozen cells (rounding ~1e-15 relative), compensated across threads
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
     for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        const float4 u = p[i];
+        const float4 u = cell_swap(p[i]);
         const double ax = u.x, ay = u.y, bx = u.z, by = u.w;
         s0 = fma(ax, ax, fma(ay, ay, s0));
         s1 = fma(bx, bx, fma(by, by, s1));
@@ -366,6 +372,12 @@ __global__ void k_state_sums(const float4 *__restrict__ state, int cells, int bl
     KVec<4> r = block_reduce<4>(acc);
     if (threadIdx.x == 0)
         for (int k = 0; k < 4; ++k) part[(size_t)blockIdx.x * 4 + k] = r.v[k].value() * scale;
+}
+
+__global__ void k_swap_cells(float4 *state, size_t n)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        state[i] = cell_swap(state[i]);
 }
 
 __global__ void k_group_reduce(const double *traj_tot, const int *first, const int *count, double *out)
@@ -493,6 +505,14 @@ void fp32_state_sums(const float4 *state, int cells, int n_traj, int blocks, dou
 {
     if (n_traj <= 0) return;
     k_state_sums<<<n_traj * blocks, 256, 0, s>>>(state, cells, blocks, scale, part);
+    g_launches++;
+}
+
+void fp32_swap_cells(float4 *state, size_t n, cudaStream_t s)
+{
+    if (n == 0) return;
+    const size_t blocks = (n + 255) / 256;
+    k_swap_cells<<<(int)(blocks > 148 * 32 ? 148 * 32 : blocks), 256, 0, s>>>(state, n);
     g_launches++;
 }
 

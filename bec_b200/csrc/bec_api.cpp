@@ -2424,8 +2424,8 @@ bec_status bec_get_state(bec_ctx *ctx, int32_t group, int32_t traj, double *ab)
     CKC(cudaStreamSynchronize(s));
     const double inv = 1.0 / ((double)one.nx * one.ny);
     for (int i = 0; i < cells; ++i) {
-        ab[2 * i] = h[i].x * inv; ab[2 * i + 1] = h[i].y * inv;
-        ab[2 * ((size_t)cells + i)] = h[i].z * inv; ab[2 * ((size_t)cells + i) + 1] = h[i].w * inv;
+        ab[2 * i] = h[i].x * inv; ab[2 * i + 1] = h[i].z * inv;
+        ab[2 * ((size_t)cells + i)] = h[i].y * inv; ab[2 * ((size_t)cells + i) + 1] = h[i].w * inv;
     }
     return BEC_OK;
 }
@@ -2455,7 +2455,7 @@ bec_status bec_set_state(bec_ctx *ctx, int32_t group, int32_t traj, const double
     if ((st = batched_resolve(ctx, false))) return st;
     std::vector<float4> h(cells);
     for (int i = 0; i < cells; ++i)
-        h[i] = make_float4((float)ab[2 * i], (float)ab[2 * i + 1], (float)ab[2 * ((size_t)cells + i)],
+        h[i] = make_float4((float)ab[2 * i], (float)ab[2 * ((size_t)cells + i)], (float)ab[2 * i + 1],
                            (float)ab[2 * ((size_t)cells + i) + 1]);
     ClassRec &c = ctx->classes[gr.cls];
     float4 *dst = c.state + (size_t)(gr.local_first + traj) * cells;
@@ -2684,7 +2684,14 @@ bec_status bec_checkpoint_save(bec_ctx *ctx, void *buf, int64_t bytes)
     } else {
         for (auto &c : ctx->classes) {
             const size_t n = sizeof(float4) * (size_t)c.geom.n_traj * c.geom.cells;
-            if (n) CKC(cudaMemcpyAsync(p, c.state, n, cudaMemcpyDeviceToHost, ctx->stream));
+            if (n) {
+                // a checkpoint holds a cell as (a.re, a.im, b.re, b.im)
+                const size_t nc = n / sizeof(float4);
+                fp32_swap_cells(c.state, nc, ctx->stream);
+                const cudaError_t e = cudaMemcpyAsync(p, c.state, n, cudaMemcpyDeviceToHost, ctx->stream);
+                fp32_swap_cells(c.state, nc, ctx->stream);
+                CKC(e);
+            }
             p += n;
         }
     }
@@ -2722,7 +2729,10 @@ bec_status bec_checkpoint_load(bec_ctx *ctx, const void *buf, int64_t bytes)
     } else {
         for (auto &c : ctx->classes) {
             const size_t n = sizeof(float4) * (size_t)c.geom.n_traj * c.geom.cells;
-            if (n) CKC(cudaMemcpyAsync(c.state, p, n, cudaMemcpyHostToDevice, ctx->stream));
+            if (n) {
+                CKC(cudaMemcpyAsync(c.state, p, n, cudaMemcpyHostToDevice, ctx->stream));
+                fp32_swap_cells(c.state, n / sizeof(float4), ctx->stream);
+            }
             p += n;
         }
     }

@@ -22,7 +22,8 @@ BEC_HD float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); 
 BEC_HD double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 BEC_HD float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 
-// float4 holds (a.re, a.im, b.re, b.im): both components of one cell.
+// float4 holds (a.re, a.im, b.re, b.im): both components of one cell (reordered from the stored order by
+// the kernels of batched_fp32.cu).
 BEC_HD float4 pmul(float4 v, float2 w)
 {
     return make_float4(v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x,

@@ -127,6 +127,8 @@ void obs_reduce(const double *obs_partial, int n_traj, int tiles, int nz, const 
 // into part[traj][block][4] (k_obs_reduce's layout with `blocks` tiles and nz = 1)
 void fp32_state_sums(const float4 *state, int cells, int n_traj, int blocks, double scale, double *part,
                      cudaStream_t s);
+// reorders n cells in place between the stored order (a.re, b.re, a.im, b.im) and (a.re, a.im, b.re, b.im)
+void fp32_swap_cells(float4 *state, size_t n, cudaStream_t s);
 void group_reduce(const double *traj_tot, const int *group_first, const int *group_count, int n_groups,
                   double *out, cudaStream_t s);
 

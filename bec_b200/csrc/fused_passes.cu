@@ -11,6 +11,7 @@
 
 namespace {
 
+using fftreg::cpair;
 using stepk::PencilArgs;
 using stepk::VBlock;
 
@@ -31,11 +32,11 @@ __device__ __forceinline__ void advance_step_if_last(uint32_t *stepp, int *done)
 }
 
 template <int N, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_plane(float4 *__restrict__ state, int nz, int cells,
+__global__ void __launch_bounds__(128, MINB) k_plane(cpair *__restrict__ state, int nz, int cells,
                                                const GroupParamsF *__restrict__ gp, const int *__restrict__ tgroup,
                                                const int *__restrict__ tlocal, uint32_t *stepp, int *done)
 {
-    extern __shared__ float4 tile[];   // 4 warps x W planes x N^2
+    extern __shared__ cpair tile[];   // 4 warps x W planes x N^2
     stepk::plane_body<N>(VBlock{(int)threadIdx.x, (int)blockIdx.x, 0, 128}, state, nz, cells, gp, tgroup, tlocal,
                          *stepp, tile);
     if (done) advance_step_if_last(stepp, done);
@@ -43,13 +44,13 @@ __global__ void __launch_bounds__(128, MINB) k_plane(float4 *__restrict__ state,
 
 // ---------------------------------------------------------------- plane pass, 32 x 32, two warps a plane
 template <int MINB>
-__global__ void __launch_bounds__(64, MINB) k_plane32s(float4 *__restrict__ state, int nz, int cells,
+__global__ void __launch_bounds__(64, MINB) k_plane32s(cpair *__restrict__ state, int nz, int cells,
                                                       const GroupParamsF *__restrict__ gp,
                                                       const int *__restrict__ tgroup, const int *__restrict__ tlocal,
                                                       uint32_t *stepp, int *done)
 {
-    __shared__ float4 tile[1024];
-    __shared__ float4 xb[512];
+    __shared__ cpair tile[1024];
+    __shared__ cpair xb[512];
     stepk::plane32_body(VBlock{(int)threadIdx.x, (int)blockIdx.x, 0, 64}, state, nz, cells, gp, tgroup, tlocal,
                         *stepp, tile, xb);
     if (done) advance_step_if_last(stepp, done);
@@ -57,13 +58,13 @@ __global__ void __launch_bounds__(64, MINB) k_plane32s(float4 *__restrict__ stat
 
 // ---------------------------------------------------------------- pencil pass
 template <int NZ, bool OBS>
-__global__ void __launch_bounds__(NZ) k_pencil(float4 *__restrict__ state, int nx, int lx, int ny, int cells,
+__global__ void __launch_bounds__(NZ, OBS ? 1 : 512 / NZ) k_pencil(cpair *__restrict__ state, int nx, int lx, int ny, int cells,
                                                int tiles, const GroupParamsF *__restrict__ gp,
                                                const int *__restrict__ tgroup, const float2 *__restrict__ tw_g,
                                                PencilArgs pa, double *__restrict__ obs, float inv_out_scale,
                                                const float2 *__restrict__ kin)
 {
-    extern __shared__ float4 dyn[];
+    extern __shared__ cpair dyn[];
     stepk::pencil_body<NZ, OBS>(VBlock{(int)threadIdx.x, (int)blockIdx.x, 0, NZ}, state, nx, lx, ny, cells, tiles,
                                 gp, tgroup, tw_g, pa, obs, inv_out_scale, kin, dyn);
 }
@@ -90,7 +91,7 @@ __global__ void k_kin_tables(float2 *__restrict__ tab, const GroupParamsF *__res
 }
 
 template <int NZ, bool OBS>
-void launch_pencil(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const float2 *tw,
+void launch_pencil(cpair *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const float2 *tw,
                    const PencilArgs &pa, double *obs, float inv_out_scale, const float2 *kin, cudaStream_t s)
 {
     const int tiles = c.nx * c.ny / 16;
@@ -102,19 +103,19 @@ void launch_pencil(float4 *state, const ClassGeom &c, const GroupParamsF *gp, co
 }
 
 template <int N, int MINB>
-void launch_plane(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
+void launch_plane(cpair *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
                   uint32_t *step, int *done, cudaStream_t s)
 {
     constexpr int W = 32 / N;
     const int planes = c.n_traj * c.nz;
-    const size_t smem = sizeof(float4) * 4 * W * N * N;
+    const size_t smem = sizeof(cpair) * 4 * W * N * N;
     ensure_smem_limit((const void *)k_plane<N, MINB>, (int)smem);
     k_plane<N, MINB><<<planes / (4 * W), 128, smem, s>>>(state, c.nz, c.cells, gp, tgroup, tlocal, step, done);
     g_launches++;
 }
 
 template <int MINB>
-void launch_plane32s(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
+void launch_plane32s(cpair *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
                      uint32_t *step, int *done, cudaStream_t s)
 {
     k_plane32s<MINB><<<c.n_traj * c.nz, 64, 0, s>>>(state, c.nz, c.cells, gp, tgroup, tlocal, step, done);
@@ -140,10 +141,11 @@ int fp32_plane_fast_ctas(const ClassGeom &c)
     return c.nx == 32 ? c.n_traj * c.nz : c.n_traj * c.nz / (4 * (32 / c.nx));
 }
 
-void fp32_plane_fast(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
+void fp32_plane_fast(float4 *cells, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
                      uint32_t *step, int occupancy, int *inc_done, cudaStream_t s)
 {
     if (c.n_traj <= 0) return;
+    cpair *state = reinterpret_cast<cpair *>(cells);
     // occupancy 0: 16 warps per SM (8x8 / 16x16: 4 CTAs of 128 threads; 32x32: 8 CTAs of 64), no register spill;
     // occupancy 1: 20 warps per SM (5 and 10 CTAs), 96 registers with a small spill
     switch (c.nx) {
@@ -173,11 +175,12 @@ void fp32_kin_tables(float2 *tab, const ClassGeom &c, const GroupParamsF *gp, co
     g_launches++;
 }
 
-void fp32_pencil_fast(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup,
+void fp32_pencil_fast(float4 *cells, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup,
                       const float2 *tw_full, float frac, float scale, const float2 *m, double *obs,
                       float out_scale, const float2 *kin, cudaStream_t s)
 {
     if (c.n_traj <= 0) return;
+    cpair *state = reinterpret_cast<cpair *>(cells);
     PencilArgs pa{};
     pa.frac = frac;
     pa.scale = scale;

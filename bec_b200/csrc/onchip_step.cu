@@ -13,18 +13,19 @@
 
 namespace {
 
+using fftreg::cpair;
 using stepk::PencilArgs;
 using stepk::VBlock;
 using stepk::ZTile;
 
 constexpr int NZ = 64, PLANE = 64, CELLS = NZ * PLANE, kThreads = 128;
-constexpr size_t kSmem = sizeof(float4) * CELLS + sizeof(float2) * (NZ + NZ + PLANE);
+constexpr size_t kSmem = sizeof(cpair) * CELLS + sizeof(float2) * (NZ + NZ + PLANE);
 
 // ZTile's buffer over 16 pencils of the resident state: buffer index e -> row z = e / 16, pencil p0 + e % 16
 struct PencilRegion {
-    float4 *st;
+    cpair *st;
     int p0;
-    __device__ __forceinline__ float4 &operator()(int e) const { return st[(e >> 4) * PLANE + p0 + (e & 15)]; }
+    __device__ __forceinline__ cpair &operator()(int e) const { return st[(e >> 4) * PLANE + p0 + (e & 15)]; }
 };
 
 __device__ __forceinline__ void group_sync(int grp)
@@ -39,7 +40,7 @@ __device__ __forceinline__ void copy_async16(void *dst_smem, const void *src)
 }
 
 // done != NULL: the last CTA also advances the Philox step index (every CTA read it at its start)
-__global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(float4 *__restrict__ state,
+__global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(cpair *__restrict__ state,
                                                              const GroupParamsF *__restrict__ gp,
                                                              const int *__restrict__ tgroup,
                                                              const int *__restrict__ tlocal,
@@ -47,12 +48,12 @@ __global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(float4 *__restric
                                                              const float2 *__restrict__ kin, float scale,
                                                              uint32_t *stepp, int *done)
 {
-    extern __shared__ float4 st[];
+    extern __shared__ cpair st[];
     float2 *tw = reinterpret_cast<float2 *>(st + CELLS);
     float2 *kzp = tw + NZ;
     float2 *kxyp = kzp + NZ;
     const int t = threadIdx.x, traj = blockIdx.x;
-    float4 *__restrict__ g = state + (size_t)traj * CELLS;
+    cpair *__restrict__ g = state + (size_t)traj * CELLS;
     const uint32_t step = *stepp;
 
     // W_64^e, this trajectory's kz and (kx, ky) kinetic factors (full kick), and the state, by asynchronous copies
@@ -80,13 +81,13 @@ __global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(float4 *__restric
     for (int round = 0; round < 2; ++round) {
         const int p0 = 16 * (2 * round + grp);
         const PencilRegion R{st, p0};
-        float4 x[16];
+        cpair x[16];
 #pragma unroll
         for (int m = 0; m < 16; ++m) x[m] = st[(j + 4 * m) * PLANE + p0 + p];
         group_sync(grp);                         // the tile is read before it is overwritten
         Z::inv1(x, R, tw, p, j);
         group_sync(grp);
-        float4 y[16];
+        cpair y[16];
         const float2 kp = kxyp[p0 + p2];
         Z::mid(y, R, tw, kzp, make_float2(pa.scale * kp.x, pa.scale * kp.y), pa, q, p2);
         group_sync(grp);                         // stage-2 reads done
@@ -126,12 +127,12 @@ __global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(float4 *__restric
 
 bool fp32_onchip_supported(const ClassGeom &c) { return c.nx == 8 && c.ny == 8 && c.nz == 64 && c.n_traj > 0; }
 
-void fp32_onchip_step(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
+void fp32_onchip_step(float4 *cells, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
                       const float2 *tw_full, const float2 *kin_full, uint32_t *d_step, int *inc_done, cudaStream_t s)
 {
     if (c.n_traj <= 0) return;
     ensure_smem_limit((const void *)k_onchip_8x8x64, (int)kSmem);
-    k_onchip_8x8x64<<<c.n_traj, kThreads, kSmem, s>>>(state, gp, tgroup, tlocal, tw_full, kin_full,
+    k_onchip_8x8x64<<<c.n_traj, kThreads, kSmem, s>>>(reinterpret_cast<cpair *>(cells), gp, tgroup, tlocal, tw_full, kin_full,
                                                        1.0f / (float)c.cells, d_step, inc_done);
     g_launches++;
 }

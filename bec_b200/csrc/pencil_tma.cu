@@ -30,6 +30,7 @@
 
 namespace {
 
+using fftreg::cpair;
 using stepk::PencilArgs;
 using stepk::ZTile;
 
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_pencil_tma(const __grid_constan
     static_assert(PEN * G == kThreads && PEN * NZ * 16 == kTileBytes, "tile shape");
     using Z = ZTile<NZ, PEN>;
     extern __shared__ __align__(1024) unsigned char smem[];
-    float4 *bufs = reinterpret_cast<float4 *>(smem);
+    cpair *bufs = reinterpret_cast<cpair *>(smem);
     float2 *tw = reinterpret_cast<float2 *>(smem + 2 * kTileBytes);
     float2 *kzp = tw + NZ;
     float2 *kxyp = kzp + NZ;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_pencil_tma(const __grid_constan
     for (int i = first; i < last; ++i) {
         const int b = (i - first) & 1;
         const uint32_t parity = (uint32_t)((i - first) >> 1) & 1u;
-        float4 *B = bufs + b * (kTileBytes / 16);
+        cpair *B = bufs + b * (kTileBytes / 16);
         const int traj = i / A.tiles_per_traj;
         const int pen0 = (i - traj * A.tiles_per_traj) * PEN;
         // this tile's kinetic factors: the kz table when the trajectory changes, the pencils' every tile
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_pencil_tma(const __grid_constan
 
         bool ok = mbar_wait_bounded(&full[b], parity, A.wait_limit_ns);
         if (A.stall && i == first && ok) ok = wait_never(A.never, A.wait_limit_ns);
-        float4 x[R];
+        cpair x[R];
 #pragma unroll
         for (int m = 0; m < R; ++m) x[m] = B[(j + G * m) * PEN + p];
         if (!ok) *abort_flag = 1;
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_pencil_tma(const __grid_constan
         Z::inv1(x, B, tw, p, j);
         stepk::copy_async_wait();
         __syncthreads();
-        float4 y[R];
+        cpair y[R];
         const float2 kp = kxyp[p2];
         Z::mid(y, B, tw, kzp, make_float2(A.pa.scale * kp.x, A.pa.scale * kp.y), A.pa, q, p2);
         __syncthreads();                                   // stage-2 reads done

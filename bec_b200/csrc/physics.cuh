@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "engine.h"
+#include "fft_reg.cuh"
 
 // Per-thread constants of a trajectory's cell step, computed once per thread from its GroupParamsF:
 // the nonlinear coefficients scaled by dt/2 and the squared loss-noise amplitudes.
@@ -67,96 +68,98 @@ __device__ __forceinline__ float2 box_muller21_scaled(uint32_t f1, uint32_t f2, 
 //     cos to t^8 (<= 0.5^10/10! = 2.7e-10), both below half an FP32 ulp of the result;
 //   exp x: Taylor to x^3 for |x| <= 1/64 (truncation <= (1/64)^4/4! = 2.5e-9).
 // Arguments outside those ranges take sincosf / expf; one branch covers all four arguments of a cell.
-__device__ __forceinline__ float2 cis_taylor(float t)
+// Both components of the cell at once, in packed pairs (fft_reg.cuh).
+__device__ __forceinline__ void cis_taylor2(fftreg::f32x2 t, fftreg::f32x2 &c, fftreg::f32x2 &s)
 {
-    const float u = t * t;
-    const float s = fmaf(t * u, fmaf(u, fmaf(u, -1.f / 5040.f, 1.f / 120.f), -1.f / 6.f), t);
-    const float c = fmaf(u, fmaf(u, fmaf(u, fmaf(u, 1.f / 40320.f, -1.f / 720.f), 1.f / 24.f), -0.5f), 1.f);
-    return make_float2(c, s);
+    using namespace fftreg;
+    const f32x2 u = mul2(t, t);
+    s = fma2(mul2(t, u), fma2(u, fma2(u, both(-1.f / 5040.f), both(1.f / 120.f)), both(-1.f / 6.f)), t);
+    c = fma2(u, fma2(u, fma2(u, fma2(u, both(1.f / 40320.f), both(-1.f / 720.f)), both(1.f / 24.f)), both(-0.5f)),
+             both(1.f));
 }
 
-__device__ __forceinline__ float exp_taylor(float x) { return fmaf(x, fmaf(x, fmaf(x, 1.f / 6.f, 0.5f), 1.f), 1.f); }
-
-// |v|^2 and complex products with every fused multiply-add written out, so that every kernel that inlines the
-// cell step rounds it the same way (the contraction of a*b + c*d left to the compiler can differ between them)
-__device__ __forceinline__ float nrm2(float2 v) { return fmaf(v.x, v.x, v.y * v.y); }
-__device__ __forceinline__ float2 cmulx(float2 a, float2 b)
+__device__ __forceinline__ fftreg::f32x2 exp_taylor2(fftreg::f32x2 x)
 {
-    return make_float2(fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x));
+    using namespace fftreg;
+    return fma2(x, fma2(x, fma2(x, both(1.f / 6.f), both(0.5f)), both(1.f)), both(1.f));
 }
 
-// The substep's factors da, db from the midpoint estimate (xa, xb).
-__device__ __forceinline__ void nonlinear_factors(float2 xa, float2 xb, float hV, float hVd, const CellConsts &K,
-                                                  float2 &da, float2 &db)
+// The substep's factor pair (da, db) from the midpoint estimate x = (xa, xb): real parts, imaginary parts and
+// negated imaginary parts. Every fused multiply-add is written out, so that every kernel that inlines the cell
+// step rounds it the same way.
+struct CellFactor {
+    fftreg::f32x2 re, im, nim;
+};
+__device__ __forceinline__ CellFactor nonlinear_factors(const fftreg::cpair &x, float hV, float hVd, const CellConsts &K)
 {
-    const float na = nrm2(xa);
-    const float nb = nrm2(xb);
+    using namespace fftreg;
+    const f32x2 n = fma2(x.re, x.re, mul2(x.im, x.im));
+    const float na = unpack2(n).x, nb = unpack2(n).y;
     const float ra = fmaf(K.hl111 * na, na, K.hl12 * nb);
     const float rb = fmaf(K.hl22, nb, K.hl12 * na);
     const float ta = fmaf(K.hg11, na, fmaf(K.hg12, nb, hV));
     const float tb = fmaf(K.hg22, nb, fmaf(K.hg12, na, hVd));
-    float2 ea, eb;
-    float ma, mb;
+    f32x2 c, s, m;
     if (fmaxf(fabsf(ta), fabsf(tb)) <= 0.5f && fmaxf(fabsf(ra), fabsf(rb)) <= 0.015625f) {
-        ea = cis_taylor(ta);
-        eb = cis_taylor(tb);
-        ma = exp_taylor(ra);
-        mb = exp_taylor(rb);
+        cis_taylor2(pack2(ta, tb), c, s);
+        m = exp_taylor2(pack2(ra, rb));
     } else {
+        float2 ea, eb;
         sincosf(ta, &ea.y, &ea.x);
         sincosf(tb, &eb.y, &eb.x);
-        ma = expf(ra);
-        mb = expf(rb);
+        c = pack2(ea.x, eb.x);
+        s = pack2(ea.y, eb.y);
+        m = pack2(expf(ra), expf(rb));
     }
-    da = make_float2(ma * ea.x, ma * ea.y);
-    db = make_float2(mb * eb.x, mb * eb.y);
+    return CellFactor{mul2(m, c), mul2(m, s), mul2(mul2(m, both(-1.f)), s)};
 }
 
 // One cell: v = (a, b) at the start of the substep, V the trap potential.
-__device__ __forceinline__ float4 nonlinear_cell(float4 v, float V, const CellConsts &K)
+__device__ __forceinline__ fftreg::cpair nonlinear_cell(const fftreg::cpair &v, float V, const CellConsts &K)
 {
-    const float2 a0 = make_float2(v.x, v.y), b0 = make_float2(v.z, v.w);
+    using namespace fftreg;
     const float hV = __fmul_rn(V, K.hdt), hVd = __fsub_rn(hV, K.hdet);   // never contracted
-    float2 da, db;
+    CellFactor d;
     if (K.itmax == 1) {
         // one midpoint iteration (every workload here): the factors of the start values, applied twice
-        nonlinear_factors(a0, b0, hV, hVd, K, da, db);
-        const float2 ao = cmulx(cmulx(a0, da), da), bo = cmulx(cmulx(b0, db), db);
-        return make_float4(ao.x, ao.y, bo.x, bo.y);
+        d = nonlinear_factors(v, hV, hVd, K);
+        return cmul2(cmul2(v, d.re, d.im, d.nim), d.re, d.im, d.nim);
     }
-    float2 xa = a0, xb = b0;
-    da = db = make_float2(0.f, 0.f);
+    cpair x = v;
+    d = CellFactor{0, 0, 0};
     for (int it = 0; it < K.itmax; ++it) {
-        nonlinear_factors(xa, xb, hV, hVd, K, da, db);
-        xa = cmulx(a0, da);
-        xb = cmulx(b0, db);
+        d = nonlinear_factors(x, hV, hVd, K);
+        x = cmul2(v, d.re, d.im, d.nim);
     }
-    const float2 ao = cmulx(xa, da), bo = cmulx(xb, db);
-    return make_float4(ao.x, ao.y, bo.x, bo.y);
+    return cmul2(x, d.re, d.im, d.nim);
 }
 
 // The loss-noise increment of one cell from its Philox output, accumulated into out as FMA chains:
 //   a += conj(a0)^2 w1 + conj(b0) w2,  b += conj(a0) w2 + conj(b0) w3.
-__device__ __forceinline__ float4 loss_noise_apply(float4 out, float4 v0, const CellConsts &K, u32x4 w)
+__device__ __forceinline__ fftreg::cpair loss_noise_apply(const fftreg::cpair &o, const fftreg::cpair &v0,
+                                                          const CellConsts &K, u32x4 w)
 {
     uint32_t f[6];
     loss_fields(w, f);
     const float2 w1 = box_muller21_scaled(f[0], f[1], K.n1);
     const float2 w2 = box_muller21_scaled(f[2], f[3], K.n2);
     const float2 w3 = box_muller21_scaled(f[4], f[5], K.n3);
-    const float ax = v0.x, ay = v0.y, bx = v0.z, by = v0.w;
+    const float2 a = fftreg::comp_a(v0), b = fftreg::comp_b(v0), oa = fftreg::comp_a(o), ob = fftreg::comp_b(o);
+    const float ax = a.x, ay = a.y, bx = b.x, by = b.y;
     const float qx = fmaf(ax, ax, -ay * ay), qy = -2.f * ax * ay;       // conj(a0)^2
-    return make_float4(fmaf(qx, w1.x, fmaf(-qy, w1.y, fmaf(bx, w2.x, fmaf(by, w2.y, out.x)))),
-                       fmaf(qx, w1.y, fmaf(qy, w1.x, fmaf(bx, w2.y, fmaf(-by, w2.x, out.y)))),
-                       fmaf(ax, w2.x, fmaf(ay, w2.y, fmaf(bx, w3.x, fmaf(by, w3.y, out.z)))),
-                       fmaf(ax, w2.y, fmaf(-ay, w2.x, fmaf(bx, w3.y, fmaf(-by, w3.x, out.w)))));
+    return fftreg::make_cpair(
+        make_float2(fmaf(qx, w1.x, fmaf(-qy, w1.y, fmaf(bx, w2.x, fmaf(by, w2.y, oa.x)))),
+                    fmaf(qx, w1.y, fmaf(qy, w1.x, fmaf(bx, w2.y, fmaf(-by, w2.x, oa.y))))),
+        make_float2(fmaf(ax, w2.x, fmaf(ay, w2.y, fmaf(bx, w3.x, fmaf(by, w3.y, ob.x)))),
+                    fmaf(ax, w2.y, fmaf(-ay, w2.x, fmaf(bx, w3.y, fmaf(-by, w3.x, ob.y))))));
 }
 
 // Adds the loss-noise increments of two cells of the same trajectory and step, evaluated at v0 and v1, to
 // out0 and out1: per cell the six normals of one Philox4x32-10 draw (loss_fields) as three complex Wiener
 // increments already scaled by their amplitudes. The two draws' rounds interleave; keys: the round keys of
 // the ensemble seed (philox_keys).
-__device__ __forceinline__ void loss_noise_cell2(float4 &out0, float4 v0, float4 &out1, float4 v1, const CellConsts &K,
+__device__ __forceinline__ void loss_noise_cell2(fftreg::cpair &out0, const fftreg::cpair &v0, fftreg::cpair &out1,
+                                                 const fftreg::cpair &v1, const CellConsts &K,
                                                  const PhiloxKeys &keys, uint32_t traj, uint32_t step,
                                                  uint32_t cell0, uint32_t cell1)
 {
@@ -168,7 +171,7 @@ __device__ __forceinline__ void loss_noise_cell2(float4 &out0, float4 v0, float4
 
 // The loss-noise increments of four consecutive cells cell0 .. cell0 + 3 of the same trajectory and step:
 // one interleaved group of four Philox4x32-10 draws.
-__device__ __forceinline__ void loss_noise_cell4(float4 out[4], const float4 v0[4], const CellConsts &K,
+__device__ __forceinline__ void loss_noise_cell4(fftreg::cpair out[4], const fftreg::cpair v0[4], const CellConsts &K,
                                                  const PhiloxKeys &keys, uint32_t traj, uint32_t step, uint32_t cell0)
 {
     const u32x4x4 w = philox4x32_10_x4(cell0, step, traj, RNG_TAG_LOSS, keys);

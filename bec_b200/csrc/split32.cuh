@@ -7,8 +7,7 @@
 // frequency with the conjugate twiddles: block layout in, x[2m + h] out, which is the layout the next
 // forward step expects. (Written as conj(FFT(conj v)) instead, the sign flips cost the real-time plane
 // pass a 52-byte register spill and 4 % of its time.) tix() is the XOR swizzle of a 32 x 32 shared tile.
-// Elements are float4 (the two components of a cell, real-time passes) or float2 (one component,
-// imaginary-time passes).
+// Elements are cpair (the two components of a cell, real-time passes) or float2 (one component).
 #pragma once
 
 #include <utility>
@@ -20,18 +19,17 @@ namespace split32 {
 __device__ __forceinline__ int kblk(int s, int h) { return s < 8 ? s + 8 * h : s + 8 + 8 * h; }
 __device__ __forceinline__ int tix(int row, int col) { return row * 32 + (col ^ (row & 7)); }
 
-// v * e^{-2 pi i K / 32} (v * e^{+2 pi i K / 32} when INV)
-template <int K, bool INV = false, typename T>
-__device__ __forceinline__ T w32(T v)
+// (x - y) e^{+2 pi i K / 32}
+template <int K, typename T>
+__device__ __forceinline__ T sub_w32(T x, T y)
 {
     if constexpr (K == 0) {
-        return v;
+        return fftreg::sub(x, y);
     } else if constexpr (K == 8) {
-        return INV ? fftreg::mul_posi(v) : fftreg::mul_negi(v);
+        return fftreg::sub_posi(x, y);
     } else {
-        constexpr fftreg::Twid t =
-            fftreg::unit_cs(fftreg::cos_2pi(K, 32), INV ? fftreg::sin_2pi(K, 32) : -fftreg::sin_2pi(K, 32));
-        return fftreg::cmulc(v, t.a, t.b);
+        constexpr fftreg::Twid t = fftreg::unit_cs(fftreg::cos_2pi(K, 32), fftreg::sin_2pi(K, 32));
+        return fftreg::cmulc(fftreg::sub(x, y), t.a, t.b);
     }
 }
 
@@ -46,10 +44,11 @@ __device__ __forceinline__ void dit_recv_one(T *v, const T *xi)
     const T e = H == 0 ? v[I] : r;
     const T o = H == 0 ? r : v[8 + I];
     constexpr int K = H == 0 ? I : 8 + I;
-    if constexpr (K == 0 || K == 8) {
-        const T t = w32<K>(o);
-        v[I] = fftreg::add(e, t);
-        v[8 + I] = fftreg::sub(e, t);
+    if constexpr (K == 0) {
+        v[I] = fftreg::add(e, o);
+        v[8 + I] = fftreg::sub(e, o);
+    } else if constexpr (K == 8) {
+        fftreg::bfly_i<false>(v[I], v[8 + I], e, o);
     } else {
         fftreg::bfly_w<K, 32, false>(v[I], v[8 + I], e, o);
     }
@@ -60,7 +59,7 @@ template <int H, int I, typename T>
 __device__ __forceinline__ void dif_send_one(T *v, T *xo)
 {
     const T a = fftreg::add(v[I], v[8 + I]);
-    const T b = w32<H == 0 ? I : 8 + I, true>(fftreg::sub(v[I], v[8 + I]));
+    const T b = sub_w32<H == 0 ? I : 8 + I>(v[I], v[8 + I]);
     if constexpr (H == 0) {
         v[I] = a;
         xo[I * 32] = b;

@@ -16,7 +16,7 @@
 //   plane from HBM (each load instruction of the warp reads consecutive 16-byte cells), transforms it
 //   along y, writes it to an XOR-swizzled shared tile, reads back row c, transforms along x, applies
 //   the nonlinear / loss / loss-noise step to its N cells, and returns the same way. Both components of
-//   a cell are one float4.
+//   a cell are one 16-byte cpair (fft_reg.cuh).
 // plane pass, 32 x 32 planes: two warps per plane, a 32-point line shared by lane L of each warp
 //   (split32.cuh).
 // pencil pass (nz = 64, 128, 256 = 16 G): 16 adjacent pencils of a trajectory per virtual block of
@@ -40,7 +40,16 @@
 
 namespace stepk {
 
+using fftreg::cpair;
 using fftreg::dft;
+using fftreg::f32x2;
+
+// a cell from L2 (ld.global.cg)
+__device__ __forceinline__ cpair ld_cg(const cpair *p)
+{
+    const ulonglong2 u = __ldcg(reinterpret_cast<const ulonglong2 *>(p));
+    return cpair{u.x, u.y};
+}
 
 // A group of nthr consecutive threads of a CTA acting as one block.
 struct VBlock {
@@ -56,13 +65,13 @@ struct VBlock {
 };
 
 // ---------------------------------------------------------------- plane pass, N = 8, 16
-// 4 warps (128 threads); tile: 4 warps x (32 / N) planes x N^2 float4
+// 4 warps (128 threads); tile: 4 warps x (32 / N) planes x N^2 cells
 // SMEM: `state` is a trajectory held in shared memory and `tile` is the same memory (the transposes run in
 // place): plain loads instead of L2-only ones, and the warp's loads all done before its first store.
 template <int N, bool SMEM = false>
-__device__ __forceinline__ void plane_body(const VBlock &vb, float4 *__restrict__ state, int nz, int cells,
+__device__ __forceinline__ void plane_body(const VBlock &vb, cpair *__restrict__ state, int nz, int cells,
                                            const GroupParamsF *__restrict__ gp, const int *__restrict__ tgroup,
-                                           const int *__restrict__ tlocal, uint32_t step, float4 *tile)
+                                           const int *__restrict__ tlocal, uint32_t step, cpair *tile)
 {
     constexpr int W = 32 / N;          // planes per warp
     constexpr int PLANE = N * N;
@@ -70,14 +79,14 @@ __device__ __forceinline__ void plane_body(const VBlock &vb, float4 *__restrict_
     const int wp = lane / N, c = lane % N;
     const int plane_id = (vb.bid * 4 + warp) * W + wp;
     const int traj = plane_id / nz, z = plane_id - traj * nz;
-    float4 *__restrict__ g = state + (size_t)traj * cells + (size_t)z * PLANE;
-    float4 *s = tile + (warp * W + wp) * PLANE;
+    cpair *__restrict__ g = state + (size_t)traj * cells + (size_t)z * PLANE;
+    cpair *s = tile + (warp * W + wp) * PLANE;
 
     const GroupParamsF P = gp[tgroup[traj]];
 
-    float4 v[N];
+    cpair v[N];
 #pragma unroll
-    for (int y = 0; y < N; ++y) v[y] = SMEM ? g[y * N + c] : __ldcg(g + y * N + c);
+    for (int y = 0; y < N; ++y) v[y] = SMEM ? g[y * N + c] : ld_cg(g + y * N + c);
     if (SMEM) __syncwarp();
 
     // Four transforms share one loop body (the kernel is otherwise bound by
@@ -110,7 +119,7 @@ __device__ __forceinline__ void plane_body(const VBlock &vb, float4 *__restrict_
             // cells in fours: the four Philox draws interleave (loss_noise_cell4)
 #pragma unroll 1
             for (int x = 0; x < N; x += 4) {
-                float4 v0[4], o[4];
+                cpair v0[4], o[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float X = fmaf(P.dx, (float)(x + q), -P.xmax);
@@ -139,27 +148,27 @@ __device__ __forceinline__ void plane_body(const VBlock &vb, float4 *__restrict_
 
 // ---------------------------------------------------------------- plane pass, 32 x 32, two warps a plane
 // 64 threads; every 32-point line is shared by lane L of warp 0 and lane L of warp 1, 16 elements
-// each, half the registers of a one-lane line, so more warps fit on an SM. tile: 1024 float4 (the
-// plane, swizzled like plane_body's), xb: 512 float4 (the line exchange slots).
-__device__ __forceinline__ void plane32_body(const VBlock &vb, float4 *__restrict__ state, int nz, int cells,
+// each, half the registers of a one-lane line, so more warps fit on an SM. tile: 1024 cells (the
+// plane, swizzled like plane_body's), xb: 512 cells (the line exchange slots).
+__device__ __forceinline__ void plane32_body(const VBlock &vb, cpair *__restrict__ state, int nz, int cells,
                                              const GroupParamsF *__restrict__ gp, const int *__restrict__ tgroup,
-                                             const int *__restrict__ tlocal, uint32_t step, float4 *tile, float4 *xb)
+                                             const int *__restrict__ tlocal, uint32_t step, cpair *tile, cpair *xb)
 {
     using namespace split32;
     const int h = vb.tid >> 5, lane = vb.tid & 31;
     const int plane_id = vb.bid;
     const int traj = plane_id / nz, z = plane_id - traj * nz;
-    float4 *__restrict__ g = state + (size_t)traj * cells + (size_t)z * 1024;
+    cpair *__restrict__ g = state + (size_t)traj * cells + (size_t)z * 1024;
     const GroupParamsF P = gp[tgroup[traj]];
     auto bar = [&vb]() { vb.sync(); };
 
-    float4 v[16];
+    cpair v[16];
     // forward along y (lane = column), then along x (lane = row); shared code body
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
         if (pass == 0) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __ldcg(g + (2 * j + h) * 32 + lane);
+            for (int j = 0; j < 16; ++j) v[j] = ld_cg(g + (2 * j + h) * 32 + lane);
         } else {
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = tile[tix(lane, 2 * j + h)];
@@ -190,10 +199,10 @@ __device__ __forceinline__ void plane32_body(const VBlock &vb, float4 *__restric
         for (int s = 0; s < 16; s += 2) {
             const int x = kblk(s, h);
             const float X0 = fmaf(P.dx, (float)x, -P.xmax), X1 = fmaf(P.dx, (float)(x + 1), -P.xmax);
-            float4 *s0 = tile + tix(r, x), *s1 = tile + tix(r, x + 1);
-            const float4 v0 = *s0, v1 = *s1;
-            float4 o0 = nonlinear_cell(v0, 0.5f * fmaf(X0, X0, base), K);
-            float4 o1 = nonlinear_cell(v1, 0.5f * fmaf(X1, X1, base), K);
+            cpair *s0 = tile + tix(r, x), *s1 = tile + tix(r, x + 1);
+            const cpair v0 = *s0, v1 = *s1;
+            cpair o0 = nonlinear_cell(v0, 0.5f * fmaf(X0, X0, base), K);
+            cpair o1 = nonlinear_cell(v1, 0.5f * fmaf(X1, X1, base), K);
             if (P.noise)
                 loss_noise_cell2(o0, v0, o1, v1, K, keys, tl, step, cell0 + x, cell0 + x + 1);
             *s0 = o0;
@@ -238,18 +247,18 @@ struct PencilArgs {
 };
 
 // The four-step z transform of a tile of PEN adjacent pencils (nz = 16 G; PEN * G threads), in three
-// stages separated by barriers of the tile's threads. buf holds PEN x NZ float4 (swizzled rows of 16).
+// stages separated by barriers of the tile's threads. buf holds PEN x NZ cells (swizzled rows of 16).
 //   inv1:  thread (p, j) = (t % PEN, t / PEN) holds z = j + G m, m < 16: inverse 16-point DFT over
 //          m -> k1, twiddle W^{-j k1}, to buf
 //   mid:   thread (q, p2) = (t % G, t / G) gathers k1 = q + G r (r < 16 / G) for all j: inverse G-point
 //          DFT over j -> k2 (k = k1 + 16 k2), kinetic phase (and pulse), forward G-point DFT, twiddle;
 //          mid_store writes it back after the caller's barrier
 //   fwd3:  thread (p, j) gathers its k1 < 16 and finishes with the forward 16-point DFT over k1 -> m
-// The buffer is a float4 pointer or an accessor (a functor mapping the buffer index to a float4 slot, e.g.
+// The buffer is a cell pointer or an accessor (a functor mapping the buffer index to a cell slot, e.g.
 // into a tile of a state held in shared memory).
-__device__ __forceinline__ float4 &zat(float4 *b, int i) { return b[i]; }
+__device__ __forceinline__ cpair &zat(cpair *b, int i) { return b[i]; }
 template <class F>
-__device__ __forceinline__ float4 &zat(const F &f, int i) { return f(i); }
+__device__ __forceinline__ cpair &zat(const F &f, int i) { return f(i); }
 
 template <int NZ, int PEN>
 struct ZTile {
@@ -259,7 +268,7 @@ struct ZTile {
     __device__ static __forceinline__ int bix(int p, int jj, int k1) { return (p * G + jj) * R + (k1 ^ (p & 7)); }
 
     template <class Buf>
-    __device__ static __forceinline__ void inv1(float4 (&x)[R], Buf buf, const float2 *tw, int p, int j)
+    __device__ static __forceinline__ void inv1(cpair (&x)[R], Buf buf, const float2 *tw, int p, int j)
     {
         dft<R, true>(x);                                            // over m -> k1 (inverse)
 #pragma unroll
@@ -273,7 +282,7 @@ struct ZTile {
 
     // pxy: the pencil's (kx, ky) factor times the scale; kzp: the kz factors
     template <class Buf>
-    __device__ static __forceinline__ void mid(float4 (&y)[R], Buf buf, const float2 *tw, const float2 *kzp,
+    __device__ static __forceinline__ void mid(cpair (&y)[R], Buf buf, const float2 *tw, const float2 *kzp,
                                                float2 pxy, const PencilArgs &pa, int q, int p2)
     {
 #pragma unroll
@@ -291,12 +300,10 @@ struct ZTile {
 #pragma unroll
             for (int k2 = 0; k2 < G; ++k2) {
                 const int k = q + G * r + R * k2;
-                float4 v = fftreg::cmulw(fftreg::cmulw(y[r * G + k2], pxy), kzp[k]);
+                cpair v = fftreg::cmulw(fftreg::cmulw(y[r * G + k2], pxy), kzp[k]);
                 if (pa.has_m) {
-                    const float2 a = make_float2(v.x, v.y), b = make_float2(v.z, v.w);
-                    const float2 an = fftreg::cmix(pa.m[0], a, pa.m[1], b);
-                    const float2 bn = fftreg::cmix(pa.m[2], a, pa.m[3], b);
-                    v = make_float4(an.x, an.y, bn.x, bn.y);
+                    const float2 a = fftreg::comp_a(v), b = fftreg::comp_b(v);
+                    v = fftreg::make_cpair(fftreg::cmix(pa.m[0], a, pa.m[1], b), fftreg::cmix(pa.m[2], a, pa.m[3], b));
                 }
                 y[r * G + k2] = v;
             }
@@ -310,7 +317,7 @@ struct ZTile {
     }
 
     template <class Buf>
-    __device__ static __forceinline__ void mid_store(const float4 (&y)[R], Buf buf, int q, int p2)
+    __device__ static __forceinline__ void mid_store(const cpair (&y)[R], Buf buf, int q, int p2)
     {
 #pragma unroll
         for (int r = 0; r < R / G; ++r)
@@ -319,7 +326,7 @@ struct ZTile {
     }
 
     template <class Buf>
-    __device__ static __forceinline__ void fwd3(float4 (&x)[R], Buf buf, int p, int j)
+    __device__ static __forceinline__ void fwd3(cpair (&x)[R], Buf buf, int p, int j)
     {
 #pragma unroll
         for (int k1 = 0; k1 < R; ++k1) x[k1] = zat(buf, bix(p, j, k1));
@@ -327,28 +334,28 @@ struct ZTile {
     }
 };
 
-// shared memory of one pencil body: 16 pencils x NZ float4, then W_NZ^e, the kz phase and the
+// shared memory of one pencil body: 16 pencils x NZ cells, then W_NZ^e, the kz phase and the
 // per-pencil (kx, ky) phase (float2 each)
 template <int NZ>
-__host__ __device__ constexpr size_t pencil_smem_bytes() { return sizeof(float4) * 16 * NZ + sizeof(float2) * (2 * NZ + 16); }
+__host__ __device__ constexpr size_t pencil_smem_bytes() { return sizeof(cpair) * 16 * NZ + sizeof(float2) * (2 * NZ + 16); }
 
 // OBS: the pass ends a step (no plane pass follows) and also writes, per z, the
 // FP64 sums over the tile's 16 pencils of |a|^2, |b|^2 and conj(a) b of the
 // z-transformed boundary state: obs[((traj * tiles + tile) * NZ + z) * 4 + k].
 // NZ threads; dyn: pencil_smem_bytes<NZ>() of shared memory.
 template <int NZ, bool OBS>
-__device__ __forceinline__ void pencil_body(const VBlock &vb, float4 *__restrict__ state, int nx, int lx, int ny,
+__device__ __forceinline__ void pencil_body(const VBlock &vb, cpair *__restrict__ state, int nx, int lx, int ny,
                                             int cells, int tiles, const GroupParamsF *__restrict__ gp,
                                             const int *__restrict__ tgroup, const float2 *__restrict__ tw_g,
                                             const PencilArgs &pa, double *__restrict__ obs, float inv_out_scale,
-                                            const float2 *__restrict__ kin, float4 *dyn)
+                                            const float2 *__restrict__ kin, cpair *dyn)
 {
     using Z = ZTile<NZ, 16>;
     constexpr int R = 16, G = NZ / 16;
     (void)gp; (void)tgroup; (void)lx;
-    float4 *buf = dyn;                                          // 16 pencils x NZ
+    cpair *buf = dyn;                                           // 16 pencils x NZ
     float2 *tw = reinterpret_cast<float2 *>(dyn + 16 * NZ);     // W_NZ^e, e < NZ
-    float2 *kzp = tw + NZ;                                      // kz phase
+    float2 *kzp = tw + NZ;                                       // kz phase
     float2 *kxyp = kzp + NZ;                                    // (kx, ky) phase x scale, per pencil
 
     const int t = vb.tid;
@@ -372,8 +379,8 @@ __device__ __forceinline__ void pencil_body(const VBlock &vb, float4 *__restrict
     }
 
     const int p = t & 15, j = t >> 4;
-    float4 *__restrict__ g = state + (size_t)traj * cells + pen0 + p;
-    float4 x[R];
+    cpair *__restrict__ g = state + (size_t)traj * cells + pen0 + p;
+    cpair x[R];
 #pragma unroll
     for (int m = 0; m < R; ++m) x[m] = g[(size_t)(j + G * m) * plane];
     copy_async_wait();
@@ -383,7 +390,7 @@ __device__ __forceinline__ void pencil_body(const VBlock &vb, float4 *__restrict
     vb.sync();
 
     const int q = t % G, p2 = t / G;
-    float4 y[R];
+    cpair y[R];
     Z::mid(y, buf, tw, kzp, kxyp[p2], pa, q, p2);
     vb.sync();                                                  // stage-2 reads done
     Z::mid_store(y, buf, q, p2);
@@ -393,13 +400,14 @@ __device__ __forceinline__ void pencil_body(const VBlock &vb, float4 *__restrict
     if constexpr (OBS) {
         // the output is out_scale * FFT_z(boundary state); undo the scale for the moments
         vb.sync();                                              // stage-3 reads of buf done
+        float4 *sums = reinterpret_cast<float4 *>(buf);
 #pragma unroll
         for (int m = 0; m < R; ++m) {
-            const float4 v = x[m];
-            const float ax = v.x * inv_out_scale, ay = v.y * inv_out_scale;
-            const float bx = v.z * inv_out_scale, by = v.w * inv_out_scale;
+            const float2 a = fftreg::comp_a(x[m]), b = fftreg::comp_b(x[m]);
+            const float ax = a.x * inv_out_scale, ay = a.y * inv_out_scale;
+            const float bx = b.x * inv_out_scale, by = b.y * inv_out_scale;
             const int z = j + G * m;
-            buf[p * NZ + (z ^ (p & 7))] = make_float4(ax * ax + ay * ay, bx * bx + by * by, ax * bx + ay * by,
+            sums[p * NZ + (z ^ (p & 7))] = make_float4(ax * ax + ay * ay, bx * bx + by * by, ax * bx + ay * by,
                                                       ax * by - ay * bx);
         }
         vb.sync();
@@ -408,7 +416,7 @@ __device__ __forceinline__ void pencil_body(const VBlock &vb, float4 *__restrict
             KSum s0, s1, s2, s3;
 #pragma unroll
             for (int q2 = 0; q2 < 16; ++q2) {
-                const float4 u = buf[q2 * NZ + (z ^ (q2 & 7))];
+                const float4 u = sums[q2 * NZ + (z ^ (q2 & 7))];
                 s0.add(u.x); s1.add(u.y); s2.add(u.z); s3.add(u.w);
             }
             double *o = obs + (((size_t)traj * tiles + tile) * NZ + z) * 4;

@@ -45,12 +45,13 @@
 
 namespace {
 
+using fftreg::cpair;
 using stepk::PencilArgs;
 using stepk::VBlock;
 
 constexpr int kThreads = 256;
 constexpr int kPlane32PerItem = 4;                              // 64-thread virtual blocks
-constexpr size_t kSmemPlane32 = sizeof(float4) * 1536;          // tile + exchange slots of one plane
+constexpr size_t kSmemPlane32 = sizeof(cpair) * 1536;          // tile + exchange slots of one plane
 constexpr size_t kSmemBytes = kSmemPlane32 * kPlane32PerItem;   // 96 KiB: the largest item's need
 
 enum { ITEM_PENCIL = 0, ITEM_PLANE = 1 };
@@ -71,43 +72,43 @@ __device__ __forceinline__ int load_acquire(const int *p)
 
 template <int NZ>
 __device__ __forceinline__ void run_pencil(const StepClassDev &c, const GroupParamsF *gp, int traj, int sub,
-                                           const PencilArgs &pa, float4 *smem)
+                                           const PencilArgs &pa, cpair *smem)
 {
     constexpr int VB = kThreads / NZ;       // tiles of 16 pencils per item
     const int v = threadIdx.x / NZ;
     PencilArgs p = pa;
     p.scale = 1.0f / (float)c.cells;        // exact: cells is a power of two
     const VBlock vb{(int)threadIdx.x % NZ, traj * c.tiles + sub * VB + v, VB == 1 ? 0 : 1 + v, NZ};
-    float4 *dyn = smem + v * (stepk::pencil_smem_bytes<NZ>() / sizeof(float4));
+    cpair *dyn = smem + v * (stepk::pencil_smem_bytes<NZ>() / sizeof(cpair));
     const float2 *kin = pa.frac == 1.0f ? c.kin[1] : pa.frac == 0.5f ? c.kin[0] : nullptr;
-    stepk::pencil_body<NZ, false>(vb, c.state, c.nx, c.lx, c.ny, c.cells, c.tiles, gp, c.tgroup, c.tw, p, nullptr,
+    stepk::pencil_body<NZ, false>(vb, reinterpret_cast<cpair *>(c.state), c.nx, c.lx, c.ny, c.cells, c.tiles, gp, c.tgroup, c.tw, p, nullptr,
                                   1.0f, kin, dyn);
 }
 
 template <int N>
 __device__ __forceinline__ void run_plane(const StepClassDev &c, const GroupParamsF *gp, int traj, int sub,
-                                          uint32_t step, float4 *smem)
+                                          uint32_t step, cpair *smem)
 {
     constexpr int W = 32 / N;
     const int v = threadIdx.x / 128;        // two 128-thread virtual blocks of 4 warps
     const int planes_per_vb = 4 * W;
     const int bid = (traj * c.nz) / planes_per_vb + sub * 2 + v;
     const VBlock vb{(int)threadIdx.x % 128, bid, 0, 128};   // warp-synchronous: no block barrier used
-    stepk::plane_body<N>(vb, c.state, c.nz, c.cells, gp, c.tgroup, c.tlocal, step, smem + v * 4 * W * N * N);
+    stepk::plane_body<N>(vb, reinterpret_cast<cpair *>(c.state), c.nz, c.cells, gp, c.tgroup, c.tlocal, step, smem + v * 4 * W * N * N);
 }
 
 __device__ __forceinline__ void run_plane32(const StepClassDev &c, const GroupParamsF *gp, int traj, int sub,
-                                            uint32_t step, float4 *smem)
+                                            uint32_t step, cpair *smem)
 {
     const int v = threadIdx.x / 64;
     const VBlock vb{(int)threadIdx.x % 64, traj * c.nz + sub * kPlane32PerItem + v, 1 + v, 64};
-    float4 *tile = smem + v * 1536;
-    stepk::plane32_body(vb, c.state, c.nz, c.cells, gp, c.tgroup, c.tlocal, step, tile, tile + 1024);
+    cpair *tile = smem + v * 1536;
+    stepk::plane32_body(vb, reinterpret_cast<cpair *>(c.state), c.nz, c.cells, gp, c.tgroup, c.tlocal, step, tile, tile + 1024);
 }
 
 __global__ void __launch_bounds__(kThreads, 2) k_step(StepLaunch L, PencilArgs pa)
 {
-    extern __shared__ float4 smem[];
+    extern __shared__ cpair smem[];
     __shared__ int4 s_item;
     __shared__ int s_last;
     const uint32_t step = *L.d_step;
