@@ -80,7 +80,7 @@ struct bec_ctx {
     int n_traj = 0;
     std::vector<GroupRec> groups;
     std::vector<ClassRec> classes;
-    std::map<int, double2 *> tw64;
+    std::map<int, double2 *> tw64, tw64_full;
     std::map<int, float2 *> tw32;
     std::map<int, float2 *> tw32_full;
     std::map<int, float2 *> tw32_nearest;
@@ -128,6 +128,8 @@ struct bec_ctx {
     size_t alloc_bytes = 0;              // bytes of the context's own device buffers
     size_t alloc_limit = 0;              // BEC_DEVICE_BYTES_LIMIT at creation (0: none)
     std::vector<WsTable> ws_tables;      // warm-start bases installed per grid
+    char *gs64_buf = nullptr;            // workspace of bec_ground_state, kept up to kGs64Keep bytes
+    size_t gs64_bytes = 0;
 };
 
 namespace {
@@ -264,6 +266,31 @@ bec_status get_tw64(bec_ctx *ctx, int n, double2 **out)
     ctx->tw64[n] = d;
     *out = d;
     return BEC_OK;
+}
+
+// all n twiddles W_n^k, k < n
+bec_status get_tw64_full(bec_ctx *ctx, int n, const double2 **out)
+{
+    auto it = ctx->tw64_full.find(n);
+    if (it != ctx->tw64_full.end()) { *out = it->second; return BEC_OK; }
+    std::vector<double2> t(n);
+    for (int k = 0; k < n; ++k) {
+        const double a = 2.0 * M_PI * (double)k / (double)n;
+        t[k] = cd(std::cos(a), -std::sin(a));
+    }
+    double2 *d = nullptr;
+    CKC(dalloc(ctx, &d, t.size()));
+    CKC(cudaMemcpyAsync(d, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->tw64_full[n] = d;
+    *out = d;
+    return BEC_OK;
+}
+
+bec_status get_gs64_tab(bec_ctx *ctx, const GeomD &g, Gs64Tab &t)
+{
+    bec_status st;
+    if ((st = get_tw64_full(ctx, g.nx, &t.x)) || (st = get_tw64_full(ctx, g.ny, &t.y))) return st;
+    return get_tw64_full(ctx, g.nz, &t.z);
 }
 
 // W_n^k = e^{-2 pi i k / n} in FP32: exact at multiples of a quarter turn, elsewhere the pair of modulus
@@ -1278,6 +1305,7 @@ void bec_destroy(bec_ctx *ctx)
     for (void *p : ctx->allocs) cudaFree(p);
     step_plan_free(ctx->plan);
     for (auto &t : ctx->ws_tables) cudaFree(t.d_basis);
+    cudaFree(ctx->gs64_buf);
     for (auto &g : ctx->step_graph)
         if (g) cudaGraphExecDestroy(g);
     for (auto &gr : ctx->groups)
@@ -1301,6 +1329,139 @@ bec_status bec_group_info(const bec_ctx *ctx, int32_t group, bec_derived *out)
 int64_t bec_total_trajectories(const bec_ctx *ctx) { return ctx ? ctx->n_traj : 0; }
 
 // ------------------------------------------------------------------------ ground state
+namespace {
+
+// mu, energy per particle, norm and residual from the sums of gs64_measures
+void fill_measures(const GeomD &g, const double *h, bec_gs_report *rep)
+{
+    const double ekin = h[3] * g.cells * g.dV, epot = h[0] * g.dV, eint = g.g11 * h[1] * g.dV, N = h[2] * g.dV;
+    rep->mu = (ekin + epot + eint) / N;
+    rep->energy = (ekin + epot + 0.5 * eint) / N;
+    rep->N = N;
+    rep->residual = std::sqrt(h[4] / h[2]);
+}
+
+// The workspace of one FP64 ground state. Contexts keep it between calls up to kGs64Keep bytes (grids up to about
+// 1.3 million cells); a larger one is given back at the end of its call.
+constexpr size_t kGs64Keep = (size_t)64 << 20;
+
+// calculateSteadyState on the fused FP64 passes (fp64_passes.cu)
+bec_status ground_state_fused(bec_ctx *ctx, GroupRec &gr, const Gs64Dims &dim, const bec_gs_opts *opts, double *psi_out,
+                              bec_gs_report *rep)
+{
+    const GeomD &g = gr.gd;
+    cudaStream_t s = ctx->stream;
+    const long long l0 = g_launches;
+    const bool mu_rule = opts->mode == BEC_GS_MU || opts->mode == BEC_GS_MU_RESIDUAL;
+    const bool ref_rule = opts->mode == BEC_GS_REFERENCE_E;
+    const size_t cells = g.cells, state = sizeof(double2) * cells;
+    const size_t n_norm = 2 * (size_t)dim.pencil_ctas();
+    const size_t n_part = std::max(5 * (size_t)dim.plane_ctas(), 2 * (size_t)dim.pencil_ctas());
+    const size_t small = sizeof(double) * (n_norm + n_part + kGs64Sums + 4) + sizeof(Gs64Par);
+    const size_t bytes = (ref_rule ? 3 : 2) * state + small + 64;
+    char *buf = ctx->gs64_buf;
+    struct Free { char *p = nullptr; cudaStream_t s; ~Free() { if (p) { cudaStreamSynchronize(s); cudaFree(p); } } } temp;
+    temp.s = s;
+    if (bytes > ctx->gs64_bytes) {
+        if (ctx->gs64_buf) {
+            CKC(cudaStreamSynchronize(s));
+            cudaFree(ctx->gs64_buf);
+            ctx->gs64_buf = nullptr;
+            ctx->gs64_bytes = 0;
+        }
+        void *p = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(ctx, BEC_ERR_OUT_OF_MEMORY, "ground-state buffers");
+        }
+        buf = static_cast<char *>(p);
+        if (bytes <= kGs64Keep) {
+            ctx->gs64_buf = buf;
+            ctx->gs64_bytes = bytes;
+        } else {
+            temp.p = buf;
+        }
+    }
+    double2 *work = reinterpret_cast<double2 *>(buf), *a = work + cells, *kout = ref_rule ? a + cells : nullptr;
+    double *norm_part = reinterpret_cast<double *>(buf + (ref_rule ? 3 : 2) * state);
+    double *part = norm_part + n_norm, *sums = part + n_part, *sums4 = sums + kGs64Sums;
+    Gs64Par *par = reinterpret_cast<Gs64Par *>(sums4 + 4);
+    Gs64Tab tab;
+    bec_status st;
+    if ((st = get_gs64_tab(ctx, g, tab))) return st;
+    const Gs64Par hp{g, gr.d.N, gr.d.mu};
+
+    CKC(cudaEventRecord(ctx->ev0, s));
+    CKC(cudaMemcpyAsync(par, &hp, sizeof hp, cudaMemcpyHostToDevice, s));
+    if (opts->warm_start) CKC(cudaMemcpyAsync(a, opts->warm_start, state, cudaMemcpyHostToDevice, s));
+    CKC(gs64_start(dim, tab, work, par, opts->warm_start ? a : nullptr, norm_part, s));   // wigner.cu:97-107
+    CKC(cudaMemsetAsync(a, 0, state, s));                           // the first check sees a full change
+
+    const int maxs = opts->max_steps > 0 ? opts->max_steps : 1;
+    const int check = opts->check_every > 0 ? opts->check_every : 1;
+    const double res_tol = opts->res_tol > 0.0 ? opts->res_tol : 10.0 * opts->tol;
+    double E = 0.0, mu_prev = 0.0, step_res = 0.0;
+    int steps = 0, converged = 0, checks = 0;
+    for (;;) {
+        CKC(gs64_plane_step(dim, tab, work, par, norm_part, s));    // :121-130
+        ++steps;
+        const bool checked = ref_rule || (mu_rule && steps % check == 0), last = steps == maxs;
+        if (!checked && !last) {
+            CKC(gs64_pencil_step(dim, tab, work, par, norm_part, s));   // :134-145, :117
+            continue;
+        }
+        CKC(gs64_boundary(dim, tab, work, par, norm_part, a, kout, part, checked ? sums : nullptr, s));
+        bool stop = false;
+        if (checked) {
+            double h[kGs64Sums];
+            CKC(cudaMemcpyAsync(h, sums, sizeof h, cudaMemcpyDeviceToHost, s));
+            CKC(cudaStreamSynchronize(s));
+            if (ref_rule) {
+                const double newE = h[4] * g.dV;
+                if (std::fabs((newE - E) / newE) < 0.000001) stop = true;   // :155
+                E = newE;
+            } else {
+                const double s2 = gr.d.N / (h[5] * g.cells * g.dV);     // the renormalisation squared
+                const double ekin = h[6] * s2 * g.cells * g.dV, epot = h[0] * g.dV, eint = g.g11 * h[1] * g.dV;
+                const double mu = (ekin + epot + eint) / (h[2] * g.dV);
+                if (!std::isfinite(mu)) return fail(ctx, BEC_ERR_NUMERICAL, "ground state diverged");
+                const double r = std::sqrt(h[3] / h[2]) / ((double)check * gr.d.dt_steady * std::fabs(mu));
+                if (checks > 0) step_res = r;
+                const bool mu_ok = mu_prev != 0.0 && std::fabs((mu - mu_prev) / mu) < opts->tol;
+                if (mu_ok && (opts->mode == BEC_GS_MU || (checks > 0 && r < res_tol))) stop = true;
+                mu_prev = mu;
+                ++checks;
+            }
+        }
+        if (stop) converged = 1;
+        if (stop || last) break;
+        CKC(gs64_resume(dim, tab, work, par, s));
+    }
+    CKC(cudaEventRecord(ctx->ev1, s));
+    CKC(cudaMemcpyAsync(psi_out, a, state, cudaMemcpyDeviceToHost, s));
+    double h[kGs64Sums];
+    if (rep) {
+        CKC(gs64_measures(dim, tab, a, work, par, part, sums4, sums, s));
+        CKC(cudaMemcpyAsync(h, sums, sizeof h, cudaMemcpyDeviceToHost, s));
+    }
+    CKC(cudaStreamSynchronize(s));
+    if (rep) {
+        std::memset(rep, 0, sizeof(*rep));
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+        rep->steps = steps;
+        rep->converged = converged;
+        rep->seconds = ms * 1e-3;
+        rep->step_residual = step_res;
+        fill_measures(g, h, rep);
+    }
+    CKL();
+    ctx->last_launches = g_launches - l0;
+    return BEC_OK;
+}
+
+} // namespace
+
 bec_status bec_ground_state(bec_ctx *ctx, int32_t group, const bec_gs_opts *opts, double *psi_out,
                             bec_gs_report *rep)
 {
@@ -1311,6 +1472,9 @@ bec_status bec_ground_state(bec_ctx *ctx, int32_t group, const bec_gs_opts *opts
         return fail(ctx, BEC_ERR_INVALID_ARG, "unknown ground-state mode");
     GroupRec &gr = ctx->groups[group];
     const GeomD &g = gr.gd;
+    Gs64Dims dim;
+    if (gs64_dims(g.nx, g.ny, g.nz, 1, dim)) return ground_state_fused(ctx, gr, dim, opts, psi_out, rep);
+    // planes too large for shared memory: one kernel per operation
     const int cells = g.cells;
     cudaStream_t s = ctx->stream;
     const long long l0 = g_launches;
@@ -1447,37 +1611,6 @@ bec_status bec_ground_state(bec_ctx *ctx, int32_t group, const bec_gs_opts *opts
 }
 
 namespace {
-
-// mu, energy per particle, norm and residual of an x-space state already on the device (FP64 kernels)
-bec_status plain_measures(bec_ctx *ctx, const GeomD &g, double2 *a, double2 *tmp, double2 *tmp2, bec_gs_report *rep)
-{
-    cudaStream_t s = ctx->stream;
-    double *sc = ctx->d_scal, *red = ctx->d_red;
-    const int cells = g.cells;
-    bec_status st;
-    plain_gs_xsums(a, g, sc + 8, red, s);
-    CKC(cudaMemcpyAsync(tmp, a, sizeof(double2) * cells, cudaMemcpyDeviceToDevice, s));
-    if ((st = plain_fft(ctx, tmp, g, 1))) return st;
-    plain_scale(tmp, cells, 1.0 / cells, s);
-    plain_gs_ksum(tmp, g, sc + 12, red, s);
-    double h[8];
-    CKC(cudaMemcpyAsync(h, sc + 8, sizeof(double) * 8, cudaMemcpyDeviceToHost, s));
-    CKC(cudaStreamSynchronize(s));
-    const double ekin = h[4] * cells * g.dV, epot = h[0] * g.dV, eint = g.g11 * h[1] * g.dV, N = h[2] * g.dV;
-    const double mu = (ekin + epot + eint) / N;
-    rep->mu = mu;
-    rep->energy = (ekin + epot + 0.5 * eint) / N;
-    rep->N = N;
-    plain_mul_k2(tmp, tmp2, g, s);
-    if ((st = plain_fft(ctx, tmp2, g, 0))) return st;
-    plain_gs_residual(a, tmp2, g, mu, sc + 16, red, s);
-    double r2;
-    CKC(cudaMemcpyAsync(&r2, sc + 16, sizeof(double), cudaMemcpyDeviceToHost, s));
-    CKC(cudaStreamSynchronize(s));
-    rep->residual = std::sqrt(r2 / h[2]);
-    CKL();
-    return BEC_OK;
-}
 
 struct GsClass {
     ClassGeom geom{};
@@ -1743,33 +1876,56 @@ bec_status gs_batched(bec_ctx *ctx, int n, const int32_t *groups, const bec_gs_o
     CKC(cudaEventSynchronize(ctx->ev1));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-    // outputs, FP64 measures of each ground state on the device
-    size_t maxc = 0;
-    for (auto &c : cls) maxc = std::max(maxc, (size_t)c.geom.cells);
-    double2 *a64 = nullptr, *t1 = nullptr, *t2 = nullptr;
-    CKC(talloc((void **)&a64, sizeof(double2) * maxc));
-    CKC(talloc((void **)&t1, sizeof(double2) * maxc));
-    CKC(talloc((void **)&t2, sizeof(double2) * maxc));
-    for (int i = 0; i < n; ++i) {
+    // outputs
+    for (int i = 0; psi_out && i < n; ++i) {
         GsClass &c = cls[cls_of[i]];
         const size_t cells = c.geom.cells;
-        const float2 *src = c.out + (size_t)idx_in[i] * cells;
-        if (psi_out) {
-            std::vector<float2> h(cells);
-            CKC(cudaMemcpyAsync(h.data(), src, sizeof(float2) * cells, cudaMemcpyDeviceToHost, s));
-            CKC(cudaStreamSynchronize(s));
-            for (size_t k = 0; k < cells; ++k) { psi_out[i][2 * k] = h[k].x; psi_out[i][2 * k + 1] = h[k].y; }
+        std::vector<float2> h(cells);
+        CKC(cudaMemcpyAsync(h.data(), c.out + (size_t)idx_in[i] * cells, sizeof(float2) * cells, cudaMemcpyDeviceToHost, s));
+        CKC(cudaStreamSynchronize(s));
+        for (size_t k = 0; k < cells; ++k) { psi_out[i][2 * k] = h[k].x; psi_out[i][2 * k + 1] = h[k].y; }
+    }
+    // FP64 measures of the ground states of each class, in launches over many of them: the loop's state buffer is
+    // free by now and holds the FP64 transforms of half the class at a time
+    for (size_t k = 0; reports && k < cls.size(); ++k) {
+        GsClass &c = cls[k];
+        const int nt = c.geom.n_traj, at_once = nt > 1 ? nt / 2 : 1;
+        const size_t cells = c.geom.cells;
+        double2 *work = reinterpret_cast<double2 *>(c.state);
+        if (nt == 1) CKC(talloc((void **)&work, sizeof(double2) * cells));
+        std::vector<Gs64Par> hpar(nt);
+        for (int t = 0; t < nt; ++t) {
+            const GroupRec &gr = ctx->groups[c.groups[t]];
+            hpar[t] = Gs64Par{gr.gd, gr.d.N, gr.d.mu};
         }
-        if (reports) {
-            bec_gs_report &r = reports[i];
+        Gs64Dims dim;
+        if (!gs64_dims(c.geom.nx, c.geom.ny, c.geom.nz, at_once, dim)) return fail(ctx, BEC_ERR_UNSUPPORTED_GRID, "measures");
+        Gs64Tab tab;
+        if ((st = get_gs64_tab(ctx, ctx->groups[c.groups[0]].gd, tab))) return st;
+        Gs64Par *dpar = nullptr;
+        double *part = nullptr, *sums4 = nullptr, *sums = nullptr;
+        CKC(talloc((void **)&dpar, sizeof(Gs64Par) * nt));
+        CKC(talloc((void **)&part, sizeof(double) * at_once * std::max(5 * dim.plane_ctas(), 2 * dim.pencil_ctas())));
+        CKC(talloc((void **)&sums4, sizeof(double) * 4 * at_once));
+        CKC(talloc((void **)&sums, sizeof(double) * kGs64Sums * nt));
+        CKC(cudaMemcpyAsync(dpar, hpar.data(), sizeof(Gs64Par) * nt, cudaMemcpyHostToDevice, s));
+        for (int t0 = 0; t0 < nt; t0 += at_once) {
+            dim.n = std::min(at_once, nt - t0);
+            CKC(gs64_measures(dim, tab, c.out + (size_t)t0 * cells, work, dpar + t0, part, sums4,
+                              sums + (size_t)kGs64Sums * t0, s));
+        }
+        std::vector<double> h((size_t)kGs64Sums * nt);
+        CKC(cudaMemcpyAsync(h.data(), sums, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s));
+        CKC(cudaStreamSynchronize(s));
+        for (int t = 0; t < nt; ++t) {
+            bec_gs_report &r = reports[c.batch[t]];
             std::memset(&r, 0, sizeof(r));
-            const double cs = conv_step[cls_of[i]][idx_in[i]];
-            r.converged = mu_mode ? (cs >= 0 ? 1 : 0) : 0;
+            const double cs = conv_step[k][t];
+            r.converged = mu_mode && cs >= 0 ? 1 : 0;
             r.steps = (mu_mode && cs >= 0) ? (int)cs : steps;
-            r.step_residual = step_res[cls_of[i]][idx_in[i]];
+            r.step_residual = step_res[k][t];
             r.seconds = ms * 1e-3;
-            gs_to_double(src, a64, cells, s);
-            if ((st = plain_measures(ctx, ctx->groups[groups[i]].gd, a64, t1, t2, &r))) return st;
+            fill_measures(ctx->groups[c.groups[t]].gd, &h[(size_t)kGs64Sums * t], &r);
         }
     }
     if (coef_out || profile_out) {

@@ -82,6 +82,45 @@ void plain_gs_residual(const double2 *ax, const double2 *hk, const GeomD &g, dou
 void plain_mul_k2(const double2 *ak, double2 *hk, const GeomD &g, cudaStream_t s);
 
 // ----------------------------------------------------------------------------
+// fp64_passes.cu: FP64 ground-state steps and measures in fused passes, n trajectories of one grid
+struct Gs64Par {
+    GeomD g;
+    double N, mu;             // target norm, Thomas-Fermi chemical potential (start profile)
+};
+struct Gs64Dims {
+    int lx, ly, lz, n;        // log2 of the grid, trajectories
+    int lppc, lp;             // log2 of the planes and of the pencils per CTA
+    int cells() const { return 1 << (lx + ly + lz); }
+    int plane_ctas() const { return 1 << (lz - lppc); }          // per trajectory
+    int pencil_ctas() const { return 1 << (lx + ly - lp); }
+};
+struct Gs64Tab {
+    const double2 *x, *y, *z; // all n twiddles W_n^k of each axis
+};
+// sums of a boundary: n V, n^2, n, |u - previous out|^2, the reference's energy integrand, |psi_k|^2 and
+// |psi_k|^2 k^2/2 before renormalisation; of gs64_measures: n V, n^2, n, |psi_k|^2 k^2/2, |(H - mu) psi|^2
+constexpr int kGs64Sums = 7;
+// fills d; false when a plane or two pencils do not fit in shared memory
+bool gs64_dims(int nx, int ny, int nz, int n_traj, Gs64Dims &d);
+// norm_part: 2 n pencil_ctas doubles; part: max(5 n plane_ctas, 2 n pencil_ctas); sums: kGs64Sums n; sums4: 4 n
+// start profile (warm x-space state or Thomas-Fermi) -> its norm and the first half kick
+cudaError_t gs64_start(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, const double2 *warm,
+                       double *norm_part, cudaStream_t s);
+cudaError_t gs64_plane_step(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, const double *norm_part,
+                            cudaStream_t s);
+cudaError_t gs64_pencil_step(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, double *norm_part,
+                             cudaStream_t s);
+// ends a step: renormalised x-space state to out; with kout also psi_k for the reference's energy; sums may be NULL
+cudaError_t gs64_boundary(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, double *norm_part,
+                          double2 *out, double2 *kout, double *part, double *sums, cudaStream_t s);
+// the first half kick of the step after a boundary
+cudaError_t gs64_resume(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, cudaStream_t s);
+cudaError_t gs64_measures(const Gs64Dims &d, const Gs64Tab &t, const double2 *psi, double2 *work, const Gs64Par *par, double *part,
+                          double *sums4, double *sums, cudaStream_t s);
+cudaError_t gs64_measures(const Gs64Dims &d, const Gs64Tab &t, const float2 *psi, double2 *work, const Gs64Par *par, double *part,
+                          double *sums4, double *sums, cudaStream_t s);
+
+// ----------------------------------------------------------------------------
 // batched_fp32.cu
 struct ZPassArgs {
     float pre;            // kick fraction before the observation (0 or 0.5)
@@ -157,8 +196,6 @@ void gs_output(float2 *state, const ClassGeom &c, const GroupParamsF *gp, const 
 void gs_pencil(float2 *state, const ClassGeom &c, const GroupParamsF *gp, const GsParamsF *gs, const int *tgroup,
                const float2 *tw_full, float frac1, float frac2, float scale, float out_scale, double *norm,
                double *ekin, cudaStream_t s, const int *active = nullptr);
-
-void gs_to_double(const float2 *in, double2 *out, size_t n, cudaStream_t s);
 
 // warmstart.cu: the 64-term correction over Thomas-Fermi (one grid per call), from the
 // built-in analytic basis or from a table of basis rows installed for that grid

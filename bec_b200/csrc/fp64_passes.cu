@@ -1,0 +1,497 @@
+// fp64_passes.cu -- FP64 imaginary-time steps of single-component states in two fused passes, and the FP64
+// measures of ground states.
+//
+// calculateSteadyState (programs/bec_wigner_3d.cuda/wigner.cu:84-175) takes a kick, three transform axes, the
+// nonlinear factor, three axes, a scaling, a kick, three axes and a renormalisation per step, each a kernel of its
+// own. Here a step is a pencil pass (IFFT_z -> 1/cells -> half kick -> norm -> half kick of the next step -> FFT_z)
+// and a plane pass (FFT_xy -> renormalise -> nonlinear factor -> IFFT_xy) over a state kept as k-space along x and
+// y, x-space along z, as in the FP32 passes. The norm after the second half kick is taken in k-space (Parseval):
+// every pencil CTA writes its partial sum, and the next plane pass adds them in a fixed order, so a step is
+// deterministic and holds no synchronisation with the host.
+//
+// What bounds it: latency. A 16x16x128 state is 512 KiB; at HBM rate the two passes would take 0.3 us. A pass is a
+// launch, one trip to L2 and back, and two to three radix-8 stages per axis in shared memory. Tiles are therefore
+// small (a plane, or two to eight pencils), so that one trajectory fills the chip. Measured on one 16x16x128 ground
+// state of 500 steps: 83.4 ms with one kernel per operation (30 launches a step), 8.43 ms here. The measures of a
+// batch (mu, energy, norm, residual) took twenty launches and two synchronisations a state; here they take eight
+// launches for half the batch (96 states of 32x32x256 with 60 steps: the whole call 42.6 -> 23.2 ms).
+#include <algorithm>
+
+#include "engine.h"
+#include "reduce.cuh"
+
+namespace {
+
+// ---------------------------------------------------------------- radix-8 transforms in shared memory
+__device__ __forceinline__ double2 mul_i(double2 v, bool inv) { return inv ? make_double2(-v.y, v.x) : make_double2(v.y, -v.x); }
+
+template <bool INV>
+__device__ __forceinline__ void dft2(double2 &a, double2 &b)
+{
+    const double2 t = a;
+    a = cadd(t, b);
+    b = csub(t, b);
+}
+template <bool INV>
+__device__ __forceinline__ void dft4(double2 &a, double2 &b, double2 &c, double2 &d)
+{
+    dft2<INV>(a, c);
+    dft2<INV>(b, d);
+    d = mul_i(d, INV);
+    dft2<INV>(a, b);
+    dft2<INV>(c, d);
+    const double2 t = b;      // natural order: a, c, b, d -> X0 X1 X2 X3
+    b = c;
+    c = t;
+}
+// x[k] <- sum_n x[n] e^{-+2 pi i n k / R}, R = 2, 4, 8
+template <int R, bool INV>
+__device__ __forceinline__ void dft_small(double2 *x)
+{
+    if constexpr (R == 2) {
+        dft2<INV>(x[0], x[1]);
+    } else if constexpr (R == 4) {
+        dft4<INV>(x[0], x[1], x[2], x[3]);
+    } else {
+        dft4<INV>(x[0], x[2], x[4], x[6]);      // even samples -> E0..E3 in x[0], x[2], x[4], x[6]
+        dft4<INV>(x[1], x[3], x[5], x[7]);
+        const double h = 0.70710678118654752440;
+        const double2 o0 = x[1], o1 = x[3], o2 = x[5], o3 = x[7];
+        const double2 i1 = mul_i(o1, INV), i3 = mul_i(o3, INV);
+        const double2 t1 = make_double2(h * (o1.x + i1.x), h * (o1.y + i1.y));       // W o1
+        const double2 t2 = mul_i(o2, INV);                                           // W^2 o2
+        const double2 t3 = make_double2(h * (i3.x - o3.x), h * (i3.y - o3.y));       // W^3 o3
+        const double2 e0 = x[0], e1 = x[2], e2 = x[4], e3 = x[6];
+        x[0] = cadd(e0, o0); x[4] = csub(e0, o0);
+        x[1] = cadd(e1, t1); x[5] = csub(e1, t1);
+        x[2] = cadd(e2, t2); x[6] = csub(e2, t2);
+        x[3] = cadd(e3, t3); x[7] = csub(e3, t3);
+    }
+}
+
+// Lines of n = 2^logn elements at base(line) + e * es: base = (line & (2^lin - 1)) * ls_in + (line >> lin) * ls_out.
+struct Lines {
+    int logn, log_lines, es, lin, ls_in, ls_out;
+    __device__ __forceinline__ int base(int line) const { return (line & ((1 << lin) - 1)) * ls_in + (line >> lin) * ls_out; }
+};
+
+// One stage of span m = 2^lm and radix R over every line. Decimation in time (DIF = false): twiddles before the
+// small transform; in frequency: after it.
+template <int R, bool INV, bool DIF>
+__device__ __forceinline__ void stage(double2 *buf, const Lines &L, const double2 *__restrict__ tw, int lm)
+{
+    constexpr int LR = R == 8 ? 3 : R == 4 ? 2 : 1;
+    const int total = 1 << (L.log_lines + L.logn - LR);
+    const int shift = L.logn - LR - lm;
+    for (int w = threadIdx.x; w < total; w += blockDim.x) {
+        const int line = w & ((1 << L.log_lines) - 1), jj = w >> L.log_lines;
+        const int j = jj & ((1 << lm) - 1);
+        double2 *p = buf + L.base(line) + (((jj >> lm) << (lm + LR)) + j) * L.es;
+        const int step = L.es << lm;
+        double2 x[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) x[r] = p[r * step];
+        if constexpr (DIF) dft_small<R, INV>(x);
+        if (lm > 0) {
+#pragma unroll
+            for (int r = 1; r < R; ++r) {
+                double2 t = tw[(j * r) << shift];
+                if (INV) t.y = -t.y;
+                x[r] = cmul(x[r], t);
+            }
+        }
+        if constexpr (!DIF) dft_small<R, INV>(x);
+#pragma unroll
+        for (int r = 0; r < R; ++r) p[r * step] = x[r];
+    }
+    __syncthreads();
+}
+
+// Position of element k of a line in the digit-reversed order that the transforms start from (in time) or end in
+// (in frequency): radix 8 as often as logn allows, a last radix of 2 or 4.
+__device__ __forceinline__ int digit_rev(int k, int logn)
+{
+    int p = 0, s = logn;
+    while (s >= 3) {
+        s -= 3;
+        p |= (k & 7) << s;
+        k >>= 3;
+    }
+    return p | k;
+}
+
+// digit-reversed -> natural, every line of the tile
+template <bool INV>
+__device__ __forceinline__ void fft_time(double2 *buf, const Lines &L, const double2 *tw)
+{
+    int lm = 0;
+    if (L.logn % 3 == 1) { stage<2, INV, false>(buf, L, tw, 0); lm = 1; }
+    else if (L.logn % 3 == 2) { stage<4, INV, false>(buf, L, tw, 0); lm = 2; }
+    for (; lm < L.logn; lm += 3) stage<8, INV, false>(buf, L, tw, lm);
+}
+// natural -> digit-reversed
+template <bool INV>
+__device__ __forceinline__ void fft_freq(double2 *buf, const Lines &L, const double2 *tw)
+{
+    int lm = L.logn - 3;
+    for (; lm >= 0; lm -= 3) stage<8, INV, true>(buf, L, tw, lm);
+    if (lm == -2) stage<2, INV, true>(buf, L, tw, 0);
+    else if (lm == -1) stage<4, INV, true>(buf, L, tw, 0);
+}
+
+__device__ __forceinline__ void copy16(double2 *dst_smem, const double2 *src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Sum of K values over the block in a fixed order, valid in every thread; red holds K * 32 + K doubles.
+template <int K>
+__device__ __forceinline__ void block_sum(double (&v)[K], double *red)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < K; ++k) red[k * 32 + warp] = v[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        double s = 0.0;
+        for (int w = 0; w < nw; ++w) s += red[k * 32 + w];
+        v[k] = s;
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ double2 load_psi(const double2 *p, size_t i) { return p[i]; }
+__device__ __forceinline__ double2 load_psi(const float2 *p, size_t i) { return make_double2(p[i].x, p[i].y); }
+
+// ---------------------------------------------------------------- plane pass
+// A CTA holds ppc planes (nx x ny, rows padded by one element against bank conflicts).
+//   START    x-space in (src, or the Thomas-Fermi profile when src is null) -> IFFT_xy -> state
+//   MEASURE  START with the sums n V, n^2, n of src per CTA
+//   STEP     state -> FFT_xy -> renormalise -> nonlinear factor -> IFFT_xy -> state
+//   OUT      state -> FFT_xy -> renormalise -> out (x-space); sums n V, n^2, n, |u - previous out|^2 and the
+//            reference's energy integrand (wigner_kernel.cu:232-258) when the k-space state kout is given
+//   RESIDUAL state (k^2/2 psi_k along z) -> FFT_xy = kinetic part; sum |(H - mu) psi|^2 of src
+enum { START, MEASURE, STEP, OUT, RESIDUAL };
+
+template <int MODE, typename S>
+__global__ void __launch_bounds__(256) k64_plane(double2 *__restrict__ state, const Gs64Par *__restrict__ par, int lx, int ly,
+                                                 int lz, int lppc, const double2 *__restrict__ tx,
+                                                 const double2 *__restrict__ ty, const double *__restrict__ norm_part,
+                                                 int norm_tiles, const S *__restrict__ src, double2 *__restrict__ out,
+                                                 const double2 *__restrict__ kout, const double *__restrict__ sums4,
+                                                 double *__restrict__ part)
+{
+    extern __shared__ double2 sm64[];
+    __shared__ double red[5 * 32];
+    const int nx = 1 << lx, ny = 1 << ly, ld = nx + 1, lplane = lx + ly;
+    const int lchunk = lppc + lplane, chunk = 1 << lchunk;
+    const int chunks = 1 << (lz - lppc);                        // per trajectory
+    const int traj = blockIdx.x >> (lz - lppc), c0 = blockIdx.x & (chunks - 1);
+    const size_t cell0 = (size_t)c0 << lchunk;
+    const size_t first = ((size_t)traj << (lplane + lz)) + cell0;
+    auto natural = [&](int i) { return (i >> lx) * ld + (i & (nx - 1)); };
+    auto reversed = [&](int i) {
+        return ((i >> lplane) * ny + digit_rev((i >> lx) & (ny - 1), ly)) * ld + digit_rev(i & (nx - 1), lx);
+    };
+    const Lines rows{lx, lppc + ly, 1, 30, ld, 0}, cols{ly, lppc + lx, ld, lx, 1, ny * ld};
+
+    if (MODE == STEP || MODE == OUT || MODE == RESIDUAL)
+        for (int i = threadIdx.x; i < chunk; i += blockDim.x) copy16(sm64 + reversed(i), state + first + i);
+    const Gs64Par &Q = par[traj];
+    const GeomD &g = Q.g;
+    double scale = 1.0;
+    if (MODE == STEP || MODE == OUT) {
+        double s[1] = {0.0};
+        for (int t = threadIdx.x; t < norm_tiles; t += blockDim.x) s[0] += norm_part[((size_t)traj * norm_tiles + t) * 2];
+        block_sum<1>(s, red);
+        scale = sqrt(Q.N / (s[0] * ((double)g.cells * g.dV)));
+    }
+    auto potential = [&](int i) {
+        const double X = -g.xmax + g.dx * (double)(i & (nx - 1));
+        const double Y = ny > 1 ? -g.ymax + g.dy * (double)((i >> lx) & (ny - 1)) : 0.0;
+        const double Z = -g.zmax + g.dz * (double)((c0 << lppc) + (i >> lplane));
+        return (X * X + Y * Y + Z * Z / (g.lambda * g.lambda)) / 2.0;
+    };
+    if (MODE == STEP || MODE == OUT || MODE == RESIDUAL) {
+        copy_wait();
+        __syncthreads();
+        fft_time<false>(sm64, rows, tx);
+        if (ly > 0) fft_time<false>(sm64, cols, ty);
+    }
+    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x) {
+        double2 &w = sm64[natural(i)];
+        if (MODE == START || MODE == MEASURE) {
+            double2 u;
+            if (src) {
+                u = load_psi(src, first + i);
+            } else {
+                const double e = Q.mu - potential(i);
+                u = make_double2(e > 0 ? sqrt(e / g.g11) : 0.0, 0.0);
+            }
+            w = u;
+            if (MODE == MEASURE) {
+                const double n = u.x * u.x + u.y * u.y;
+                v[0] += n * potential(i);
+                v[1] += n * n;
+                v[2] += n;
+            }
+        } else if (MODE == STEP) {
+            // propagateXSpaceOneComponent (wigner_kernel.cu:154-181)
+            const double V = potential(i);
+            const double2 a0 = cscale(w, scale);
+            double2 x = a0;
+            double d = 0.0;
+            for (int it = 0; it < g.itmax; ++it) {
+                d = exp(g.dt_steady / 2.0 * (-V - g.g11 * (x.x * x.x + x.y * x.y)));
+                x = cscale(a0, d);
+            }
+            w = cscale(x, d);
+        } else if (MODE == OUT) {
+            const double2 u = cscale(w, scale), p = out[first + i];
+            out[first + i] = u;
+            const double V = potential(i), n = u.x * u.x + u.y * u.y;
+            v[0] += n * V;
+            v[1] += n * n;
+            v[2] += n;
+            const double dx = u.x - p.x, dy = u.y - p.y;
+            v[3] += dx * dx + dy * dy;
+            if (kout) {
+                const int x = i & (nx - 1), y = (i >> lx) & (ny - 1), z = (c0 << lppc) + (i >> lplane);
+                const double kx = getk<double>(x, g.dkx, nx), ky = ny > 1 ? getk<double>(y, g.dky, ny) : 0.0;
+                const double kz = getk<double>(z, g.dkz, 1 << lz);
+                const double2 ak = cscale(kout[first + i], scale * ((kx * kx + ky * ky + kz * kz) / 2.0));
+                v[4] += n * (V + g.g11 * n / 2.0) + (u.x * ak.x - u.y * ak.y);
+            }
+        } else {
+            const double2 u = load_psi(src, first + i);
+            const double *m = sums4 + 4 * (size_t)traj;            // n V, n^2, n, kinetic
+            const double mu = (m[3] * g.cells + m[0] + g.g11 * m[1]) / m[2];
+            const double f = potential(i) + g.g11 * (u.x * u.x + u.y * u.y) - mu;
+            const double hx = w.x + u.x * f, hy = w.y + u.y * f;
+            v[0] += hx * hx + hy * hy;
+        }
+    }
+    if (MODE == START || MODE == MEASURE || MODE == STEP) {
+        __syncthreads();
+        if (ly > 0) fft_freq<true>(sm64, cols, ty);
+        fft_freq<true>(sm64, rows, tx);
+        for (int i = threadIdx.x; i < chunk; i += blockDim.x) state[first + i] = sm64[reversed(i)];
+    }
+    if (MODE == MEASURE || MODE == OUT || MODE == RESIDUAL) {
+        constexpr int K = MODE == MEASURE ? 3 : MODE == OUT ? 5 : 1;
+        double s[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) s[k] = v[k];
+        block_sum<K>(s, red);
+        if (threadIdx.x == 0)
+#pragma unroll
+            for (int k = 0; k < K; ++k) part[(size_t)blockIdx.x * K + k] = s[k];
+    }
+}
+
+// ---------------------------------------------------------------- pencil pass
+// A CTA holds 2^lp adjacent pencils of a trajectory, laid out [z][pencil]: IFFT_z -> scale -> [half kick] -> [sums
+// |psi_k|^2 and |psi_k|^2 k^2/2 per CTA] -> [psi_k to kout] -> [half kick, or k^2/2] -> FFT_z.
+enum { KICK1 = 1, SUMS = 2, KICK2 = 4, TIMES_K2 = 8 };
+
+__global__ void __launch_bounds__(256) k64_pencil(double2 *__restrict__ state, const Gs64Par *__restrict__ par, int lx, int ly,
+                                                  int lz, int lp, const double2 *__restrict__ tz, double scale, int what,
+                                                  double *__restrict__ part, double2 *__restrict__ kout)
+{
+    extern __shared__ double2 sm64[];
+    __shared__ double red[2 * 32];
+    __shared__ double exy[8], kxy[8];
+    const int nx = 1 << lx, nz = 1 << lz, lplane = lx + ly, P = 1 << lp, chunk = nz << lp;
+    double *ez = reinterpret_cast<double *>(sm64 + chunk);     // half-kick factors per kz, then kz^2/2
+    double *kz2 = ez + nz;
+    const int traj = blockIdx.x >> (lplane - lp), pen0 = (blockIdx.x & ((1 << (lplane - lp)) - 1)) << lp;
+    double2 *g0 = state + ((size_t)traj << (lplane + lz)) + pen0;
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x)
+        copy16(sm64 + (digit_rev(i >> lp, lz) << lp) + (i & (P - 1)), g0 + ((size_t)(i >> lp) << lplane) + (i & (P - 1)));
+    const Gs64Par &Q = par[traj];
+    const GeomD &g = Q.g;
+    for (int i = threadIdx.x; i < nz + P; i += blockDim.x) {
+        double k2;
+        if (i < nz) {
+            const double kz = getk<double>(i, g.dkz, nz);
+            k2 = kz * kz / 2.0;
+        } else {
+            const int pen = pen0 + i - nz;
+            const double kx = getk<double>(pen & (nx - 1), g.dkx, nx);
+            const double ky = ly > 0 ? getk<double>(pen >> lx, g.dky, 1 << ly) : 0.0;
+            k2 = (kx * kx + ky * ky) / 2.0;
+        }
+        const double e = (what & (KICK1 | KICK2)) ? exp(-g.dt_steady / 2.0 * k2) : 1.0;   // wigner_kernel.cu:128-134
+        if (i < nz) { ez[i] = e; kz2[i] = k2; }
+        else { exy[i - nz] = e; kxy[i - nz] = k2; }
+    }
+    copy_wait();
+    __syncthreads();
+    const Lines L{lz, lp, P, 30, 1, 0};
+    fft_time<true>(sm64, L, tz);
+    double v[2] = {0.0, 0.0};
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x) {
+        const int z = i >> lp, p = i & (P - 1);
+        const double e = ez[z] * exy[p], k2 = kz2[z] + kxy[p];
+        double2 u = cscale(sm64[i], scale);
+        if (what & KICK1) u = cscale(u, e);
+        if (what & SUMS) {
+            const double n = u.x * u.x + u.y * u.y;
+            v[0] += n;
+            v[1] += n * k2;
+        }
+        if (kout) kout[((size_t)traj << (lplane + lz)) + ((size_t)z << lplane) + pen0 + p] = u;
+        if (what & KICK2) u = cscale(u, e);
+        if (what & TIMES_K2) u = cscale(u, k2);
+        sm64[i] = u;
+    }
+    __syncthreads();
+    fft_freq<false>(sm64, L, tz);
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x)
+        g0[((size_t)(i >> lp) << lplane) + (i & (P - 1))] = sm64[(digit_rev(i >> lp, lz) << lp) + (i & (P - 1))];
+    if (what & SUMS) {
+        block_sum<2>(v, red);
+        if (threadIdx.x == 0) {
+            part[(size_t)blockIdx.x * 2] = v[0];
+            part[(size_t)blockIdx.x * 2 + 1] = v[1];
+        }
+    }
+}
+
+// out[traj * stride + off + k] = sum over n of part[(traj * n + i) * K + first + k], k < count; one block per trajectory
+__global__ void k64_fold(const double *__restrict__ part, int n, int K, int first, int count, double *__restrict__ out,
+                         int stride, int off)
+{
+    __shared__ double red[32];
+    for (int k = 0; k < count; ++k) {
+        double s[1] = {0.0};
+        for (int i = threadIdx.x; i < n; i += blockDim.x) s[0] += part[((size_t)blockIdx.x * n + i) * K + first + k];
+        block_sum<1>(s, red);
+        if (threadIdx.x == 0) out[(size_t)blockIdx.x * stride + off + k] = s[0];
+    }
+}
+
+size_t plane_smem(int lx, int ly, int lppc) { return sizeof(double2) * (((size_t)1 << (ly + lppc)) * ((1 << lx) + 1)); }
+size_t pencil_smem(int lz, int lp) { return sizeof(double2) * ((size_t)1 << (lz + lp)) + sizeof(double) * 2 * ((size_t)1 << lz); }
+constexpr size_t kMaxSmem = 200 * 1024;
+
+int ilog(int n) { int r = 0; while ((1 << r) < n) ++r; return r; }
+int threads_for(int log_elems) { return log_elems >= 11 ? 256 : 128; }
+
+template <int MODE, typename S>
+cudaError_t plane_launch(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, const double *norm_part,
+                         const S *src, double2 *out, const double2 *kout, const double *sums4, double *part, cudaStream_t s)
+{
+    const size_t smem = plane_smem(d.lx, d.ly, d.lppc);
+    cudaError_t e = ensure_smem_limit((const void *)k64_plane<MODE, S>, (int)kMaxSmem);
+    if (e) return e;
+    k64_plane<MODE, S><<<d.n * d.plane_ctas(), threads_for(d.lppc + d.lx + d.ly), smem, s>>>(
+        state, par, d.lx, d.ly, d.lz, d.lppc, t.x, t.y, norm_part, d.pencil_ctas(), src, out, kout, sums4, part);
+    g_launches++;
+    return cudaGetLastError();
+}
+
+cudaError_t pencil_launch(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, double scale, int what,
+                          double *part, double2 *kout, cudaStream_t s)
+{
+    cudaError_t e = ensure_smem_limit((const void *)k64_pencil, (int)kMaxSmem);
+    if (e) return e;
+    k64_pencil<<<d.n * d.pencil_ctas(), threads_for(d.lz + d.lp), pencil_smem(d.lz, d.lp), s>>>(
+        state, par, d.lx, d.ly, d.lz, d.lp, t.z, scale, what, part, kout);
+    g_launches++;
+    return cudaGetLastError();
+}
+
+void fold_launch(const Gs64Dims &d, const double *part, int n, int K, int first, int count, double *out, int off, cudaStream_t s)
+{
+    k64_fold<<<d.n, 128, 0, s>>>(part, n, K, first, count, out, kGs64Sums, off);
+    g_launches++;
+}
+
+} // namespace
+
+// Tiles: a plane pass takes planes up to 256 cells together, a pencil pass 8 pencils (128-byte rows), fewer while one
+// launch has fewer CTAs than the chip has SMs (down to 2: 32-byte sectors) or the tile would not fit.
+bool gs64_dims(int nx, int ny, int nz, int n_traj, Gs64Dims &d)
+{
+    d.lx = ilog(nx); d.ly = ilog(ny); d.lz = ilog(nz);
+    d.n = n_traj;
+    d.lppc = std::max(0, std::min(8 - d.lx - d.ly, d.lz));
+    d.lp = std::min(3, d.lx + d.ly);
+    while (d.lp > 1 && ((long long)d.n * d.pencil_ctas() < 148 || pencil_smem(d.lz, d.lp) > 64 * 1024)) --d.lp;
+    return d.lx >= 1 && d.lz >= 1 && d.lx <= 10 && d.ly <= 10 && d.lz <= 10 &&
+           plane_smem(d.lx, d.ly, d.lppc) <= kMaxSmem && pencil_smem(d.lz, d.lp) <= kMaxSmem &&
+           (long long)d.n * std::max(d.plane_ctas(), d.pencil_ctas()) < (1ll << 31);
+}
+
+cudaError_t gs64_start(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, const double2 *warm,
+                       double *norm_part, cudaStream_t s)
+{
+    cudaError_t e = plane_launch<START, double2>(d, t, state, par, nullptr, warm, nullptr, nullptr, nullptr, nullptr, s);
+    return e ? e : pencil_launch(d, t, state, par, 1.0 / d.cells(), SUMS | KICK2, norm_part, nullptr, s);
+}
+
+cudaError_t gs64_plane_step(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, const double *norm_part,
+                            cudaStream_t s)
+{
+    return plane_launch<STEP, double2>(d, t, state, par, norm_part, nullptr, nullptr, nullptr, nullptr, nullptr, s);
+}
+
+cudaError_t gs64_pencil_step(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, double *norm_part,
+                             cudaStream_t s)
+{
+    return pencil_launch(d, t, state, par, 1.0 / d.cells(), KICK1 | SUMS | KICK2, norm_part, nullptr, s);
+}
+
+cudaError_t gs64_boundary(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, double *norm_part,
+                          double2 *out, double2 *kout, double *part, double *sums, cudaStream_t s)
+{
+    cudaError_t e = pencil_launch(d, t, state, par, 1.0 / d.cells(), KICK1 | SUMS, norm_part, kout, s);
+    if (e) return e;
+    e = plane_launch<OUT, double2>(d, t, state, par, norm_part, nullptr, out, kout, nullptr, part, s);
+    if (e || !sums) return e;
+    fold_launch(d, part, d.plane_ctas(), 5, 0, 5, sums, 0, s);
+    fold_launch(d, norm_part, d.pencil_ctas(), 2, 0, 2, sums, 5, s);
+    return cudaGetLastError();
+}
+
+cudaError_t gs64_resume(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, cudaStream_t s)
+{
+    return pencil_launch(d, t, state, par, 1.0 / (1 << d.lz), KICK2, nullptr, nullptr, s);
+}
+
+template <typename S>
+static cudaError_t measures(const Gs64Dims &d, const Gs64Tab &t, const S *psi, double2 *work, const Gs64Par *par, double *part,
+                            double *sums4, double *sums, cudaStream_t s)
+{
+    cudaError_t e = plane_launch<MEASURE, S>(d, t, work, par, nullptr, psi, nullptr, nullptr, nullptr, part, s);
+    if (e) return e;
+    k64_fold<<<d.n, 128, 0, s>>>(part, d.plane_ctas(), 3, 0, 3, sums4, 4, 0);
+    if ((e = pencil_launch(d, t, work, par, 1.0 / d.cells(), SUMS | TIMES_K2, part, nullptr, s))) return e;
+    k64_fold<<<d.n, 128, 0, s>>>(part, d.pencil_ctas(), 2, 1, 1, sums4, 4, 3);
+    if ((e = plane_launch<RESIDUAL, S>(d, t, work, par, nullptr, psi, nullptr, nullptr, sums4, part, s))) return e;
+    fold_launch(d, sums4, 1, 4, 0, 4, sums, 0, s);
+    fold_launch(d, part, d.plane_ctas(), 1, 0, 1, sums, 4, s);
+    g_launches += 2;
+    return cudaGetLastError();
+}
+
+cudaError_t gs64_measures(const Gs64Dims &d, const Gs64Tab &t, const double2 *psi, double2 *work, const Gs64Par *par, double *part,
+                          double *sums4, double *sums, cudaStream_t s)
+{
+    return measures(d, t, psi, work, par, part, sums4, sums, s);
+}
+cudaError_t gs64_measures(const Gs64Dims &d, const Gs64Tab &t, const float2 *psi, double2 *work, const Gs64Par *par, double *part,
+                          double *sums4, double *sums, cudaStream_t s)
+{
+    return measures(d, t, psi, work, par, part, sums4, sums, s);
+}

@@ -346,22 +346,6 @@ void dispatch_plane(float2 *state, const ClassGeom &c, const GroupParamsF *gp, c
 
 } // namespace
 
-namespace {
-__global__ void k_to_double(const float2 *in, double2 *out, size_t n)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = make_double2(in[i].x, in[i].y);
-}
-} // namespace
-
-void gs_to_double(const float2 *in, double2 *out, size_t n, cudaStream_t s)
-{
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 4096) blocks = 4096;
-    k_to_double<<<blocks, 256, 0, s>>>(in, out, n);
-    g_launches++;
-}
-
 bool gs_batched_supported(const ClassGeom &c)
 {
     return fp32_fast_plane_supported(c) && fp32_fast_pencil_supported(c);
