@@ -15,6 +15,18 @@
 // BF16 rounding level and its warm starts needed 1.6x the steps of the same
 // network trained in FP32). Master weights, Adam moments, activations' pre-images
 // and gradients are FP32.
+//
+// What bounds it: latency. A training step of the 256-wide network at batch 256 is
+// 0.23 GFLOP and 4 MB, under a microsecond of either; it is a chain of dependent
+// GEMMs. So a step is one launch per link of that chain (four forward, four backward)
+// and nothing else: every GEMM's epilogue applies the bias, the activation or its
+// derivative, the loss or Adam, and writes its result as the split operands that the
+// next GEMMs read, plain and transposed, already in the tiles' shared-memory layout; a
+// layer's weight gradient, bias gradient and input gradient share a launch, and the
+// next minibatch is gathered beside the first layer's. Weights' operands alternate
+// between two buffers, so that a launch can update a layer that another tile of it
+// still reads. 87 us a step (batch 256, 400 steps with the set-up) against 314 us with one kernel per
+// operation.
 #include <algorithm>
 #include <cstdlib>
 #include <cmath>
@@ -29,24 +41,104 @@
 
 namespace {
 
+typedef __nv_bfloat16 bf16;
+
+// ---------------------------------------------------------------- operands
+// A split matrix [R x K] (R, K multiples of 64) as its hi and its lo values, each in the K-major canonical order of
+// the tensor core without swizzle: 64 columns after another, 8-row groups of 1024 bytes, in a group 16-byte chunks of 8
+// columns (128 bytes apart) of 8 rows (16 bytes apart). The rows r0 .. r0 + T of a 64-column block are then T * 128
+// contiguous bytes: one bulk copy brings an operand tile to shared memory.
+struct Split {
+    bf16 *hi, *lo;
+};
+__host__ __device__ __forceinline__ size_t blk(int R, int r, int k)
+{
+    return ((size_t)(k >> 6) * (R >> 3) + (r >> 3)) * 512 + ((k >> 3) & 7) * 64 + (r & 7) * 8 + (k & 7);
+}
+
+// the split of an FP32 value into hi = bf16(v) and lo = bf16(v - hi)
+__device__ __forceinline__ void split_bf16(float v, bf16 &hi, bf16 &lo)
+{
+    hi = __float2bfloat16(v);
+    lo = __float2bfloat16(v - __bfloat162float(hi));
+}
+
 // ---------------------------------------------------------------- GEMM on the 5th-generation tensor cores
-// C[M x N] = A[M x K] * B[N x K]^T (+ bias[N]) with A = A_hi + A_lo, B = B_hi + B_lo (BF16 row-major, K contiguous);
-// C FP32; M, N, K multiples of 64. One CTA of 128 threads per 128 x 64 tile of C. The FP32 accumulator lives in
-// tensor memory (64 columns, lane i = row i of the tile). K runs in groups of up to four 64-wide stages: the threads
-// copy every stage's four tiles (A and B, hi and lo) to shared memory at once (cp.async, 16 bytes each) in the
-// K-major canonical layout without swizzle (8-row x 16-byte core matrices; the two 16-byte K chunks of one
-// instruction 128 B apart, consecutive 8-row groups 1024 B apart), then one thread issues, per 16-wide K step, the
-// three tcgen05.mma (M 128, N 64, K 16, BF16 in, FP32 accumulate) lo*hi, hi*lo, hi*hi, and tcgen05.commit arrives
-// on an mbarrier when they are done; every wait is bounded. Rows of a last 64-row tile (M = 64 mod 128) are zero in
-// A and not stored. The epilogue reads the accumulator with tcgen05.ld (warp w owns lanes 32w..32w+31), adds the
-// bias and stores FP32 rows.
-constexpr int GM = 128, GN = 64, GK = 64, GSTAGES = 4;
-constexpr int kTileA = GM * GK * 2, kTileB = GN * GK * 2;     // 16 KiB, 8 KiB
-constexpr int kStageBytes = 2 * (kTileA + kTileB);          // hi and lo of both: 48 KiB
-constexpr int kGemmSmem = GSTAGES * kStageBytes + 64;       // + mbarrier and TMEM slot: 192 KiB, one CTA per SM
-// instruction descriptor, kind::f16: D F32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1), both K-major,
-// N >> 3 at bits 17-22, M >> 4 at bits 24-28
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GN >> 3) << 17) | ((uint32_t)(GM >> 4) << 24);
+// C[M x N] = A[M x K] * B[N x K]^T with A = A_hi + A_lo, B = B_hi + B_lo; M, N, K multiples of 64. One CTA of 128
+// threads per 128 x tn tile of C (tn = 16, 32 or 64: the narrowest that keeps a launch within one CTA per SM, so that
+// a 256 x 256 product spreads over 32 SMs instead of 8). The FP32 accumulator lives in tensor memory (lane i = row i
+// of the tile). K runs in 64-wide stages through a ring of four: one thread issues the bulk copies of a stage's four
+// tiles onto an mbarrier, and, as each stage lands, per 16-wide K step the three tcgen05.mma (M 128, N tn, K 16, BF16
+// in, FP32 accumulate) lo*hi, hi*lo, hi*hi; tcgen05.commit arrives on the stage's second mbarrier when they are done.
+// Every wait is bounded. Rows of a last 64-row tile (M = 64 mod 128) are not loaded and not stored. The epilogue reads
+// the accumulator with tcgen05.ld (warp w owns lanes 32w..32w+31).
+constexpr int GM = 128, GK = 64, GSTAGES = 4;
+constexpr int kTileA = GM * GK * 2;                           // 16 KiB each of hi and lo
+__host__ __device__ constexpr int stage_bytes(int tn) { return 2 * (kTileA + tn * GK * 2); }
+__host__ __device__ constexpr int gemm_smem(int tn) { return GSTAGES * stage_bytes(tn) + 128; }   // + mbarriers and TMEM slot
+
+enum Epilogue {
+    EPI_TANH,       // y = tanh(acc + bias): f32 and operands
+    EPI_LINEAR,     // y = acc + bias
+    EPI_LOSS,       // the output layer in training: y = acc + bias, dz = 2 (y - t) / (valid * real_cols), loss
+    EPI_DX,         // dz = acc (1 - y^2): f32 and operands
+    EPI_GRAD,       // the weight gradient: f32
+    EPI_ADAM        // the weight gradient applied at once: master weight, moments, operands
+};
+
+struct AdamArgs {
+    float lr, c1, c2;           // step size, 1 - beta1^t, 1 - beta2^t
+};
+struct GemmJob {
+    const bf16 *Ahi, *Alo, *Bhi, *Blo;   // operands; Ahi == nullptr: no job
+    int Ra, Rb;                 // rows of the operand matrices
+    int M, N, K, tn, ctas;
+    int epi;
+    const float *bias;          // [N]
+    float *f32;                 // row-major [M x N] result (y, dz, gradient), may be NULL
+    int f32_ld, f32_rows, f32_cols;      // ... stored for rows and columns below these
+    Split out, outT;            // [M x N] and [N x M] operands, may be NULL
+    const float *y;             // EPI_DX: activation [M x N]
+    const float *tgt;           // EPI_LOSS: targets [M x N]
+    int valid, real_cols;
+    float *loss;
+    float *w, *m, *v;           // EPI_ADAM: master weights and moments, [M x N]
+    AdamArgs adam;
+};
+struct BiasJob {                // db[c] = sum_r dz[r][c], rows in order
+    const float *dz;
+    int rows, cols, ctas;
+    float *g;                   // gradient out, or NULL: Adam on w, m, v
+    float *w, *m, *v;
+    AdamArgs adam;
+};
+struct GatherJob {              // a minibatch: rows idx[r] (or r) of x, zero rows past valid and columns past in_real
+    const float *x, *t;
+    const int *idx;
+    int rows, valid, in_real, in, out_real, out, ctas;
+    Split X, XT;                // [rows x in], [in x rows]; XT and tgt may be NULL
+    float *tgt;                 // [rows x out]
+};
+struct Jobs {
+    GemmJob gemm[2];
+    BiasJob bias;
+    GatherJob gather;
+    int *err;
+    const int *never;
+    int stall;
+    unsigned long long limit_ns;
+};
+
+__device__ __forceinline__ float adam_update(float &w, float &m, float &v, float gi, const AdamArgs &a)
+{
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    const float mi = b1 * m + (1.0f - b1) * gi;
+    const float vi = b2 * v + (1.0f - b2) * gi * gi;
+    m = mi;
+    v = vi;
+    w -= a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + eps);
+    return w;
+}
 
 __device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -98,33 +190,128 @@ __device__ __noinline__ bool wait_flag(const int *flag, unsigned long long limit
 }
 
 // one tcgen05.mma of the tile: D (+)= A B^T from the shared-memory descriptors; accumulate = 0 overwrites D
-__device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t accumulate)
+__device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(tmem), "l"(ad), "l"(bd), "r"(kIdesc), "r"(accumulate)
+                 ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate)
                  : "memory");
 }
 
-__global__ void __launch_bounds__(128) k_gemm_tc(const __nv_bfloat16 *__restrict__ A, const __nv_bfloat16 *__restrict__ Alo,
-                                                 const __nv_bfloat16 *__restrict__ B, const __nv_bfloat16 *__restrict__ Blo,
-                                                 float *__restrict__ C, const float *__restrict__ bias, int M, int N,
-                                                 int K, int *err, const int *never, int stall,
-                                                 unsigned long long limit_ns)
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
 {
-    extern __shared__ __align__(1024) unsigned char sm[];
-    // stage g at g * kStageBytes: A_hi (128 rows x 64 K), B_hi (64 rows x 64 K), A_lo, B_lo
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + GSTAGES * kStageBytes);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + GSTAGES * kStageBytes + 8);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// 16 consecutive columns of one row, as operands: two 16-byte chunks of the plain matrix, and of the transposed one
+// a 2-byte value per column (8 rows of consecutive lanes make a chunk)
+__device__ __forceinline__ void store_operands(const GemmJob &J, int row, int col, const float (&o)[16])
+{
+    __align__(16) bf16 hi[16], lo[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) split_bf16(o[q], hi[q], lo[q]);
+    if (J.out.hi) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const size_t at = blk(J.M, row, col + 8 * h);
+            *reinterpret_cast<uint4 *>(J.out.hi + at) = reinterpret_cast<const uint4 *>(hi)[h];
+            *reinterpret_cast<uint4 *>(J.out.lo + at) = reinterpret_cast<const uint4 *>(lo)[h];
+        }
+    }
+    if (J.outT.hi) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const size_t at = blk(J.N, col + q, row);
+            J.outT.hi[at] = hi[q];
+            J.outT.lo[at] = lo[q];
+        }
+    }
+}
+
+__device__ __forceinline__ void load16(float (&o)[16], const float *p)
+{
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float4 v = reinterpret_cast<const float4 *>(p)[q];
+        o[4 * q] = v.x; o[4 * q + 1] = v.y; o[4 * q + 2] = v.z; o[4 * q + 3] = v.w;
+    }
+}
+__device__ __forceinline__ void store16(float *p, const float (&o)[16])
+{
+#pragma unroll
+    for (int q = 0; q < 4; ++q) reinterpret_cast<float4 *>(p)[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+}
+
+// row's 16 accumulator columns from col on; returns the row's share of the loss (EPI_LOSS)
+__device__ __forceinline__ float epilogue(const GemmJob &J, int row, int col, float (&o)[16])
+{
+    float l = 0.0f, b[16];
+    const size_t at = (size_t)row * J.N + col;
+    if (J.epi <= EPI_LOSS) {
+        load16(b, J.bias + col);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) o[q] += b[q];
+    }
+    if (J.epi == EPI_TANH) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) o[q] = tanhf(o[q]);
+    } else if (J.epi == EPI_LOSS) {
+        // the padding columns of y and t are zero, padding rows get no gradient
+        load16(b, J.tgt + at);
+        const float s = 2.0f / ((float)J.valid * J.real_cols);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const float d = row < J.valid ? o[q] - b[q] : 0.0f;
+            l += d * d;
+            o[q] = s * d;
+        }
+    } else if (J.epi == EPI_DX) {
+        load16(b, J.y + at);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) o[q] *= 1.0f - b[q] * b[q];
+    } else if (J.epi == EPI_ADAM) {
+        float w[16], m[16], v[16];
+        load16(w, J.w + at);
+        load16(m, J.m + at);
+        load16(v, J.v + at);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) o[q] = adam_update(w[q], m[q], v[q], o[q], J.adam);
+        store16(J.w + at, w);
+        store16(J.m + at, m);
+        store16(J.v + at, v);
+    }
+    if (J.f32 && row < J.f32_rows) {
+        float *dst = J.f32 + (size_t)row * J.f32_ld + col;
+        if (col + 16 <= J.f32_cols && (J.f32_ld & 3) == 0) {
+            store16(dst, o);
+        } else {
+            for (int q = 0; q < 16; ++q)
+                if (col + q < J.f32_cols) dst[q] = o[q];
+        }
+    }
+    store_operands(J, row, col, o);
+    return l;
+}
+
+__device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned char *sm)
+{
+    const int tn = J.tn, tiles_n = J.N / tn, sbytes = stage_bytes(tn);
     const int t = threadIdx.x, warp = t >> 5;
-    const int m0 = blockIdx.y * GM, n0 = blockIdx.x * GN;
+    const int m0 = tile / tiles_n * GM, n0 = tile % tiles_n * tn;
+    const int rows = min(GM, J.M - m0), nk = J.K / GK;
+    // stage g at g * sbytes: A_hi (128 rows x 64 K), A_lo, B_hi (tn rows x 64 K), B_lo; then full and done barriers
+    const uint32_t full = saddr(sm + GSTAGES * sbytes), done = full + 8 * GSTAGES;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + GSTAGES * sbytes + 16 * GSTAGES);
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(saddr(tslot)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (t == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(bar)) : "memory");
+        for (int g = 0; g < 2 * GSTAGES; ++g)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + 8 * g) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -132,99 +319,83 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const __nv_bfloat16 *__restrict
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
 
-    uint32_t parity = 0;
-    bool failed = false;
-    for (int kg = 0; kg < K; kg += GSTAGES * GK) {
-        const int stages = min(GSTAGES, (K - kg) / GK);
-        // chunk c (16 bytes = 8 K values) of a tile sits at byte 16 c: 8-row group c / 64, K chunk (c / 8) % 8,
-        // row c % 8; A rows past M are zero-filled (source size 0)
-        for (int g = 0; g < stages; ++g) {
-            const int k0 = kg + g * GK;
-            unsigned char *As = sm + g * kStageBytes, *Bs = As + kTileA, *Als = Bs + kTileB, *Bls = Als + kTileA;
-            for (int c = t; c < GM * 8; c += 128) {
-                const int row = (c >> 6) * 8 + (c & 7), kc = (c >> 3) & 7;
-                const bool in = m0 + row < M;
-                const size_t off = (size_t)(in ? m0 + row : 0) * K + k0 + kc * 8;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr(As + 16 * c)), "l"(A + off),
-                             "r"(in ? 16 : 0)
-                             : "memory");
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr(Als + 16 * c)), "l"(Alo + off),
-                             "r"(in ? 16 : 0)
-                             : "memory");
-            }
-            for (int c = t; c < GN * 8; c += 128) {
-                const int row = (c >> 6) * 8 + (c & 7), kc = (c >> 3) & 7;
-                const size_t off = (size_t)(n0 + row) * K + k0 + kc * 8;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(Bs + 16 * c)), "l"(B + off)
-                             : "memory");
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(Bls + 16 * c)), "l"(Blo + off)
-                             : "memory");
-            }
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tiles, visible to the tensor core
-        __syncthreads();
-        if (t == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int g = 0; g < stages; ++g) {
-                const uint32_t as = saddr(sm + g * kStageBytes), bs = as + kTileA, als = bs + kTileB,
-                               bls = als + kTileA;
+    bool ok = true;
+    if (t == 0) {
+        // instruction descriptor, kind::f16: D F32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1), both K-major,
+        // N >> 3 at bits 17-22, M >> 4 at bits 24-28
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(GM >> 4) << 24);
+        auto load = [&](int kb) {
+            const int g = kb % GSTAGES;
+            const uint32_t dst = saddr(sm + g * sbytes), bar = full + 8 * g;
+            const uint32_t ab = rows * GK * 2, bb = tn * GK * 2;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * (ab + bb)) : "memory");
+            const size_t a0 = blk(J.Ra, m0, kb * GK), b0 = blk(J.Rb, n0, kb * GK);
+            bulk_load(dst, J.Ahi + a0, ab, bar);
+            bulk_load(dst + kTileA, J.Alo + a0, ab, bar);
+            bulk_load(dst + 2 * kTileA, J.Bhi + b0, bb, bar);
+            bulk_load(dst + 2 * kTileA + bb, J.Blo + b0, bb, bar);
+        };
+        auto landed = [&](int kb) { return mbar_wait_bounded(full + 8 * (kb % GSTAGES), (kb / GSTAGES) & 1, all.limit_ns); };
+        auto multiplied = [&](int kb) { return mbar_wait_bounded(done + 8 * (kb % GSTAGES), (kb / GSTAGES) & 1, all.limit_ns); };
+        int loaded = 0, waited = 0, issued = 0;
+        while (loaded < min(GSTAGES, nk)) load(loaded++);
+        for (int kb = 0; kb < nk && ok; ++kb) {
+            ok = landed(kb);
+            // stall (fault injection): the first stage also waits for a flag that nothing sets
+            if (ok) ++waited;
+            if (ok && all.stall && kb == 0) ok = wait_flag(all.never, all.limit_ns);
+            if (!ok) break;
+            const uint32_t as = saddr(sm + (kb % GSTAGES) * sbytes), als = as + kTileA, bs = als + kTileA, bls = bs + tn * GK * 2;
 #pragma unroll
-                for (int kk = 0; kk < GK / 16; ++kk) {
-                    const uint64_t ad = kmajor_desc(as + 256 * kk), bd = kmajor_desc(bs + 256 * kk);
-                    const uint64_t ald = kmajor_desc(als + 256 * kk), bld = kmajor_desc(bls + 256 * kk);
-                    // the small products first; only the very first MMA of the tile starts D afresh
-                    mma_f16(tmem, ald, bd, (kg > 0 || g > 0 || kk > 0) ? 1u : 0u);
-                    mma_f16(tmem, ad, bld, 1u);
-                    mma_f16(tmem, ad, bd, 1u);
-                }
+            for (int kk = 0; kk < GK / 16; ++kk) {
+                const uint64_t ad = kmajor_desc(as + 256 * kk), bd = kmajor_desc(bs + 256 * kk);
+                const uint64_t ald = kmajor_desc(als + 256 * kk), bld = kmajor_desc(bls + 256 * kk);
+                // the small products first; only the very first MMA of the tile starts D afresh
+                mma_f16(tmem, ald, bd, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+                mma_f16(tmem, ad, bld, idesc, 1u);
+                mma_f16(tmem, ad, bd, idesc, 1u);
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         ::"r"(saddr(bar)) : "memory");
-        }
-        // the group's MMAs read the tiles: every thread waits for them before the next group overwrites them;
-        // stall (fault injection): the first group also waits for a flag that nothing sets
-        bool ok = mbar_wait_bounded(saddr(bar), parity, limit_ns);
-        if (stall && kg == 0 && ok) ok = wait_flag(never, limit_ns);
-        if (__syncthreads_or(!ok)) {
-            failed = true;
-            break;
-        }
-        parity ^= 1u;
-    }
-    if (failed) {
-        // a wait that ran out: report it, give the group's MMAs once more the limit, free the columns
-        if (t == 0) atomicExch(err, 1);
-        mbar_wait_bounded(saddr(bar), parity, limit_ns);
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
-        return;
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int row = m0 + warp * 32 + (t & 31);
-#pragma unroll
-    for (int cb = 0; cb < GN; cb += 16) {
-        uint32_t r[16];
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                     "%13, %14, %15}, [%16];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                       "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                       "=r"(r[15])
-                     : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)cb));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row < M) {
-            float4 *dst = reinterpret_cast<float4 *>(C + (size_t)row * N + n0 + cb);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                float4 o = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
-                                       __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
-                if (bias) {
-                    const float4 b = *reinterpret_cast<const float4 *>(bias + n0 + cb + 4 * q);
-                    o.x += b.x; o.y += b.y; o.z += b.z; o.w += b.w;
-                }
-                dst[q] = o;
+                         ::"r"(done + 8 * (kb % GSTAGES)) : "memory");
+            ++issued;
+            // refill the stage before this one once its MMAs have read it
+            if (kb >= 1 && loaded < nk) {
+                ok = multiplied(kb - 1);
+                if (ok) load(loaded++);
             }
+        }
+        if (ok) ok = multiplied(nk - 1);
+        if (!ok) {
+            // a wait that ran out: report it and give the copies and MMAs in flight once more the limit
+            atomicExch(all.err, 1);
+            for (int kb = waited; kb < loaded; ++kb) landed(kb);
+            if (issued) multiplied(issued - 1);
+        }
+    }
+    const bool failed = __syncthreads_or(!ok);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (!failed) {
+        const int lr = warp * 32 + (t & 31);
+        float l = 0.0f;
+        for (int cb = 0; cb < tn; cb += 16) {
+            uint32_t r[16];
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+                         "%13, %14, %15}, [%16];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                           "=r"(r[15])
+                         : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)cb));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (lr < rows) {
+                float o[16];
+#pragma unroll
+                for (int q = 0; q < 16; ++q) o[q] = __uint_as_float(r[q]);
+                l += epilogue(J, m0 + lr, n0 + cb, o);
+            }
+        }
+        if (J.epi == EPI_LOSS) {
+            for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
+            if ((t & 31) == 0) atomicAdd(J.loss, l / ((float)J.valid * J.real_cols));
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -232,89 +403,72 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const __nv_bfloat16 *__restrict
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
 }
 
-// the split of an FP32 value into hi = bf16(v) and lo = bf16(v - hi)
-__device__ __forceinline__ void split_bf16(float v, __nv_bfloat16 &hi, __nv_bfloat16 &lo)
+__device__ __forceinline__ void bias_columns(const BiasJob &J, int cta)
 {
-    hi = __float2bfloat16(v);
-    lo = __float2bfloat16(v - __bfloat162float(hi));
-}
-
-// y = tanh(z) (or z on the output layer), FP32, and its split (yhi, ylo) for the next GEMM
-__global__ void k_act(const float *z, float *y, __nv_bfloat16 *yhi, __nv_bfloat16 *ylo, size_t n, int linear)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float v = linear ? z[i] : tanhf(z[i]);
-        y[i] = v;
-        split_bf16(v, yhi[i], ylo[i]);
-    }
-}
-
-// dZ = dY * (1 - y^2) (tanh) or dY (linear)
-__global__ void k_act_back(const float *dy, const float *y, float *dz, size_t n, int linear)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        dz[i] = linear ? dy[i] : dy[i] * (1.0f - y[i] * y[i]);
-}
-
-// (hi, lo)[c][r] = split(in[r][c]) for an R x Cn FP32 matrix (also plain splits with transpose = 0)
-__global__ void k_cast_t(const float *in, __nv_bfloat16 *hi, __nv_bfloat16 *lo, int R, int Cn, int transpose)
-{
-    const size_t n = (size_t)R * Cn;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / Cn), c = (int)(i - (size_t)r * Cn);
-        const size_t o = transpose ? (size_t)c * R + r : i;
-        split_bf16(in[i], hi[o], lo[o]);
-    }
-}
-
-// db[c] = sum_r dz[r][c]
-__global__ void k_colsum(const float *dz, float *db, int R, int Cn)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= Cn) return;
+    const int c = cta * 128 + threadIdx.x;
+    if (c >= J.cols) return;
     float s = 0.0f;
-    for (int r = 0; r < R; ++r) s += dz[(size_t)r * Cn + c];
-    db[c] = s;
+#pragma unroll 16
+    for (int r = 0; r < J.rows; ++r) s += J.dz[(size_t)r * J.cols + c];
+    if (J.g) J.g[c] = s;
+    else adam_update(J.w[c], J.m[c], J.v[c], s, J.adam);
 }
 
-// dY = 2 (y - t) / (B * out) over the first `valid` rows (padding rows get 0), out = the caller's output width
-// (real_cols; the padding columns of y and t are zero); loss partials
-__global__ void k_mse(const float *y, const float *tgt, float *dy, int rows, int valid, int cols, int real_cols,
-                      float *loss)
+// a row group (8 rows) of a minibatch per CTA
+__device__ __forceinline__ void gather_rows(const GatherJob &J, int cta)
 {
-    const size_t n = (size_t)rows * cols;
-    float l = 0.0f;
-    const float s = 2.0f / ((float)valid * real_cols);
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / cols);
-        const float d = (r < valid) ? y[i] - tgt[i] : 0.0f;
-        dy[i] = s * d;
-        l += d * d;
+    for (int e = threadIdx.x; e < 8 * J.in; e += 128) {
+        const int r = cta * 8 + (e & 7), c = e >> 3;
+        float x = 0.0f;
+        if (r < J.valid && c < J.in_real) x = J.x[(size_t)(J.idx ? J.idx[r] : r) * J.in_real + c];
+        bf16 hi, lo;
+        split_bf16(x, hi, lo);
+        J.X.hi[blk(J.rows, r, c)] = hi;
+        J.X.lo[blk(J.rows, r, c)] = lo;
+        if (J.XT.hi) {
+            J.XT.hi[blk(J.in, c, r)] = hi;
+            J.XT.lo[blk(J.in, c, r)] = lo;
+        }
     }
-    for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l / ((float)valid * real_cols));
+    if (J.tgt)
+        for (int e = threadIdx.x; e < 8 * J.out; e += 128) {
+            const int r = cta * 8 + e / J.out, c = e % J.out;
+            J.tgt[(size_t)r * J.out + c] =
+                r < J.valid && c < J.out_real ? J.t[(size_t)(J.idx ? J.idx[r] : r) * J.out_real + c] : 0.0f;
+        }
 }
 
-__global__ void k_adam(float *w, float *m, float *v, const float *g, size_t n, float lr, float b1, float b2, float eps,
-                       float c1, float c2)
+// one link of the chain: the tiles of up to two GEMMs, a bias gradient, the gathering of a minibatch
+__global__ void __launch_bounds__(128) k_mlp(const __grid_constant__ Jobs jobs)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    extern __shared__ __align__(1024) unsigned char sm[];
+    int b = blockIdx.x;
+    for (int j = 0; j < 2; ++j) {
+        if (b < jobs.gemm[j].ctas) {
+            gemm_tile(jobs.gemm[j], jobs, b, sm);
+            return;
+        }
+        b -= jobs.gemm[j].ctas;
     }
+    if (b < jobs.bias.ctas) {
+        bias_columns(jobs.bias, b);
+        return;
+    }
+    gather_rows(jobs.gather, b - jobs.bias.ctas);
 }
 
-// gather rows idx[r] of src (n_src x cols) into dst (rows x cols), zero rows past `valid`
-__global__ void k_gather(const float *src, const int *idx, float *dst, int rows, int valid, int cols)
+// the operands of a weight matrix [out x in]: plain and transposed
+__global__ void k_split_weights(const float *__restrict__ w, int out, int in, Split W, Split WT)
 {
-    const size_t n = (size_t)rows * cols;
+    const size_t n = (size_t)out * in;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / cols), c = (int)(i - (size_t)r * cols);
-        dst[i] = (r < valid) ? src[(size_t)idx[r] * cols + c] : 0.0f;
+        const int r = (int)(i / in), c = (int)(i - (size_t)r * in);
+        bf16 hi, lo;
+        split_bf16(w[i], hi, lo);
+        W.hi[blk(out, r, c)] = hi;
+        W.lo[blk(out, r, c)] = lo;
+        WT.hi[blk(in, c, r)] = hi;
+        WT.lo[blk(in, c, r)] = lo;
     }
 }
 
@@ -328,77 +482,298 @@ struct bec_mlp {
     int L = 0;                       // weight layers
     std::vector<size_t> woff, boff;  // offsets into the parameter vector
     size_t n_params = 0;
+    // device memory, one slab per use, each allocated by the first call that needs it: parameters and their operands;
+    // the gradient vector; Adam moments and the second set of operands; the buffers of a batch for inference, for its
+    // gradients, and for training
+    char *slab[6] = {};
+    int cap[6] = {};                 // 1, or the batch capacity of slabs 3 to 5
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;   // FP32 params, grads, Adam moments
-    __nv_bfloat16 *pbf = nullptr, *plo = nullptr;   // the weights' split [out x in] (hi, lo)
-    __nv_bfloat16 *wt = nullptr, *wtlo = nullptr;   // scratch for the split of W^T
-    int cap = 0;                     // batch capacity of the activation buffers
-    std::vector<float *> z, y;       // per layer: pre-activation, activation (FP32) [cap x w]
-    std::vector<__nv_bfloat16 *> xbf, xlo;   // per layer the input's split [cap x w]
-    float *dy = nullptr, *dz = nullptr, *loss = nullptr;
-    __nv_bfloat16 *tA = nullptr, *tB = nullptr, *tAlo = nullptr, *tBlo = nullptr;   // split scratch operands
-    int *idx = nullptr;
+    std::vector<Split> W[2], WT[2];  // per layer the weights' operands, plain and transposed: the current set and the
+    int cur = 0;                     // one that a training step writes
+    std::vector<float *> y, dz;      // per layer: activation, its gradient before the activation (FP32) [cap x w]
+    std::vector<Split> X, XT, D, DT; // their operands, plain and transposed
+    Split X0[2], XT0[2];             // the operands of the inputs of this minibatch and of the next
+    float *tgt[2] = {nullptr, nullptr};
+    float *io = nullptr;             // raw inputs, and the raw result
+    float *raw_t = nullptr;          // raw targets
+    float *loss = nullptr;
     int *d_err = nullptr;            // [0] set by a GEMM whose wait ran out, [1] a flag nothing sets
-    float *xin = nullptr, *tgt = nullptr;
+    int sms = 148;
     long long adam_t = 0;
     cudaStream_t s = nullptr;
     std::string err;
-    std::vector<void *> allocs;
+    // waits of the device side (read from the environment at every call): limit, fault injection
+    int stall = 0;
+    unsigned long long limit_ns = 2000000000ull;
 };
 
 namespace {
 
-bec_status mlp_alloc(bec_mlp *m, void **p, size_t bytes)
-{
-    if (cudaMalloc(p, bytes ? bytes : 16) != cudaSuccess) { cudaGetLastError(); return BEC_ERR_OUT_OF_MEMORY; }
-    m->allocs.push_back(*p);
-    return BEC_OK;
-}
-
 int round_up(int v, int q) { return (v + q - 1) / q * q; }
 
-bec_status mlp_reserve(bec_mlp *m, int batch)
-{
-    if (batch <= m->cap) return BEC_OK;
-    const int cap = round_up(batch, 64);
-    int maxw = 0;
-    for (int v : m->w) maxw = std::max(maxw, v);
-    m->z.assign(m->L + 1, nullptr);
-    m->y.assign(m->L + 1, nullptr);
-    m->xbf.assign(m->L + 1, nullptr);
-    m->xlo.assign(m->L + 1, nullptr);
-    bec_status st;
-    for (int l = 0; l <= m->L; ++l) {
-        if ((st = mlp_alloc(m, (void **)&m->z[l], sizeof(float) * cap * m->w[l]))) return st;
-        if ((st = mlp_alloc(m, (void **)&m->y[l], sizeof(float) * cap * m->w[l]))) return st;
-        if ((st = mlp_alloc(m, (void **)&m->xbf[l], sizeof(__nv_bfloat16) * cap * m->w[l]))) return st;
-        if ((st = mlp_alloc(m, (void **)&m->xlo[l], sizeof(__nv_bfloat16) * cap * m->w[l]))) return st;
+// hands out 256-byte aligned pieces of a slab; with base == NULL it only counts
+struct Carve {
+    char *base;
+    size_t used = 0;
+    template <typename T>
+    T *take(size_t n)
+    {
+        T *p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+        used += (n * sizeof(T) + 255) / 256 * 256;
+        return p;
     }
-    if ((st = mlp_alloc(m, (void **)&m->dy, sizeof(float) * cap * maxw))) return st;
-    if ((st = mlp_alloc(m, (void **)&m->dz, sizeof(float) * cap * maxw))) return st;
-    if ((st = mlp_alloc(m, (void **)&m->tA, sizeof(__nv_bfloat16) * cap * maxw))) return st;
-    if ((st = mlp_alloc(m, (void **)&m->tB, sizeof(__nv_bfloat16) * cap * maxw))) return st;
-    if ((st = mlp_alloc(m, (void **)&m->tAlo, sizeof(__nv_bfloat16) * cap * maxw))) return st;
-    if ((st = mlp_alloc(m, (void **)&m->tBlo, sizeof(__nv_bfloat16) * cap * maxw))) return st;
-    if ((st = mlp_alloc(m, (void **)&m->tgt, sizeof(float) * cap * m->w[m->L]))) return st;
-    m->cap = cap;
+    Split split(size_t n)
+    {
+        Split s;
+        s.hi = take<bf16>(n);
+        s.lo = take<bf16>(n);
+        return s;
+    }
+};
+
+enum Slab { SLAB_PARAMS, SLAB_GRADS, SLAB_ADAM, SLAB_FORWARD, SLAB_BACKWARD, SLAB_TRAIN };
+
+size_t carve(bec_mlp *m, Slab which, char *base, int cap)
+{
+    Carve c{base};
+    const int L = m->L;
+    auto operands = [&](int k) {
+        m->W[k].resize(L);
+        m->WT[k].resize(L);
+        for (int l = 0; l < L; ++l) {
+            m->W[k][l] = c.split((size_t)m->w[l] * m->w[l + 1]);
+            m->WT[k][l] = c.split((size_t)m->w[l] * m->w[l + 1]);
+        }
+    };
+    switch (which) {
+    case SLAB_PARAMS:
+        m->p = c.take<float>(m->n_params);
+        operands(0);
+        m->loss = c.take<float>(1);
+        m->d_err = c.take<int>(2);
+        break;
+    case SLAB_GRADS:
+        m->g = c.take<float>(m->n_params);
+        break;
+    case SLAB_ADAM:
+        m->m = c.take<float>(m->n_params);
+        m->v = c.take<float>(m->n_params);
+        operands(1);
+        break;
+    case SLAB_FORWARD:
+        m->X.assign(L + 1, Split{nullptr, nullptr});
+        m->X0[0] = c.split((size_t)cap * m->w[0]);
+        for (int l = 1; l < L; ++l) m->X[l] = c.split((size_t)cap * m->w[l]);
+        m->io = c.take<float>((size_t)cap * (m->w_real[0] + m->w_real[L]) + 64);
+        break;
+    case SLAB_BACKWARD:
+        m->y.assign(L + 1, nullptr);
+        m->dz.assign(L + 1, nullptr);
+        for (auto *v : {&m->XT, &m->D, &m->DT}) v->assign(L + 1, Split{nullptr, nullptr});
+        m->XT0[0] = c.split((size_t)cap * m->w[0]);
+        m->tgt[0] = c.take<float>((size_t)cap * m->w[L]);
+        m->raw_t = c.take<float>((size_t)cap * m->w_real[L]);
+        for (int l = 1; l <= L; ++l) {
+            const size_t n = (size_t)cap * m->w[l];
+            m->dz[l] = c.take<float>(n);
+            m->D[l] = c.split(n);
+            m->DT[l] = c.split(n);
+            if (l < L) {
+                m->y[l] = c.take<float>(n);
+                m->XT[l] = c.split(n);
+            }
+        }
+        break;
+    case SLAB_TRAIN:
+        m->X0[1] = c.split((size_t)cap * m->w[0]);
+        m->XT0[1] = c.split((size_t)cap * m->w[0]);
+        m->tgt[1] = c.take<float>((size_t)cap * m->w[L]);
+        break;
+    }
+    return c.used;
+}
+
+bec_status slab_alloc(char **p, size_t bytes)
+{
+    if (cudaMalloc((void **)p, bytes) != cudaSuccess) { cudaGetLastError(); *p = nullptr; return BEC_ERR_OUT_OF_MEMORY; }
     return BEC_OK;
 }
 
-// C[M x N] = A[M x K] B[N x K]^T (+ bias) on m's stream; A and B each as their split (hi, lo)
-void gemm_bt(bec_mlp *m, const __nv_bfloat16 *A, const __nv_bfloat16 *Alo, const __nv_bfloat16 *B,
-             const __nv_bfloat16 *Blo, float *C, const float *bias, int M, int N, int K)
+// makes a slab hold at least cap rows (batch slabs; 1 for the others)
+bec_status reserve(bec_mlp *m, Slab which, int cap)
 {
-    ensure_smem_limit((const void *)k_gemm_tc, kGemmSmem);
-    // BEC_STEP_WAIT_LIMIT_MS bounds the device-side waits (2 s by default); BEC_GEMM_INJECT_STALL=1 makes the
-    // first K group of every CTA also wait for a flag that nothing sets (the error path, without a fault)
-    unsigned long long limit_ns = 2000000000ull;
-    if (const char *v = std::getenv("BEC_STEP_WAIT_LIMIT_MS")) limit_ns = 1000000ull * std::strtoull(v, nullptr, 10);
+    if (cap <= m->cap[which]) return BEC_OK;
+    if (m->slab[which]) {
+        cudaStreamSynchronize(m->s);
+        cudaFree(m->slab[which]);
+        m->slab[which] = nullptr;
+        m->cap[which] = 0;
+    }
+    bec_status st = slab_alloc(&m->slab[which], carve(m, which, nullptr, cap));
+    if (st) return st;
+    carve(m, which, m->slab[which], cap);
+    m->cap[which] = cap;
+    if (which == SLAB_ADAM && (cudaMemsetAsync(m->m, 0, sizeof(float) * m->n_params, m->s) != cudaSuccess ||
+                               cudaMemsetAsync(m->v, 0, sizeof(float) * m->n_params, m->s) != cudaSuccess))
+        return BEC_ERR_CUDA;
+    return BEC_OK;
+}
+
+// BEC_STEP_WAIT_LIMIT_MS bounds the device-side waits (2 s by default); BEC_GEMM_INJECT_STALL=1 makes the
+// first stage of every tile also wait for a flag that nothing sets (the error path, without a fault)
+void read_env(bec_mlp *m)
+{
+    m->limit_ns = 2000000000ull;
+    if (const char *v = std::getenv("BEC_STEP_WAIT_LIMIT_MS")) m->limit_ns = 1000000ull * std::strtoull(v, nullptr, 10);
     const char *inj = std::getenv("BEC_GEMM_INJECT_STALL");
-    const int stall = inj && std::atoi(inj) ? 1 : 0;
-    dim3 grid(N / GN, (M + GM - 1) / GM);
-    k_gemm_tc<<<grid, 128, kGemmSmem, m->s>>>(A, Alo, B, Blo, C, bias, M, N, K, m->d_err, m->d_err + 1, stall,
-                                             limit_ns);
+    m->stall = inj && std::atoi(inj) ? 1 : 0;
+}
+
+GemmJob make_job(const Split &A, int Ra, const Split &B, int Rb, int M, int N, int K, int epi)
+{
+    GemmJob j{};
+    j.Ahi = A.hi; j.Alo = A.lo; j.Bhi = B.hi; j.Blo = B.lo;
+    j.Ra = Ra; j.Rb = Rb;
+    j.M = M; j.N = N; j.K = K;
+    j.epi = epi;
+    return j;
+}
+
+// launches the jobs: column tiles as narrow as one CTA per SM allows
+void launch(bec_mlp *m, Jobs &J)
+{
+    J.err = m->d_err;
+    J.never = m->d_err + 1;
+    J.stall = m->stall;
+    J.limit_ns = m->limit_ns;
+    int tn = 16, total = 0;
+    for (;; tn *= 2) {
+        total = J.bias.ctas + J.gather.ctas;
+        for (auto &g : J.gemm) {
+            g.tn = tn;
+            g.ctas = g.Ahi ? (g.M + GM - 1) / GM * (g.N / tn) : 0;
+            total += g.ctas;
+        }
+        if (total <= m->sms || tn == 64) break;
+    }
+    const bool gemm = J.gemm[0].Ahi != nullptr;
+    if (gemm) ensure_smem_limit((const void *)k_mlp, gemm_smem(64));
+    k_mlp<<<total, 128, gemm ? gemm_smem(tn) : 0, m->s>>>(J);
     g_launches++;
+}
+
+GatherJob gather_job(bec_mlp *m, int k, const float *x, const float *t, const int *idx, int rows, int valid, bool train)
+{
+    GatherJob g{};
+    g.x = x; g.t = t; g.idx = idx;
+    g.rows = rows; g.valid = valid;
+    g.in_real = m->w_real[0]; g.in = m->w[0];
+    g.out_real = m->w_real[m->L]; g.out = m->w[m->L];
+    g.ctas = rows / 8;
+    g.X = m->X0[k];
+    if (train) {
+        g.XT = m->XT0[k];
+        g.tgt = m->tgt[k];
+    }
+    return g;
+}
+
+// the forward chain on the inputs in buffer k; train: up to the loss and the output layer's dz, else the outputs of the
+// first `valid` rows to out
+void forward_chain(bec_mlp *m, int k, int rows, int valid, bool train, float *out, float *loss)
+{
+    for (int l = 0; l < m->L; ++l) {
+        const int in = m->w[l], ow = m->w[l + 1];
+        const bool last = l == m->L - 1;
+        Jobs J{};
+        GemmJob &g = J.gemm[0];
+        g = make_job(l ? m->X[l] : m->X0[k], rows, m->W[m->cur][l], ow, rows, ow, in, !last ? EPI_TANH : train ? EPI_LOSS : EPI_LINEAR);
+        g.bias = m->p + m->boff[l];
+        if (!last) {
+            g.out = m->X[l + 1];
+            if (train) {
+                g.outT = m->XT[l + 1];
+                g.f32 = m->y[l + 1];
+            }
+        } else if (train) {
+            g.tgt = m->tgt[k];
+            g.valid = valid;
+            g.real_cols = m->w_real[m->L];
+            g.loss = loss;
+            g.f32 = m->dz[l + 1];
+            g.out = m->D[l + 1];
+            g.outT = m->DT[l + 1];
+        } else {
+            g.f32 = out;
+        }
+        g.f32_ld = last && !train ? m->w_real[m->L] : ow;
+        g.f32_rows = last && !train ? valid : rows;
+        g.f32_cols = last && !train ? m->w_real[m->L] : ow;
+        launch(m, J);
+    }
+}
+
+// the backward chain from the output layer's dz: gradients into m->g, or (adam) applied to the weights, whose operands go
+// to the other set; next: gathered beside the first layer's gradient
+void backward_chain(bec_mlp *m, int k, int rows, const AdamArgs *adam, const GatherJob *next)
+{
+    for (int l = m->L - 1; l >= 0; --l) {
+        const int in = m->w[l], ow = m->w[l + 1];
+        Jobs J{};
+        // dW [out x in] = dZ^T [out x rows] * (X^T [in x rows])^T
+        GemmJob &g = J.gemm[0];
+        g = make_job(m->DT[l + 1], ow, l ? m->XT[l] : m->XT0[k], in, ow, in, rows, adam ? EPI_ADAM : EPI_GRAD);
+        if (adam) {
+            g.w = m->p + m->woff[l];
+            g.m = m->m + m->woff[l];
+            g.v = m->v + m->woff[l];
+            g.adam = *adam;
+            g.out = m->W[1 - m->cur][l];
+            g.outT = m->WT[1 - m->cur][l];
+        } else {
+            g.f32 = m->g + m->woff[l];
+            g.f32_ld = in;
+            g.f32_rows = ow;
+            g.f32_cols = in;
+        }
+        if (l > 0) {
+            // dX [rows x in] = dZ [rows x out] * (W^T [in x out])^T, times the tanh derivative: the next layer's dZ
+            GemmJob &d = J.gemm[1];
+            d = make_job(m->D[l + 1], rows, m->WT[m->cur][l], in, rows, in, ow, EPI_DX);
+            d.y = m->y[l];
+            d.f32 = m->dz[l];
+            d.f32_ld = in;
+            d.f32_rows = rows;
+            d.f32_cols = in;
+            d.out = m->D[l];
+            d.outT = m->DT[l];
+        }
+        BiasJob &b = J.bias;
+        b.dz = m->dz[l + 1];
+        b.rows = rows;
+        b.cols = ow;
+        b.ctas = (ow + 127) / 128;
+        if (adam) {
+            b.w = m->p + m->boff[l];
+            b.m = m->m + m->boff[l];
+            b.v = m->v + m->boff[l];
+            b.adam = *adam;
+        } else {
+            b.g = m->g + m->boff[l];
+        }
+        if (l == 0 && next) J.gather = *next;
+        launch(m, J);
+    }
+    if (adam) m->cur = 1 - m->cur;
+}
+
+void split_weights(bec_mlp *m)
+{
+    for (int l = 0; l < m->L; ++l) {
+        k_split_weights<<<grid_for((size_t)m->w[l] * m->w[l + 1]), 256, 0, m->s>>>(
+            m->p + m->woff[l], m->w[l + 1], m->w[l], m->W[m->cur][l], m->WT[m->cur][l]);
+        g_launches++;
+    }
 }
 
 // BEC_ERR_CUDA when a GEMM since the last check gave up a wait (synchronises the stream)
@@ -416,73 +791,6 @@ bec_status check_gemm(bec_mlp *m)
         return BEC_ERR_CUDA;
     }
     return BEC_OK;
-}
-
-// forward on the first `rows` (multiple of 64) rows of y[0] (FP32 inputs, padded)
-void mlp_forward_dev(bec_mlp *m, int rows)
-{
-    cudaStream_t s = m->s;
-    k_cast_t<<<grid_for((size_t)rows * m->w[0]), 256, 0, s>>>(m->y[0], m->xbf[0], m->xlo[0], rows, m->w[0], 0);
-    for (int l = 0; l < m->L; ++l) {
-        const int in = m->w[l], out = m->w[l + 1];
-        gemm_bt(m, m->xbf[l], m->xlo[l], m->pbf + m->woff[l], m->plo + m->woff[l], m->z[l + 1], m->p + m->boff[l],
-                rows, out, in);
-        const int linear = (l == m->L - 1);
-        k_act<<<grid_for((size_t)rows * out), 256, 0, s>>>(m->z[l + 1], m->y[l + 1], m->xbf[l + 1], m->xlo[l + 1],
-                                                           (size_t)rows * out, linear);
-        g_launches++;
-    }
-    g_launches++;
-}
-
-// gradients of the MSE loss into m->g, after mlp_forward_dev; targets in m->tgt
-void mlp_backward_dev(bec_mlp *m, int rows, int valid)
-{
-    cudaStream_t s = m->s;
-    const int outw = m->w[m->L];
-    cudaMemsetAsync(m->loss, 0, sizeof(float), s);
-    k_mse<<<grid_for((size_t)rows * outw), 256, 0, s>>>(m->y[m->L], m->tgt, m->dy, rows, valid, outw,
-                                                        m->w_real[m->L], m->loss);
-    g_launches++;
-    for (int l = m->L - 1; l >= 0; --l) {
-        const int in = m->w[l], out = m->w[l + 1];
-        const int linear = (l == m->L - 1);
-        k_act_back<<<grid_for((size_t)rows * out), 256, 0, s>>>(m->dy, m->y[l + 1], m->dz, (size_t)rows * out, linear);
-        k_colsum<<<(out + 127) / 128, 128, 0, s>>>(m->dz, m->g + m->boff[l], rows, out);
-        // dW [out x in] = dZ^T [out x rows] * (X^T [in x rows])^T
-        k_cast_t<<<grid_for((size_t)rows * out), 256, 0, s>>>(m->dz, m->tA, m->tAlo, rows, out, 1);
-        k_cast_t<<<grid_for((size_t)rows * in), 256, 0, s>>>(m->y[l], m->tB, m->tBlo, rows, in, 1);
-        gemm_bt(m, m->tA, m->tAlo, m->tB, m->tBlo, m->g + m->woff[l], nullptr, out, in, rows);
-        g_launches += 4;
-        if (l > 0) {
-            // dX [rows x in] = dZ [rows x out] * W [out x in] = dZ * (W^T [in x out])^T
-            k_cast_t<<<grid_for((size_t)rows * out), 256, 0, s>>>(m->dz, m->tA, m->tAlo, rows, out, 0);
-            k_cast_t<<<grid_for((size_t)out * in), 256, 0, s>>>(m->p + m->woff[l], m->wt, m->wtlo, out, in, 1);
-            gemm_bt(m, m->tA, m->tAlo, m->wt, m->wtlo, m->dy, nullptr, rows, in, out);
-            g_launches += 2;
-        }
-    }
-}
-
-void mlp_sync_bf16(bec_mlp *m)
-{
-    for (int l = 0; l < m->L; ++l) {
-        k_cast_t<<<grid_for((size_t)m->w[l] * m->w[l + 1]), 256, 0, m->s>>>(m->p + m->woff[l], m->pbf + m->woff[l],
-                                                                             m->plo + m->woff[l], m->w[l + 1], m->w[l],
-                                                                             0);
-        g_launches++;
-    }
-}
-
-// host x (batch x real_in) -> device y[0] (rows x padded_in)
-bec_status upload_inputs(bec_mlp *m, const float *x, int batch, int rows)
-{
-    std::vector<float> h((size_t)rows * m->w[0], 0.0f);
-    for (int r = 0; r < batch; ++r)
-        for (int c = 0; c < m->w_real[0]; ++c) h[(size_t)r * m->w[0] + c] = x[(size_t)r * m->w_real[0] + c];
-    if (cudaMemcpyAsync(m->y[0], h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice, m->s) != cudaSuccess)
-        return BEC_ERR_CUDA;
-    return cudaStreamSynchronize(m->s) == cudaSuccess ? BEC_OK : BEC_ERR_CUDA;
 }
 
 } // namespace
@@ -511,19 +819,11 @@ bec_status bec_mlp_create(const int32_t *widths, int32_t n_layers, uint64_t seed
     }
     auto bail = [&](bec_status st) { bec_mlp_destroy(m); return st; };
     bec_status st;
-    if (cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking) != cudaSuccess) return bail(BEC_ERR_CUDA);
-    if ((st = mlp_alloc(m, (void **)&m->p, sizeof(float) * m->n_params))) return bail(st);
-    if ((st = mlp_alloc(m, (void **)&m->g, sizeof(float) * m->n_params))) return bail(st);
-    if ((st = mlp_alloc(m, (void **)&m->m, sizeof(float) * m->n_params))) return bail(st);
-    if ((st = mlp_alloc(m, (void **)&m->v, sizeof(float) * m->n_params))) return bail(st);
-    if ((st = mlp_alloc(m, (void **)&m->pbf, sizeof(__nv_bfloat16) * m->n_params))) return bail(st);
-    if ((st = mlp_alloc(m, (void **)&m->plo, sizeof(__nv_bfloat16) * m->n_params))) return bail(st);
-    int maxw = 0;
-    for (int v : m->w) maxw = std::max(maxw, v);
-    if ((st = mlp_alloc(m, (void **)&m->wt, sizeof(__nv_bfloat16) * maxw * maxw))) return bail(st);
-    if ((st = mlp_alloc(m, (void **)&m->wtlo, sizeof(__nv_bfloat16) * maxw * maxw))) return bail(st);
-    if ((st = mlp_alloc(m, (void **)&m->loss, sizeof(float)))) return bail(st);
-    if ((st = mlp_alloc(m, (void **)&m->d_err, 2 * sizeof(int)))) return bail(st);
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking) != cudaSuccess)
+        return bail(BEC_ERR_CUDA);
+    if ((st = reserve(m, SLAB_PARAMS, 1))) return bail(st);
     if (cudaMemsetAsync(m->d_err, 0, 2 * sizeof(int), m->s) != cudaSuccess) return bail(BEC_ERR_CUDA);
     // Glorot-uniform weights on the real block, zero padding and biases
     std::vector<float> h(m->n_params, 0.0f);
@@ -535,9 +835,7 @@ bec_status bec_mlp_create(const int32_t *widths, int32_t n_layers, uint64_t seed
             for (int i = 0; i < widths[l]; ++i) h[m->woff[l] + (size_t)o * m->w[l] + i] = U(rng);
     }
     cudaMemcpyAsync(m->p, h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice, m->s);
-    cudaMemsetAsync(m->m, 0, sizeof(float) * m->n_params, m->s);
-    cudaMemsetAsync(m->v, 0, sizeof(float) * m->n_params, m->s);
-    mlp_sync_bf16(m);
+    split_weights(m);
     if (cudaStreamSynchronize(m->s) != cudaSuccess) return bail(BEC_ERR_CUDA);
     *out = m;
     return BEC_OK;
@@ -547,7 +845,7 @@ void bec_mlp_destroy(bec_mlp *m)
 {
     if (!m) return;
     if (m->s) cudaStreamSynchronize(m->s);
-    for (void *p : m->allocs) cudaFree(p);
+    for (char *p : m->slab) cudaFree(p);
     if (m->s) cudaStreamDestroy(m->s);
     delete m;
 }
@@ -587,7 +885,7 @@ bec_status bec_mlp_set_params(bec_mlp *m, const float *params)
         for (int o = 0; o < m->w_real[l + 1]; ++o) h[m->boff[l] + o] = params[k++];
     }
     if (cudaMemcpyAsync(m->p, h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice, m->s) != cudaSuccess) return BEC_ERR_CUDA;
-    mlp_sync_bf16(m);
+    split_weights(m);
     return cudaStreamSynchronize(m->s) == cudaSuccess ? BEC_OK : BEC_ERR_CUDA;
 }
 
@@ -596,17 +894,18 @@ bec_status bec_mlp_forward(bec_mlp *m, const float *x, int32_t batch, float *y)
     if (!m || !x || !y || batch < 1) return BEC_ERR_INVALID_ARG;
     const int rows = round_up(batch, 64);
     bec_status st;
-    if ((st = mlp_reserve(m, rows))) return st;
-    if ((st = upload_inputs(m, x, batch, rows))) return st;
-    mlp_forward_dev(m, rows);
-    const int ow = m->w[m->L];
-    std::vector<float> h((size_t)rows * ow);
-    if (cudaMemcpyAsync(h.data(), m->y[m->L], sizeof(float) * h.size(), cudaMemcpyDeviceToHost, m->s) != cudaSuccess)
-        return BEC_ERR_CUDA;
-    if ((st = check_gemm(m))) return st;
-    for (int r = 0; r < batch; ++r)
-        for (int c = 0; c < m->w_real[m->L]; ++c) y[(size_t)r * m->w_real[m->L] + c] = h[(size_t)r * ow + c];
-    return BEC_OK;
+    if ((st = reserve(m, SLAB_FORWARD, rows))) return st;
+    read_env(m);
+    const size_t nx = (size_t)batch * m->w_real[0], ny = (size_t)batch * m->w_real[m->L];
+    float *out = m->io + (nx + 63) / 64 * 64;     // aligned for 16-byte stores
+    // x is pageable or pinned memory that the caller may reuse on return: this call waits for its result
+    if (cudaMemcpyAsync(m->io, x, sizeof(float) * nx, cudaMemcpyHostToDevice, m->s) != cudaSuccess) return BEC_ERR_CUDA;
+    Jobs J{};
+    J.gather = gather_job(m, 0, m->io, nullptr, nullptr, rows, batch, false);
+    launch(m, J);
+    forward_chain(m, 0, rows, batch, false, out, nullptr);
+    if (cudaMemcpyAsync(y, out, sizeof(float) * ny, cudaMemcpyDeviceToHost, m->s) != cudaSuccess) return BEC_ERR_CUDA;
+    return check_gemm(m);
 }
 
 // Loss and gradients of mean((y - target)^2) over the batch (host params layout).
@@ -616,15 +915,19 @@ bec_status bec_mlp_gradients(bec_mlp *m, const float *x, const float *target, in
     if (!m || !x || !target || batch < 1) return BEC_ERR_INVALID_ARG;
     const int rows = round_up(batch, 64);
     bec_status st;
-    if ((st = mlp_reserve(m, rows))) return st;
-    if ((st = upload_inputs(m, x, batch, rows))) return st;
-    const int ow = m->w[m->L];
-    std::vector<float> t((size_t)rows * ow, 0.0f);
-    for (int r = 0; r < batch; ++r)
-        for (int c = 0; c < m->w_real[m->L]; ++c) t[(size_t)r * ow + c] = target[(size_t)r * m->w_real[m->L] + c];
-    cudaMemcpyAsync(m->tgt, t.data(), sizeof(float) * t.size(), cudaMemcpyHostToDevice, m->s);
-    mlp_forward_dev(m, rows);
-    mlp_backward_dev(m, rows, batch);
+    if ((st = reserve(m, SLAB_FORWARD, rows)) || (st = reserve(m, SLAB_BACKWARD, rows)) || (st = reserve(m, SLAB_GRADS, 1)))
+        return st;
+    read_env(m);
+    const size_t nx = (size_t)batch * m->w_real[0], ny = (size_t)batch * m->w_real[m->L];
+    if (cudaMemcpyAsync(m->io, x, sizeof(float) * nx, cudaMemcpyHostToDevice, m->s) != cudaSuccess ||
+        cudaMemcpyAsync(m->raw_t, target, sizeof(float) * ny, cudaMemcpyHostToDevice, m->s) != cudaSuccess ||
+        cudaMemsetAsync(m->loss, 0, sizeof(float), m->s) != cudaSuccess)
+        return BEC_ERR_CUDA;
+    Jobs J{};
+    J.gather = gather_job(m, 0, m->io, m->raw_t, nullptr, rows, batch, true);
+    launch(m, J);
+    forward_chain(m, 0, rows, batch, true, nullptr, m->loss);
+    backward_chain(m, 0, rows, nullptr, nullptr);
     float l = 0.f;
     cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->s);
     std::vector<float> h(m->n_params);
@@ -634,79 +937,91 @@ bec_status bec_mlp_gradients(bec_mlp *m, const float *x, const float *target, in
     if (grads) {
         size_t k = 0;
         for (int li = 0; li < m->L; ++li) {
-            for (int o = 0; o < m->w_real[li + 1]; ++o)
-                for (int i = 0; i < m->w_real[li]; ++i) grads[k++] = h[m->woff[li] + (size_t)o * m->w[li] + i];
-            for (int o = 0; o < m->w_real[li + 1]; ++o) grads[k++] = h[m->boff[li] + o];
+            for (int o = 0; o < m->w_real[li + 1]; ++o, k += m->w_real[li])
+                std::memcpy(grads + k, &h[m->woff[li] + (size_t)o * m->w[li]], sizeof(float) * m->w_real[li]);
+            std::memcpy(grads + k, &h[m->boff[li]], sizeof(float) * m->w_real[li + 1]);
+            k += m->w_real[li + 1];
         }
     }
     return BEC_OK;
 }
 
-// Adam on minibatches drawn (seeded) from n samples; loss_history[s] = loss of step s. Every
-// minibatch's indices are drawn up front and uploaded once, and the losses stay on the device
-// until the end, so the step loop issues work without waiting on the GPU.
+// Adam on minibatches drawn (seeded) from n samples; loss_history[s] = loss of step s. The samples are uploaded once and
+// the losses stay on the device until the end; the indices of kDrawSteps minibatches at a time are drawn and uploaded
+// while the GPU works on earlier ones, so the step loop issues work without waiting on the GPU.
 bec_status bec_mlp_train(bec_mlp *m, const float *x, const float *target, int32_t n, int32_t batch, int32_t steps,
                          float lr, int32_t schedule, uint64_t seed, float *loss_history)
 {
     if (!m || !x || !target || n < 1 || batch < 1 || steps < 0) return BEC_ERR_INVALID_ARG;
     if (schedule != BEC_LR_CONSTANT && schedule != BEC_LR_COSINE) return BEC_ERR_INVALID_ARG;
+    constexpr int kDrawSteps = 64;
     const int rows = round_up(batch, 64);
     bec_status st;
-    if ((st = mlp_reserve(m, rows))) return st;
-    const int in_r = m->w_real[0], out_r = m->w_real[m->L], inw = m->w[0], ow = m->w[m->L];
+    read_env(m);
+    if (steps == 0) return check_gemm(m);
+    if ((st = reserve(m, SLAB_ADAM, 1)) || (st = reserve(m, SLAB_FORWARD, rows)) || (st = reserve(m, SLAB_BACKWARD, rows)) ||
+        (st = reserve(m, SLAB_TRAIN, rows)))
+        return st;
+    const int in_r = m->w_real[0], out_r = m->w_real[m->L];
+    const int valid = std::min(batch, n);
     float *dx = nullptr, *dt = nullptr, *dhist = nullptr;
     int *didx = nullptr;
-    std::vector<void *> loc;
-    auto lalloc = [&](void **p, size_t b) {
-        cudaError_t e = cudaMalloc(p, b > 0 ? b : 16);
-        if (e == cudaSuccess) loc.push_back(*p);
-        return e;
+    auto samples = [&](char *base) {
+        Carve c{base};
+        dx = c.take<float>((size_t)n * in_r);
+        dt = c.take<float>((size_t)n * out_r);
+        dhist = c.take<float>(steps);
+        didx = c.take<int>((size_t)valid * steps);
+        return c.used;
     };
-    struct F { std::vector<void *> &v; cudaStream_t s; ~F() { cudaStreamSynchronize(s); for (void *p : v) cudaFree(p); } } f{loc, m->s};
-    if (lalloc((void **)&dx, sizeof(float) * (size_t)n * inw) || lalloc((void **)&dt, sizeof(float) * (size_t)n * ow) ||
-        lalloc((void **)&didx, sizeof(int) * (size_t)rows * steps) || lalloc((void **)&dhist, sizeof(float) * steps))
-        return BEC_ERR_OUT_OF_MEMORY;
-    {
-        std::vector<float> hx((size_t)n * inw, 0.0f), ht((size_t)n * ow, 0.0f);
-        for (int r = 0; r < n; ++r) {
-            for (int c = 0; c < in_r; ++c) hx[(size_t)r * inw + c] = x[(size_t)r * in_r + c];
-            for (int c = 0; c < out_r; ++c) ht[(size_t)r * ow + c] = target[(size_t)r * out_r + c];
-        }
-        cudaMemcpyAsync(dx, hx.data(), sizeof(float) * hx.size(), cudaMemcpyHostToDevice, m->s);
-        cudaMemcpyAsync(dt, ht.data(), sizeof(float) * ht.size(), cudaMemcpyHostToDevice, m->s);
-    }
+    char *slab = nullptr;
+    if ((st = slab_alloc(&slab, samples(nullptr)))) return st;
+    struct F { char *p; cudaStream_t s; ~F() { cudaStreamSynchronize(s); cudaFree(p); } } f{slab, m->s};
+    samples(slab);
+    if (cudaMemcpyAsync(dx, x, sizeof(float) * (size_t)n * in_r, cudaMemcpyHostToDevice, m->s) != cudaSuccess ||
+        cudaMemcpyAsync(dt, target, sizeof(float) * (size_t)n * out_r, cudaMemcpyHostToDevice, m->s) != cudaSuccess ||
+        cudaMemsetAsync(dhist, 0, sizeof(float) * steps, m->s) != cudaSuccess)
+        return BEC_ERR_CUDA;
     // minibatches: consecutive slices of seeded shuffles of the n samples
     std::mt19937_64 rng(seed);
-    std::vector<int> order(n);
+    std::vector<int> order(n), drawn;
     for (int i = 0; i < n; ++i) order[i] = i;
-    int pos = n;
-    const int valid = std::min(batch, n);
-    std::vector<int> hidx((size_t)rows * steps, 0);
-    for (int s = 0; s < steps; ++s)
-        for (int r = 0; r < valid; ++r) {
+    int pos = n, ready = 0;
+    auto draw = [&]() -> bec_status {
+        const int k = std::min(kDrawSteps, steps - ready);
+        drawn.resize((size_t)valid * k);
+        for (int &i : drawn) {
             if (pos >= n) { std::shuffle(order.begin(), order.end(), rng); pos = 0; }
-            hidx[(size_t)s * rows + r] = order[pos++];
+            i = order[pos++];
         }
-    if (steps > 0) cudaMemcpyAsync(didx, hidx.data(), sizeof(int) * hidx.size(), cudaMemcpyHostToDevice, m->s);
+        // the copy from this pageable buffer is staged before the call returns
+        const cudaError_t e = cudaMemcpyAsync(didx + (size_t)valid * ready, drawn.data(), sizeof(int) * drawn.size(),
+                                              cudaMemcpyHostToDevice, m->s);
+        ready += k;
+        return e == cudaSuccess ? BEC_OK : BEC_ERR_CUDA;
+    };
+    auto minibatch = [&](int s) { return gather_job(m, s & 1, dx, dt, didx + (size_t)valid * s, rows, valid, true); };
     const double pi = 3.14159265358979323846;
     for (int s = 0; s < steps; ++s) {
-        const int *bidx = didx + (size_t)s * rows;
-        k_gather<<<grid_for((size_t)rows * inw), 256, 0, m->s>>>(dx, bidx, m->y[0], rows, valid, inw);
-        k_gather<<<grid_for((size_t)rows * ow), 256, 0, m->s>>>(dt, bidx, m->tgt, rows, valid, ow);
-        mlp_forward_dev(m, rows);
-        mlp_backward_dev(m, rows, valid);
+        if (s == 0) {
+            if ((st = draw())) return st;
+            Jobs J{};
+            J.gather = minibatch(0);
+            launch(m, J);
+        }
+        if (s + 1 < steps && s + 1 == ready && (st = draw())) return st;
+        forward_chain(m, s & 1, rows, valid, true, nullptr, dhist + s);
         ++m->adam_t;
-        const float b1 = 0.9f, b2 = 0.999f;
-        const float c1 = 1.0f - std::pow(b1, (float)m->adam_t), c2 = 1.0f - std::pow(b2, (float)m->adam_t);
-        const float lr_s = schedule == BEC_LR_COSINE ? (float)(lr * 0.5 * (1.0 + std::cos(pi * s / steps))) : lr;
-        k_adam<<<grid_for(m->n_params), 256, 0, m->s>>>(m->p, m->m, m->v, m->g, m->n_params, lr_s, b1, b2, 1e-8f, c1,
-                                                        c2);
-        mlp_sync_bf16(m);
-        cudaMemcpyAsync(dhist + s, m->loss, sizeof(float), cudaMemcpyDeviceToDevice, m->s);
-        g_launches += 3;
+        AdamArgs a;
+        a.c1 = 1.0f - std::pow(0.9f, (float)m->adam_t);
+        a.c2 = 1.0f - std::pow(0.999f, (float)m->adam_t);
+        a.lr = schedule == BEC_LR_COSINE ? (float)(lr * 0.5 * (1.0 + std::cos(pi * s / steps))) : lr;
+        GatherJob next{};
+        if (s + 1 < steps) next = minibatch(s + 1);
+        backward_chain(m, s & 1, rows, &a, s + 1 < steps ? &next : nullptr);
     }
     std::vector<float> hist(steps, 0.0f);
-    if (steps > 0) cudaMemcpyAsync(hist.data(), dhist, sizeof(float) * steps, cudaMemcpyDeviceToHost, m->s);
+    cudaMemcpyAsync(hist.data(), dhist, sizeof(float) * steps, cudaMemcpyDeviceToHost, m->s);
     if ((st = check_gemm(m))) return st;
     if (loss_history)
         for (int s = 0; s < steps; ++s) loss_history[s] = hist[s];
