@@ -1357,7 +1357,8 @@ bec_status ground_state_fused(bec_ctx *ctx, GroupRec &gr, const Gs64Dims &dim, c
     const size_t cells = g.cells, state = sizeof(double2) * cells;
     const size_t n_norm = 2 * (size_t)dim.pencil_ctas();
     const size_t n_part = std::max(5 * (size_t)dim.plane_ctas(), 2 * (size_t)dim.pencil_ctas());
-    const size_t small = sizeof(double) * (n_norm + n_part + kGs64Sums + 4) + sizeof(Gs64Par);
+    const size_t n_kick = (size_t)g.nz + (size_t)g.nx * g.ny;
+    const size_t small = sizeof(double) * (n_norm + n_part + kGs64Sums + 4 + n_kick) + sizeof(Gs64Par);
     const size_t bytes = (ref_rule ? 3 : 2) * state + small + 64;
     char *buf = ctx->gs64_buf;
     struct Free { char *p = nullptr; cudaStream_t s; ~Free() { if (p) { cudaStreamSynchronize(s); cudaFree(p); } } } temp;
@@ -1385,10 +1386,12 @@ bec_status ground_state_fused(bec_ctx *ctx, GroupRec &gr, const Gs64Dims &dim, c
     double2 *work = reinterpret_cast<double2 *>(buf), *a = work + cells, *kout = ref_rule ? a + cells : nullptr;
     double *norm_part = reinterpret_cast<double *>(buf + (ref_rule ? 3 : 2) * state);
     double *part = norm_part + n_norm, *sums = part + n_part, *sums4 = sums + kGs64Sums;
-    Gs64Par *par = reinterpret_cast<Gs64Par *>(sums4 + 4);
+    double *kick = sums4 + 4;
+    Gs64Par *par = reinterpret_cast<Gs64Par *>(kick + n_kick);
     Gs64Tab tab;
     bec_status st;
     if ((st = get_gs64_tab(ctx, g, tab))) return st;
+    tab.kick = kick;
     const Gs64Par hp{g, gr.d.N, gr.d.mu};
 
     CKC(cudaEventRecord(ctx->ev0, s));

@@ -96,6 +96,7 @@ struct Gs64Dims {
 };
 struct Gs64Tab {
     const double2 *x, *y, *z; // all n twiddles W_n^k of each axis
+    double *kick = nullptr;   // half-kick factors of the steps, nz + nx ny doubles, filled by gs64_start (one trajectory)
 };
 // sums of a boundary: n V, n^2, n, |u - previous out|^2, the reference's energy integrand, |psi_k|^2 and
 // |psi_k|^2 k^2/2 before renormalisation; of gs64_measures: n V, n^2, n, |psi_k|^2 k^2/2, |(H - mu) psi|^2

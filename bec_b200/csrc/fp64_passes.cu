@@ -12,12 +12,14 @@
 // What bounds it: latency. A 16x16x128 state is 512 KiB; at HBM rate the two passes would take 0.3 us. A pass is a
 // launch, one trip to L2 and back, and two to three radix-8 stages per axis in shared memory. Tiles are therefore
 // small (a plane, or two to eight pencils), so that one trajectory fills the chip. Measured on one 16x16x128 ground
-// state of 500 steps: 83.4 ms with one kernel per operation (30 launches a step), 8.43 ms here. The measures of a
+// state of 500 steps: 83.4 ms with one kernel per operation (30 launches a step), 5.33 ms here (8.43 ms before the
+// twiddles and kick factors lay in shared memory at the pass's start and a launch overlapped the end of the one before). The measures of a
 // batch (mu, energy, norm, residual) took twenty launches and two synchronisations a state; here they take eight
 // launches for half the batch (96 states of 32x32x256 with 60 steps: the whole call 42.6 -> 23.2 ms).
 #include <algorithm>
 
 #include "engine.h"
+#include "launch.cuh"
 #include "reduce.cuh"
 
 namespace {
@@ -78,7 +80,7 @@ struct Lines {
 // One stage of span m = 2^lm and radix R over every line. Decimation in time (DIF = false): twiddles before the
 // small transform; in frequency: after it.
 template <int R, bool INV, bool DIF>
-__device__ __forceinline__ void stage(double2 *buf, const Lines &L, const double2 *__restrict__ tw, int lm)
+__device__ __forceinline__ void stage(double2 *buf, const Lines &L, const double2 *tw, int lm)
 {
     constexpr int LR = R == 8 ? 3 : R == 4 ? 2 : 1;
     const int total = 1 << (L.log_lines + L.logn - LR);
@@ -184,11 +186,11 @@ enum { START, MEASURE, STEP, OUT, RESIDUAL };
 template <int MODE, typename S>
 __global__ void __launch_bounds__(256) k64_plane(double2 *__restrict__ state, const Gs64Par *__restrict__ par, int lx, int ly,
                                                  int lz, int lppc, const double2 *__restrict__ tx,
-                                                 const double2 *__restrict__ ty, const double *__restrict__ norm_part,
-                                                 int norm_tiles, const S *__restrict__ src, double2 *__restrict__ out,
-                                                 const double2 *__restrict__ kout, const double *__restrict__ sums4,
-                                                 double *__restrict__ part)
+                                                 const double2 *__restrict__ ty, const double *norm_part, int norm_tiles,
+                                                 const S *src, double2 *out, const double2 *kout, const double *sums4,
+                                                 double *part)
 {
+    // (what the kernel before this one writes is not declared __restrict__: such loads might move above the wait)
     extern __shared__ double2 sm64[];
     __shared__ double red[5 * 32];
     const int nx = 1 << lx, ny = 1 << ly, ld = nx + 1, lplane = lx + ly;
@@ -202,7 +204,13 @@ __global__ void __launch_bounds__(256) k64_plane(double2 *__restrict__ state, co
         return ((i >> lplane) * ny + digit_rev((i >> lx) & (ny - 1), ly)) * ld + digit_rev(i & (nx - 1), lx);
     };
     const Lines rows{lx, lppc + ly, 1, 30, ld, 0}, cols{ly, lppc + lx, ld, lx, 1, ny * ld};
+    // the twiddles beside the tile: read from L2 stage by stage they would add a trip to every barrier
+    double2 *twx = sm64 + ((ny << lppc) * ld), *twy = twx + nx;
+    for (int i = threadIdx.x; i < nx; i += blockDim.x) copy16(twx + i, tx + i);
+    for (int i = threadIdx.x; i < ny; i += blockDim.x) copy16(twy + i, ty + i);
 
+    wait_predecessor();
+    allow_successor();
     if (MODE == STEP || MODE == OUT || MODE == RESIDUAL)
         for (int i = threadIdx.x; i < chunk; i += blockDim.x) copy16(sm64 + reversed(i), state + first + i);
     const Gs64Par &Q = par[traj];
@@ -223,8 +231,8 @@ __global__ void __launch_bounds__(256) k64_plane(double2 *__restrict__ state, co
     if (MODE == STEP || MODE == OUT || MODE == RESIDUAL) {
         copy_wait();
         __syncthreads();
-        fft_time<false>(sm64, rows, tx);
-        if (ly > 0) fft_time<false>(sm64, cols, ty);
+        fft_time<false>(sm64, rows, twx);
+        if (ly > 0) fft_time<false>(sm64, cols, twy);
     }
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     for (int i = threadIdx.x; i < chunk; i += blockDim.x) {
@@ -281,9 +289,10 @@ __global__ void __launch_bounds__(256) k64_plane(double2 *__restrict__ state, co
         }
     }
     if (MODE == START || MODE == MEASURE || MODE == STEP) {
+        copy_wait();
         __syncthreads();
-        if (ly > 0) fft_freq<true>(sm64, cols, ty);
-        fft_freq<true>(sm64, rows, tx);
+        if (ly > 0) fft_freq<true>(sm64, cols, twy);
+        fft_freq<true>(sm64, rows, twx);
         for (int i = threadIdx.x; i < chunk; i += blockDim.x) state[first + i] = sm64[reversed(i)];
     }
     if (MODE == MEASURE || MODE == OUT || MODE == RESIDUAL) {
@@ -304,19 +313,19 @@ __global__ void __launch_bounds__(256) k64_plane(double2 *__restrict__ state, co
 enum { KICK1 = 1, SUMS = 2, KICK2 = 4, TIMES_K2 = 8 };
 
 __global__ void __launch_bounds__(256) k64_pencil(double2 *__restrict__ state, const Gs64Par *__restrict__ par, int lx, int ly,
-                                                  int lz, int lp, const double2 *__restrict__ tz, double scale, int what,
+                                                  int lz, int lp, const double2 *__restrict__ tz,
+                                                  const double *__restrict__ kick, double scale, int what,
                                                   double *__restrict__ part, double2 *__restrict__ kout)
 {
     extern __shared__ double2 sm64[];
     __shared__ double red[2 * 32];
     __shared__ double exy[8], kxy[8];
     const int nx = 1 << lx, nz = 1 << lz, lplane = lx + ly, P = 1 << lp, chunk = nz << lp;
-    double *ez = reinterpret_cast<double *>(sm64 + chunk);     // half-kick factors per kz, then kz^2/2
+    double2 *tw = sm64 + chunk;
+    double *ez = reinterpret_cast<double *>(tw + nz);          // half-kick factors per kz, then kz^2/2
     double *kz2 = ez + nz;
     const int traj = blockIdx.x >> (lplane - lp), pen0 = (blockIdx.x & ((1 << (lplane - lp)) - 1)) << lp;
     double2 *g0 = state + ((size_t)traj << (lplane + lz)) + pen0;
-    for (int i = threadIdx.x; i < chunk; i += blockDim.x)
-        copy16(sm64 + (digit_rev(i >> lp, lz) << lp) + (i & (P - 1)), g0 + ((size_t)(i >> lp) << lplane) + (i & (P - 1)));
     const Gs64Par &Q = par[traj];
     const GeomD &g = Q.g;
     for (int i = threadIdx.x; i < nz + P; i += blockDim.x) {
@@ -330,14 +339,20 @@ __global__ void __launch_bounds__(256) k64_pencil(double2 *__restrict__ state, c
             const double ky = ly > 0 ? getk<double>(pen >> lx, g.dky, 1 << ly) : 0.0;
             k2 = (kx * kx + ky * ky) / 2.0;
         }
-        const double e = (what & (KICK1 | KICK2)) ? exp(-g.dt_steady / 2.0 * k2) : 1.0;   // wigner_kernel.cu:128-134
+        // the half-kick factors come from k64_kick's table
+        const double e = (what & (KICK1 | KICK2)) ? kick[i < nz ? i : i + pen0] : 1.0;
         if (i < nz) { ez[i] = e; kz2[i] = k2; }
         else { exy[i - nz] = e; kxy[i - nz] = k2; }
     }
+    for (int i = threadIdx.x; i < nz; i += blockDim.x) copy16(tw + i, tz + i);
+    wait_predecessor();
+    allow_successor();
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x)
+        copy16(sm64 + (digit_rev(i >> lp, lz) << lp) + (i & (P - 1)), g0 + ((size_t)(i >> lp) << lplane) + (i & (P - 1)));
     copy_wait();
     __syncthreads();
     const Lines L{lz, lp, P, 30, 1, 0};
-    fft_time<true>(sm64, L, tz);
+    fft_time<true>(sm64, L, tw);
     double v[2] = {0.0, 0.0};
     for (int i = threadIdx.x; i < chunk; i += blockDim.x) {
         const int z = i >> lp, p = i & (P - 1);
@@ -355,7 +370,7 @@ __global__ void __launch_bounds__(256) k64_pencil(double2 *__restrict__ state, c
         sm64[i] = u;
     }
     __syncthreads();
-    fft_freq<false>(sm64, L, tz);
+    fft_freq<false>(sm64, L, tw);
     for (int i = threadIdx.x; i < chunk; i += blockDim.x)
         g0[((size_t)(i >> lp) << lplane) + (i & (P - 1))] = sm64[(digit_rev(i >> lp, lz) << lp) + (i & (P - 1))];
     if (what & SUMS) {
@@ -364,6 +379,27 @@ __global__ void __launch_bounds__(256) k64_pencil(double2 *__restrict__ state, c
             part[(size_t)blockIdx.x * 2] = v[0];
             part[(size_t)blockIdx.x * 2 + 1] = v[1];
         }
+    }
+}
+
+// half-kick factors exp(-dt/2 k^2/2) of one trajectory (propagateKSpaceImaginaryTime, wigner_kernel.cu:128-134): nz of the
+// kz, then nx ny of (kx, ky)
+__global__ void k64_kick(const Gs64Par *__restrict__ par, int lx, int ly, int lz, double *__restrict__ kick)
+{
+    const GeomD &g = par->g;
+    const int nx = 1 << lx, nz = 1 << lz, n = nz + (1 << (lx + ly));
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        double k2;
+        if (i < nz) {
+            const double kz = getk<double>(i, g.dkz, nz);
+            k2 = kz * kz / 2.0;
+        } else {
+            const int pen = i - nz;
+            const double kx = getk<double>(pen & (nx - 1), g.dkx, nx);
+            const double ky = ly > 0 ? getk<double>(pen >> lx, g.dky, 1 << ly) : 0.0;
+            k2 = (kx * kx + ky * ky) / 2.0;
+        }
+        kick[i] = exp(-g.dt_steady / 2.0 * k2);
     }
 }
 
@@ -380,8 +416,11 @@ __global__ void k64_fold(const double *__restrict__ part, int n, int K, int firs
     }
 }
 
-size_t plane_smem(int lx, int ly, int lppc) { return sizeof(double2) * (((size_t)1 << (ly + lppc)) * ((1 << lx) + 1)); }
-size_t pencil_smem(int lz, int lp) { return sizeof(double2) * ((size_t)1 << (lz + lp)) + sizeof(double) * 2 * ((size_t)1 << lz); }
+size_t plane_smem(int lx, int ly, int lppc)
+{
+    return sizeof(double2) * ((((size_t)1 << (ly + lppc)) * ((1 << lx) + 1)) + ((size_t)1 << lx) + ((size_t)1 << ly));
+}
+size_t pencil_smem(int lz, int lp) { return sizeof(double2) * (((size_t)1 << (lz + lp)) + ((size_t)2 << lz)); }
 constexpr size_t kMaxSmem = 200 * 1024;
 
 int ilog(int n) { int r = 0; while ((1 << r) < n) ++r; return r; }
@@ -394,10 +433,8 @@ cudaError_t plane_launch(const Gs64Dims &d, const Gs64Tab &t, double2 *state, co
     const size_t smem = plane_smem(d.lx, d.ly, d.lppc);
     cudaError_t e = ensure_smem_limit((const void *)k64_plane<MODE, S>, (int)kMaxSmem);
     if (e) return e;
-    k64_plane<MODE, S><<<d.n * d.plane_ctas(), threads_for(d.lppc + d.lx + d.ly), smem, s>>>(
-        state, par, d.lx, d.ly, d.lz, d.lppc, t.x, t.y, norm_part, d.pencil_ctas(), src, out, kout, sums4, part);
-    g_launches++;
-    return cudaGetLastError();
+    return launch_after(k64_plane<MODE, S>, d.n * d.plane_ctas(), threads_for(d.lppc + d.lx + d.ly), smem, s, state, par, d.lx,
+                        d.ly, d.lz, d.lppc, t.x, t.y, norm_part, d.pencil_ctas(), src, out, kout, sums4, part);
 }
 
 cudaError_t pencil_launch(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, double scale, int what,
@@ -405,10 +442,8 @@ cudaError_t pencil_launch(const Gs64Dims &d, const Gs64Tab &t, double2 *state, c
 {
     cudaError_t e = ensure_smem_limit((const void *)k64_pencil, (int)kMaxSmem);
     if (e) return e;
-    k64_pencil<<<d.n * d.pencil_ctas(), threads_for(d.lz + d.lp), pencil_smem(d.lz, d.lp), s>>>(
-        state, par, d.lx, d.ly, d.lz, d.lp, t.z, scale, what, part, kout);
-    g_launches++;
-    return cudaGetLastError();
+    return launch_after(k64_pencil, d.n * d.pencil_ctas(), threads_for(d.lz + d.lp), pencil_smem(d.lz, d.lp), s, state, par, d.lx,
+                        d.ly, d.lz, d.lp, t.z, t.kick, scale, what, part, kout);
 }
 
 void fold_launch(const Gs64Dims &d, const double *part, int n, int K, int first, int count, double *out, int off, cudaStream_t s)
@@ -436,6 +471,8 @@ bool gs64_dims(int nx, int ny, int nz, int n_traj, Gs64Dims &d)
 cudaError_t gs64_start(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, const double2 *warm,
                        double *norm_part, cudaStream_t s)
 {
+    k64_kick<<<(d.cells() >> d.lz) / 128 + 1, 128, 0, s>>>(par, d.lx, d.ly, d.lz, t.kick);
+    g_launches++;
     cudaError_t e = plane_launch<START, double2>(d, t, state, par, nullptr, warm, nullptr, nullptr, nullptr, nullptr, s);
     return e ? e : pencil_launch(d, t, state, par, 1.0 / d.cells(), SUMS | KICK2, norm_part, nullptr, s);
 }

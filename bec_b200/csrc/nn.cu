@@ -23,9 +23,10 @@
 // derivative, the loss or Adam, and writes its result as the split operands that the
 // next GEMMs read, plain and transposed, already in the tiles' shared-memory layout; a
 // layer's weight gradient, bias gradient and input gradient share a launch, and the
-// next minibatch is gathered beside the first layer's. Weights' operands alternate
+// next minibatch is gathered beside the first layer's. A launch sets itself up (barriers, tensor memory) while the one
+// before it finishes (launch.cuh), and an epilogue fetches what it reads while the tile's operands load. Weights' operands alternate
 // between two buffers, so that a launch can update a layer that another tile of it
-// still reads. 87 us a step (batch 256, 400 steps with the set-up) against 314 us with one kernel per
+// still reads. 78 us a step (batch 256, 400 steps with the set-up) against 314 us with one kernel per
 // operation.
 #include <algorithm>
 #include <cstdlib>
@@ -38,6 +39,7 @@
 #include <cuda_bf16.h>
 
 #include "engine.h"
+#include "launch.cuh"
 
 namespace {
 
@@ -244,43 +246,53 @@ __device__ __forceinline__ void store16(float *p, const float (&o)[16])
     for (int q = 0; q < 4; ++q) reinterpret_cast<float4 *>(p)[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
 }
 
-// row's 16 accumulator columns from col on; returns the row's share of the loss (EPI_LOSS)
-__device__ __forceinline__ float epilogue(const GemmJob &J, int row, int col, float (&o)[16])
+// what the epilogue reads beside the accumulator: the tile's first 16 columns are fetched while its operands load
+struct Aux {
+    float a[16], b[16], c[16];
+};
+__device__ __forceinline__ void load_aux(const GemmJob &J, Aux &x, int row, int col)
 {
-    float l = 0.0f, b[16];
+    const size_t at = (size_t)row * J.N + col;
+    if (J.epi <= EPI_LOSS) load16(x.a, J.bias + col);
+    if (J.epi == EPI_LOSS) load16(x.b, J.tgt + at);
+    if (J.epi == EPI_DX) load16(x.a, J.y + at);
+    if (J.epi == EPI_ADAM) {
+        load16(x.a, J.w + at);
+        load16(x.b, J.m + at);
+        load16(x.c, J.v + at);
+    }
+}
+
+// row's 16 accumulator columns from col on; returns the row's share of the loss (EPI_LOSS)
+__device__ __forceinline__ float epilogue(const GemmJob &J, int row, int col, float (&o)[16], Aux &x)
+{
+    float l = 0.0f;
     const size_t at = (size_t)row * J.N + col;
     if (J.epi <= EPI_LOSS) {
-        load16(b, J.bias + col);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) o[q] += b[q];
+        for (int q = 0; q < 16; ++q) o[q] += x.a[q];
     }
     if (J.epi == EPI_TANH) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) o[q] = tanhf(o[q]);
     } else if (J.epi == EPI_LOSS) {
         // the padding columns of y and t are zero, padding rows get no gradient
-        load16(b, J.tgt + at);
         const float s = 2.0f / ((float)J.valid * J.real_cols);
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
-            const float d = row < J.valid ? o[q] - b[q] : 0.0f;
+            const float d = row < J.valid ? o[q] - x.b[q] : 0.0f;
             l += d * d;
             o[q] = s * d;
         }
     } else if (J.epi == EPI_DX) {
-        load16(b, J.y + at);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) o[q] *= 1.0f - b[q] * b[q];
+        for (int q = 0; q < 16; ++q) o[q] *= 1.0f - x.a[q] * x.a[q];
     } else if (J.epi == EPI_ADAM) {
-        float w[16], m[16], v[16];
-        load16(w, J.w + at);
-        load16(m, J.m + at);
-        load16(v, J.v + at);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) o[q] = adam_update(w[q], m[q], v[q], o[q], J.adam);
-        store16(J.w + at, w);
-        store16(J.m + at, m);
-        store16(J.v + at, v);
+        for (int q = 0; q < 16; ++q) o[q] = adam_update(x.a[q], x.b[q], x.c[q], o[q], J.adam);
+        store16(J.w + at, x.a);
+        store16(J.m + at, x.b);
+        store16(J.v + at, x.c);
     }
     if (J.f32 && row < J.f32_rows) {
         float *dst = J.f32 + (size_t)row * J.f32_ld + col;
@@ -319,6 +331,11 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
 
+    wait_predecessor();
+    allow_successor();
+    const int lr = warp * 32 + (t & 31);
+    Aux x;
+    if (lr < rows) load_aux(J, x, m0 + lr, n0);
     bool ok = true;
     if (t == 0) {
         // instruction descriptor, kind::f16: D F32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1), both K-major,
@@ -375,7 +392,6 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
     const bool failed = __syncthreads_or(!ok);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!failed) {
-        const int lr = warp * 32 + (t & 31);
         float l = 0.0f;
         for (int cb = 0; cb < tn; cb += 16) {
             uint32_t r[16];
@@ -390,7 +406,8 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
                 float o[16];
 #pragma unroll
                 for (int q = 0; q < 16; ++q) o[q] = __uint_as_float(r[q]);
-                l += epilogue(J, m0 + lr, n0 + cb, o);
+                if (cb > 0) load_aux(J, x, m0 + lr, n0 + cb);
+                l += epilogue(J, m0 + lr, n0 + cb, o, x);
             }
         }
         if (J.epi == EPI_LOSS) {
@@ -403,13 +420,29 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
 }
 
-__device__ __forceinline__ void bias_columns(const BiasJob &J, int cta)
+// 32 columns per CTA, 128 rows at a time through shared memory, so that the loads overlap while the sum keeps its order
+constexpr int kBiasCols = 32, kBiasRows = 128;
+__device__ __forceinline__ void bias_columns(const BiasJob &J, int cta, float *sm)
 {
-    const int c = cta * 128 + threadIdx.x;
-    if (c >= J.cols) return;
+    const int t = threadIdx.x, c = cta * kBiasCols + (t & 31);
     float s = 0.0f;
+    for (int r0 = 0; r0 < J.rows; r0 += kBiasRows) {
+        const int n = min(kBiasRows, J.rows - r0);
+        float v[kBiasRows / 4];
+#pragma unroll
+        for (int i = 0; i < kBiasRows / 4; ++i) {
+            const int r = i * 4 + (t >> 5);
+            v[i] = r < n ? J.dz[(size_t)(r0 + r) * J.cols + c] : 0.0f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kBiasRows / 4; ++i) sm[(i * 4 + (t >> 5)) * 32 + (t & 31)] = v[i];
+        __syncthreads();
+        if (t < 32)
 #pragma unroll 16
-    for (int r = 0; r < J.rows; ++r) s += J.dz[(size_t)r * J.cols + c];
+            for (int r = 0; r < n; ++r) s += sm[r * 32 + t];
+    }
+    if (t >= 32) return;
     if (J.g) J.g[c] = s;
     else adam_update(J.w[c], J.m[c], J.v[c], s, J.adam);
 }
@@ -450,8 +483,10 @@ __global__ void __launch_bounds__(128) k_mlp(const __grid_constant__ Jobs jobs)
         }
         b -= jobs.gemm[j].ctas;
     }
+    wait_predecessor();
+    allow_successor();
     if (b < jobs.bias.ctas) {
-        bias_columns(jobs.bias, b);
+        bias_columns(jobs.bias, b, reinterpret_cast<float *>(sm));
         return;
     }
     gather_rows(jobs.gather, b - jobs.bias.ctas);
@@ -482,11 +517,11 @@ struct bec_mlp {
     int L = 0;                       // weight layers
     std::vector<size_t> woff, boff;  // offsets into the parameter vector
     size_t n_params = 0;
-    // device memory, one slab per use, each allocated by the first call that needs it: parameters and their operands;
-    // the gradient vector; Adam moments and the second set of operands; the buffers of a batch for inference, for its
-    // gradients, and for training
-    char *slab[6] = {};
-    int cap[6] = {};                 // 1, or the batch capacity of slabs 3 to 5
+    // device memory, one slab per use: parameters and their operands; Adam moments and the second set of operands; the
+    // buffers of a batch for inference, for its gradients, and for training. The first and, for kFirstBatch rows, the third
+    // exist from the start, the others from the first call that needs them.
+    char *slab[5] = {};
+    int cap[5] = {};                 // 1, or the batch capacity of slabs 2 to 4
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;   // FP32 params, grads, Adam moments
     std::vector<Split> W[2], WT[2];  // per layer the weights' operands, plain and transposed: the current set and the
     int cur = 0;                     // one that a training step writes
@@ -531,7 +566,8 @@ struct Carve {
     }
 };
 
-enum Slab { SLAB_PARAMS, SLAB_GRADS, SLAB_ADAM, SLAB_FORWARD, SLAB_BACKWARD, SLAB_TRAIN };
+enum Slab { SLAB_PARAMS, SLAB_ADAM, SLAB_FORWARD, SLAB_BACKWARD, SLAB_TRAIN };
+constexpr int kFirstBatch = 256;
 
 size_t carve(bec_mlp *m, Slab which, char *base, int cap)
 {
@@ -552,9 +588,6 @@ size_t carve(bec_mlp *m, Slab which, char *base, int cap)
         m->loss = c.take<float>(1);
         m->d_err = c.take<int>(2);
         break;
-    case SLAB_GRADS:
-        m->g = c.take<float>(m->n_params);
-        break;
     case SLAB_ADAM:
         m->m = c.take<float>(m->n_params);
         m->v = c.take<float>(m->n_params);
@@ -570,6 +603,7 @@ size_t carve(bec_mlp *m, Slab which, char *base, int cap)
         m->y.assign(L + 1, nullptr);
         m->dz.assign(L + 1, nullptr);
         for (auto *v : {&m->XT, &m->D, &m->DT}) v->assign(L + 1, Split{nullptr, nullptr});
+        m->g = c.take<float>(m->n_params);
         m->XT0[0] = c.split((size_t)cap * m->w[0]);
         m->tgt[0] = c.take<float>((size_t)cap * m->w[L]);
         m->raw_t = c.take<float>((size_t)cap * m->w_real[L]);
@@ -658,8 +692,7 @@ void launch(bec_mlp *m, Jobs &J)
     }
     const bool gemm = J.gemm[0].Ahi != nullptr;
     if (gemm) ensure_smem_limit((const void *)k_mlp, gemm_smem(64));
-    k_mlp<<<total, 128, gemm ? gemm_smem(tn) : 0, m->s>>>(J);
-    g_launches++;
+    launch_after(k_mlp, total, 128, gemm ? gemm_smem(tn) : 0, m->s, J);
 }
 
 GatherJob gather_job(bec_mlp *m, int k, const float *x, const float *t, const int *idx, int rows, int valid, bool train)
@@ -752,7 +785,7 @@ void backward_chain(bec_mlp *m, int k, int rows, const AdamArgs *adam, const Gat
         b.dz = m->dz[l + 1];
         b.rows = rows;
         b.cols = ow;
-        b.ctas = (ow + 127) / 128;
+        b.ctas = ow / kBiasCols;
         if (adam) {
             b.w = m->p + m->boff[l];
             b.m = m->m + m->boff[l];
@@ -823,7 +856,7 @@ bec_status bec_mlp_create(const int32_t *widths, int32_t n_layers, uint64_t seed
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking) != cudaSuccess)
         return bail(BEC_ERR_CUDA);
-    if ((st = reserve(m, SLAB_PARAMS, 1))) return bail(st);
+    if ((st = reserve(m, SLAB_PARAMS, 1)) || (st = reserve(m, SLAB_FORWARD, kFirstBatch))) return bail(st);
     if (cudaMemsetAsync(m->d_err, 0, 2 * sizeof(int), m->s) != cudaSuccess) return bail(BEC_ERR_CUDA);
     // Glorot-uniform weights on the real block, zero padding and biases
     std::vector<float> h(m->n_params, 0.0f);
@@ -915,8 +948,7 @@ bec_status bec_mlp_gradients(bec_mlp *m, const float *x, const float *target, in
     if (!m || !x || !target || batch < 1) return BEC_ERR_INVALID_ARG;
     const int rows = round_up(batch, 64);
     bec_status st;
-    if ((st = reserve(m, SLAB_FORWARD, rows)) || (st = reserve(m, SLAB_BACKWARD, rows)) || (st = reserve(m, SLAB_GRADS, 1)))
-        return st;
+    if ((st = reserve(m, SLAB_FORWARD, rows)) || (st = reserve(m, SLAB_BACKWARD, rows))) return st;
     read_env(m);
     const size_t nx = (size_t)batch * m->w_real[0], ny = (size_t)batch * m->w_real[m->L];
     if (cudaMemcpyAsync(m->io, x, sizeof(float) * nx, cudaMemcpyHostToDevice, m->s) != cudaSuccess ||
