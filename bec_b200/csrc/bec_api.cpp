@@ -71,6 +71,8 @@ struct ClassRec {
     double pencil_ms[2] = {-1.0, -1.0};        // autotuner: ms per launch of each pencil kernel
     bool onchip = false;      // the tuned schedules run this class's steady steps as one on-chip launch
     double plane_ms = -1.0, onchip_ms = -1.0;  // autotuner: its plane launch, its on-chip step
+    bool split_pencil = false, split_plane = false;   // the tuned schedules run this pass with four cells per thread
+    double pair_ms[4] = {-1.0, -1.0, -1.0, -1.0};     // autotuner: a captured step's two launches; 1: split pencil, 2: split plane
 };
 
 } // namespace
@@ -390,7 +392,12 @@ bec_status plain_step(bec_ctx *ctx, GroupRec &gr, int t)
 // a class whose steady step runs as one on-chip launch in the step being launched
 bool onchip_now(const bec_ctx *ctx, const ClassRec &c)
 {
-    return ctx->step_onchip && ctx->pencil_tuned && c.onchip && c.kin_tab[1] && fp32_onchip_supported(c.geom);
+    return ctx->step_onchip && ctx->pencil_tuned && c.onchip && !c.split_pencil && !c.split_plane && c.kin_tab[1] &&
+           fp32_onchip_supported(c.geom);
+}
+bool split_plane_now(const bec_ctx *ctx, const ClassRec &c)
+{
+    return ctx->use_fast && ctx->pencil_tuned && c.split_plane && fp32_plane_split_supported(c.geom);
 }
 
 bec_status batched_zpass_all(bec_ctx *ctx, float pre, float post, bool observe, const double2 *m2,
@@ -443,7 +450,9 @@ bec_status batched_zpass_all(bec_ctx *ctx, float pre, float post, bool observe, 
             const float frac = kf;
             const float2 *kin = frac == 1.0f ? c.kin_tab[1] : frac == 0.5f ? c.kin_tab[0] : nullptr;
             const int kind = !observe && ctx->pencil_tuned ? c.pencil_kind : kPencilRegister;
-            if (kind == kPencilTma && fp32_pencil_tma_supported(c.geom))
+            if (!observe && ctx->pencil_tuned && c.split_pencil)
+                fp32_pencil_split(c.state, c.geom, twf, z.scale * z.out_scale, mf, kin, ctx->stream);
+            else if (kind == kPencilTma && fp32_pencil_tma_supported(c.geom))
                 CKC(fp32_pencil_tma(c.state, c.geom, twf, frac, z.scale * z.out_scale, mf, kin, ctx->d_pflags,
                                     ctx->d_pflags + 1, ctx->stream));
             else
@@ -484,8 +493,10 @@ bec_status batched_ppass_all(bec_ctx *ctx, std::pair<cudaEvent_t, cudaEvent_t> *
     };
     auto onchip = [&](int ci) { return onchip_now(ctx, ctx->classes[ci]); };
     auto fast = [&](int ci) { return onchip(ci) || (ctx->use_fast && fp32_fast_plane_supported(ctx->classes[ci].geom)); };
+    auto split = [&](int ci) { return split_plane_now(ctx, ctx->classes[ci]); };
     auto ctas = [&](int ci) {
-        return onchip(ci) ? ctx->classes[ci].geom.n_traj : fp32_plane_fast_ctas(ctx->classes[ci].geom);
+        const ClassGeom &g = ctx->classes[ci].geom;
+        return onchip(ci) ? g.n_traj : split(ci) ? fp32_plane_split_ctas(g) : fp32_plane_fast_ctas(g);
     };
     int carrier = -1;
     if (advanced) {
@@ -505,6 +516,9 @@ bec_status batched_ppass_all(bec_ctx *ctx, std::pair<cudaEvent_t, cudaEvent_t> *
             bec_status st;
             if ((st = get_tw32_full(ctx, c.geom.nz, &twf))) return st;
             fp32_onchip_step(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, twf, c.kin_tab[1], ctx->d_step,
+                             ci == carrier ? ctx->d_pflags + 2 : nullptr, ctx->stream);
+        } else if (split(ci)) {
+            fp32_plane_split(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, ctx->d_step,
                              ci == carrier ? ctx->d_pflags + 2 : nullptr, ctx->stream);
         } else if (fast(ci)) {
             fp32_plane_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, ctx->d_step, ctx->plane_occupancy,
@@ -564,7 +578,7 @@ bec_status batched_step(bec_ctx *ctx, float pre, bool put_step)
 constexpr int kPerPassCandidates = 4;
 constexpr int kAllCandidates = kPerPassCandidates + kStepCandidates;
 const char *const kPerPassNames[kPerPassCandidates] = {"unfused", "unfused-20", "unfused-tma", "unfused-20-tma"};
-constexpr size_t kPickClasses = 11;   // classes whose picks the plan cache keeps (two bits each above bit 8)
+constexpr size_t kPickClasses = 13;   // classes whose picks the plan cache keeps (four bits each above bit 8)
 
 std::string candidate_name(int c)
 {
@@ -580,56 +594,127 @@ bec_status check_step_error(bec_ctx *ctx);
 // kernel (16 pencils per CTA of nz threads, 16 warps per SM) or the persistent TMA kernel (three CTAs per SM,
 // the next tile's load in flight). Both compute the same bits; each is timed over three launches after one
 // warm-up on the current state (the caller restores it).
+// ms of what enqueue() launches, replayed from a captured graph; left alone (-1) when it cannot be captured
+template <class F>
+bec_status time_captured(bec_ctx *ctx, double *ms, F &&enqueue)
+{
+    constexpr int kTimes = 16;
+    const long long l0 = g_launches;
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+        for (int i = 0; i < kTimes; ++i) enqueue();
+        if (cudaStreamEndCapture(ctx->stream, &graph) == cudaSuccess && graph) cudaGraphInstantiate(&exec, graph, 0);
+        if (graph) cudaGraphDestroy(graph);
+    }
+    g_launches = l0;
+    cudaGetLastError();
+    if (!exec) return BEC_OK;
+    struct Destroy { cudaGraphExec_t e; ~Destroy() { cudaGraphExecDestroy(e); } } destroy{exec};
+    for (int r = 0; r < 3; ++r) {
+        if (r == 1) CKC(cudaEventRecord(ctx->ev0, ctx->stream));
+        CKC(cudaGraphLaunch(exec, ctx->stream));
+    }
+    CKC(cudaEventRecord(ctx->ev1, ctx->stream));
+    CKC(cudaEventSynchronize(ctx->ev1));
+    float t = 0.f;
+    CKC(cudaEventElapsedTime(&t, ctx->ev0, ctx->ev1));
+    *ms = t / (2 * kTimes);
+    return BEC_OK;
+}
+
+// Classes up to this many cells try the split passes: beyond it the chip is full with sixteen cells per thread (64
+// trajectories of 16x16x128: 42.2 us a step against 43.3; 32: 26.2 against 25.4).
+constexpr long long kSplitCells = 1 << 21;
+
 bec_status pick_pencil_kernels(bec_ctx *ctx)
 {
     for (auto &c : ctx->classes) {
         c.pencil_kind = kPencilRegister;
         c.pencil_ms[0] = c.pencil_ms[1] = -1.0;
-        c.onchip = false;
+        c.onchip = c.split_pencil = c.split_plane = false;
         c.plane_ms = c.onchip_ms = -1.0;
+        for (double &ms : c.pair_ms) ms = -1.0;
         if (c.geom.n_traj == 0 || !ctx->use_fast || !fp32_fast_pencil_supported(c.geom) || !c.kin_tab[1]) continue;
         float2 *twf;
         bec_status st;
         if ((st = get_tw32_full(ctx, c.geom.nz, &twf))) return st;
         const float scale = (float)(1.0 / (double)c.geom.cells);
-        for (int kind = 0; kind < kPencilKinds; ++kind) {
-            if (kind == kPencilTma && !fp32_pencil_tma_supported(c.geom)) continue;
-            for (int r = 0; r < 4; ++r) {
-                if (r == 1) CKC(cudaEventRecord(ctx->ev0, ctx->stream));
-                if (kind == kPencilRegister)
-                    fp32_pencil_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, twf, 1.0f, scale, nullptr, nullptr,
-                                     1.0f, c.kin_tab[1], ctx->stream);
-                else
-                    CKC(fp32_pencil_tma(c.state, c.geom, twf, 1.0f, scale, nullptr, c.kin_tab[1], ctx->d_pflags,
-                                        ctx->d_pflags + 1, ctx->stream));
-            }
-            CKC(cudaEventRecord(ctx->ev1, ctx->stream));
-            CKC(cudaEventSynchronize(ctx->ev1));
-            float ms = 0.f;
-            CKC(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-            c.pencil_ms[kind] = ms / 3.0;
-            if (c.pencil_ms[kind] < c.pencil_ms[c.pencil_kind]) c.pencil_kind = kind;
-        }
-        // an 8x8x64 class: its steady step as one on-chip launch against its faster pencil launch plus its plane
-        // launch (the step index is left alone: no launch here advances it)
-        if (fp32_onchip_supported(c.geom) && fp32_fast_plane_supported(c.geom)) {
-            for (int kind = 0; kind < 2; ++kind) {
-                for (int r = 0; r < 4; ++r) {
+        // ms per launch: three launches after one warm-up, and launches of a few microseconds again over thirty, which the
+        // events' resolution needs (no launch advances the step index)
+        auto time_launch = [&](double *ms, auto &&launch) -> bec_status {
+            for (int n : {3, 30}) {
+                for (int r = 0; r <= n; ++r) {
                     if (r == 1) CKC(cudaEventRecord(ctx->ev0, ctx->stream));
-                    if (kind == 0)
-                        fp32_plane_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, ctx->d_step,
-                                        ctx->plane_occupancy, nullptr, ctx->stream);
-                    else
-                        fp32_onchip_step(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, twf, c.kin_tab[1],
-                                         ctx->d_step, nullptr, ctx->stream);
+                    launch();
+                    CKL();
                 }
                 CKC(cudaEventRecord(ctx->ev1, ctx->stream));
                 CKC(cudaEventSynchronize(ctx->ev1));
-                float ms = 0.f;
-                CKC(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-                (kind == 0 ? c.plane_ms : c.onchip_ms) = ms / 3.0;
+                float t = 0.f;
+                CKC(cudaEventElapsedTime(&t, ctx->ev0, ctx->ev1));
+                *ms = t / n;
+                if (*ms > 0.05) break;
             }
-            c.onchip = c.onchip_ms < c.pencil_ms[c.pencil_kind] + c.plane_ms;
+            return BEC_OK;
+        };
+        for (int kind = 0; kind < kPencilKinds; ++kind) {
+            if (kind == kPencilTma && !fp32_pencil_tma_supported(c.geom)) continue;
+            if ((st = time_launch(&c.pencil_ms[kind], [&] {
+                     if (kind == kPencilRegister)
+                         fp32_pencil_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, twf, 1.0f, scale, nullptr, nullptr,
+                                          1.0f, c.kin_tab[1], ctx->stream);
+                     else
+                         fp32_pencil_tma(c.state, c.geom, twf, 1.0f, scale, nullptr, c.kin_tab[1], ctx->d_pflags,
+                                         ctx->d_pflags + 1, ctx->stream);
+                 })))
+                return st;
+            if (c.pencil_ms[kind] < c.pencil_ms[c.pencil_kind]) c.pencil_kind = kind;
+        }
+        const double pencil_ms = c.pencil_ms[c.pencil_kind];
+        auto pencil = [&](bool split) {
+            if (split)
+                fp32_pencil_split(c.state, c.geom, twf, scale, nullptr, c.kin_tab[1], ctx->stream);
+            else if (c.pencil_kind == kPencilTma)
+                fp32_pencil_tma(c.state, c.geom, twf, 1.0f, scale, nullptr, c.kin_tab[1], ctx->d_pflags, ctx->d_pflags + 1,
+                                ctx->stream);
+            else
+                fp32_pencil_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, twf, 1.0f, scale, nullptr, nullptr, 1.0f,
+                                 c.kin_tab[1], ctx->stream);
+        };
+        const bool fast_plane = fp32_fast_plane_supported(c.geom), split_plane = fp32_plane_split_supported(c.geom);
+        auto plane = [&](bool split) {
+            if (split)
+                fp32_plane_split(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, ctx->d_step, nullptr, ctx->stream);
+            else if (fast_plane)
+                fp32_plane_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, ctx->d_step, ctx->plane_occupancy,
+                                nullptr, ctx->stream);
+        };
+        if (fast_plane && (st = time_launch(&c.plane_ms, [&] { plane(false); }))) return st;
+        // a small class: the two launches of a step with four cells per thread in either, both or none, timed as a captured
+        // step runs them (launched one by one, launches this short show the host's pace)
+        if ((long long)c.geom.n_traj * c.geom.cells <= kSplitCells) {
+            int best = 0;
+            for (int k = 0; k < 4; ++k) {
+                if ((k & 2) && !split_plane) continue;
+                if ((st = time_captured(ctx, &c.pair_ms[k], [&] { pencil(k & 1); plane(k & 2); }))) return st;
+                if (c.pair_ms[k] > 0 && c.pair_ms[k] < c.pair_ms[best]) best = k;
+            }
+            c.split_pencil = best & 1;
+            c.split_plane = best & 2;
+        }
+        if (!fast_plane) continue;
+        // an 8x8x64 class: its steady step as one on-chip launch against its faster pencil launch plus its plane launch
+        if (fp32_onchip_supported(c.geom)) {
+            if ((st = time_launch(&c.onchip_ms, [&] {
+                     fp32_onchip_step(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, twf, c.kin_tab[1], ctx->d_step,
+                                      nullptr, ctx->stream);
+                 })))
+                return st;
+            c.onchip = c.onchip_ms < pencil_ms + c.plane_ms;
+            // the split launches, where they are faster still, go before it
+            const int k = (c.split_pencil ? 1 : 0) | (c.split_plane ? 2 : 0);
+            if (c.onchip && k && c.onchip_ms <= c.pair_ms[k]) c.split_pencil = c.split_plane = false;
         }
     }
     return BEC_OK;
@@ -641,7 +726,9 @@ bec_status ensure_plan(bec_ctx *ctx)
     ctx->fused.assign(ctx->classes.size(), 0);
     const char *force = std::getenv("BEC_STEP_PLAN");
     const std::string fs = force ? force : "";
-    std::vector<ClassGeom> geoms;
+    std::vector<ClassGeom> geoms, all_geoms;
+    for (auto &c : ctx->classes) all_geoms.push_back(c.geom);
+    long long cached = 0;
     std::vector<StepClassDev> devs;
     std::vector<int> offs, idx;
     if (ctx->use_fast) {
@@ -691,7 +778,7 @@ bec_status ensure_plan(bec_ctx *ctx)
         cand = named;                                  // "-tma": every class on the TMA pencil kernel
         for (auto &c : ctx->classes) {
             c.pencil_kind = named < 2 ? kPencilRegister : kPencilTma;
-            c.onchip = false;
+            c.onchip = c.split_pencil = c.split_plane = false;
         }
         how = "forced";
     } else if (fs == "unfused-onchip") {
@@ -699,6 +786,7 @@ bec_status ensure_plan(bec_ctx *ctx)
         for (auto &c : ctx->classes) {
             c.pencil_kind = kPencilRegister;
             c.onchip = fp32_onchip_supported(c.geom);
+            c.split_pencil = c.split_plane = false;
         }
         how = "forced";
     } else if (!fs.empty()) {
@@ -707,13 +795,17 @@ bec_status ensure_plan(bec_ctx *ctx)
             return fail(ctx, BEC_ERR_INVALID_ARG, "BEC_STEP_PLAN: no such fused work list for this context");
         cand = kPerPassCandidates + k;
         how = "forced";
-    } else if (step_plan_cached(geoms, &cand)) {
-        // the candidate, and above bit 8 two bits per class: its pencil kernel, its on-chip step
+    } else if (step_plan_cached(all_geoms, &cached)) {
+        // the candidate, and above bit 8 four bits per class: its pencil kernel, its on-chip step, its split passes
         for (size_t ci = 0; ci < ctx->classes.size() && ci < kPickClasses; ++ci) {
-            ctx->classes[ci].pencil_kind = (cand >> (8 + 2 * ci)) & 1;
-            ctx->classes[ci].onchip = (cand >> (9 + 2 * ci)) & 1;
+            ClassRec &c = ctx->classes[ci];
+            const int b = (int)(cached >> (8 + 4 * ci)) & 15;
+            c.pencil_kind = b & 1;
+            c.onchip = b >> 1 & 1;
+            c.split_pencil = b >> 2 & 1;
+            c.split_plane = b >> 3 & 1;
         }
-        cand &= 0xFF;
+        cand = (int)(cached & 0xFF);
         how = "cached";
     } else {
         const char *at = std::getenv("BEC_AUTOTUNE");
@@ -737,7 +829,8 @@ bec_status ensure_plan(bec_ctx *ctx)
                 double best = 1e30;
                 for (int k = 0; k < n_cand && st == BEC_OK; ++k) {
                     if ((st = apply(k))) break;
-                    for (int r = 0; r < 4 && st == BEC_OK; ++r) {
+                    const int reps = best < 0.2 ? 20 : 3;          // short steps need more of them
+                    for (int r = 0; r <= reps && st == BEC_OK; ++r) {
                         if (r == 1) cudaEventRecord(ctx->ev0, ctx->stream);
                         st = batched_step(ctx, 0.5f, true);
                     }
@@ -749,7 +842,7 @@ bec_status ensure_plan(bec_ctx *ctx)
                     }
                     float ms = 0.f;
                     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-                    tms[k] = ms / 3.0;
+                    tms[k] = ms / reps;
                     if (tms[k] < best) { best = tms[k]; cand = k; }
                 }
                 o = 0;
@@ -764,11 +857,12 @@ bec_status ensure_plan(bec_ctx *ctx)
                 if (st) return st;
                 if ((st = check_step_error(ctx))) return st;
                 how = "autotuned";
-                int picks = 0;
-                for (size_t ci = 0; ci < ctx->classes.size() && ci < kPickClasses; ++ci)
-                    picks |= (ctx->classes[ci].pencil_kind << (8 + 2 * ci)) |
-                             ((ctx->classes[ci].onchip ? 1 : 0) << (9 + 2 * ci));
-                step_plan_remember(geoms, cand | picks);
+                long long picks = 0;
+                for (size_t ci = 0; ci < ctx->classes.size() && ci < kPickClasses; ++ci) {
+                    const ClassRec &c = ctx->classes[ci];
+                    picks |= (long long)(c.pencil_kind | c.onchip << 1 | c.split_pencil << 2 | c.split_plane << 3) << (8 + 4 * ci);
+                }
+                step_plan_remember(all_geoms, cand | picks);
             } else {
                 cudaGetLastError();
             }
@@ -780,7 +874,7 @@ bec_status ensure_plan(bec_ctx *ctx)
     const bool fused = cand >= kPerPassCandidates;
     int n_classes = 0;
     for (auto &c : ctx->classes) n_classes += c.geom.n_traj > 0;
-    char buf[256];
+    char buf[512];
     std::string j = "{\"plan\": \"" + candidate_name(cand) + "\", \"candidate\": " + std::to_string(cand) +
                     ", \"chosen\": \"" + how + "\", \"fused_classes\": " + std::to_string(fused ? (int)idx.size() : 0) +
                     ", \"launches_per_step\": " +
@@ -793,11 +887,14 @@ bec_status ensure_plan(bec_ctx *ctx)
         if (c.geom.n_traj == 0) continue;
         const int kind = ctx->pencil_tuned ? c.pencil_kind : kPencilRegister;
         const bool oc = ctx->pencil_tuned && c.onchip && fp32_onchip_supported(c.geom);
+        const int sp = ctx->pencil_tuned ? (c.split_pencil ? 1 : 0) | (c.split_plane ? 2 : 0) : 0;
         std::snprintf(buf, sizeof buf,
                       "%s{\"grid\": [%d, %d, %d], \"kernel\": \"%s\", \"register_ms\": %.4f, \"tma_ms\": %.4f, "
-                      "\"onchip\": %s, \"plane_ms\": %.4f, \"onchip_ms\": %.4f}",
+                      "\"onchip\": %s, \"plane_ms\": %.4f, \"onchip_ms\": %.4f, \"split_pencil\": %s, "
+                      "\"split_plane\": %s, \"pair_ms\": [%.4f, %.4f, %.4f, %.4f]}",
                       firstc ? "" : ", ", c.geom.nx, c.geom.ny, c.geom.nz, kPencilNames[kind], c.pencil_ms[0],
-                      c.pencil_ms[1], oc ? "true" : "false", c.plane_ms, c.onchip_ms);
+                      c.pencil_ms[1], oc ? "true" : "false", c.plane_ms, c.onchip_ms, sp & 1 ? "true" : "false",
+                      sp & 2 ? "true" : "false", c.pair_ms[0], c.pair_ms[1], c.pair_ms[2], c.pair_ms[3]);
         j += buf;
         firstc = false;
     }

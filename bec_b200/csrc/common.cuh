@@ -118,13 +118,13 @@ __device__ __forceinline__ u32x4x2 philox4x32_10_x2(uint32_t a0, uint32_t a1, ui
 struct u32x4x4 { u32x4 a, b, c, d; };
 
 __device__ __forceinline__ u32x4x4 philox4x32_10_x4(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
-                                                    const PhiloxKeys &K)
+                                                    const PhiloxKeys &K, uint32_t d = 1u)
 {
-    // counters (c0 + i, c1, c2, c3), i < 4
+    // counters (c0 + i d, c1, c2, c3), i < 4
     uint32_t a0 = c0, a1 = c1, a2 = c2, a3 = c3;
-    uint32_t b0 = c0 + 1u, b1 = c1, b2 = c2, b3 = c3;
-    uint32_t e0 = c0 + 2u, e1 = c1, e2 = c2, e3 = c3;
-    uint32_t d0 = c0 + 3u, d1 = c1, d2 = c2, d3 = c3;
+    uint32_t b0 = c0 + d, b1 = c1, b2 = c2, b3 = c3;
+    uint32_t e0 = c0 + 2u * d, e1 = c1, e2 = c2, e3 = c3;
+    uint32_t d0 = c0 + 3u * d, d1 = c1, d2 = c2, d3 = c3;
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
         uint32_t la0, ha0, la1, ha1, lb0, hb0, lb1, hb1, le0, he0, le1, he1, ld0, hd0, ld1, hd1;

@@ -242,6 +242,15 @@ void fp32_pencil_fast(float4 *state, const ClassGeom &c, const GroupParamsF *gp,
 // = e^{+i kz_i^2/2 dt frac} for i < nz, then e^{+i (kx^2 + ky^2)/2 dt frac} per pencil (y * nx + x)
 void fp32_kin_tables(float2 *tab, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, float frac,
                      cudaStream_t s);
+// split_passes.cu: the plane pass (8x8 and 16x16 planes) and the non-observing pencil pass (nz = 64, 128, 256) with four
+// cells per thread, for classes with too few trajectories to fill the chip; the same bits as fp32_plane_fast and
+// fp32_pencil_fast
+bool fp32_plane_split_supported(const ClassGeom &c);
+int fp32_plane_split_ctas(const ClassGeom &c);
+void fp32_plane_split(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
+                      uint32_t *d_step, int *inc_done, cudaStream_t s);
+void fp32_pencil_split(float4 *state, const ClassGeom &c, const float2 *tw_full, float scale, const float2 *m,
+                       const float2 *kin, cudaStream_t s);
 // onchip_step.cu: a steady step (full kick, no pulse, no observation) of an 8x8x64 class with each trajectory's
 // state in shared memory, one launch instead of its pencil and plane launches; kin_full: the class's full-kick
 // kinetic table; inc_done as fp32_plane_fast
@@ -304,5 +313,5 @@ void step_launch(const StepPlan &P, const GroupParamsF *gp, uint32_t *d_step, fl
 // *err = 1 if a dependency wait of a launch since the plan was built gave up (synchronises s)
 cudaError_t step_read_error(const StepPlan &P, int *err, cudaStream_t s);
 // per-process cache of the autotuned candidate for a class mix on this device (-1: per-pass launches)
-bool step_plan_cached(const std::vector<ClassGeom> &geoms, int *candidate);
-void step_plan_remember(const std::vector<ClassGeom> &geoms, int candidate);
+bool step_plan_cached(const std::vector<ClassGeom> &geoms, long long *candidate);
+void step_plan_remember(const std::vector<ClassGeom> &geoms, long long candidate);

@@ -169,12 +169,13 @@ __device__ __forceinline__ void loss_noise_cell2(fftreg::cpair &out0, const fftr
 }
 
 
-// The loss-noise increments of four consecutive cells cell0 .. cell0 + 3 of the same trajectory and step:
+// The loss-noise increments of four cells cell0 + d i, i < 4, of the same trajectory and step:
 // one interleaved group of four Philox4x32-10 draws.
 __device__ __forceinline__ void loss_noise_cell4(fftreg::cpair out[4], const fftreg::cpair v0[4], const CellConsts &K,
-                                                 const PhiloxKeys &keys, uint32_t traj, uint32_t step, uint32_t cell0)
+                                                 const PhiloxKeys &keys, uint32_t traj, uint32_t step, uint32_t cell0,
+                                                 uint32_t d = 1u)
 {
-    const u32x4x4 w = philox4x32_10_x4(cell0, step, traj, RNG_TAG_LOSS, keys);
+    const u32x4x4 w = philox4x32_10_x4(cell0, step, traj, RNG_TAG_LOSS, keys, d);
     out[0] = loss_noise_apply(out[0], v0[0], K, w.a);
     out[1] = loss_noise_apply(out[1], v0[1], K, w.b);
     out[2] = loss_noise_apply(out[2], v0[2], K, w.c);

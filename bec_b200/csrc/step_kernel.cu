@@ -187,7 +187,7 @@ struct PlanKey {
 };
 
 std::mutex g_plan_mutex;
-std::map<PlanKey, int> g_plan_cache;   // chosen candidate per class mix and SM count
+std::map<PlanKey, long long> g_plan_cache;   // chosen candidate and picks per class mix and SM count
 
 PlanKey plan_key(const std::vector<ClassGeom> &geoms)
 {
@@ -364,7 +364,7 @@ cudaError_t step_read_error(const StepPlan &P, int *err, cudaStream_t s)
     return e;
 }
 
-bool step_plan_cached(const std::vector<ClassGeom> &geoms, int *candidate)
+bool step_plan_cached(const std::vector<ClassGeom> &geoms, long long *candidate)
 {
     PlanKey k = plan_key(geoms);
     std::lock_guard<std::mutex> lock(g_plan_mutex);
@@ -374,7 +374,7 @@ bool step_plan_cached(const std::vector<ClassGeom> &geoms, int *candidate)
     return true;
 }
 
-void step_plan_remember(const std::vector<ClassGeom> &geoms, int candidate)
+void step_plan_remember(const std::vector<ClassGeom> &geoms, long long candidate)
 {
     PlanKey k = plan_key(geoms);
     std::lock_guard<std::mutex> lock(g_plan_mutex);

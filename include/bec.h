@@ -366,7 +366,8 @@ int32_t bec_step_graphs(const bec_ctx *ctx);
  * first step an autotuner times the candidates on a copy of the state -- per-pass launches with
  * the plane passes at 16 or at 20 warps per SM, each with the register pencil kernel or with every
  * class's pencil pass on the faster of the register kernel and a persistent TMA kernel (timed per
- * class: "pencil_kernels" in the JSON), and the work list run in two phases or interleaving each
+ * class: "pencil_kernels" in the JSON; classes of few trajectories also try passes with four cells
+ * per thread, "split_pencil" and "split_plane"), and the work list run in two phases or interleaving each
  * trajectory's plane items 0.5 to 4 waves of the grid after its pencil items -- and keeps the
  * fastest for this class mix and device (cached per process). BEC_STEP_PLAN in the environment
  * forces one (unfused, unfused-20, unfused-tma and unfused-20-tma with every class on the TMA
