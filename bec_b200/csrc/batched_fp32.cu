@@ -1,4 +1,4 @@
-// batched_fp32.cu -- the batched FP32 split-step path.
+// batched_fp32.cu -- the general FP32 passes: any power-of-two grid, the initial states, and the reductions.
 //
 // One split step of the reference (propagate, programs/bec_wigner_3d.cuda/
 // wigner.cu:178-199: K/2 -> FFT -> N(dt) -> IFFT -> 1/cells -> K/2) is
@@ -6,7 +6,7 @@
 //
 //   z pass (pencils along z):  IFFT_z -> 1/cells -> K (the previous step's
 //                              second half-kick merged with this step's first)
-//                              [-> pulse] [-> observe] -> FFT_z
+//                              [-> pulse] -> FFT_z [-> observe]
 //   plane pass (x-y planes):   FFT_xy -> nonlinear + losses + loss noise
 //                              -> IFFT_xy
 //
@@ -16,198 +16,346 @@
 // IFFT_xy(psi_x) (unnormalised, nx*ny times larger), which the next z pass
 // turns into ifftn(psi_x) with its 1/cells. A z pass that ends a step (no
 // plane pass follows) multiplies by nx*ny on the way out so the state is
-// again in the form a z pass reads. Both components of a cell travel together as one float4,
-// stored (a.re, b.re, a.im, b.im): the register passes operate on the two components as packed
-// pairs (fft_reg.cuh). Every load and store is a 16-byte vector and the nonlinear step sees both
-// components in registers; the kernels of this file reorder a cell to (a.re, a.im, b.re, b.im)
-// on its way in and back on its way out. The FFTs run in shared memory (fft_smem.cuh); each pass reads and writes the state once.
+// again in the form a z pass reads. Both components of a cell travel together as one 16-byte
+// value (a.re, b.re, a.im, b.im).
+//
+// The shapes that most runs use take the register passes (fused_passes.cu); these kernels
+// serve the others (2D slices, planes that are not square or not 8, 16 or 32 wide, other nz), and the transforms of
+// every grid's initial and fetched states. They are bound by latency: a run on such a grid has a few thousand to a few
+// hundred thousand cells, whose HBM time is well under a microsecond. So a CTA's tile is small (a plane or a few, 128 cells
+// or more; two to sixteen pencils), which fills the chip with one trajectory, three radix-2 stages share a barrier, and the
+// kinetic phases, the same at every step, come from a table per ensemble. A step of one 32x128 slice takes 6.6 us and one
+// of a 4x4x512 trajectory 9.9 us; with 2048-cell tiles, a barrier per stage and the phases evaluated in FP64 in every pass
+// they took 21.9 and 51.5 us, with the same bits. (256 trajectories of 64x32x16: 516 us a step, 887 then.)
+#include <algorithm>
+
+#include "common.cuh"
 #include "engine.h"
-#include "fft_smem.cuh"
+#include "launch.cuh"
 #include "reduce.cuh"
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kTileElems = 2048;   // float4 elements per CTA tile (32 KiB)
+// ---------------------------------------------------------------- cells
+// A cell in the stored order (a.re, b.re, a.im, b.im), and the operations of the transforms on it.
+struct __align__(16) Cell {
+    float ar, br, ai, bi;
+};
+__device__ __forceinline__ Cell make_cell(float2 a, float2 b) { return Cell{a.x, b.x, a.y, b.y}; }
+__device__ __forceinline__ float2 cell_a(const Cell &v) { return make_float2(v.ar, v.ai); }
+__device__ __forceinline__ float2 cell_b(const Cell &v) { return make_float2(v.br, v.bi); }
+__device__ __forceinline__ Cell cell_add(Cell p, Cell q) { return Cell{p.ar + q.ar, p.br + q.br, p.ai + q.ai, p.bi + q.bi}; }
+__device__ __forceinline__ Cell cell_sub(Cell p, Cell q) { return Cell{p.ar - q.ar, p.br - q.br, p.ai - q.ai, p.bi - q.bi}; }
+__device__ __forceinline__ Cell cell_scale(Cell v, float s) { return Cell{v.ar * s, v.br * s, v.ai * s, v.bi * s}; }
+__device__ __forceinline__ Cell cell_mul(Cell v, float2 w) { return make_cell(cmul(cell_a(v), w), cmul(cell_b(v), w)); }
 
-inline int planes_per_cta(const ClassGeom &c)
+// ---------------------------------------------------------------- transforms in shared memory
+// Radix-2 butterflies over lines of n = 2^logn cells at base(line) + e * es, base = (line & (2^lin - 1)) * ls_in + (line >>
+// lin) * ls_out: decimation in time (bit-reversed -> natural) and in frequency (natural -> bit-reversed), one after the
+// other in tw = W_n^k = e^{-2 pi i k / n} (conjugated when INV). A thread takes the 2^LR cells that LR consecutive stages
+// combine through its registers, so a barrier separates three stages instead of one.
+struct Lines {
+    int logn, log_lines, es, lin, ls_in, ls_out;
+    __device__ __forceinline__ int base(int line) const { return (line & ((1 << lin) - 1)) * ls_in + (line >> lin) * ls_out; }
+};
+
+// stages s .. s + LR - 1 in time
+template <int LR, bool INV>
+__device__ __forceinline__ void stages_time(Cell *buf, const Lines &L, const float2 *tw, int s)
 {
-    int ppc = kTileElems / (c.nx * c.ny);
-    if (ppc < 1) ppc = 1;
-    if (ppc > c.nz) ppc = c.nz;
-    return ppc;
+    constexpr int R = 1 << LR;
+    const int total = 1 << (L.log_lines + L.logn - LR);
+    for (int w = threadIdx.x; w < total; w += blockDim.x) {
+        const int line = w & ((1 << L.log_lines) - 1), jj = w >> L.log_lines;
+        const int j = jj & ((1 << s) - 1);
+        Cell *p = buf + L.base(line) + (((jj >> s) << (s + LR)) + j) * L.es;
+        const int step = L.es << s;
+        Cell x[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) x[r] = p[r * step];
+#pragma unroll
+        for (int q = 0; q < LR; ++q) {
+            const int shift = L.logn - 1 - s - q;       // stage s + q: W_n^{pos << shift}, pos < 2^(s + q)
+#pragma unroll
+            for (int m = 0; m < 1 << q; ++m) {
+                float2 t = tw[(j + (m << s)) << shift];
+                if (INV) t.y = -t.y;
+#pragma unroll
+                for (int r = m; r < R; r += 2 << q) {
+                    const Cell u = x[r], v = cell_mul(x[r + (1 << q)], t);
+                    x[r] = cell_add(u, v);
+                    x[r + (1 << q)] = cell_sub(u, v);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) p[r * step] = x[r];
+    }
+    __syncthreads();
 }
 
-inline void ztile(const ClassGeom &c, int &tx, int &ty)
+// stages s + LR - 1 .. s in frequency
+template <int LR, bool INV>
+__device__ __forceinline__ void stages_freq(Cell *buf, const Lines &L, const float2 *tw, int s)
 {
-    tx = c.nx < 16 ? c.nx : 16;
-    ty = kTileElems / (tx * c.nz);
-    if (ty < 1) ty = 1;
-    if (ty > c.ny) ty = c.ny;
+    constexpr int R = 1 << LR;
+    const int total = 1 << (L.log_lines + L.logn - LR);
+    for (int w = threadIdx.x; w < total; w += blockDim.x) {
+        const int line = w & ((1 << L.log_lines) - 1), jj = w >> L.log_lines;
+        const int j = jj & ((1 << s) - 1);
+        Cell *p = buf + L.base(line) + (((jj >> s) << (s + LR)) + j) * L.es;
+        const int step = L.es << s;
+        Cell x[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) x[r] = p[r * step];
+#pragma unroll
+        for (int q = LR - 1; q >= 0; --q) {
+            const int shift = L.logn - 1 - s - q;
+#pragma unroll
+            for (int m = 0; m < 1 << q; ++m) {
+                float2 t = tw[(j + (m << s)) << shift];
+                if (INV) t.y = -t.y;
+#pragma unroll
+                for (int r = m; r < R; r += 2 << q) {
+                    const Cell u = x[r], v = x[r + (1 << q)];
+                    x[r] = cell_add(u, v);
+                    x[r + (1 << q)] = cell_mul(cell_sub(u, v), t);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) p[r * step] = x[r];
+    }
+    __syncthreads();
 }
 
-// (a.re, b.re, a.im, b.im) <-> (a.re, a.im, b.re, b.im)
-__device__ __forceinline__ float4 cell_swap(float4 v) { return make_float4(v.x, v.z, v.y, v.w); }
+template <bool INV>
+__device__ __forceinline__ void fft_time(Cell *buf, const Lines &L, const float2 *tw)
+{
+    const int first = L.logn % 3;
+    if (first == 1) stages_time<1, INV>(buf, L, tw, 0);
+    else if (first == 2) stages_time<2, INV>(buf, L, tw, 0);
+    for (int s = first; s < L.logn; s += 3) stages_time<3, INV>(buf, L, tw, s);
+}
+template <bool INV>
+__device__ __forceinline__ void fft_freq(Cell *buf, const Lines &L, const float2 *tw)
+{
+    const int first = L.logn % 3;
+    for (int s = L.logn - 3; s >= first; s -= 3) stages_freq<3, INV>(buf, L, tw, s);
+    if (first == 1) stages_freq<1, INV>(buf, L, tw, 0);
+    else if (first == 2) stages_freq<2, INV>(buf, L, tw, 0);
+}
 
-// ---------------------------------------------------------------- init
+__device__ __forceinline__ void copy16(Cell *dst_smem, const Cell *src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy8(float2 *dst_smem, const float2 *src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// ---------------------------------------------------------------- initial states
 // initializeEnsembles (wigner_kernel.cu:295-317): x-space a = gs + Va eta_a / sqrt(dV),
 // b = Vb eta_b / sqrt(dV), eta = (n0 + i n1) / 2 from Philox or injected.
-__global__ void k_init(float4 *state, int cells, int ne, GroupParamsF gp, const double2 *gs, const float2 *noise)
+__device__ __forceinline__ Cell initial_cell(float2 g, const GroupParamsF &P, float2 ea, float2 eb)
 {
-    const size_t n = (size_t)cells * ne;
-    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
-        const int t = (int)(idx / cells);
-        const int i = (int)(idx - (size_t)t * cells);
-        float2 ea, eb;
-        if (noise) {
-            ea = noise[((size_t)t * 2 + 0) * cells + i];
-            eb = noise[((size_t)t * 2 + 1) * cells + i];
-        } else {
-            float r[4];
-            const uint64_t seed = ((uint64_t)gp.seed_hi << 32) | gp.seed_lo;
-            normals4<float>(seed, (uint32_t)t, 0u, (uint32_t)i, RNG_TAG_INIT, r);
-            ea = make_float2(0.5f * r[0], 0.5f * r[1]);
-            eb = make_float2(0.5f * r[2], 0.5f * r[3]);
-        }
-        const double2 g = gs[i];
-        state[idx] = make_float4((float)g.x + gp.init_a * ea.x, gp.init_b * eb.x,
-                                 (float)g.y + gp.init_a * ea.y, gp.init_b * eb.y);
-    }
+    return Cell{g.x + P.init_a * ea.x, P.init_b * eb.x, g.y + P.init_a * ea.y, P.init_b * eb.y};
+}
+__device__ __forceinline__ Cell initial_cell_philox(float2 g, const GroupParamsF &P, uint32_t traj, uint32_t cell)
+{
+    float r[4];
+    const uint64_t seed = ((uint64_t)P.seed_hi << 32) | P.seed_lo;
+    normals4<float>(seed, traj, 0u, cell, RNG_TAG_INIT, r);
+    return initial_cell(g, P, make_float2(0.5f * r[0], 0.5f * r[1]), make_float2(0.5f * r[2], 0.5f * r[3]));
 }
 
+// sources of the x-space cells of a preparation pass, by trajectory t of the launch and cell i
+// the state itself, (a.re, a.im, b.re, b.im) as float4 (an uploaded trajectory)
+struct FromState {
+    const float4 *x;
+    __device__ __forceinline__ Cell operator()(size_t at, int, int) const
+    {
+        const float4 v = x[at];
+        return Cell{v.x, v.z, v.y, v.w};
+    }
+};
+// one ensemble's ground state and its noise (injected, or Philox stream t)
+struct FromGroup {
+    GroupParamsF P;
+    const double2 *gs;
+    const float2 *noise;
+    int cells;
+    __device__ __forceinline__ Cell operator()(size_t, int t, int i) const
+    {
+        const float2 g = make_float2((float)gs[i].x, (float)gs[i].y);
+        if (noise) return initial_cell(g, P, noise[((size_t)t * 2 + 0) * cells + i], noise[((size_t)t * 2 + 1) * cells + i]);
+        return initial_cell_philox(g, P, (uint32_t)t, (uint32_t)i);
+    }
+};
 // ground-state value i of a complex128 (double2), complex64 (float2) or real FP32 (float) array, as float2
 __device__ __forceinline__ float2 gs_value(const double2 *p, int i) { return make_float2((float)p[i].x, (float)p[i].y); }
 __device__ __forceinline__ float2 gs_value(const float2 *p, int i) { return p[i]; }
 __device__ __forceinline__ float2 gs_value(const float *p, int i) { return make_float2(p[i], 0.f); }
-
-// The same initial state as k_init for a run of trajectories of one grid class that may belong to many
-// ensembles: trajectory t of the run takes its ensemble's parameters gp[tgroup[t]], its ground state
-// gs_ptrs[tgroup[t]] (complex128, complex64 or real FP32 values, by T), and its Philox stream tlocal[t].
+// the same initial states for a run of trajectories that may belong to many ensembles: trajectory t takes its ensemble's
+// parameters, its ground state gs_ptrs[tgroup[t]] and its Philox stream tlocal[t]
 template <typename T>
-__global__ void k_init_batched(float4 *state, int cells, int n_traj, const int *__restrict__ tgroup,
-                               const int *__restrict__ tlocal, const GroupParamsF *__restrict__ gp,
-                               const void *const *__restrict__ gs_ptrs)
-{
-    const size_t n = (size_t)cells * n_traj;
-    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
-        const int t = (int)(idx / cells);
-        const int i = (int)(idx - (size_t)t * cells);
+struct FromGroups {
+    const int *tgroup, *tlocal;
+    const GroupParamsF *gp;
+    const void *const *gs_ptrs;
+    __device__ __forceinline__ Cell operator()(size_t, int t, int i) const
+    {
         const int grp = tgroup[t];
-        const GroupParamsF &P = gp[grp];
-        float r[4];
-        const uint64_t seed = ((uint64_t)P.seed_hi << 32) | P.seed_lo;
-        normals4<float>(seed, (uint32_t)tlocal[t], 0u, (uint32_t)i, RNG_TAG_INIT, r);
-        const float2 ea = make_float2(0.5f * r[0], 0.5f * r[1]);
-        const float2 eb = make_float2(0.5f * r[2], 0.5f * r[3]);
-        const float2 g = gs_value(static_cast<const T *>(gs_ptrs[grp]), i);
-        state[idx] = make_float4(g.x + P.init_a * ea.x, P.init_b * eb.x, g.y + P.init_a * ea.y, P.init_b * eb.y);
+        return initial_cell_philox(gs_value(static_cast<const T *>(gs_ptrs[grp]), i), gp[grp], (uint32_t)tlocal[t], (uint32_t)i);
+    }
+};
+
+// ---------------------------------------------------------------- plane passes
+// A CTA holds 2^lppc planes, rows padded by one cell against bank conflicts.
+struct PlaneTile {
+    int lx, ly, lz, lppc;
+    const float2 *tx, *ty;      // W_nx^k, k < nx / 2, and W_ny^k (global; copied beside the tile)
+    __host__ __device__ __forceinline__ int ld() const { return (1 << lx) + 1; }
+    __device__ __forceinline__ int natural(int i) const { return (i >> lx) * ld() + (i & ((1 << lx) - 1)); }
+    __device__ __forceinline__ int reversed(int i) const
+    {
+        const int y = (i >> lx) & ((1 << ly) - 1);
+        return (((i >> (lx + ly)) << ly) + brev_bits(y, ly)) * ld() + brev_bits(i & ((1 << lx) - 1), lx);
+    }
+    __device__ __forceinline__ Lines rows() const { return Lines{lx, lppc + ly, 1, 30, ld(), 0}; }
+    __device__ __forceinline__ Lines cols() const { return Lines{ly, lppc + lx, ld(), lx, 1, ld() << ly}; }
+    __host__ __device__ __forceinline__ int cells() const { return ld() << (ly + lppc); }
+    __device__ __forceinline__ float2 *tw(Cell *sm) const { return reinterpret_cast<float2 *>(sm + cells()); }
+    // the twiddles beside the tile: read from L2 stage by stage they would add a trip to every barrier
+    __device__ __forceinline__ void fetch_twiddles(Cell *sm) const
+    {
+        const int hx = 1 << lx >> 1, hy = 1 << ly >> 1;
+        for (int i = threadIdx.x; i < hx + hy; i += blockDim.x) copy8(tw(sm) + i, i < hx ? tx + i : ty + i - hx);
+    }
+    __device__ __forceinline__ void forward(Cell *sm) const
+    {
+        fft_time<false>(sm, rows(), tw(sm));
+        if (ly > 0) fft_time<false>(sm, cols(), tw(sm) + (1 << lx >> 1));
+    }
+    __device__ __forceinline__ void inverse(Cell *sm) const
+    {
+        if (ly > 0) fft_freq<true>(sm, cols(), tw(sm) + (1 << lx >> 1));
+        fft_freq<true>(sm, rows(), tw(sm));
+    }
+};
+
+// x-space cells of src -> IFFT_xy -> stored representation
+template <typename Src>
+__global__ void __launch_bounds__(256) k_prep(Cell *__restrict__ state, PlaneTile T, Src src)
+{
+    extern __shared__ Cell smw[];
+    const int lchunk = T.lppc + T.lx + T.ly, lcells = T.lx + T.ly + T.lz;
+    const size_t first = (size_t)blockIdx.x << lchunk;
+    const int traj = (int)(first >> lcells), cell0 = (int)(first & ((1u << lcells) - 1));
+    T.fetch_twiddles(smw);
+    for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) smw[T.natural(i)] = src(first + i, traj, cell0 + i);
+    copy_wait();
+    __syncthreads();
+    T.inverse(smw);
+    for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) state[first + i] = smw[T.reversed(i)];
+}
+
+// stored representation -> FFT_xy -> x-space cells (a.re, a.im, b.re, b.im) to out
+__global__ void __launch_bounds__(256) k_unprep(const Cell *__restrict__ state, PlaneTile T, float4 *__restrict__ out)
+{
+    extern __shared__ Cell smw[];
+    const int lchunk = T.lppc + T.lx + T.ly;
+    const size_t first = (size_t)blockIdx.x << lchunk;
+    T.fetch_twiddles(smw);
+    for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) copy16(smw + T.reversed(i), state + first + i);
+    copy_wait();
+    __syncthreads();
+    T.forward(smw);
+    for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) {
+        const Cell v = smw[T.natural(i)];
+        out[first + i] = make_float4(v.ar, v.ai, v.br, v.bi);
     }
 }
 
-// ---------------------------------------------------------------- plane pass
-// mode 0: full step (load bit-reversed, FFT_xy, nonlinear, IFFT_xy, store bit-reversed)
-// mode 1: prep (x-space natural in -> IFFT_xy -> stored representation)
-// mode 2: unprep (stored representation -> FFT_xy -> x-space natural out)
-template <int MODE>
-__global__ void __launch_bounds__(kThreads) k_ppass(float4 *state, ClassGeom c, int ppc, const GroupParamsF *gp,
-                                                   const int *tgroup, const int *tlocal, const float2 *tw_x,
-                                                   const float2 *tw_y, const uint32_t *stepp)
+// the plane pass of a step; done != NULL: the last CTA advances the step index (fused_passes.cu)
+__global__ void __launch_bounds__(256) k_plane_any(Cell *__restrict__ state, PlaneTile T, const GroupParamsF *__restrict__ gp,
+                                                   const int *__restrict__ tgroup, const int *__restrict__ tlocal,
+                                                   uint32_t *stepp, int *done)
 {
-    extern __shared__ float4 sm4[];
-    const uint32_t step = stepp ? *stepp : 0u;   // Philox step index (device scalar, see fp32_put_step)
-    const int plane = c.nx * c.ny;
-    const int chunk = ppc * plane;
-    float4 *buf = sm4;
-    float2 *twx = reinterpret_cast<float2 *>(sm4 + chunk);
-    float2 *twy = twx + (c.nx / 2 > 0 ? c.nx / 2 : 1);
-    load_twiddles(twx, tw_x, c.nx / 2);
-    load_twiddles(twy, tw_y, c.ny / 2);
-
-    const int chunks_per_traj = c.nz / ppc;
-    const int traj = blockIdx.x / chunks_per_traj;
-    const int z0 = (blockIdx.x - traj * chunks_per_traj) * ppc;
-    float4 *g = state + (size_t)traj * c.cells + (size_t)z0 * plane;
-
-    const bool brev_in = (MODE == 0 || MODE == 2);
-    for (int idx = threadIdx.x; idx < chunk; idx += blockDim.x) {
-        const int x = idx & (c.nx - 1);
-        const int y = (idx >> c.lx) & (c.ny - 1);
-        const int p = idx >> (c.lx + c.ly);
-        const int dst = brev_in ? (p * plane + brev_bits(y, c.ly) * c.nx + brev_bits(x, c.lx)) : idx;
-        buf[dst] = cell_swap(g[idx]);
+    extern __shared__ Cell smw[];
+    const int lplane = T.lx + T.ly, lchunk = T.lppc + lplane, lcells = lplane + T.lz;
+    const size_t first = (size_t)blockIdx.x << lchunk;
+    const int traj = (int)(first >> lcells), cell0 = (int)(first & ((1u << lcells) - 1));
+    T.fetch_twiddles(smw);
+    const GroupParamsF P = gp[tgroup[traj]];
+    const uint32_t tl = (uint32_t)tlocal[traj];
+    wait_predecessor();
+    allow_successor();
+    for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) copy16(smw + T.reversed(i), state + first + i);
+    const uint32_t step = *stepp;                 // Philox step index (device scalar, see fp32_put_step)
+    const uint64_t seed = ((uint64_t)P.seed_hi << 32) | P.seed_lo;
+    const float hdt = P.dt * 0.5f;
+    copy_wait();
+    __syncthreads();
+    T.forward(smw);
+    for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) {
+        const int cell = cell0 + i;
+        const int x = cell & ((1 << T.lx) - 1), y = (cell >> T.lx) & ((1 << T.ly) - 1), z = cell >> lplane;
+        const float X = -P.xmax + P.dx * (float)x;
+        const float Y = (T.ly > 0) ? -P.ymax + P.dy * (float)y : 0.0f;
+        const float Z = -P.zmax + P.dz * (float)z;
+        const float V = (X * X + Y * Y + Z * Z * P.inv_lambda2) * 0.5f;
+        Cell *at = smw + T.natural(i);
+        float2 a0 = cell_a(*at), b0 = cell_b(*at);
+        float2 xa = a0, xb = b0, da = make_float2(0.f, 0.f), db = make_float2(0.f, 0.f);
+        for (int it = 0; it < P.itmax; ++it) {
+            const float na = xa.x * xa.x + xa.y * xa.y;
+            const float nb = xb.x * xb.x + xb.y * xb.y;
+            // propagateXSpaceTwoComponent (wigner_kernel.cu:203-223), reference sign
+            // (fused multiply-adds written out where the compiler's choice could change with the code around them)
+            const float pa_re = -fmaf(P.l111 * na, na, P.l12 * nb) * 0.5f;
+            const float pa_im = V + P.g11 * na + P.g12 * nb;
+            const float pb_re = -fmaf(P.l12, na, P.l22 * nb) * 0.5f;
+            const float pb_im = V + P.g22 * nb + P.g12 * na - P.detuning;
+            float sa, ca, sb, cb;
+            sincosf(pa_im * hdt, &sa, &ca);
+            sincosf(pb_im * hdt, &sb, &cb);
+            const float ma = expf(pa_re * hdt), mb = expf(pb_re * hdt);
+            da = make_float2(ma * ca, ma * sa);
+            db = make_float2(mb * cb, mb * sb);
+            xa = cmul(a0, da);
+            xb = cmul(b0, db);
+        }
+        float2 ao = cmul(xa, da), bo = cmul(xb, db);
+        if (P.noise) {
+            float r[6];
+            loss_normals6<float>(seed, tl, step, (uint32_t)cell, r);
+            const float s = P.noise_amp;
+            const float2 w1 = make_float2(s * r[0], s * r[1]);
+            const float2 w2 = make_float2(s * r[2], s * r[3]);
+            const float2 w3 = make_float2(s * r[4], s * r[5]);
+            const float2 ca2 = cconj(a0), cb2 = cconj(b0);
+            ao = cadd(ao, cadd(cmul(cscale(cmul(ca2, ca2), P.c1), w1), cmul(cscale(cb2, P.c2), w2)));
+            bo = cadd(bo, cadd(cmul(cscale(ca2, P.c2), w2), cmul(cscale(cb2, P.c3), w3)));
+        }
+        *at = make_cell(ao, bo);
     }
     __syncthreads();
-
-    const LineMap mx{c.lx, ppc * c.ny, 1, c.nx, ppc * c.ny, 0, 0};
-    const LineMap my{c.ly, ppc * c.nx, c.nx, 1, c.nx, plane, 1};
-
-    if (MODE == 0 || MODE == 2) {
-        fft_dit(buf, mx, twx, false);
-        fft_dit(buf, my, twy, false);
-    }
-    if (MODE == 0) {
-        const int gi = tgroup[traj];
-        const GroupParamsF P = gp[gi];
-        const uint32_t tl = (uint32_t)tlocal[traj];
-        const uint64_t seed = ((uint64_t)P.seed_hi << 32) | P.seed_lo;
-        const float hdt = P.dt * 0.5f;
-        for (int idx = threadIdx.x; idx < chunk; idx += blockDim.x) {
-            const int x = idx & (c.nx - 1);
-            const int y = (idx >> c.lx) & (c.ny - 1);
-            const int p = idx >> (c.lx + c.ly);
-            const float X = -P.xmax + P.dx * (float)x;
-            const float Y = (c.ny > 1) ? -P.ymax + P.dy * (float)y : 0.0f;
-            const float Z = -P.zmax + P.dz * (float)(z0 + p);
-            const float V = (X * X + Y * Y + Z * Z * P.inv_lambda2) * 0.5f;
-            const float4 v0 = buf[idx];
-            float2 a0 = make_float2(v0.x, v0.y), b0 = make_float2(v0.z, v0.w);
-            float2 xa = a0, xb = b0, da = make_float2(0.f, 0.f), db = make_float2(0.f, 0.f);
-            for (int it = 0; it < P.itmax; ++it) {
-                const float na = xa.x * xa.x + xa.y * xa.y;
-                const float nb = xb.x * xb.x + xb.y * xb.y;
-                // propagateXSpaceTwoComponent (wigner_kernel.cu:203-223), reference sign
-                const float pa_re = -(P.l111 * na * na + P.l12 * nb) * 0.5f;
-                const float pa_im = V + P.g11 * na + P.g12 * nb;
-                const float pb_re = -(P.l22 * nb + P.l12 * na) * 0.5f;
-                const float pb_im = V + P.g22 * nb + P.g12 * na - P.detuning;
-                float sa, ca, sb, cb;
-                sincosf(pa_im * hdt, &sa, &ca);
-                sincosf(pb_im * hdt, &sb, &cb);
-                const float ma = expf(pa_re * hdt), mb = expf(pb_re * hdt);
-                da = make_float2(ma * ca, ma * sa);
-                db = make_float2(mb * cb, mb * sb);
-                xa = cmul(a0, da);
-                xb = cmul(b0, db);
-            }
-            float2 ao = cmul(xa, da), bo = cmul(xb, db);
-            if (P.noise) {
-                const uint32_t cell = (uint32_t)((z0 + p) * plane + y * c.nx + x);
-                float r[6];
-                loss_normals6<float>(seed, tl, step, cell, r);
-                const float s = P.noise_amp;
-                const float2 w1 = make_float2(s * r[0], s * r[1]);
-                const float2 w2 = make_float2(s * r[2], s * r[3]);
-                const float2 w3 = make_float2(s * r[4], s * r[5]);
-                const float2 ca2 = cconj(a0), cb2 = cconj(b0);
-                ao = cadd(ao, cadd(cmul(cscale(cmul(ca2, ca2), P.c1), w1), cmul(cscale(cb2, P.c2), w2)));
-                bo = cadd(bo, cadd(cmul(cscale(ca2, P.c2), w2), cmul(cscale(cb2, P.c3), w3)));
-            }
-            buf[idx] = make_float4(ao.x, ao.y, bo.x, bo.y);
-        }
+    T.inverse(smw);
+    for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) state[first + i] = smw[T.reversed(i)];
+    if (done) {
         __syncthreads();
-    }
-    if (MODE == 0 || MODE == 1) {
-        fft_dif(buf, my, twy, true);
-        fft_dif(buf, mx, twx, true);
-    }
-
-    const bool brev_out = (MODE == 0 || MODE == 1);
-    for (int idx = threadIdx.x; idx < chunk; idx += blockDim.x) {
-        const int x = idx & (c.nx - 1);
-        const int y = (idx >> c.lx) & (c.ny - 1);
-        const int p = idx >> (c.lx + c.ly);
-        const int src = brev_out ? (p * plane + brev_bits(y, c.ly) * c.nx + brev_bits(x, c.lx)) : idx;
-        g[idx] = cell_swap(buf[src]);
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
+                *done = 0;
+                atomicAdd(stepp, 1u);
+            }
+        }
     }
 }
 
@@ -216,108 +364,107 @@ __global__ void __launch_bounds__(kThreads) k_ppass(float4 *state, ClassGeom c, 
 // (report.tex rotation matrix; applyHalfPiPulse / applyPiPulse,
 // wigner_kernel.cu:320-341). It acts identically on every cell, so it
 // commutes with the transforms and the kinetic phase.
-__device__ __forceinline__ float4 apply_m(const float2 *m, float4 v)
+__device__ __forceinline__ Cell apply_m(const float2 *m, Cell v)
 {
-    const float2 a = make_float2(v.x, v.y), b = make_float2(v.z, v.w);
-    const float2 an = cadd(cmul(m[0], a), cmul(m[1], b));
-    const float2 bn = cadd(cmul(m[2], a), cmul(m[3], b));
-    return make_float4(an.x, an.y, bn.x, bn.y);
+    const float2 a = cell_a(v), b = cell_b(v);
+    return make_cell(cadd(cmul(m[0], a), cmul(m[1], b)), cadd(cmul(m[2], a), cmul(m[3], b)));
 }
 
-__global__ void __launch_bounds__(kThreads) k_zpass(float4 *state, ClassGeom c, int tx, int ty,
-                                                   const GroupParamsF *gp, const int *tgroup,
-                                                   const float2 *tw_z, ZPassArgs za, double *obs_partial)
+// v times a kinetic phase, with the fused multiply-adds written out (as above)
+__device__ __forceinline__ float2 kick(float2 v, float2 w)
 {
-    extern __shared__ float4 sm4[];
-    const int npen = tx * ty;
-    const int n = c.nz;
-    float4 *buf = sm4;
-    float2 *twz = reinterpret_cast<float2 *>(sm4 + npen * n);
-    load_twiddles(twz, tw_z, n / 2);
+    return make_float2(fmaf(v.x, w.x, -(v.y * w.y)), fmaf(v.y, w.x, v.x * w.y));
+}
+__device__ __forceinline__ Cell kick_cell(Cell v, float2 w) { return make_cell(kick(cell_a(v), w), kick(cell_b(v), w)); }
 
-    const int tiles_x = c.nx / tx, tiles_y = c.ny / ty;
-    const int tiles = tiles_x * tiles_y;
-    const int traj = blockIdx.x / tiles;
-    const int tile = blockIdx.x - traj * tiles;
-    const int x0 = (tile % tiles_x) * tx, y0 = (tile / tiles_x) * ty;
-    const int plane = c.nx * c.ny;
-    float4 *g = state + (size_t)traj * c.cells;
+// e^{+i k^2/2 dt frac} of cell i of an ensemble (wigner_kernel.cu:143-144)
+__device__ __forceinline__ float2 kick_phase(const GroupParamsF &P, int x, int y, int z, int nx, int ny, int nz, float frac)
+{
+    const int ix = kidx(x, nx), iy = ny > 1 ? kidx(y, ny) : 0, iz = kidx(z, nz);
+    const double k2h = P.kin_x * (double)(ix * ix) + P.kin_y * (double)(iy * iy) + P.kin_z * (double)(iz * iz);
+    return kin_phase(k2h * (double)frac);
+}
 
-    for (int idx = threadIdx.x; idx < npen * n; idx += blockDim.x) {
-        const int xl = idx % tx;
-        const int r = idx / tx;
-        const int yl = r % ty;
-        const int z = r / ty;
-        buf[(yl * tx + xl) * n + brev_bits(z, c.lz)] =
-            cell_swap(g[(size_t)z * plane + (y0 + yl) * c.nx + x0 + xl]);
-    }
-    __syncthreads();
+// the phases of every cell of each of the class's ensembles (ensemble e: parameters gp[groups[e]])
+__global__ void k_kick_table(float2 *__restrict__ tab, const GroupParamsF *__restrict__ gp, const int *__restrict__ groups,
+                             int lx, int ly, int lz, float frac)
+{
+    const GroupParamsF &P = gp[groups[blockIdx.y]];
+    const int cells = 1 << (lx + ly + lz);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += gridDim.x * blockDim.x)
+        tab[(size_t)blockIdx.y * cells + i] = kick_phase(P, i & ((1 << lx) - 1), (i >> lx) & ((1 << ly) - 1), i >> (lx + ly),
+                                                         1 << lx, 1 << ly, 1 << lz, frac);
+}
 
-    const LineMap mz{c.lz, npen, 1, n, npen, 0, 0};
-    fft_dit(buf, mz, twz, true);     // IFFT_z: now full k-space (unnormalised)
+struct ZArgs {
+    int lx, ly, lz, lp;          // 2^lp pencils per CTA
+    const float2 *tz;            // W_nz^k, k < nz / 2
+    const float2 *kick;          // k_kick_table of the kick fraction, or NULL: evaluated here
+    const int *tindex;           // ensemble of the table per trajectory
+    float frac;                  // 0: no kick
+    float scale, out_scale;      // 1/cells; nx ny when the pass ends a step, else 1
+    int has_m;
+    float2 m[4];
+};
 
+// OBS: the pass ends a step and writes, per z, the FP64 sums of |a|^2, |b|^2 and conj(a) b over the tile's pencils
+template <bool OBS>
+__global__ void __launch_bounds__(256) k_z_any(Cell *__restrict__ state, ZArgs A, const GroupParamsF *__restrict__ gp,
+                                               const int *__restrict__ tgroup, double *__restrict__ obs)
+{
+    extern __shared__ Cell smw[];
+    const int lplane = A.lx + A.ly, P2 = 1 << A.lp, nz = 1 << A.lz, chunk = nz << A.lp;
+    float2 *tw = reinterpret_cast<float2 *>(smw + chunk);
+    const int tile = blockIdx.x & ((1 << (lplane - A.lp)) - 1), traj = blockIdx.x >> (lplane - A.lp);
+    const int pen0 = tile << A.lp;
+    Cell *__restrict__ g = state + ((size_t)traj << (lplane + A.lz)) + pen0;
+    for (int i = threadIdx.x; i < nz / 2; i += blockDim.x) copy8(tw + i, A.tz + i);
     const GroupParamsF P = gp[tgroup[traj]];
-    const float kick_first = za.observe ? za.pre : (za.pre + za.post);
-    for (int idx = threadIdx.x; idx < npen * n; idx += blockDim.x) {
-        const int pen = idx / n, z = idx - pen * n;
-        const int xl = pen % tx, yl = pen / tx;
-        const int ix = kidx(x0 + xl, c.nx), iy = c.ny > 1 ? kidx(y0 + yl, c.ny) : 0, iz = kidx(z, n);
-        const double k2h = P.kin_x * (double)(ix * ix) + P.kin_y * (double)(iy * iy) + P.kin_z * (double)(iz * iz);
-        float4 v = pscale(buf[idx], za.observe ? za.scale : za.scale * za.out_scale);
-        if (kick_first != 0.0f)
-            v = pmul(v, kin_phase(k2h * (double)kick_first));   // e^{+i k^2/2 dt}, wigner_kernel.cu:143-144
-        if (za.has_m1) v = apply_m(za.m1, v);
-        if (!za.observe && za.has_m2) v = apply_m(za.m2, v);
-        buf[idx] = v;
+    const float2 *table = A.kick ? A.kick + ((size_t)A.tindex[traj] << (lplane + A.lz)) + pen0 : nullptr;
+    wait_predecessor();
+    allow_successor();
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x)
+        copy16(smw + (brev_bits(i >> A.lp, A.lz) << A.lp) + (i & (P2 - 1)), g + ((size_t)(i >> A.lp) << lplane) + (i & (P2 - 1)));
+    copy_wait();
+    __syncthreads();
+    const Lines L{A.lz, A.lp, P2, 30, 1, 0};
+    fft_time<true>(smw, L, tw);       // IFFT_z: now full k-space (unnormalised)
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x) {
+        const int z = i >> A.lp, p = i & (P2 - 1);
+        Cell v = cell_scale(smw[i], OBS ? A.scale : A.scale * A.out_scale);
+        if (A.frac != 0.0f)
+            v = kick_cell(v, table ? table[((size_t)z << lplane) + p]
+                                 : kick_phase(P, (pen0 + p) & ((1 << A.lx) - 1), (pen0 + p) >> A.lx, z, 1 << A.lx, 1 << A.ly, nz,
+                                              A.frac));
+        if (A.has_m) v = apply_m(A.m, v);
+        smw[i] = v;
     }
     __syncthreads();
-
-    if (za.observe) {
+    if (OBS) {
         // per-z moments: transform the boundary state along z, sum over the tile's pencils
-        fft_dif(buf, mz, twz, false);
-        const int tiles_total = tiles;
-        for (int z = threadIdx.x; z < n; z += blockDim.x) {
-            const int pos = brev_bits(z, c.lz);
+        fft_freq<false>(smw, L, tw);
+        for (int z = threadIdx.x; z < nz; z += blockDim.x) {
+            const Cell *row = smw + (brev_bits(z, A.lz) << A.lp);
             KSum s0, s1, s2, s3;
-            for (int pen = 0; pen < npen; ++pen) {
-                const float4 v = buf[pen * n + pos];
-                s0.add((double)v.x * v.x + (double)v.y * v.y);
-                s1.add((double)v.z * v.z + (double)v.w * v.w);
-                s2.add((double)v.x * v.z + (double)v.y * v.w);
-                s3.add((double)v.x * v.w - (double)v.y * v.z);
+            for (int p = 0; p < P2; ++p) {
+                const Cell v = row[p];
+                s0.add((double)v.ar * v.ar + (double)v.ai * v.ai);
+                s1.add((double)v.br * v.br + (double)v.bi * v.bi);
+                s2.add((double)v.ar * v.br + (double)v.ai * v.bi);
+                s3.add((double)v.ar * v.bi - (double)v.ai * v.br);
             }
-            double *o = obs_partial + (((size_t)traj * tiles_total + tile) * n + z) * 4;
+            double *o = obs + ((size_t)blockIdx.x * nz + z) * 4;
             o[0] = s0.value(); o[1] = s1.value(); o[2] = s2.value(); o[3] = s3.value();
         }
         __syncthreads();
-        fft_dit(buf, mz, twz, true);   // back to k-space (times nz)
-        const float inv_n = za.out_scale / (float)n;
-        for (int idx = threadIdx.x; idx < npen * n; idx += blockDim.x) {
-            const int pen = idx / n, z = idx - pen * n;
-            const int xl = pen % tx, yl = pen / tx;
-            float4 v = pscale(buf[idx], inv_n);
-            if (za.has_m2) v = apply_m(za.m2, v);
-            if (za.post != 0.0f) {
-                const int ix = kidx(x0 + xl, c.nx), iy = c.ny > 1 ? kidx(y0 + yl, c.ny) : 0, iz = kidx(z, n);
-                const double k2h =
-                    P.kin_x * (double)(ix * ix) + P.kin_y * (double)(iy * iy) + P.kin_z * (double)(iz * iz);
-                v = pmul(v, kin_phase(k2h * (double)za.post));
-            }
-            buf[idx] = v;
-        }
+        fft_time<true>(smw, L, tw);   // back to k-space (times nz)
+        const float inv_n = A.out_scale / (float)nz;
+        for (int i = threadIdx.x; i < chunk; i += blockDim.x) smw[i] = cell_scale(smw[i], inv_n);
         __syncthreads();
     }
-
-    fft_dif(buf, mz, twz, false);    // FFT_z back to the stored representation (bit-reversed slots)
-
-    for (int idx = threadIdx.x; idx < npen * n; idx += blockDim.x) {
-        const int xl = idx % tx;
-        const int r = idx / tx;
-        const int yl = r % ty;
-        const int z = r / ty;
-        g[(size_t)z * plane + (y0 + yl) * c.nx + x0 + xl] =
-            cell_swap(buf[(yl * tx + xl) * n + brev_bits(z, c.lz)]);
-    }
+    fft_freq<false>(smw, L, tw);      // FFT_z back to the stored representation (bit-reversed slots)
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x)
+        g[((size_t)(i >> A.lp) << lplane) + (i & (P2 - 1))] = smw[(brev_bits(i >> A.lp, A.lz) << A.lp) + (i & (P2 - 1))];
 }
 
 // obs_partial[traj][tile][z][4] -> traj_axial[traj][z][4] (scaled), traj_tot[traj][4]
@@ -357,8 +504,8 @@ __global__ void k_state_sums(const float4 *__restrict__ state, int cells, int bl
     // plain FP64 sums over a thread's few dozen cells (rounding ~1e-15 relative), compensated across threads
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
     for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        const float4 u = cell_swap(p[i]);
-        const double ax = u.x, ay = u.y, bx = u.z, by = u.w;
+        const float4 v = p[i];
+        const double ax = v.x, bx = v.y, ay = v.z, by = v.w;
         s0 = fma(ax, ax, fma(ay, ay, s0));
         s1 = fma(bx, bx, fma(by, by, s1));
         s2 = fma(ax, bx, fma(ay, by, s2));
@@ -374,10 +521,11 @@ __global__ void k_state_sums(const float4 *__restrict__ state, int cells, int bl
         for (int k = 0; k < 4; ++k) part[(size_t)blockIdx.x * 4 + k] = r.v[k].value() * scale;
 }
 
+// (a.re, b.re, a.im, b.im) <-> (a.re, a.im, b.re, b.im)
 __global__ void k_swap_cells(float4 *state, size_t n)
 {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        state[i] = cell_swap(state[i]);
+        state[i] = make_float4(state[i].x, state[i].z, state[i].y, state[i].w);
 }
 
 __global__ void k_group_reduce(const double *traj_tot, const int *first, const int *count, double *out)
@@ -391,66 +539,86 @@ __global__ void k_group_reduce(const double *traj_tot, const int *first, const i
         for (int k = 0; k < 4; ++k) out[(size_t)gidx * 4 + k] = r.v[k].value();
 }
 
-size_t ppass_smem(const ClassGeom &c, int ppc)
+
+// ---------------------------------------------------------------- tiles
+constexpr size_t kMaxTile = 64 * 1024;      // shared memory of a z tile
+constexpr int kEnoughCtas = 2 * 148;
+
+// Planes per CTA: as many as 1024 cells hold while the launch keeps two CTAs per SM, at least one, at least 128 cells (a
+// cell per thread).
+PlaneTile plane_tile(const ClassGeom &c, const float2 *tx, const float2 *ty)
 {
-    return sizeof(float4) * (size_t)ppc * c.nx * c.ny + sizeof(float2) * (size_t)((c.nx / 2 > 0 ? c.nx / 2 : 1) + (c.ny / 2 > 0 ? c.ny / 2 : 1));
+    PlaneTile T{c.lx, c.ly, c.lz, 0, tx, ty};
+    const int lplane = c.lx + c.ly;
+    T.lppc = std::max(0, std::min(10 - lplane, c.lz));
+    while (T.lppc > 0 && T.lppc + lplane > 7 && ((long long)c.n_traj << (c.lz - T.lppc)) < kEnoughCtas) --T.lppc;
+    return T;
+}
+int plane_ctas(const ClassGeom &c, const PlaneTile &T) { return c.n_traj << (c.lz - T.lppc); }
+int tile_threads(int log_cells) { return log_cells >= 10 ? 256 : 128; }
+size_t plane_bytes(const PlaneTile &T) { return sizeof(Cell) * (size_t)T.cells() + sizeof(float2) * ((1 << T.lx >> 1) + (1 << T.ly >> 1)); }
+constexpr int kMaxPlaneBytes = 16 * 3 * 1024 + 8 * 1024;    // planes of up to 2048 cells, rows of two padded to three
+
+// Pencils per CTA: 16 (256-byte rows) for observing passes, whose sums take memory per tile; else 8 (128 bytes), fewer, down
+// to two 32-byte sectors' worth, while the launch has fewer than two CTAs per SM; never more than fit.
+int z_log_pencils(const ClassGeom &c, bool observe)
+{
+    int lp = std::min(observe ? 4 : 3, c.lx + c.ly);
+    while (lp > 0 && (sizeof(Cell) << (lp + c.lz)) > kMaxTile) --lp;
+    while (!observe && lp > 1 && ((long long)c.n_traj << (c.lx + c.ly - lp)) < kEnoughCtas) --lp;
+    return lp;
 }
 
-template <int MODE>
-void launch_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                  const float2 *tw_x, const float2 *tw_y, const uint32_t *step, cudaStream_t s)
+template <typename Src>
+void launch_prep(float4 *state, const ClassGeom &c, const float2 *tx, const float2 *ty, const Src &src, cudaStream_t s)
 {
     if (c.n_traj <= 0) return;
-    const int ppc = planes_per_cta(c);
-    const int blocks = c.n_traj * (c.nz / ppc);
-    const size_t smem = ppass_smem(c, ppc);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_ppass<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_ppass<MODE><<<blocks, kThreads, smem, s>>>(state, c, ppc, gp, tgroup, tlocal, tw_x, tw_y, step);
+    const PlaneTile T = plane_tile(c, tx, ty);
+    ensure_smem_limit((const void *)k_prep<Src>, kMaxPlaneBytes);
+    k_prep<Src><<<plane_ctas(c, T), tile_threads(T.lppc + c.lx + c.ly), plane_bytes(T), s>>>(reinterpret_cast<Cell *>(state), T, src);
     g_launches++;
 }
 
 } // namespace
 
-void fp32_init_group(float4 *state, int cells, int ne, const GroupParamsF &gp, const double2 *gs,
-                     const float2 *noise, cudaStream_t s)
+void fp32_init_group(float4 *state, const ClassGeom &c, const GroupParamsF &gp, const double2 *gs, const float2 *noise,
+                     const float2 *tx, const float2 *ty, cudaStream_t s)
 {
-    size_t n = (size_t)cells * ne;
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 148 * 32) blocks = 148 * 32;
-    k_init<<<blocks, 256, 0, s>>>(state, cells, ne, gp, gs, noise);
+    launch_prep(state, c, tx, ty, FromGroup{gp, gs, noise, c.cells}, s);
+}
+
+void fp32_init_batched(float4 *state, const ClassGeom &c, const int *tgroup, const int *tlocal, const GroupParamsF *gp,
+                       const void *const *gs_ptrs, int host_type, const float2 *tx, const float2 *ty, cudaStream_t s)
+{
+    if (host_type == BEC_HOST_R32) launch_prep(state, c, tx, ty, FromGroups<float>{tgroup, tlocal, gp, gs_ptrs}, s);
+    else if (host_type == BEC_HOST_C64) launch_prep(state, c, tx, ty, FromGroups<float2>{tgroup, tlocal, gp, gs_ptrs}, s);
+    else launch_prep(state, c, tx, ty, FromGroups<double2>{tgroup, tlocal, gp, gs_ptrs}, s);
+}
+
+void fp32_prep(float4 *state, const ClassGeom &c, const float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s)
+{
+    launch_prep(state, c, tx, ty, FromState{x}, s);
+}
+
+void fp32_unprep(const float4 *state, const ClassGeom &c, float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s)
+{
+    if (c.n_traj <= 0) return;
+    const PlaneTile T = plane_tile(c, tx, ty);
+    ensure_smem_limit((const void *)k_unprep, kMaxPlaneBytes);
+    k_unprep<<<plane_ctas(c, T), tile_threads(T.lppc + c.lx + c.ly), plane_bytes(T), s>>>(reinterpret_cast<const Cell *>(state), T, x);
     g_launches++;
 }
 
-void fp32_init_batched(float4 *state, int cells, int n_traj, const int *tgroup, const int *tlocal,
-                       const GroupParamsF *gp, const void *const *gs_ptrs, int host_type, cudaStream_t s)
-{
-    size_t n = (size_t)cells * n_traj;
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 148 * 32) blocks = 148 * 32;
-    if (host_type == BEC_HOST_R32)
-        k_init_batched<float><<<blocks, 256, 0, s>>>(state, cells, n_traj, tgroup, tlocal, gp, gs_ptrs);
-    else if (host_type == BEC_HOST_C64)
-        k_init_batched<float2><<<blocks, 256, 0, s>>>(state, cells, n_traj, tgroup, tlocal, gp, gs_ptrs);
-    else
-        k_init_batched<double2><<<blocks, 256, 0, s>>>(state, cells, n_traj, tgroup, tlocal, gp, gs_ptrs);
-    g_launches++;
-}
-
-void fp32_prep(float4 *state, const ClassGeom &c, const float2 *tw_x, const float2 *tw_y, cudaStream_t s)
-{
-    launch_ppass<1>(state, c, nullptr, nullptr, nullptr, tw_x, tw_y, nullptr, s);
-}
-
-void fp32_unprep(float4 *state, const ClassGeom &c, const float2 *tw_x, const float2 *tw_y, cudaStream_t s)
-{
-    launch_ppass<2>(state, c, nullptr, nullptr, nullptr, tw_x, tw_y, nullptr, s);
-}
+int fp32_ppass_ctas(const ClassGeom &c) { return plane_ctas(c, plane_tile(c, nullptr, nullptr)); }
 
 void fp32_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                const float2 *tw_x, const float2 *tw_y, const uint32_t *d_step, cudaStream_t s)
+                const float2 *tx, const float2 *ty, uint32_t *d_step, int *inc_done, cudaStream_t s)
 {
-    launch_ppass<0>(state, c, gp, tgroup, tlocal, tw_x, tw_y, d_step, s);
+    if (c.n_traj <= 0) return;
+    const PlaneTile T = plane_tile(c, tx, ty);
+    ensure_smem_limit((const void *)k_plane_any, kMaxPlaneBytes);
+    launch_after(k_plane_any, plane_ctas(c, T), tile_threads(T.lppc + c.lx + c.ly), plane_bytes(T), s,
+                 reinterpret_cast<Cell *>(state), T, gp, tgroup, tlocal, d_step, inc_done);
 }
 
 namespace {
@@ -470,26 +638,44 @@ void fp32_inc_step(uint32_t *d_step, cudaStream_t s)
     g_launches++;
 }
 
-int fp32_zpass_tiles(const ClassGeom &c)
+int fp32_zpass_tiles(const ClassGeom &c) { return (c.nx * c.ny) >> z_log_pencils(c, true); }
+
+void fp32_kick_table(float2 *tab, const ClassGeom &c, const GroupParamsF *gp, const int *groups, int n_groups, float frac,
+                     cudaStream_t s)
 {
-    int tx, ty;
-    ztile(c, tx, ty);
-    return (c.nx / tx) * (c.ny / ty);
+    if (n_groups <= 0) return;
+    k_kick_table<<<dim3((unsigned)std::min((c.cells + 127) / 128, 1024), (unsigned)n_groups), 128, 0, s>>>(tab, gp, groups, c.lx,
+                                                                                                          c.ly, c.lz, frac);
+    g_launches++;
 }
 
-void fp32_zpass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const float2 *tw_z,
-                const ZPassArgs &z, double *obs_partial, cudaStream_t s)
+void fp32_zpass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const float2 *tz,
+                const float2 *kick, const int *tindex, float frac, float scale, float out_scale, const float2 *m, double *obs,
+                cudaStream_t s)
 {
     if (c.n_traj <= 0) return;
-    int tx, ty;
-    ztile(c, tx, ty);
-    const int tiles = (c.nx / tx) * (c.ny / ty);
-    const int blocks = c.n_traj * tiles;
-    const size_t smem = sizeof(float4) * (size_t)tx * ty * c.nz + sizeof(float2) * (size_t)(c.nz / 2);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_zpass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_zpass<<<blocks, kThreads, smem, s>>>(state, c, tx, ty, gp, tgroup, tw_z, z, obs_partial);
-    g_launches++;
+    ZArgs A{};
+    A.lx = c.lx; A.ly = c.ly; A.lz = c.lz;
+    A.lp = z_log_pencils(c, obs != nullptr);
+    A.tz = tz;
+    A.kick = kick;
+    A.tindex = tindex;
+    A.frac = frac;
+    A.scale = scale;
+    A.out_scale = out_scale;
+    A.has_m = m ? 1 : 0;
+    for (int i = 0; m && i < 4; ++i) A.m[i] = m[i];
+    const int ctas = c.n_traj << (c.lx + c.ly - A.lp), threads = tile_threads(c.lz + A.lp);
+    const size_t bytes = (sizeof(Cell) << (c.lz + A.lp)) + sizeof(float2) * ((size_t)c.nz / 2);
+    const int most = (int)(kMaxTile + sizeof(float2) * 256);
+    Cell *st = reinterpret_cast<Cell *>(state);
+    if (obs) {
+        ensure_smem_limit((const void *)k_z_any<true>, most);
+        launch_after(k_z_any<true>, ctas, threads, bytes, s, st, A, gp, tgroup, obs);
+    } else {
+        ensure_smem_limit((const void *)k_z_any<false>, most);
+        launch_after(k_z_any<false>, ctas, threads, bytes, s, st, A, gp, tgroup, obs);
+    }
 }
 
 void obs_reduce(const double *obs_partial, int n_traj, int tiles, int nz, const double *traj_scale,

@@ -67,6 +67,8 @@ struct ClassRec {
     int traj_offset = 0;      // global index of the class's first trajectory
     std::vector<int> groups;  // group indices in this class
     float2 *kin_tab[2] = {nullptr, nullptr};   // kinetic phase tables for kick fractions 0.5 and 1 (register pencils)
+    float2 *kick_tab[2] = {nullptr, nullptr};  // the general z pass: phases of every cell per ensemble (fractions 0.5, 1)
+    int *d_tindex = nullptr;  // ... the trajectory's ensemble in them
     int pencil_kind = 0;      // the tuned per-pass schedules' pencil kernel for this class (kPencilRegister ...)
     double pencil_ms[2] = {-1.0, -1.0};        // autotuner: ms per launch of each pencil kernel
     bool onchip = false;      // the tuned schedules run this class's steady steps as one on-chip launch
@@ -83,7 +85,6 @@ struct bec_ctx {
     std::vector<GroupRec> groups;
     std::vector<ClassRec> classes;
     std::map<int, double2 *> tw64, tw64_full;
-    std::map<int, float2 *> tw32;
     std::map<int, float2 *> tw32_full;
     std::map<int, float2 *> tw32_nearest;
     bool use_fast = true;                // register-resident passes where the shape allows
@@ -310,20 +311,6 @@ float2 tw32_unit(int k, int n)
     return make_float2(t.a, t.b);
 }
 
-bec_status get_tw32(bec_ctx *ctx, int n, float2 **out)
-{
-    auto it = ctx->tw32.find(n);
-    if (it != ctx->tw32.end()) { *out = it->second; return BEC_OK; }
-    std::vector<float2> f(n / 2 > 0 ? n / 2 : 1, make_float2(1.f, 0.f));
-    for (int k = 0; k < n / 2; ++k) f[k] = tw32_unit(k, n);
-    float2 *d = nullptr;
-    CKC(dalloc(ctx, &d, f.size()));
-    CKC(cudaMemcpyAsync(d, f.data(), f.size() * sizeof(float2), cudaMemcpyHostToDevice, ctx->stream));
-    ctx->tw32[n] = d;
-    *out = d;
-    return BEC_OK;
-}
-
 // all n twiddles W_n^e, e < n (the pencil pass indexes products j * k1 < n)
 bec_status get_tw32_full(bec_ctx *ctx, int n, float2 **out)
 {
@@ -386,9 +373,6 @@ bec_status plain_step(bec_ctx *ctx, GroupRec &gr, int t)
 }
 
 // ---------------------------------------------------------------- batched z pass
-// ends_step: no plane pass follows, so the pass leaves the state in the form a z pass reads
-// ev (optional): per class (start, stop) events recorded around that class's launch
-// skip_fused: leave out the classes of the fused step plan (their pencil pass runs inside it)
 // a class whose steady step runs as one on-chip launch in the step being launched
 bool onchip_now(const bec_ctx *ctx, const ClassRec &c)
 {
@@ -400,69 +384,46 @@ bool split_plane_now(const bec_ctx *ctx, const ClassRec &c)
     return ctx->use_fast && ctx->pencil_tuned && c.split_plane && fp32_plane_split_supported(c.geom);
 }
 
-bec_status batched_zpass_all(bec_ctx *ctx, float pre, float post, bool observe, const double2 *m2,
-                             bool ends_step = false, std::pair<cudaEvent_t, cudaEvent_t> *ev = nullptr,
-                             bool skip_fused = false)
+// frac: the kick in units of dt (0, 0.5 or 1)
+// ends_step: no plane pass follows, so the pass leaves the state in the form a z pass reads; observing passes end a step
+// ev (optional): per class (start, stop) events recorded around that class's launch
+// skip_fused: leave out the classes of the fused step plan (their pencil pass runs inside it)
+bec_status batched_zpass_all(bec_ctx *ctx, float frac, bool observe, bool ends_step = false,
+                             std::pair<cudaEvent_t, cudaEvent_t> *ev = nullptr, bool skip_fused = false)
 {
-    ZPassArgs z{};
-    z.pre = pre;
-    z.post = post;
-    z.observe = observe ? 1 : 0;
-    if (ctx->has_pulse) {
-        z.has_m1 = 1;
-        for (int i = 0; i < 4; ++i) z.m1[i] = make_float2((float)ctx->pulse[i].x, (float)ctx->pulse[i].y);
-    }
-    if (m2) {
-        z.has_m2 = 1;
-        for (int i = 0; i < 4; ++i) z.m2[i] = make_float2((float)m2[i].x, (float)m2[i].y);
-    }
-    // without an observation the two pulse matrices collapse into one
-    float2 mfused[4];
+    float2 m[4];
     const float2 *mf = nullptr;
-    if ((!observe && (z.has_m1 || z.has_m2)) || (observe && z.has_m1 && !z.has_m2)) {
-        double2 a[4], b[4], r[4];
-        for (int i = 0; i < 4; ++i) {
-            a[i] = z.has_m2 ? m2[i] : cd(i == 0 || i == 3 ? 1.0 : 0.0, 0.0);
-            b[i] = z.has_m1 ? ctx->pulse[i] : cd(i == 0 || i == 3 ? 1.0 : 0.0, 0.0);
-        }
-        matmul2(a, b, r);
-        for (int i = 0; i < 4; ++i) mfused[i] = make_float2((float)r[i].x, (float)r[i].y);
-        mf = mfused;
+    if (ctx->has_pulse) {
+        for (int i = 0; i < 4; ++i) m[i] = make_float2((float)ctx->pulse[i].x, (float)ctx->pulse[i].y);
+        mf = m;
     }
+    const int half = frac == 1.0f ? 1 : 0;              // the tables' index of this kick fraction
     for (auto &c : ctx->classes) {
         if (c.geom.n_traj == 0) continue;
         if (skip_fused && ctx->fused[&c - &ctx->classes[0]]) continue;
         if (onchip_now(ctx, c)) continue;           // its plane-pass slot runs the whole step
         bec_status st;
-        z.scale = (float)(1.0 / (double)c.geom.cells);
-        z.out_scale = ends_step ? (float)(c.geom.nx * c.geom.ny) : 1.0f;
+        const float scale = (float)(1.0 / (double)c.geom.cells), out_scale = ends_step ? (float)(c.geom.nx * c.geom.ny) : 1.0f;
         const size_t ci = &c - &ctx->classes[0];
+        double *obs = observe ? c.obs_partial : nullptr;
+        float2 *tw;
+        if ((st = get_tw32_full(ctx, c.geom.nz, &tw))) return st;
         if (ev) CKC(cudaEventRecord(ev[ci].first, ctx->stream));
-        // the register pencil pass observes only when it also ends the step (post = 0), and kicks by the
-        // fractions its kinetic tables hold (0.5, 1) or not at all
-        const float kf = pre + post;
-        const bool fast = ctx->use_fast && fp32_fast_pencil_supported(c.geom) &&
-                          (kf == 0.0f || kf == 0.5f || kf == 1.0f) &&
-                          (!observe || (post == 0.0f && ends_step && !z.has_m2));
-        if (fast) {
-            float2 *twf;
-            if ((st = get_tw32_full(ctx, c.geom.nz, &twf))) return st;
-            const float frac = kf;
-            const float2 *kin = frac == 1.0f ? c.kin_tab[1] : frac == 0.5f ? c.kin_tab[0] : nullptr;
+        if (ctx->use_fast && fp32_fast_pencil_supported(c.geom)) {
+            const float2 *kin = frac == 0.0f ? nullptr : c.kin_tab[half];
             const int kind = !observe && ctx->pencil_tuned ? c.pencil_kind : kPencilRegister;
             if (!observe && ctx->pencil_tuned && c.split_pencil)
-                fp32_pencil_split(c.state, c.geom, twf, z.scale * z.out_scale, mf, kin, ctx->stream);
+                fp32_pencil_split(c.state, c.geom, tw, scale * out_scale, mf, kin, ctx->stream);
             else if (kind == kPencilTma && fp32_pencil_tma_supported(c.geom))
-                CKC(fp32_pencil_tma(c.state, c.geom, twf, frac, z.scale * z.out_scale, mf, kin, ctx->d_pflags,
-                                    ctx->d_pflags + 1, ctx->stream));
+                CKC(fp32_pencil_tma(c.state, c.geom, tw, frac, scale * out_scale, mf, kin, ctx->d_pflags, ctx->d_pflags + 1,
+                                    ctx->stream));
             else
-                fp32_pencil_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, twf, frac, z.scale * z.out_scale,
-                                 mf, observe ? c.obs_partial : nullptr, z.out_scale, kin, ctx->stream);
+                fp32_pencil_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, tw, frac, scale * out_scale, mf, obs, out_scale,
+                                 kin, ctx->stream);
             if (observe) c.obs_tiles = fp32_fast_pencil_tiles(c.geom);
         } else {
-            float2 *tz;
-            if ((st = get_tw32(ctx, c.geom.nz, &tz))) return st;
-            fp32_zpass(c.state, c.geom, ctx->d_gparams, c.d_tgroup, tz, z, c.obs_partial, ctx->stream);
+            fp32_zpass(c.state, c.geom, ctx->d_gparams, c.d_tgroup, tw, c.kick_tab[half], c.d_tindex, frac, scale, out_scale,
+                       mf, obs, ctx->stream);
             if (observe) c.obs_tiles = c.tiles;
         }
         if (ev) CKC(cudaEventRecord(ev[ci].second, ctx->stream));
@@ -474,10 +435,11 @@ bec_status batched_zpass_all(bec_ctx *ctx, float pre, float post, bool observe, 
 
 // put_step: write ctx->step into the device step scalar first (eager launches; a captured step graph
 // leaves it to the step before); skip_fused: leave out the classes of the fused step plan. advanced != NULL:
-// the step index is advanced in the same pass where a class can carry it -- the register-path plane launch
+// the step index is advanced in the same pass where a class can carry it -- the plane launch
 // with the fewest CTAs (at most kMaxCarrierCtas, one atomic each) runs last and its last CTA increments the
 // index -- and *advanced tells the caller whether that happened.
 constexpr int kMaxCarrierCtas = 16384;
+constexpr size_t kKickTableBytes = (size_t)256 << 20;   // phase tables of a class of the general z pass, at most
 
 bec_status batched_ppass_all(bec_ctx *ctx, std::pair<cudaEvent_t, cudaEvent_t> *ev = nullptr, bool put_step = true,
                              bool skip_fused = false, bool *advanced = nullptr)
@@ -496,12 +458,12 @@ bec_status batched_ppass_all(bec_ctx *ctx, std::pair<cudaEvent_t, cudaEvent_t> *
     auto split = [&](int ci) { return split_plane_now(ctx, ctx->classes[ci]); };
     auto ctas = [&](int ci) {
         const ClassGeom &g = ctx->classes[ci].geom;
-        return onchip(ci) ? g.n_traj : split(ci) ? fp32_plane_split_ctas(g) : fp32_plane_fast_ctas(g);
+        return onchip(ci) ? g.n_traj : split(ci) ? fp32_plane_split_ctas(g) : fast(ci) ? fp32_plane_fast_ctas(g) : fp32_ppass_ctas(g);
     };
     int carrier = -1;
     if (advanced) {
         for (int ci = 0; ci < nc; ++ci)
-            if (launched(ci) && fast(ci) && ctas(ci) <= kMaxCarrierCtas && (carrier < 0 || ctas(ci) < ctas(carrier)))
+            if (launched(ci) && ctas(ci) <= kMaxCarrierCtas && (carrier < 0 || ctas(ci) < ctas(carrier)))
                 carrier = ci;
         *advanced = carrier >= 0;
     }
@@ -526,9 +488,10 @@ bec_status batched_ppass_all(bec_ctx *ctx, std::pair<cudaEvent_t, cudaEvent_t> *
         } else {
             float2 *tx, *ty;
             bec_status st;
-            if ((st = get_tw32(ctx, c.geom.nx, &tx))) return st;
-            if ((st = get_tw32(ctx, c.geom.ny, &ty))) return st;
-            fp32_ppass(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, tx, ty, ctx->d_step, ctx->stream);
+            if ((st = get_tw32_full(ctx, c.geom.nx, &tx))) return st;
+            if ((st = get_tw32_full(ctx, c.geom.ny, &ty))) return st;
+            fp32_ppass(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, tx, ty, ctx->d_step,
+                       ci == carrier ? ctx->d_pflags + 2 : nullptr, ctx->stream);
         }
         if (ev) CKC(cudaEventRecord(ev[ci].second, ctx->stream));
         CKL();
@@ -557,7 +520,7 @@ bec_status batched_step(bec_ctx *ctx, float pre, bool put_step)
     // a steady step (the previous step's second half kick pending, no pulse): the on-chip classes take one launch
     ctx->step_onchip = !fused && pre == 0.5f && !has_m;
     struct Clear { bool &f; ~Clear() { f = false; } } clear{ctx->step_onchip};
-    if ((st = batched_zpass_all(ctx, pre, 0.5f, false, nullptr, false, nullptr, fused))) return st;
+    if ((st = batched_zpass_all(ctx, pre + 0.5f, false, false, nullptr, fused))) return st;
     bool advanced = false;
     if ((st = batched_ppass_all(ctx, nullptr, false, fused, fused ? nullptr : &advanced))) return st;
     if (fused) step_launch(ctx->plan, ctx->d_gparams, ctx->d_step, pre + 0.5f, has_m ? mf : nullptr, ctx->stream);
@@ -951,7 +914,7 @@ bec_status batched_moments_stored(bec_ctx *ctx)
 bec_status batched_resolve(bec_ctx *ctx, bool observe)
 {
     if (!ctx->pending && !ctx->has_pulse && !observe) return BEC_OK;
-    bec_status st = batched_zpass_all(ctx, ctx->pending ? 0.5f : 0.0f, 0.0f, observe, nullptr, true);
+    bec_status st = batched_zpass_all(ctx, ctx->pending ? 0.5f : 0.0f, observe, true);
     if (st) return st;
     ctx->pending = false;
     return BEC_OK;
@@ -1379,7 +1342,28 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
             CKA(cudaMemcpyAsync(c.d_tgroup, tg.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream));
             CKA(cudaMemcpyAsync(c.d_tlocal, tl.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream));
             CKA(cudaMemcpyAsync(c.d_traj_scale, ts.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, ctx->stream));
-            if (fp32_fast_pencil_supported(c.geom)) {
+            if (!fp32_fast_pencil_supported(c.geom)) {
+                // the general z pass evaluates its phases in FP64: a table per ensemble where it stays small
+                const size_t n = c.groups.size();
+                if (2 * sizeof(float2) * n * c.geom.cells <= kKickTableBytes) {
+                    std::vector<int> ti(nt);
+                    for (size_t e = 0; e < n; ++e)
+                        for (int t = 0; t < ctx->groups[c.groups[e]].p.ne; ++t) ti[ctx->groups[c.groups[e]].local_first + t] = (int)e;
+                    int *d_groups = nullptr;
+                    float2 *tab[2] = {nullptr, nullptr};
+                    // (without them, for want of memory or under a byte limit, the pass evaluates the phases itself)
+                    if (dalloc(ctx, &tab[0], n * c.geom.cells) == cudaSuccess && dalloc(ctx, &tab[1], n * c.geom.cells) == cudaSuccess &&
+                        dalloc(ctx, &d_groups, n) == cudaSuccess && dalloc(ctx, &c.d_tindex, nt) == cudaSuccess) {
+                        CKA(cudaMemcpyAsync(c.d_tindex, ti.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream));
+                        CKA(cudaMemcpyAsync(d_groups, c.groups.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
+                        for (int k = 0; k < 2; ++k) {
+                            fp32_kick_table(tab[k], c.geom, ctx->d_gparams, d_groups, (int)n, k ? 1.0f : 0.5f, ctx->stream);
+                            c.kick_tab[k] = tab[k];
+                        }
+                    }
+                    if (cudaGetLastError() != cudaSuccess && c.kick_tab[0]) return bail(BEC_ERR_CUDA);
+                }
+            } else {
                 for (int k = 0; k < 2; ++k) {
                     CKA(dalloc(ctx, &c.kin_tab[k], nt * (size_t)(c.geom.nz + c.geom.nx * c.geom.ny)));
                     fp32_kin_tables(c.kin_tab[k], c.geom, ctx->d_gparams, c.d_tgroup, k ? 1.0f : 0.5f, ctx->stream);
@@ -2181,8 +2165,9 @@ bec_status bec_init_group(bec_ctx *ctx, int32_t group, const double *psi_gs, con
         if (nz) { cudaStreamSynchronize(s); cudaFree(nz); }
         CKL();
     } else {
-        // bring the other groups to a clean step boundary first
-        if ((st = batched_resolve(ctx, false))) return st;
+        // bring the other groups to a clean step boundary first (without others, the state is overwritten as it is)
+        if (ctx->groups.size() == 1) ctx->pending = ctx->has_pulse = false;
+        else if ((st = batched_resolve(ctx, false))) return st;
         if ((st = gs_stage_ready(ctx))) return st;
         size_t off = 0;
         for (int g = 0; g < group; ++g) off += sizeof(double2) * (size_t)ctx->groups[g].gd.cells;
@@ -2201,15 +2186,14 @@ bec_status bec_init_group(bec_ctx *ctx, int32_t group, const double *psi_gs, con
         }
         ClassRec &c = ctx->classes[gr.cls];
         float4 *base = c.state + (size_t)gr.local_first * cells;
-        fp32_init_group(base, cells, ne, gr.gf, gr.gs_dev, nz, s);
         ClassGeom sub = c.geom;
         sub.n_traj = ne;
         float2 *tx, *ty;
-        if ((st = get_tw32(ctx, sub.nx, &tx)) || (st = get_tw32(ctx, sub.ny, &ty))) {
+        if ((st = get_tw32_full(ctx, sub.nx, &tx)) || (st = get_tw32_full(ctx, sub.ny, &ty))) {
             if (nz) { cudaStreamSynchronize(s); cudaFree(nz); }
             return st;
         }
-        fp32_prep(base, sub, tx, ty, s);
+        fp32_init_group(base, sub, gr.gf, gr.gs_dev, nz, tx, ty, s);
         if (nz) { cudaStreamSynchronize(s); cudaFree(nz); }
         CKL();
     }
@@ -2256,7 +2240,8 @@ bec_status bec_init_groups(bec_ctx *ctx, int32_t n, const int32_t *groups, const
         ctx->last_launches = g_launches - l0;
         return BEC_OK;
     }
-    if ((st = batched_resolve(ctx, false))) return st;
+    if (n == ng) ctx->pending = ctx->has_pulse = false;      // every group listed: the whole state is overwritten
+    else if ((st = batched_resolve(ctx, false))) return st;
     const long long l0 = g_launches;
     cudaStream_t s = ctx->stream;
     if (!ctx->d_gs_ptrs) CKC(dalloc(ctx, &ctx->d_gs_ptrs, (size_t)ng));
@@ -2284,7 +2269,7 @@ bec_status bec_init_groups(bec_ctx *ctx, int32_t n, const int32_t *groups, const
         ctx->gs_ptrs_host = tab;
     }
     CKC(cudaEventRecord(ctx->ev_h2d, s));
-    // one initialisation kernel and one preparation pass per run of consecutive listed trajectories
+    // one initialisation pass per run of consecutive listed trajectories
     for (auto &c : ctx->classes) {
         std::vector<std::pair<int, int>> runs;    // (first local trajectory, count)
         std::vector<int> gl;
@@ -2298,14 +2283,12 @@ bec_status bec_init_groups(bec_ctx *ctx, int32_t n, const int32_t *groups, const
         }
         for (const auto &r : runs) {
             float4 *base = c.state + (size_t)r.first * c.geom.cells;
-            fp32_init_batched(base, c.geom.cells, r.second, c.d_tgroup + r.first, c.d_tlocal + r.first, ctx->d_gparams,
-                              ctx->d_gs_ptrs, host_type, s);
-            CKL();
             ClassGeom sub = c.geom;
             sub.n_traj = r.second;
             float2 *tx, *ty;
-            if ((st = get_tw32(ctx, sub.nx, &tx)) || (st = get_tw32(ctx, sub.ny, &ty))) return st;
-            fp32_prep(base, sub, tx, ty, s);
+            if ((st = get_tw32_full(ctx, sub.nx, &tx)) || (st = get_tw32_full(ctx, sub.ny, &ty))) return st;
+            fp32_init_batched(base, sub, c.d_tgroup + r.first, c.d_tlocal + r.first, ctx->d_gparams, ctx->d_gs_ptrs,
+                              host_type, tx, ty, s);
             CKL();
         }
     }
@@ -2483,12 +2466,10 @@ bec_status bec_render_projections(bec_ctx *ctx, int32_t group, float *xy_a, floa
     ClassGeom one = c.geom;
     one.n_traj = 1;
     float2 *tx, *ty;
-    if ((st = get_tw32(ctx, one.nx, &tx)) || (st = get_tw32(ctx, one.ny, &ty))) return st;
+    if ((st = get_tw32_full(ctx, one.nx, &tx)) || (st = get_tw32_full(ctx, one.ny, &ty))) return st;
     const float sub = (float)(gr.d.V / (2.0 * gr.d.dV));
     for (int t = 0; t < gr.p.ne; ++t) {
-        CKC(cudaMemcpyAsync(ctx->scratch4, c.state + (size_t)(gr.local_first + t) * c.geom.cells,
-                            sizeof(float4) * c.geom.cells, cudaMemcpyDeviceToDevice, s));
-        fp32_unprep(ctx->scratch4, one, tx, ty, s);
+        fp32_unprep(c.state + (size_t)(gr.local_first + t) * c.geom.cells, one, ctx->scratch4, tx, ty, s);
         render_project(ctx->scratch4, one, 1.0f / (float)nxy, sub, lxa, lxb, lza, lzb, s);
     }
     const double scale = 3.0 * gr.d.N * gr.p.ne / ((double)gr.d.cells * gr.d.dV);    // wigner.cu:418
@@ -2667,21 +2648,19 @@ bec_status bec_get_state(bec_ctx *ctx, int32_t group, int32_t traj, double *ab)
     }
     if ((st = batched_resolve(ctx, false))) return st;
     ClassRec &c = ctx->classes[gr.cls];
-    CKC(cudaMemcpyAsync(ctx->scratch4, c.state + (size_t)(gr.local_first + traj) * cells, sizeof(float4) * cells,
-                        cudaMemcpyDeviceToDevice, s));
     ClassGeom one = c.geom;
     one.n_traj = 1;
     float2 *tx, *ty;
-    if ((st = get_tw32(ctx, one.nx, &tx)) || (st = get_tw32(ctx, one.ny, &ty))) return st;
-    fp32_unprep(ctx->scratch4, one, tx, ty, s);
+    if ((st = get_tw32_full(ctx, one.nx, &tx)) || (st = get_tw32_full(ctx, one.ny, &ty))) return st;
+    fp32_unprep(c.state + (size_t)(gr.local_first + traj) * cells, one, ctx->scratch4, tx, ty, s);
     // the stored representation carries the unnormalised x-y inverse transform
     std::vector<float4> h(cells);
     CKC(cudaMemcpyAsync(h.data(), ctx->scratch4, sizeof(float4) * cells, cudaMemcpyDeviceToHost, s));
     CKC(cudaStreamSynchronize(s));
     const double inv = 1.0 / ((double)one.nx * one.ny);
     for (int i = 0; i < cells; ++i) {
-        ab[2 * i] = h[i].x * inv; ab[2 * i + 1] = h[i].z * inv;
-        ab[2 * ((size_t)cells + i)] = h[i].y * inv; ab[2 * ((size_t)cells + i) + 1] = h[i].w * inv;
+        ab[2 * i] = h[i].x * inv; ab[2 * i + 1] = h[i].y * inv;
+        ab[2 * ((size_t)cells + i)] = h[i].z * inv; ab[2 * ((size_t)cells + i) + 1] = h[i].w * inv;
     }
     return BEC_OK;
 }
@@ -2711,16 +2690,16 @@ bec_status bec_set_state(bec_ctx *ctx, int32_t group, int32_t traj, const double
     if ((st = batched_resolve(ctx, false))) return st;
     std::vector<float4> h(cells);
     for (int i = 0; i < cells; ++i)
-        h[i] = make_float4((float)ab[2 * i], (float)ab[2 * ((size_t)cells + i)], (float)ab[2 * i + 1],
+        h[i] = make_float4((float)ab[2 * i], (float)ab[2 * i + 1], (float)ab[2 * ((size_t)cells + i)],
                            (float)ab[2 * ((size_t)cells + i) + 1]);
     ClassRec &c = ctx->classes[gr.cls];
     float4 *dst = c.state + (size_t)(gr.local_first + traj) * cells;
-    CKC(cudaMemcpyAsync(dst, h.data(), sizeof(float4) * cells, cudaMemcpyHostToDevice, s));
+    CKC(cudaMemcpyAsync(ctx->scratch4, h.data(), sizeof(float4) * cells, cudaMemcpyHostToDevice, s));
     ClassGeom one = c.geom;
     one.n_traj = 1;
     float2 *tx, *ty;
-    if ((st = get_tw32(ctx, one.nx, &tx)) || (st = get_tw32(ctx, one.ny, &ty))) return st;
-    fp32_prep(dst, one, tx, ty, s);
+    if ((st = get_tw32_full(ctx, one.nx, &tx)) || (st = get_tw32_full(ctx, one.ny, &ty))) return st;
+    fp32_prep(dst, one, ctx->scratch4, tx, ty, s);
     CKC(cudaStreamSynchronize(s));
     CKL();
     gr.initialised = true;
@@ -2763,7 +2742,7 @@ bec_status bec_profile_steps(bec_ctx *ctx, int32_t n_steps, int32_t max_classes,
                 marks[((size_t)i * nc + c) * 2] = zev[c];
                 marks[((size_t)i * nc + c) * 2 + 1] = pev[c];
             }
-            if ((st = batched_zpass_all(ctx, ctx->pending ? 0.5f : 0.0f, 0.5f, false, nullptr, false, zev.data())))
+            if ((st = batched_zpass_all(ctx, ctx->pending ? 1.0f : 0.5f, false, false, zev.data())))
                 return st;
             ctx->pending = true;
             if ((st = batched_ppass_all(ctx, pev.data()))) return st;
@@ -2824,7 +2803,7 @@ bec_status bec_profile_fused_step(bec_ctx *ctx, int32_t n_steps, double *ms_per_
     long long l0 = g_launches;
     for (int i = 0; i < n_steps; ++i) {
         fp32_put_step(ctx->d_step, (uint32_t)ctx->step, ctx->stream);
-        if ((st = batched_zpass_all(ctx, 0.5f, 0.5f, false, nullptr, false, nullptr, true))) return st;
+        if ((st = batched_zpass_all(ctx, 1.0f, false, false, nullptr, true))) return st;
         if ((st = batched_ppass_all(ctx, nullptr, false, true))) return st;
         CKC(cudaEventRecord(ctx->ev0, ctx->stream));
         step_launch(ctx->plan, ctx->d_gparams, ctx->d_step, 1.0f, nullptr, ctx->stream);

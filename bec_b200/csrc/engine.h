@@ -123,41 +123,37 @@ cudaError_t gs64_measures(const Gs64Dims &d, const Gs64Tab &t, const float2 *psi
 
 // ----------------------------------------------------------------------------
 // batched_fp32.cu
-struct ZPassArgs {
-    float pre;            // kick fraction before the observation (0 or 0.5)
-    float post;           // kick fraction after it (0 or 0.5)
-    float scale;          // applied after the inverse z transform (1 / cells)
-    float out_scale;      // applied before the forward z transform: 1 when a plane pass
-                          // follows, nx*ny when the pass ends a step (see batched_fp32.cu)
-    int has_m1;           // 1: apply matrix m1 before the observation
-    float2 m1[4];         // row-major 2x2 (m11, m12, m21, m22)
-    int observe;          // 1: write per-z partial moments
-    int has_m2;           // 1: apply matrix m2 after the observation
-    float2 m2[4];
-};
-
-// x-space initial state of ne consecutive trajectories of one group (GS + vacuum noise);
+// twiddle tables tx, ty, tz: W_n^k of an axis, k < n / 2 at least
+// initial state of c.n_traj consecutive trajectories of one group (GS + vacuum noise), in the stored representation;
 // noise == NULL draws from Philox, else [traj][a|b][cell] float2
-void fp32_init_group(float4 *state, int cells, int ne, const GroupParamsF &gp, const double2 *gs,
-                     const float2 *noise, cudaStream_t s);
-// k_init for n_traj consecutive trajectories of a class from many ensembles: tgroup / tlocal of the run,
+void fp32_init_group(float4 *state, const ClassGeom &c, const GroupParamsF &gp, const double2 *gs, const float2 *noise,
+                     const float2 *tx, const float2 *ty, cudaStream_t s);
+// the same for c.n_traj consecutive trajectories of a class from many ensembles: tgroup / tlocal of the run,
 // gs_ptrs[group] the ensemble's device ground state, in the element type of host_type (BEC_HOST_*)
-void fp32_init_batched(float4 *state, int cells, int n_traj, const int *tgroup, const int *tlocal,
-                       const GroupParamsF *gp, const void *const *gs_ptrs, int host_type, cudaStream_t s);
-// x-space -> stored representation (inverse transform over x and y)
-void fp32_prep(float4 *state, const ClassGeom &c, const float2 *tw_x, const float2 *tw_y, cudaStream_t s);
-// stored representation -> x-space (forward transform over x and y)
-void fp32_unprep(float4 *state, const ClassGeom &c, const float2 *tw_x, const float2 *tw_y, cudaStream_t s);
-void fp32_zpass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup,
-                const float2 *tw_z, const ZPassArgs &z, double *obs_partial, cudaStream_t s);
-void fp32_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup,
-                const int *tlocal, const float2 *tw_x, const float2 *tw_y, const uint32_t *d_step, cudaStream_t s);
+void fp32_init_batched(float4 *state, const ClassGeom &c, const int *tgroup, const int *tlocal, const GroupParamsF *gp,
+                       const void *const *gs_ptrs, int host_type, const float2 *tx, const float2 *ty, cudaStream_t s);
+// x-space cells (a.re, a.im, b.re, b.im) -> stored representation (inverse transform over x and y), and back
+void fp32_prep(float4 *state, const ClassGeom &c, const float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s);
+void fp32_unprep(const float4 *state, const ClassGeom &c, float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s);
+// kinetic phases of every cell of n_groups ensembles of a class (groups: their indices, device) for kick fraction frac
+void fp32_kick_table(float2 *tab, const ClassGeom &c, const GroupParamsF *gp, const int *groups, int n_groups, float frac,
+                     cudaStream_t s);
+// frac: kick in units of dt; kick: its table, by ensemble tindex[trajectory], or NULL to evaluate the phases in place;
+// scale: 1/cells; out_scale: nx ny when the pass ends a step (no plane pass follows), else 1; m: optional pulse matrix
+// (row-major); obs: when not NULL the pass ends a step and writes per-z partial moments
+void fp32_zpass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const float2 *tz,
+                const float2 *kick, const int *tindex, float frac, float scale, float out_scale, const float2 *m, double *obs,
+                cudaStream_t s);
+// inc_done as fp32_plane_fast; CTAs of the launch
+void fp32_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
+                const float2 *tx, const float2 *ty, uint32_t *d_step, int *inc_done, cudaStream_t s);
+int fp32_ppass_ctas(const ClassGeom &c);
 // the plane passes read the Philox step index from a device scalar, so a captured step graph can replay:
 // an eagerly launched step writes it (fp32_put_step); a step advances it at its end (fp32_inc_step, or the
 // last CTA of a plane launch given inc_done, or of the fused step kernel)
 void fp32_put_step(uint32_t *d_step, uint32_t v, cudaStream_t s);
 void fp32_inc_step(uint32_t *d_step, cudaStream_t s);
-int fp32_zpass_tiles(const ClassGeom &c);   // tiles per trajectory of the z pass (obs_partial layout)
+int fp32_zpass_tiles(const ClassGeom &c);   // tiles per trajectory of an observing z pass (obs_partial layout)
 // obs_partial[traj][tile][z][4] -> traj_axial[traj][z][4] * traj_scale[traj] (1 if NULL),
 // traj_tot[traj][4] = sum over z; traj_axial may be NULL
 void obs_reduce(const double *obs_partial, int n_traj, int tiles, int nz, const double *traj_scale,

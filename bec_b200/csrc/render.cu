@@ -19,7 +19,7 @@ __global__ void k_project(const float4 *x, int nx, int lx, int ny, int ly, int n
     const int cells = nx * ny * nz;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += gridDim.x * blockDim.x) {
         const float4 v = x[i];
-        const float ar = v.x * in_scale, br = v.y * in_scale, ai = v.z * in_scale, bi = v.w * in_scale;
+        const float ar = v.x * in_scale, ai = v.y * in_scale, br = v.z * in_scale, bi = v.w * in_scale;
         // a - i b = (ar + bi) + i (ai - br); -i a + b = (ai + br) + i (bi - ar); |.|^2 / 2 from the 1/sqrt2
         const float pa = ((ar + bi) * (ar + bi) + (ai - br) * (ai - br)) * 0.5f - sub;
         const float pb = ((ai + br) * (ai + br) + (bi - ar) * (bi - ar)) * 0.5f - sub;
