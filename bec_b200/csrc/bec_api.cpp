@@ -46,6 +46,7 @@ struct GroupRec {
     int traj_first = 0;       // global trajectory index of the first trajectory
     int local_first = 0;      // index within the class
     double2 *a = nullptr, *b = nullptr;   // plain path: k-space state [ne][cells]
+    Evo64 evo;                            // plain path: the fused passes' tiles and tables
     double2 *gs_dev = nullptr;            // batched path: x-space ground state (in the context's gs_stage)
     bool initialised = false;
 };
@@ -113,7 +114,8 @@ struct bec_ctx {
     double *d_scal = nullptr;            // device scalars
     double *d_plain_obs = nullptr;       // plain path per-trajectory per-z sums [n_traj][nzmax][4]
     double *d_plain_axial = nullptr;     // [n_traj][nzmax][4]
-    double2 *scratch_a = nullptr, *scratch_b = nullptr;  // plain: x-space copies (max cells)
+    double2 *scratch_a = nullptr, *scratch_b = nullptr;  // plain: x-space copies (scratch_cells each)
+    size_t scratch_cells = 0;
     float4 *scratch4 = nullptr;          // batched: one trajectory (max cells)
     int max_cells = 0, max_nz = 0;
     cudaStream_t stream = nullptr;
@@ -356,20 +358,62 @@ bec_status plain_fft(bec_ctx *ctx, double2 *data, const GeomD &g, int inv)
 }
 
 // ---------------------------------------------------------------- plain step
-// propagate (wigner.cu:178-199) for one trajectory
-bec_status plain_step(bec_ctx *ctx, GroupRec &gr, int t)
+// n steps of an ensemble (propagate, wigner.cu:178-199): the fused passes over all its trajectories, or one kernel per
+// operation and trajectory
+bec_status plain_steps(bec_ctx *ctx, GroupRec &gr, int n)
 {
     const GeomD &g = gr.gd;
-    double2 *a = gr.a + (size_t)t * g.cells, *b = gr.b + (size_t)t * g.cells;
+    if (gr.evo.ready) {
+        CKC(evo64_steps(gr.evo, gr.a, gr.b, gr.p.ne, (uint32_t)ctx->step, n, ctx->stream));
+        return BEC_OK;
+    }
     bec_status st;
-    plain_kick(a, b, g, 1.0, 0, ctx->stream);
-    if ((st = plain_fft(ctx, a, g, 0))) return st;
-    if ((st = plain_fft(ctx, b, g, 0))) return st;
-    plain_nl(a, b, g, (uint32_t)t, (uint32_t)ctx->step, ctx->stream);
-    if ((st = plain_fft(ctx, a, g, 1))) return st;
-    if ((st = plain_fft(ctx, b, g, 1))) return st;
-    plain_kick(a, b, g, 1.0 / g.cells, 1, ctx->stream);
+    for (int i = 0; i < n; ++i)
+        for (int t = 0; t < gr.p.ne; ++t) {
+            double2 *a = gr.a + (size_t)t * g.cells, *b = gr.b + (size_t)t * g.cells;
+            plain_kick(a, b, g, 1.0, 0, ctx->stream);
+            if ((st = plain_fft(ctx, a, g, 0))) return st;
+            if ((st = plain_fft(ctx, b, g, 0))) return st;
+            plain_nl(a, b, g, (uint32_t)t, (uint32_t)(ctx->step + i), ctx->stream);
+            if ((st = plain_fft(ctx, a, g, 1))) return st;
+            if ((st = plain_fft(ctx, b, g, 1))) return st;
+            plain_kick(a, b, g, 1.0 / g.cells, 1, ctx->stream);
+        }
     return BEC_OK;
+}
+
+// n trajectories of x-space in (a, b) to k-space, in place
+bec_status plain_from_x(bec_ctx *ctx, GroupRec &gr, double2 *a, double2 *b, int n)
+{
+    const GeomD &g = gr.gd;
+    if (gr.evo.ready) {
+        CKC(evo64_from_x(gr.evo, a, b, n, ctx->stream));
+        return BEC_OK;
+    }
+    bec_status st;
+    for (int t = 0; t < n; ++t, a += g.cells, b += g.cells) {
+        if ((st = plain_fft(ctx, a, g, 1))) return st;
+        if ((st = plain_fft(ctx, b, g, 1))) return st;
+        plain_scale(a, g.cells, 1.0 / g.cells, ctx->stream);
+        plain_scale(b, g.cells, 1.0 / g.cells, ctx->stream);
+    }
+    return BEC_OK;
+}
+
+// a trajectory's x-space state to (scratch_a, scratch_b)
+bec_status plain_to_x(bec_ctx *ctx, GroupRec &gr, int t)
+{
+    const GeomD &g = gr.gd;
+    const size_t off = (size_t)t * g.cells;
+    if (gr.evo.ready) {
+        CKC(evo64_to_x(gr.evo, gr.a + off, gr.b + off, ctx->scratch_a, ctx->scratch_b, 1, ctx->stream));
+        return BEC_OK;
+    }
+    CKC(cudaMemcpyAsync(ctx->scratch_a, gr.a + off, sizeof(double2) * g.cells, cudaMemcpyDeviceToDevice, ctx->stream));
+    CKC(cudaMemcpyAsync(ctx->scratch_b, gr.b + off, sizeof(double2) * g.cells, cudaMemcpyDeviceToDevice, ctx->stream));
+    bec_status st;
+    if ((st = plain_fft(ctx, ctx->scratch_a, g, 0))) return st;
+    return plain_fft(ctx, ctx->scratch_b, g, 0);
 }
 
 // ---------------------------------------------------------------- batched z pass
@@ -439,6 +483,7 @@ bec_status batched_zpass_all(bec_ctx *ctx, float frac, bool observe, bool ends_s
 // with the fewest CTAs (at most kMaxCarrierCtas, one atomic each) runs last and its last CTA increments the
 // index -- and *advanced tells the caller whether that happened.
 constexpr int kMaxCarrierCtas = 16384;
+constexpr size_t kPlainScratch = (size_t)1 << 21;       // cells of each x-space copy of the FP64 path, at most
 constexpr size_t kKickTableBytes = (size_t)256 << 20;   // phase tables of a class of the general z pass, at most
 
 bec_status batched_ppass_all(bec_ctx *ctx, std::pair<cudaEvent_t, cudaEvent_t> *ev = nullptr, bool put_step = true,
@@ -1019,16 +1064,18 @@ bec_status plain_observe(bec_ctx *ctx)
     CKC(cudaMemsetAsync(ctx->d_plain_obs, 0, sizeof(double) * (size_t)ctx->n_traj * ctx->max_nz * 4, ctx->stream));
     for (auto &gr : ctx->groups) {
         const GeomD &g = gr.gd;
-        for (int t = 0; t < gr.p.ne; ++t) {
-            CKC(cudaMemcpyAsync(ctx->scratch_a, gr.a + (size_t)t * g.cells, sizeof(double2) * g.cells,
-                                cudaMemcpyDeviceToDevice, ctx->stream));
-            CKC(cudaMemcpyAsync(ctx->scratch_b, gr.b + (size_t)t * g.cells, sizeof(double2) * g.cells,
-                                cudaMemcpyDeviceToDevice, ctx->stream));
+        double *obs = ctx->d_plain_obs + (size_t)gr.traj_first * ctx->max_nz * 4;
+        const int at_once = gr.evo.ready ? (int)std::min<size_t>(gr.p.ne, ctx->scratch_cells / g.cells) : 1;
+        for (int t = 0; t < gr.p.ne; t += at_once, obs += (size_t)at_once * ctx->max_nz * 4) {
+            if (gr.evo.ready) {
+                const size_t off = (size_t)t * g.cells;
+                CKC(evo64_observe(gr.evo, gr.a + off, gr.b + off, ctx->scratch_a, ctx->scratch_b, std::min(at_once, gr.p.ne - t), obs,
+                                  ctx->max_nz, ctx->stream));
+                continue;
+            }
             bec_status st;
-            if ((st = plain_fft(ctx, ctx->scratch_a, g, 0))) return st;
-            if ((st = plain_fft(ctx, ctx->scratch_b, g, 0))) return st;
-            plain_axial_sums(ctx->scratch_a, ctx->scratch_b, g,
-                             ctx->d_plain_obs + (size_t)(gr.traj_first + t) * ctx->max_nz * 4, ctx->stream);
+            if ((st = plain_to_x(ctx, gr, t))) return st;
+            plain_axial_sums(ctx->scratch_a, ctx->scratch_b, g, obs, ctx->stream);
             CKL();
         }
     }
@@ -1053,14 +1100,11 @@ bec_status do_evolve(bec_ctx *ctx, int n)
 {
     bec_status st;
     if (ctx->path == BEC_PATH_FP64_PLAIN) {
-        for (int s = 0; s < n; ++s) {
-            for (auto &gr : ctx->groups)
-                for (int t = 0; t < gr.p.ne; ++t)
-                    if ((st = plain_step(ctx, gr, t))) return st;
-            CKL();
-            ctx->step++;
-            ctx->evo_steps++;
-        }
+        for (auto &gr : ctx->groups)
+            if ((st = plain_steps(ctx, gr, n))) return st;
+        CKL();
+        ctx->step += n;
+        ctx->evo_steps += n;
     } else {
         int s = 0;
         if ((st = ensure_plan(ctx))) return st;
@@ -1302,10 +1346,38 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
             CKA(dalloc(ctx, &gr.a, (size_t)gr.p.ne * gr.d.cells));
             CKA(dalloc(ctx, &gr.b, (size_t)gr.p.ne * gr.d.cells));
         }
-        CKA(dalloc(ctx, &ctx->scratch_a, (size_t)ctx->max_cells));
-        CKA(dalloc(ctx, &ctx->scratch_b, (size_t)ctx->max_cells));
         CKA(dalloc(ctx, &ctx->d_plain_obs, (size_t)ctx->n_traj * ctx->max_nz * 4));
         CKA(dalloc(ctx, &ctx->d_plain_axial, (size_t)ctx->n_traj * ctx->max_nz * 4));
+        // the fused passes' tables, and x-space copies of as many trajectories as an observation takes at once; without
+        // room for them, one kernel per operation, and one trajectory
+        size_t elems = 0, wide = 0;
+        for (auto &gr : ctx->groups)
+            if (evo64_dims(gr.gd, gr.p.ne, gr.evo)) {
+                elems += (size_t)gr.evo.kick_elems();
+                wide = std::max(wide, std::min((size_t)gr.p.ne * gr.d.cells, kPlainScratch));
+            }
+        ctx->scratch_cells = std::max((size_t)ctx->max_cells, wide);
+        if (dalloc(ctx, &ctx->scratch_a, 2 * ctx->scratch_cells)) {
+            cudaGetLastError();
+            ctx->scratch_cells = (size_t)ctx->max_cells;
+            CKA(dalloc(ctx, &ctx->scratch_a, 2 * ctx->scratch_cells));
+        }
+        ctx->scratch_b = ctx->scratch_a + ctx->scratch_cells;
+        double2 *kick = nullptr;
+        const bool room = dalloc(ctx, &kick, elems) == cudaSuccess;
+        for (auto &gr : ctx->groups) {
+            Evo64 &e = gr.evo;
+            Gs64Tab t;
+            if (!e.ready || !room || get_gs64_tab(ctx, gr.gd, t)) {
+                e.ready = false;
+                continue;
+            }
+            e.x = t.x; e.y = t.y; e.z = t.z;
+            e.kick = kick;
+            kick += e.kick_elems();
+            evo64_kick_table(e, ctx->stream);
+        }
+        cudaGetLastError();
     } else {
         std::vector<GroupParamsF> gfs(ng);
         for (int g = 0; g < ng; ++g) gfs[g] = ctx->groups[g].gf;
@@ -1342,28 +1414,7 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
             CKA(cudaMemcpyAsync(c.d_tgroup, tg.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream));
             CKA(cudaMemcpyAsync(c.d_tlocal, tl.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream));
             CKA(cudaMemcpyAsync(c.d_traj_scale, ts.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, ctx->stream));
-            if (!fp32_fast_pencil_supported(c.geom)) {
-                // the general z pass evaluates its phases in FP64: a table per ensemble where it stays small
-                const size_t n = c.groups.size();
-                if (2 * sizeof(float2) * n * c.geom.cells <= kKickTableBytes) {
-                    std::vector<int> ti(nt);
-                    for (size_t e = 0; e < n; ++e)
-                        for (int t = 0; t < ctx->groups[c.groups[e]].p.ne; ++t) ti[ctx->groups[c.groups[e]].local_first + t] = (int)e;
-                    int *d_groups = nullptr;
-                    float2 *tab[2] = {nullptr, nullptr};
-                    // (without them, for want of memory or under a byte limit, the pass evaluates the phases itself)
-                    if (dalloc(ctx, &tab[0], n * c.geom.cells) == cudaSuccess && dalloc(ctx, &tab[1], n * c.geom.cells) == cudaSuccess &&
-                        dalloc(ctx, &d_groups, n) == cudaSuccess && dalloc(ctx, &c.d_tindex, nt) == cudaSuccess) {
-                        CKA(cudaMemcpyAsync(c.d_tindex, ti.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream));
-                        CKA(cudaMemcpyAsync(d_groups, c.groups.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
-                        for (int k = 0; k < 2; ++k) {
-                            fp32_kick_table(tab[k], c.geom, ctx->d_gparams, d_groups, (int)n, k ? 1.0f : 0.5f, ctx->stream);
-                            c.kick_tab[k] = tab[k];
-                        }
-                    }
-                    if (cudaGetLastError() != cudaSuccess && c.kick_tab[0]) return bail(BEC_ERR_CUDA);
-                }
-            } else {
+            if (fp32_fast_pencil_supported(c.geom)) {
                 for (int k = 0; k < 2; ++k) {
                     CKA(dalloc(ctx, &c.kin_tab[k], nt * (size_t)(c.geom.nz + c.geom.nx * c.geom.ny)));
                     fp32_kin_tables(c.kin_tab[k], c.geom, ctx->d_gparams, c.d_tgroup, k ? 1.0f : 0.5f, ctx->stream);
@@ -1372,6 +1423,31 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
             }
         }
         CKA(dalloc(ctx, &ctx->scratch4, (size_t)ctx->max_cells));
+        // the general z pass evaluates its phases in FP64: a table per ensemble where it stays small, after all that a
+        // context cannot do without
+        for (auto &c : ctx->classes) {
+            if (fp32_fast_pencil_supported(c.geom)) continue;
+            const size_t nt = (size_t)c.geom.n_traj;
+            const size_t n = c.groups.size();
+            if (2 * sizeof(float2) * n * c.geom.cells <= kKickTableBytes) {
+                std::vector<int> ti(nt);
+                for (size_t e = 0; e < n; ++e)
+                    for (int t = 0; t < ctx->groups[c.groups[e]].p.ne; ++t) ti[ctx->groups[c.groups[e]].local_first + t] = (int)e;
+                int *d_groups = nullptr;
+                float2 *tab[2] = {nullptr, nullptr};
+                // (without them, for want of memory or under a byte limit, the pass evaluates the phases itself)
+                if (dalloc(ctx, &tab[0], n * c.geom.cells) == cudaSuccess && dalloc(ctx, &tab[1], n * c.geom.cells) == cudaSuccess &&
+                    dalloc(ctx, &d_groups, n) == cudaSuccess && dalloc(ctx, &c.d_tindex, nt) == cudaSuccess) {
+                    CKA(cudaMemcpyAsync(c.d_tindex, ti.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream));
+                    CKA(cudaMemcpyAsync(d_groups, c.groups.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
+                    for (int k = 0; k < 2; ++k) {
+                        fp32_kick_table(tab[k], c.geom, ctx->d_gparams, d_groups, (int)n, k ? 1.0f : 0.5f, ctx->stream);
+                        c.kick_tab[k] = tab[k];
+                    }
+                }
+                if (cudaGetLastError() != cudaSuccess && c.kick_tab[0]) return bail(BEC_ERR_CUDA);
+            }
+        }
     }
 #undef CKA
     (void)st;
@@ -2153,16 +2229,10 @@ bec_status bec_init_group(bec_ctx *ctx, int32_t group, const double *psi_gs, con
                                             cudaMemcpyHostToDevice, s);
             if (e != cudaSuccess) { cudaFree(p); return fail(ctx, BEC_ERR_CUDA, cudaGetErrorString(e)); }
         }
-        for (int t = 0; t < ne; ++t) {
-            double2 *a = gr.a + (size_t)t * cells, *b = gr.b + (size_t)t * cells;
-            plain_init(a, b, gs, nz ? nz + (size_t)(2 * t) * cells : nullptr,
-                       nz ? nz + (size_t)(2 * t + 1) * cells : nullptr, g, (uint32_t)t, s);
-            if ((st = plain_fft(ctx, a, g, 1))) { if (nz) { cudaStreamSynchronize(s); cudaFree(nz); } return st; }
-            if ((st = plain_fft(ctx, b, g, 1))) { if (nz) { cudaStreamSynchronize(s); cudaFree(nz); } return st; }
-            plain_scale(a, cells, 1.0 / cells, s);
-            plain_scale(b, cells, 1.0 / cells, s);
-        }
+        plain_init(gr.a, gr.b, gs, nz, g, ne, s);
+        st = plain_from_x(ctx, gr, gr.a, gr.b, ne);
         if (nz) { cudaStreamSynchronize(s); cudaFree(nz); }
+        if (st) return st;
         CKL();
     } else {
         // bring the other groups to a clean step boundary first (without others, the state is overwritten as it is)
@@ -2519,8 +2589,12 @@ bec_status bec_run(bec_ctx *ctx, const bec_schedule *sch, bec_moments *samples, 
         return BEC_OK;
     };
     if (ctx->path == BEC_PATH_FP64_PLAIN) {
-        for (int i = 1; i <= n; ++i) {
-            if ((st = do_evolve(ctx, 1))) return st;
+        for (int i = 0; i < n;) {
+            // the steps up to the next sample or pulse
+            int len = std::min(n - i, every - i % every);
+            if (sch->pi_pulse_step > i) len = std::min(len, sch->pi_pulse_step - i);
+            if ((st = do_evolve(ctx, len))) return st;
+            i += len;
             if (i % every == 0 && sample < n_samples) {
                 if ((st = plain_observe(ctx))) return st;
                 if ((st = take_sample())) return st;
@@ -2635,12 +2709,7 @@ bec_status bec_get_state(bec_ctx *ctx, int32_t group, int32_t traj, double *ab)
     cudaStream_t s = ctx->stream;
     bec_status st;
     if (ctx->path == BEC_PATH_FP64_PLAIN) {
-        CKC(cudaMemcpyAsync(ctx->scratch_a, gr.a + (size_t)traj * cells, sizeof(double2) * cells,
-                            cudaMemcpyDeviceToDevice, s));
-        CKC(cudaMemcpyAsync(ctx->scratch_b, gr.b + (size_t)traj * cells, sizeof(double2) * cells,
-                            cudaMemcpyDeviceToDevice, s));
-        if ((st = plain_fft(ctx, ctx->scratch_a, gr.gd, 0))) return st;
-        if ((st = plain_fft(ctx, ctx->scratch_b, gr.gd, 0))) return st;
+        if ((st = plain_to_x(ctx, gr, traj))) return st;
         CKC(cudaMemcpyAsync(ab, ctx->scratch_a, sizeof(double2) * cells, cudaMemcpyDeviceToHost, s));
         CKC(cudaMemcpyAsync(ab + 2 * (size_t)cells, ctx->scratch_b, sizeof(double2) * cells, cudaMemcpyDeviceToHost, s));
         CKC(cudaStreamSynchronize(s));
@@ -2678,10 +2747,7 @@ bec_status bec_set_state(bec_ctx *ctx, int32_t group, int32_t traj, const double
         double2 *a = gr.a + (size_t)traj * cells, *b = gr.b + (size_t)traj * cells;
         CKC(cudaMemcpyAsync(a, ab, sizeof(double2) * cells, cudaMemcpyHostToDevice, s));
         CKC(cudaMemcpyAsync(b, ab + 2 * (size_t)cells, sizeof(double2) * cells, cudaMemcpyHostToDevice, s));
-        if ((st = plain_fft(ctx, a, gr.gd, 1))) return st;
-        if ((st = plain_fft(ctx, b, gr.gd, 1))) return st;
-        plain_scale(a, cells, 1.0 / cells, s);
-        plain_scale(b, cells, 1.0 / cells, s);
+        if ((st = plain_from_x(ctx, gr, a, b, 1))) return st;
         CKC(cudaStreamSynchronize(s));
         CKL();
         gr.initialised = true;
@@ -2730,8 +2796,7 @@ bec_status bec_profile_steps(bec_ctx *ctx, int32_t n_steps, int32_t max_classes,
                 mk.first = new_event();
                 mk.second = new_event();
                 CKC(cudaEventRecord(mk.first, s));
-                for (int t = 0; t < gr.p.ne; ++t)
-                    if ((st = plain_step(ctx, gr, t))) return st;
+                if ((st = plain_steps(ctx, gr, 1))) return st;
                 CKC(cudaEventRecord(mk.second, s));
             }
         } else {

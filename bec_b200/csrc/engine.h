@@ -54,8 +54,8 @@ void plain_nl(double2 *a, double2 *b, const GeomD &g, uint32_t traj, uint32_t st
 void plain_scale(double2 *a, int n, double scale, cudaStream_t s);
 void plain_pulse(double2 *a, double2 *b, int n, double2 m11, double2 m12, double2 m21, double2 m22,
                  cudaStream_t s);
-void plain_init(double2 *a, double2 *b, const double2 *gs, const double2 *noise_a, const double2 *noise_b,
-                const GeomD &g, uint32_t traj, cudaStream_t s);
+// ne trajectories; noise: two fields (a, b) per trajectory, or NULL for the ensemble's own
+void plain_init(double2 *a, double2 *b, const double2 *gs, const double2 *noise, const GeomD &g, int ne, cudaStream_t s);
 // per-z sums (|a|^2, |b|^2, Re, Im conj(a) b) of x-space arrays into out[nz][4], accumulating
 void plain_axial_sums(const double2 *a, const double2 *b, const GeomD &g, double *out, cudaStream_t s);
 // ground state
@@ -120,6 +120,26 @@ cudaError_t gs64_measures(const Gs64Dims &d, const Gs64Tab &t, const double2 *ps
                           double *sums4, double *sums, cudaStream_t s);
 cudaError_t gs64_measures(const Gs64Dims &d, const Gs64Tab &t, const float2 *psi, double2 *work, const Gs64Par *par, double *part,
                           double *sums4, double *sums, cudaStream_t s);
+
+// FP64 real-time steps of both components, n trajectories of one ensemble; a and b in k-space unless said otherwise
+struct Evo64 {
+    GeomD g;
+    int lppc = 0, lp = 0;                    // log2 of the planes and of the pencils per CTA
+    bool ready = false;                      // false: one kernel per operation (plain_fp64.cu)
+    const double2 *x = nullptr, *y = nullptr, *z = nullptr;   // all n twiddles W_n^k of each axis
+    double2 *kick = nullptr;                 // half-kick phases, kick_elems()
+    int kick_elems() const { return g.nz + g.nx * g.ny; }
+};
+// fills e.g and the tiles; false when a plane of both components or two pencils do not fit in shared memory
+bool evo64_dims(const GeomD &g, int n, Evo64 &e);
+void evo64_kick_table(const Evo64 &e, cudaStream_t s);
+cudaError_t evo64_steps(const Evo64 &e, double2 *a, double2 *b, int n, uint32_t step, int n_steps, cudaStream_t s);
+// per-z sums (|a|^2, |b|^2, Re, Im conj(a) b) dV into obs[n][row][4]; wa, wb: n trajectories of workspace
+cudaError_t evo64_observe(const Evo64 &e, const double2 *a, const double2 *b, double2 *wa, double2 *wb, int n, double *obs, int row,
+                          cudaStream_t s);
+// x-space to (wa, wb); and x-space to k-space in place
+cudaError_t evo64_to_x(const Evo64 &e, const double2 *a, const double2 *b, double2 *wa, double2 *wb, int n, cudaStream_t s);
+cudaError_t evo64_from_x(const Evo64 &e, double2 *a, double2 *b, int n, cudaStream_t s);
 
 // ----------------------------------------------------------------------------
 // batched_fp32.cu

@@ -1,6 +1,7 @@
-// fp64_passes.cu -- FP64 imaginary-time steps of single-component states in two fused passes, and the FP64
-// measures of ground states.
+// fp64_passes.cu -- FP64 imaginary-time steps of single-component states and real-time steps of both components, each in
+// two fused passes, and the FP64 measures of ground states.
 //
+// Imaginary time:
 // calculateSteadyState (programs/bec_wigner_3d.cuda/wigner.cu:84-175) takes a kick, three transform axes, the
 // nonlinear factor, three axes, a scaling, a kick, three axes and a renormalisation per step, each a kernel of its
 // own. Here a step is a pencil pass (IFFT_z -> 1/cells -> half kick -> norm -> half kick of the next step -> FFT_z)
@@ -16,6 +17,8 @@
 // twiddles and kick factors lay in shared memory at the pass's start and a launch overlapped the end of the one before). The measures of a
 // batch (mu, energy, norm, residual) took twenty launches and two synchronisations a state; here they take eight
 // launches for half the batch (96 states of 32x32x256 with 60 steps: the whole call 42.6 -> 23.2 ms).
+//
+// Real time (wigner.cu:178-199): the passes of k64_evo_plane and k64_evo_pencil below, over every trajectory of an ensemble.
 #include <algorithm>
 
 #include "engine.h"
@@ -416,10 +419,210 @@ __global__ void k64_fold(const double *__restrict__ part, int n, int K, int firs
     }
 }
 
+// ---------------------------------------------------------------- real time
+// Between calls an ensemble's state is k-space on every axis, as the reference keeps it. n steps take 2 n + 1 launches:
+//   pencils   k-space -> half kick -> FFT_z                      \
+//   planes    FFT_xy -> nonlinear step, loss noise -> IFFT_xy     | the last pencil pass ends
+//   pencils   IFFT_z -> 1/cells, two half kicks -> FFT_z         /  after one half kick, in k-space
+// The two half kicks between steps are applied one after the other, so that a run has the same bits however it is cut
+// into calls. Where one kernel per operation and trajectory moved the state nine times a step, it moves twice. The plane
+// pass is bound by FP64 arithmetic (most of it exp, sincos and the normals): 15 us of a step of four 16x16x128
+// trajectories, whose pencil pass takes 7, near its latency. Measured, a step: 22.9 us for those four, 199 for 64, and 183
+// for eight of 32x32x256; with one kernel per operation and trajectory 565, 9154 and 1311.
+
+// A CTA holds ppc planes of both components, the second's after the first's.
+//   E_STEP    state -> FFT_xy -> midpoint iteration (wigner_kernel.cu:184-229) and loss noise -> IFFT_xy -> state
+//   E_OBSERVE state -> FFT_xy -> per-z sums |a|^2, |b|^2, Re and Im conj(a) b, times dV
+//   E_TO_X    state -> FFT_xy -> state;   E_FROM_X  state -> IFFT_xy -> state
+enum { E_STEP, E_OBSERVE, E_TO_X, E_FROM_X };
+
+__device__ __forceinline__ double2 cexp64(double re, double im)
+{
+    double s, c;
+    sincos(im, &s, &c);
+    const double m = exp(re);
+    return make_double2(m * c, m * s);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(256) k64_evo_plane(double2 *A, double2 *B, const GeomD g, int lppc, const double2 *__restrict__ tx,
+                                                     const double2 *__restrict__ ty, uint32_t traj0, uint32_t step, double *obs,
+                                                     int row)
+{
+    extern __shared__ double2 sm64[];
+    const int lx = g.lx, ly = g.ly, nx = 1 << lx, ny = 1 << ly, ld = nx + 1, lplane = lx + ly;
+    const int lchunk = lppc + lplane, chunk = 1 << lchunk;
+    const int lcta = g.lz - lppc;                               // CTAs per trajectory
+    const int traj = blockIdx.x >> lcta, c0 = blockIdx.x & ((1 << lcta) - 1);
+    const size_t cell0 = (size_t)c0 << lchunk;
+    const size_t first = ((size_t)traj << (lplane + g.lz)) + cell0;
+    double2 *const gA = A + first, *const gB = B + first;
+    auto natural = [&](int i) { return (i >> lx) * ld + (i & (nx - 1)); };
+    auto reversed = [&](int i) {
+        return ((i >> lplane) * ny + digit_rev((i >> lx) & (ny - 1), ly)) * ld + digit_rev(i & (nx - 1), lx);
+    };
+    const Lines rows{lx, lppc + ly + 1, 1, 30, ld, 0}, cols{ly, lppc + lx + 1, ld, lx, 1, ny * ld};
+    double2 *twx = sm64 + ((2 * ny << lppc) * ld), *twy = twx + nx;
+    for (int i = threadIdx.x; i < nx; i += blockDim.x) copy16(twx + i, tx + i);
+    for (int i = threadIdx.x; i < ny; i += blockDim.x) copy16(twy + i, ty + i);
+    wait_predecessor();
+    allow_successor();
+    for (int i = threadIdx.x; i < 2 * chunk; i += blockDim.x)
+        copy16(sm64 + (MODE == E_FROM_X ? natural(i) : reversed(i)), i < chunk ? gA + i : gB + (i - chunk));
+    copy_wait();
+    __syncthreads();
+    if (MODE != E_FROM_X) {
+        fft_time<false>(sm64, rows, twx);
+        if (ly > 0) fft_time<false>(sm64, cols, twy);
+    }
+    if (MODE == E_STEP) {
+        const double dt = g.dt_evo, h = dt / 2.0, iz = 1.0 / (g.lambda * g.lambda);
+        const double ns = sqrt(dt / (2.0 * g.dV));
+        const double c1 = sqrt(g.l111 / 6.0) * 3.0, c2 = sqrt(g.l12 / 2.0), c3 = sqrt(g.l22);
+        for (int i = threadIdx.x; i < chunk; i += blockDim.x) {
+            double2 &wa = sm64[natural(i)], &wb = sm64[natural(i + chunk)];
+            const double X = -g.xmax + g.dx * (double)(i & (nx - 1));
+            const double Y = ny > 1 ? -g.ymax + g.dy * (double)((i >> lx) & (ny - 1)) : 0.0;
+            const double Z = -g.zmax + g.dz * (double)((c0 << lppc) + (i >> lplane));
+            const double V = (X * X + Y * Y + Z * Z * iz) / 2.0;
+            const double2 a0 = wa, b0 = wb;
+            double2 x = a0, y = b0, da = make_double2(0, 0), db = make_double2(0, 0);
+            for (int it = 0; it < g.itmax; ++it) {
+                const double na = x.x * x.x + x.y * x.y, nb = y.x * y.x + y.y * y.y;
+                const double pa_re = -(g.l111 * na * na + g.l12 * nb) / 2.0, pb_re = -(g.l22 * nb + g.l12 * na) / 2.0;
+                const double pa_im = V + g.g11 * na + g.g12 * nb, pb_im = V + g.g22 * nb + g.g12 * na - g.detuning;
+                da = cexp64(pa_re * h, pa_im * h);
+                db = cexp64(pb_re * h, pb_im * h);
+                x = cmul(a0, da);
+                y = cmul(b0, db);
+            }
+            double2 ao = cmul(x, da), bo = cmul(y, db);
+            if (g.noise) {
+                double r[6];
+                loss_normals6<double>(g.seed, traj0 + (uint32_t)traj, step, (uint32_t)(cell0 + i), r);
+                const double2 w1 = make_double2(ns * r[0], ns * r[1]), w2 = make_double2(ns * r[2], ns * r[3]),
+                              w3 = make_double2(ns * r[4], ns * r[5]);
+                const double2 ca = cconj(a0), cb = cconj(b0);
+                ao = cadd(ao, cadd(cmul(cscale(cmul(ca, ca), c1), w1), cmul(cscale(cb, c2), w2)));
+                bo = cadd(bo, cadd(cmul(cscale(ca, c2), w2), cmul(cscale(cb, c3), w3)));
+            }
+            wa = ao;
+            wb = bo;
+        }
+        __syncthreads();
+    }
+    if (MODE == E_STEP || MODE == E_FROM_X) {
+        if (ly > 0) fft_freq<true>(sm64, cols, twy);
+        fft_freq<true>(sm64, rows, twx);
+    }
+    if (MODE == E_OBSERVE) {
+        const int plane = 1 << lplane;
+        auto sums = [&](int pl, int i0, int di) {
+            KVec<4> acc;
+            for (int i = i0; i < plane; i += di) {
+                const double2 u = sm64[natural((pl << lplane) + i)], v = sm64[natural(chunk + (pl << lplane) + i)];
+                acc.v[0].add(u.x * u.x + u.y * u.y);
+                acc.v[1].add(v.x * v.x + v.y * v.y);
+                acc.v[2].add(u.x * v.x + u.y * v.y);
+                acc.v[3].add(u.x * v.y - u.y * v.x);
+            }
+            return acc;
+        };
+        double *o = obs + ((size_t)traj * row + ((size_t)c0 << lppc)) * 4;
+        if (lppc == 0) {
+            const KVec<4> r = block_reduce<4>(sums(0, threadIdx.x, blockDim.x));
+            if (threadIdx.x == 0)
+                for (int k = 0; k < 4; ++k) o[k] = r.v[k].value() * g.dV;
+        } else {                                                // planes of 128 cells at most: a warp each
+            for (int pl = threadIdx.x >> 5; pl < 1 << lppc; pl += blockDim.x >> 5) {
+                KVec<4> r = sums(pl, threadIdx.x & 31, 32);
+                for (int k = 0; k < 4; ++k)
+                    for (int off = 16; off > 0; off >>= 1)
+                        ksum_merge(r.v[k], __shfl_down_sync(0xffffffffu, r.v[k].s, off),
+                                   __shfl_down_sync(0xffffffffu, r.v[k].c, off));
+                if ((threadIdx.x & 31) == 0)
+                    for (int k = 0; k < 4; ++k) o[4 * pl + k] = r.v[k].value() * g.dV;
+            }
+        }
+        return;
+    }
+    for (int i = threadIdx.x; i < 2 * chunk; i += blockDim.x)
+        (i < chunk ? gA + i : gB + (i - chunk))[0] = sm64[MODE == E_TO_X ? natural(i) : reversed(i)];
+}
+
+// A CTA holds 2^lp adjacent pencils of one component: [IFFT_z ->] scale -> `kicks` half kicks [-> FFT_z], from (sA, sB) to
+// (dA, dB), which may be the same. kick: e^{i k^2/2 dt/2}, nz of the kz, then nx ny of (kx, ky).
+template <bool FROM_Z, bool TO_Z>
+__global__ void __launch_bounds__(256) k64_evo_pencil(const double2 *sA, const double2 *sB, double2 *dA, double2 *dB, int lx, int ly,
+                                                      int lz, int lp, int n, const double2 *__restrict__ tz,
+                                                      const double2 *__restrict__ kick, double scale, int kicks)
+{
+    extern __shared__ double2 sm64[];
+    const int nz = 1 << lz, lplane = lx + ly, P = 1 << lp, chunk = nz << lp, ltiles = lplane - lp;
+    double2 *tw = sm64 + chunk, *ez = tw + nz, *exy = ez + nz;
+    const bool second = (int)blockIdx.x >= n << ltiles;
+    const int blk = second ? blockIdx.x - (n << ltiles) : blockIdx.x;
+    const int traj = blk >> ltiles, pen0 = (blk & ((1 << ltiles) - 1)) << lp;
+    const size_t off = ((size_t)traj << (lplane + lz)) + pen0;
+    const double2 *src = (second ? sB : sA) + off;
+    double2 *dst = (second ? dB : dA) + off;
+    for (int i = threadIdx.x; i < nz; i += blockDim.x) copy16(tw + i, tz + i);
+    if (kicks) {
+        for (int i = threadIdx.x; i < nz; i += blockDim.x) copy16(ez + i, kick + i);
+        if (threadIdx.x < P) copy16(exy + threadIdx.x, kick + nz + pen0 + threadIdx.x);
+    }
+    wait_predecessor();
+    allow_successor();
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x)
+        copy16(sm64 + (FROM_Z ? (digit_rev(i >> lp, lz) << lp) + (i & (P - 1)) : i), src + ((size_t)(i >> lp) << lplane) + (i & (P - 1)));
+    copy_wait();
+    __syncthreads();
+    const Lines L{lz, lp, P, 30, 1, 0};
+    if (FROM_Z) fft_time<true>(sm64, L, tw);
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x) {
+        double2 u = cscale(sm64[i], scale);
+        if (kicks) {
+            const double2 e = cmul(ez[i >> lp], exy[i & (P - 1)]);
+            u = cmul(u, e);
+            if (kicks > 1) u = cmul(u, e);
+        }
+        if (TO_Z) sm64[i] = u;
+        else dst[((size_t)(i >> lp) << lplane) + (i & (P - 1))] = u;
+    }
+    if (!TO_Z) return;
+    __syncthreads();
+    fft_freq<false>(sm64, L, tw);
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x)
+        dst[((size_t)(i >> lp) << lplane) + (i & (P - 1))] = sm64[(digit_rev(i >> lp, lz) << lp) + (i & (P - 1))];
+}
+
+// e^{i k^2/2 dt/2} (propagateKSpaceRealTime, wigner_kernel.cu:137-151): nz of the kz, then nx ny of (kx, ky)
+__global__ void k64_evo_kick(const GeomD g, double2 *__restrict__ kick)
+{
+    const int n = g.nz + g.nx * g.ny;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        double k2;
+        if (i < g.nz) {
+            const double kz = getk<double>(i, g.dkz, g.nz);
+            k2 = kz * kz / 2.0;
+        } else {
+            const int pen = i - g.nz;
+            const double kx = getk<double>(pen & (g.nx - 1), g.dkx, g.nx);
+            const double ky = g.ly > 0 ? getk<double>(pen >> g.lx, g.dky, g.ny) : 0.0;
+            k2 = (kx * kx + ky * ky) / 2.0;
+        }
+        double s, c;
+        sincos(k2 * g.dt_evo / 2.0, &s, &c);
+        kick[i] = make_double2(c, s);
+    }
+}
+
 size_t plane_smem(int lx, int ly, int lppc)
 {
     return sizeof(double2) * ((((size_t)1 << (ly + lppc)) * ((1 << lx) + 1)) + ((size_t)1 << lx) + ((size_t)1 << ly));
 }
+size_t evo_plane_smem(int lx, int ly, int lppc) { return 2 * plane_smem(lx, ly, lppc); }    // (the twiddles' share is ample)
+size_t evo_pencil_smem(int lz, int lp) { return sizeof(double2) * (((size_t)1 << (lz + lp)) + ((size_t)2 << lz) + 8); }
 size_t pencil_smem(int lz, int lp) { return sizeof(double2) * (((size_t)1 << (lz + lp)) + ((size_t)2 << lz)); }
 constexpr size_t kMaxSmem = 200 * 1024;
 
@@ -452,7 +655,80 @@ void fold_launch(const Gs64Dims &d, const double *part, int n, int K, int first,
     g_launches++;
 }
 
+template <bool FROM_Z, bool TO_Z>
+cudaError_t evo_pencil(const Evo64 &e, const double2 *sA, const double2 *sB, double2 *dA, double2 *dB, int n, double scale, int kicks,
+                       cudaStream_t s)
+{
+    cudaError_t err = ensure_smem_limit((const void *)k64_evo_pencil<FROM_Z, TO_Z>, (int)kMaxSmem);
+    if (err) return err;
+    const GeomD &g = e.g;
+    return launch_after(k64_evo_pencil<FROM_Z, TO_Z>, 2 * n << (g.lx + g.ly - e.lp), threads_for(g.lz + e.lp),
+                        evo_pencil_smem(g.lz, e.lp), s, sA, sB, dA, dB, g.lx, g.ly, g.lz, e.lp, n, e.z, (const double2 *)e.kick, scale,
+                        kicks);
+}
+
+template <int MODE>
+cudaError_t evo_plane(const Evo64 &e, double2 *A, double2 *B, int n, uint32_t traj0, uint32_t step, double *obs, int row,
+                      cudaStream_t s)
+{
+    cudaError_t err = ensure_smem_limit((const void *)k64_evo_plane<MODE>, (int)kMaxSmem);
+    if (err) return err;
+    const GeomD &g = e.g;
+    return launch_after(k64_evo_plane<MODE>, n << (g.lz - e.lppc), threads_for(e.lppc + g.lx + g.ly),
+                        evo_plane_smem(g.lx, g.ly, e.lppc), s, A, B, g, e.lppc, e.x, e.y, traj0, step, obs, row);
+}
+
 } // namespace
+
+// As gs64_dims; both components of a plane lie in shared memory.
+bool evo64_dims(const GeomD &g, int n, Evo64 &e)
+{
+    e.g = g;
+    e.lppc = std::max(0, std::min(8 - g.lx - g.ly, g.lz));
+    e.lp = std::min(3, g.lx + g.ly);
+    while (e.lp > 1 && (((long long)2 * n << (g.lx + g.ly - e.lp)) < 148 || evo_pencil_smem(g.lz, e.lp) > 64 * 1024)) --e.lp;
+    e.ready = g.lx >= 1 && g.lz >= 1 && g.lx <= 10 && g.ly <= 10 && g.lz <= 10 && evo_plane_smem(g.lx, g.ly, e.lppc) <= kMaxSmem &&
+              evo_pencil_smem(g.lz, e.lp) <= kMaxSmem && ((long long)2 * n << (g.lx + g.ly - e.lp)) < (1ll << 31) &&
+              ((long long)n << (g.lz - e.lppc)) < (1ll << 31);
+    return e.ready;
+}
+
+void evo64_kick_table(const Evo64 &e, cudaStream_t s)
+{
+    k64_evo_kick<<<(e.kick_elems() + 127) / 128, 128, 0, s>>>(e.g, e.kick);
+    g_launches++;
+}
+
+cudaError_t evo64_steps(const Evo64 &e, double2 *a, double2 *b, int n, uint32_t step, int n_steps, cudaStream_t s)
+{
+    const double norm = 1.0 / e.g.cells;
+    cudaError_t err = n_steps > 0 ? evo_pencil<false, true>(e, a, b, a, b, n, 1.0, 1, s) : cudaSuccess;
+    for (int i = 0; i < n_steps && !err; ++i) {
+        if ((err = evo_plane<E_STEP>(e, a, b, n, 0, step + (uint32_t)i, nullptr, 0, s))) break;
+        err = i + 1 < n_steps ? evo_pencil<true, true>(e, a, b, a, b, n, norm, 2, s)
+                              : evo_pencil<true, false>(e, a, b, a, b, n, norm, 1, s);
+    }
+    return err;
+}
+
+cudaError_t evo64_observe(const Evo64 &e, const double2 *a, const double2 *b, double2 *wa, double2 *wb, int n, double *obs, int row,
+                          cudaStream_t s)
+{
+    const cudaError_t err = evo_pencil<false, true>(e, a, b, wa, wb, n, 1.0, 0, s);
+    return err ? err : evo_plane<E_OBSERVE>(e, wa, wb, n, 0, 0, obs, row, s);
+}
+
+cudaError_t evo64_to_x(const Evo64 &e, const double2 *a, const double2 *b, double2 *wa, double2 *wb, int n, cudaStream_t s)
+{
+    const cudaError_t err = evo_pencil<false, true>(e, a, b, wa, wb, n, 1.0, 0, s);
+    return err ? err : evo_plane<E_TO_X>(e, wa, wb, n, 0, 0, nullptr, 0, s);
+}
+
+cudaError_t evo64_from_x(const Evo64 &e, double2 *a, double2 *b, int n, cudaStream_t s)
+{
+    const cudaError_t err = evo_plane<E_FROM_X>(e, a, b, n, 0, 0, nullptr, 0, s);
+    return err ? err : evo_pencil<true, false>(e, a, b, a, b, n, 1.0 / e.g.cells, 0, s);
+}
 
 // Tiles: a plane pass takes planes up to 256 cells together, a pencil pass 8 pencils (128-byte rows), fewer while one
 // launch has fewer CTAs than the chip has SMs (down to 2: 32-byte sectors) or the tile would not fit.

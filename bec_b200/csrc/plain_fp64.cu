@@ -1,11 +1,11 @@
-// plain_fp64.cu -- the plain per-trajectory FP64 path.
+// plain_fp64.cu -- FP64 kernels, one per operation.
 //
 // Structured like the reference's propagate() (programs/bec_wigner_3d.cuda/
-// wigner.cu:178-199): one kernel per operation, one trajectory at a time,
-// separate passes for the k-space kick, each FFT axis, the nonlinear step and
-// the 1/cells scaling. It is the FP64 parity path (matches the CPU oracle to
-// ~1e-12 relative) and the baseline that the batched FP32 path is measured
-// against. FFT axes use this library's shared-memory radix-2 stages
+// wigner.cu:178-199): one trajectory at a time, separate passes for the k-space
+// kick, each FFT axis, the nonlinear step and the 1/cells scaling. The FP64 path
+// takes its initial states and pulses from here, and its steps and transforms
+// where a plane does not fit in shared memory for the fused passes
+// (fp64_passes.cu). FFT axes use this library's shared-memory radix-2 stages
 // (fft_smem.cuh) in place of cuFFT + transposes (batchfft.cu:130-180).
 #include <mutex>
 #include <set>
@@ -170,25 +170,27 @@ __global__ void k_pulse(double2 *a, double2 *b, int n, double2 m11, double2 m12,
     b[i] = cadd(cmul(m21, u), cmul(m22, v));
 }
 
-// initializeEnsembles (wigner_kernel.cu:295-317) for one trajectory, x-space.
-__global__ void k_init(double2 *a, double2 *b, const double2 *gs, const double2 *na, const double2 *nb, GeomD g,
-                       uint32_t traj)
+// initializeEnsembles (wigner_kernel.cu:295-317), x-space, every trajectory
+__global__ void k_init(double2 *a, double2 *b, const double2 *gs, const double2 *noise, GeomD g, int ne)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.cells) return;
     const double coeff = 1.0 / sqrt(g.dV);
-    double2 ea, eb;
-    if (na) {
-        ea = na[i];
-        eb = nb[i];
-    } else {
-        double r[4];
-        normals4<double>(g.seed, traj, 0u, (uint32_t)i, RNG_TAG_INIT, r);
-        ea = make_double2(0.5 * r[0], 0.5 * r[1]);
-        eb = make_double2(0.5 * r[2], 0.5 * r[3]);
+    const size_t n = (size_t)ne * g.cells;
+    for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (size_t)gridDim.x * blockDim.x) {
+        const int i = (int)(j & (size_t)(g.cells - 1));
+        const size_t t = j >> (g.lx + g.ly + g.lz);
+        double2 ea, eb;
+        if (noise) {
+            ea = noise[j + t * g.cells];
+            eb = noise[j + (t + 1) * g.cells];
+        } else {
+            double r[4];
+            normals4<double>(g.seed, (uint32_t)t, 0u, (uint32_t)i, RNG_TAG_INIT, r);
+            ea = make_double2(0.5 * r[0], 0.5 * r[1]);
+            eb = make_double2(0.5 * r[2], 0.5 * r[3]);
+        }
+        a[j] = cadd(gs[i], cscale(cscale(ea, g.Va), coeff));
+        b[j] = cscale(cscale(eb, g.Vb), coeff);
     }
-    a[i] = cadd(gs[i], cscale(cscale(ea, g.Va), coeff));
-    b[i] = cscale(cscale(eb, g.Vb), coeff);
 }
 
 // per-z sums of one x-space trajectory, one block per z plane
@@ -377,10 +379,10 @@ void plain_pulse(double2 *a, double2 *b, int n, double2 m11, double2 m12, double
     g_launches++;
 }
 
-void plain_init(double2 *a, double2 *b, const double2 *gs, const double2 *noise_a, const double2 *noise_b,
-                const GeomD &g, uint32_t traj, cudaStream_t s)
+void plain_init(double2 *a, double2 *b, const double2 *gs, const double2 *noise, const GeomD &g, int ne, cudaStream_t s)
 {
-    k_init<<<nblk(g.cells), 256, 0, s>>>(a, b, gs, noise_a, noise_b, g, traj);
+    const size_t blocks = ((size_t)ne * g.cells + 255) / 256;
+    k_init<<<(unsigned)(blocks < 65536 ? blocks : 65536), 256, 0, s>>>(a, b, gs, noise, g, ne);
     g_launches++;
 }
 

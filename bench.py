@@ -489,7 +489,7 @@ def main():
     extras = {}
     cpu = None
     if rank == 0 and ws == 1 and not args.no_extras:
-        # plain per-trajectory FP64 path on a sample with the batch's grid mix
+        # the FP64 path on a sample with the batch's grid mix (per ensemble: here one trajectory each)
         sample = mix_sample(groups, 24)
         plain = Engine(sample, path=BEC_PATH_FP64_PLAIN)
         for g, d in enumerate(plain.derived):

@@ -44,8 +44,10 @@ typedef enum bec_status {
 
 /* Execution paths. */
 enum {
-    /* One trajectory at a time, one kernel per operation, FP64 throughout:
-     * structured like the reference's propagate() (wigner.cu:178-199). */
+    /* FP64 throughout (the reference's propagate(), wigner.cu:178-199), one
+     * ensemble at a time: all its trajectories in two fused passes a step, or
+     * one kernel per operation and trajectory where a plane of both components
+     * does not fit in shared memory. */
     BEC_PATH_FP64_PLAIN = 0,
     /* All trajectories of all groups in fused FP32 passes with FP64
      * compensated reductions; the product path. */
