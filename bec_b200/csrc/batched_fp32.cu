@@ -281,10 +281,10 @@ __global__ void __launch_bounds__(256) k_unprep(const Cell *__restrict__ state, 
     }
 }
 
-// the plane pass of a step; done != NULL: the last CTA advances the step index (fused_passes.cu)
+// the plane pass of a step
 __global__ void __launch_bounds__(256) k_plane_any(Cell *__restrict__ state, PlaneTile T, const GroupParamsF *__restrict__ gp,
                                                    const int *__restrict__ tgroup, const int *__restrict__ tlocal,
-                                                   uint32_t *stepp, int *done)
+                                                   const StepRef sr)
 {
     extern __shared__ Cell smw[];
     const int lplane = T.lx + T.ly, lchunk = T.lppc + lplane, lcells = lplane + T.lz;
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(256) k_plane_any(Cell *__restrict__ state, Pla
     wait_predecessor();
     allow_successor();
     for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) copy16(smw + T.reversed(i), state + first + i);
-    const uint32_t step = *stepp;                 // Philox step index (device scalar, see fp32_put_step)
+    const uint32_t step = *sr.step + sr.off;                 // Philox step index (device scalar, see fp32_put_step)
     const uint64_t seed = ((uint64_t)P.seed_hi << 32) | P.seed_lo;
     const float hdt = P.dt * 0.5f;
     copy_wait();
@@ -347,16 +347,7 @@ __global__ void __launch_bounds__(256) k_plane_any(Cell *__restrict__ state, Pla
     __syncthreads();
     T.inverse(smw);
     for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) state[first + i] = smw[T.reversed(i)];
-    if (done) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
-                *done = 0;
-                atomicAdd(stepp, 1u);
-            }
-        }
-    }
+    advance_step(sr);
 }
 
 // ---------------------------------------------------------------- z pass
@@ -609,32 +600,26 @@ void fp32_unprep(const float4 *state, const ClassGeom &c, float4 *x, const float
     g_launches++;
 }
 
-int fp32_ppass_ctas(const ClassGeom &c) { return plane_ctas(c, plane_tile(c, nullptr, nullptr)); }
-
 void fp32_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                const float2 *tx, const float2 *ty, uint32_t *d_step, int *inc_done, cudaStream_t s)
+                const float2 *tx, const float2 *ty, const StepRef &sr, cudaStream_t s)
 {
     if (c.n_traj <= 0) return;
     const PlaneTile T = plane_tile(c, tx, ty);
     ensure_smem_limit((const void *)k_plane_any, kMaxPlaneBytes);
     launch_after(k_plane_any, plane_ctas(c, T), tile_threads(T.lppc + c.lx + c.ly), plane_bytes(T), s,
-                 reinterpret_cast<Cell *>(state), T, gp, tgroup, tlocal, d_step, inc_done);
+                 reinterpret_cast<Cell *>(state), T, gp, tgroup, tlocal, sr);
 }
 
 namespace {
-__global__ void k_put_step(uint32_t *d, uint32_t v) { *d = v; }
-__global__ void k_inc_step(uint32_t *d) { *d += 1u; }
+__global__ void k_put_step(uint32_t *d, int n, uint32_t v)
+{
+    for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = v;
+}
 } // namespace
 
-void fp32_put_step(uint32_t *d_step, uint32_t v, cudaStream_t s)
+void fp32_put_step(uint32_t *d_step, int n, uint32_t v, cudaStream_t s)
 {
-    k_put_step<<<1, 1, 0, s>>>(d_step, v);
-    g_launches++;
-}
-
-void fp32_inc_step(uint32_t *d_step, cudaStream_t s)
-{
-    k_inc_step<<<1, 1, 0, s>>>(d_step);
+    k_put_step<<<1, 32, 0, s>>>(d_step, n, v);
     g_launches++;
 }
 

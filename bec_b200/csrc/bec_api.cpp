@@ -89,7 +89,11 @@ struct bec_ctx {
     std::map<int, float2 *> tw32_full;
     std::map<int, float2 *> tw32_nearest;
     bool use_fast = true;                // register-resident passes where the shape allows
-    uint32_t *d_step = nullptr;          // batched: Philox step index the plane passes read
+    uint32_t *d_step = nullptr;          // batched: Philox step index the plane passes read; one per class of a captured stretch
+    int *d_done = nullptr;               // ... CTAs finished in the plane launch that advances it
+    int n_steps_dev = 0;                 // ... of them
+    std::vector<cudaStream_t> side;      // streams on which a captured stretch forks
+    cudaEvent_t ev_chain = nullptr;
     bool use_graphs = true;              // batched: steady steps replay captured CUDA graphs
     bool graphs_failed = false;
     StepPlan plan;                       // batched: the fused step of the register-path classes
@@ -98,11 +102,11 @@ struct bec_ctx {
     int plane_occupancy = 0;             // per-pass plane launches: 0 = 16 warps per SM, 1 = 20
     bool pencil_tuned = false;           // per-pass pencil launches: each class's own pencil kernel (pencil_kind)
     bool step_onchip = false;            // the step being launched is steady: classes with `onchip` take one launch
-    int *d_pflags = nullptr;             // batched: [0] error flag of the TMA pencil pass, [1] a flag nothing sets,
-                                         // [2] CTAs finished in the plane launch that advances the step index
+    int *d_pflags = nullptr;             // batched: [0] error flag of the TMA pencil pass, [1] a flag nothing sets
     std::string plan_desc;               // the chosen plan and the autotuner's timings (JSON)
-    cudaGraphExec_t step_graph[2] = {nullptr, nullptr};   // kGraphSteps steps, 1 step
-    long long graph_kernels[2] = {0, 0};                  // kernels per replay of each
+    cudaGraphExec_t step_graph[3] = {nullptr, nullptr, nullptr};   // kGraphSteps steps, 1 step, kLongSteps
+    long long graph_kernels[3] = {0, 0, 0};               // kernels per replay of each
+    bool long_failed = false;            // the kLongSteps graph could not be captured
     GroupParamsF *d_gparams = nullptr;
     const void **d_gs_ptrs = nullptr;   // batched: device ground-state pointer of every group (bec_init_groups)
     std::vector<const void *> gs_ptrs_host;   // the table last copied to d_gs_ptrs
@@ -428,6 +432,34 @@ bool split_plane_now(const bec_ctx *ctx, const ClassRec &c)
     return ctx->use_fast && ctx->pencil_tuned && c.split_plane && fp32_plane_split_supported(c.geom);
 }
 
+// the z pass of one class
+bec_status zpass_class(bec_ctx *ctx, ClassRec &c, float frac, bool observe, bool ends_step, const float2 *mf, cudaStream_t s)
+{
+    if (onchip_now(ctx, c)) return BEC_OK;          // its plane-pass slot runs the whole step
+    const int half = frac == 1.0f ? 1 : 0;          // the tables' index of this kick fraction
+    const float scale = (float)(1.0 / (double)c.geom.cells), out_scale = ends_step ? (float)(c.geom.nx * c.geom.ny) : 1.0f;
+    double *obs = observe ? c.obs_partial : nullptr;
+    float2 *tw;
+    bec_status st;
+    if ((st = get_tw32_full(ctx, c.geom.nz, &tw))) return st;
+    if (ctx->use_fast && fp32_fast_pencil_supported(c.geom)) {
+        const float2 *kin = frac == 0.0f ? nullptr : c.kin_tab[half];
+        const int kind = !observe && ctx->pencil_tuned ? c.pencil_kind : kPencilRegister;
+        if (!observe && ctx->pencil_tuned && c.split_pencil)
+            fp32_pencil_split(c.state, c.geom, tw, scale * out_scale, mf, kin, s);
+        else if (kind == kPencilTma && fp32_pencil_tma_supported(c.geom))
+            CKC(fp32_pencil_tma(c.state, c.geom, tw, frac, scale * out_scale, mf, kin, ctx->d_pflags, ctx->d_pflags + 1, s));
+        else
+            fp32_pencil_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, tw, frac, scale * out_scale, mf, obs, out_scale, kin, s);
+        if (observe) c.obs_tiles = fp32_fast_pencil_tiles(c.geom);
+    } else {
+        fp32_zpass(c.state, c.geom, ctx->d_gparams, c.d_tgroup, tw, c.kick_tab[half], c.d_tindex, frac, scale, out_scale, mf, obs, s);
+        if (observe) c.obs_tiles = c.tiles;
+    }
+    CKL();
+    return BEC_OK;
+}
+
 // frac: the kick in units of dt (0, 0.5 or 1)
 // ends_step: no plane pass follows, so the pass leaves the state in the form a z pass reads; observing passes end a step
 // ev (optional): per class (start, stop) events recorded around that class's launch
@@ -441,105 +473,59 @@ bec_status batched_zpass_all(bec_ctx *ctx, float frac, bool observe, bool ends_s
         for (int i = 0; i < 4; ++i) m[i] = make_float2((float)ctx->pulse[i].x, (float)ctx->pulse[i].y);
         mf = m;
     }
-    const int half = frac == 1.0f ? 1 : 0;              // the tables' index of this kick fraction
     for (auto &c : ctx->classes) {
         if (c.geom.n_traj == 0) continue;
-        if (skip_fused && ctx->fused[&c - &ctx->classes[0]]) continue;
-        if (onchip_now(ctx, c)) continue;           // its plane-pass slot runs the whole step
-        bec_status st;
-        const float scale = (float)(1.0 / (double)c.geom.cells), out_scale = ends_step ? (float)(c.geom.nx * c.geom.ny) : 1.0f;
         const size_t ci = &c - &ctx->classes[0];
-        double *obs = observe ? c.obs_partial : nullptr;
-        float2 *tw;
-        if ((st = get_tw32_full(ctx, c.geom.nz, &tw))) return st;
+        if (skip_fused && ctx->fused[ci]) continue;
+        bec_status st;
         if (ev) CKC(cudaEventRecord(ev[ci].first, ctx->stream));
-        if (ctx->use_fast && fp32_fast_pencil_supported(c.geom)) {
-            const float2 *kin = frac == 0.0f ? nullptr : c.kin_tab[half];
-            const int kind = !observe && ctx->pencil_tuned ? c.pencil_kind : kPencilRegister;
-            if (!observe && ctx->pencil_tuned && c.split_pencil)
-                fp32_pencil_split(c.state, c.geom, tw, scale * out_scale, mf, kin, ctx->stream);
-            else if (kind == kPencilTma && fp32_pencil_tma_supported(c.geom))
-                CKC(fp32_pencil_tma(c.state, c.geom, tw, frac, scale * out_scale, mf, kin, ctx->d_pflags, ctx->d_pflags + 1,
-                                    ctx->stream));
-            else
-                fp32_pencil_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, tw, frac, scale * out_scale, mf, obs, out_scale,
-                                 kin, ctx->stream);
-            if (observe) c.obs_tiles = fp32_fast_pencil_tiles(c.geom);
-        } else {
-            fp32_zpass(c.state, c.geom, ctx->d_gparams, c.d_tgroup, tw, c.kick_tab[half], c.d_tindex, frac, scale, out_scale,
-                       mf, obs, ctx->stream);
-            if (observe) c.obs_tiles = c.tiles;
-        }
+        if ((st = zpass_class(ctx, c, frac, observe, ends_step, mf, ctx->stream))) return st;
         if (ev) CKC(cudaEventRecord(ev[ci].second, ctx->stream));
-        CKL();
     }
     ctx->has_pulse = false;
     return BEC_OK;
 }
 
-// put_step: write ctx->step into the device step scalar first (eager launches; a captured step graph
-// leaves it to the step before); skip_fused: leave out the classes of the fused step plan. advanced != NULL:
-// the step index is advanced in the same pass where a class can carry it -- the plane launch
-// with the fewest CTAs (at most kMaxCarrierCtas, one atomic each) runs last and its last CTA increments the
-// index -- and *advanced tells the caller whether that happened.
-constexpr int kMaxCarrierCtas = 16384;
 constexpr size_t kPlainScratch = (size_t)1 << 21;       // cells of each x-space copy of the FP64 path, at most
 constexpr size_t kKickTableBytes = (size_t)256 << 20;   // phase tables of a class of the general z pass, at most
 
+// the plane pass of one class; for a class whose steady step is one on-chip launch, that step
+bec_status ppass_class(bec_ctx *ctx, const ClassRec &c, const StepRef &sr, cudaStream_t s)
+{
+    bec_status st;
+    if (onchip_now(ctx, c)) {
+        float2 *twf;
+        if ((st = get_tw32_full(ctx, c.geom.nz, &twf))) return st;
+        fp32_onchip_step(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, twf, c.kin_tab[1], sr, s);
+    } else if (split_plane_now(ctx, c)) {
+        fp32_plane_split(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, sr, s);
+    } else if (ctx->use_fast && fp32_fast_plane_supported(c.geom)) {
+        fp32_plane_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, sr, ctx->plane_occupancy, s);
+    } else {
+        float2 *tx, *ty;
+        if ((st = get_tw32_full(ctx, c.geom.nx, &tx))) return st;
+        if ((st = get_tw32_full(ctx, c.geom.ny, &ty))) return st;
+        fp32_ppass(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, tx, ty, sr, s);
+    }
+    CKL();
+    return BEC_OK;
+}
+
+// put_step: write ctx->step into the device step index first; skip_fused: leave out the classes of the fused step plan
 bec_status batched_ppass_all(bec_ctx *ctx, std::pair<cudaEvent_t, cudaEvent_t> *ev = nullptr, bool put_step = true,
-                             bool skip_fused = false, bool *advanced = nullptr)
+                             bool skip_fused = false)
 {
     if (put_step) {
-        fp32_put_step(ctx->d_step, (uint32_t)ctx->step, ctx->stream);
+        fp32_put_step(ctx->d_step, 1, (uint32_t)ctx->step, ctx->stream);
         CKL();
     }
-    const int nc = (int)ctx->classes.size();
-    auto launched = [&](int ci) {
+    for (size_t ci = 0; ci < ctx->classes.size(); ++ci) {
         const ClassRec &c = ctx->classes[ci];
-        return c.geom.n_traj > 0 && !(skip_fused && ctx->fused[ci]);
-    };
-    auto onchip = [&](int ci) { return onchip_now(ctx, ctx->classes[ci]); };
-    auto fast = [&](int ci) { return onchip(ci) || (ctx->use_fast && fp32_fast_plane_supported(ctx->classes[ci].geom)); };
-    auto split = [&](int ci) { return split_plane_now(ctx, ctx->classes[ci]); };
-    auto ctas = [&](int ci) {
-        const ClassGeom &g = ctx->classes[ci].geom;
-        return onchip(ci) ? g.n_traj : split(ci) ? fp32_plane_split_ctas(g) : fast(ci) ? fp32_plane_fast_ctas(g) : fp32_ppass_ctas(g);
-    };
-    int carrier = -1;
-    if (advanced) {
-        for (int ci = 0; ci < nc; ++ci)
-            if (launched(ci) && ctas(ci) <= kMaxCarrierCtas && (carrier < 0 || ctas(ci) < ctas(carrier)))
-                carrier = ci;
-        *advanced = carrier >= 0;
-    }
-    for (int k = 0; k < nc; ++k) {
-        // the carrier, if any, goes last
-        const int ci = carrier < 0 ? k : (k < carrier ? k : k + 1 < nc ? k + 1 : carrier);
-        if (!launched(ci)) continue;
-        ClassRec &c = ctx->classes[ci];
+        if (c.geom.n_traj == 0 || (skip_fused && ctx->fused[ci])) continue;
+        bec_status st;
         if (ev) CKC(cudaEventRecord(ev[ci].first, ctx->stream));
-        if (onchip(ci)) {
-            float2 *twf;
-            bec_status st;
-            if ((st = get_tw32_full(ctx, c.geom.nz, &twf))) return st;
-            fp32_onchip_step(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, twf, c.kin_tab[1], ctx->d_step,
-                             ci == carrier ? ctx->d_pflags + 2 : nullptr, ctx->stream);
-        } else if (split(ci)) {
-            fp32_plane_split(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, ctx->d_step,
-                             ci == carrier ? ctx->d_pflags + 2 : nullptr, ctx->stream);
-        } else if (fast(ci)) {
-            fp32_plane_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, ctx->d_step, ctx->plane_occupancy,
-                            ci == carrier ? ctx->d_pflags + 2 : nullptr, ctx->stream);
-        } else {
-            float2 *tx, *ty;
-            bec_status st;
-            if ((st = get_tw32_full(ctx, c.geom.nx, &tx))) return st;
-            if ((st = get_tw32_full(ctx, c.geom.ny, &ty))) return st;
-            fp32_ppass(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, tx, ty, ctx->d_step,
-                       ci == carrier ? ctx->d_pflags + 2 : nullptr, ctx->stream);
-        }
+        if ((st = ppass_class(ctx, c, StepRef{ctx->d_step}, ctx->stream))) return st;
         if (ev) CKC(cudaEventRecord(ev[ci].second, ctx->stream));
-        CKL();
     }
     return BEC_OK;
 }
@@ -547,13 +533,12 @@ bec_status batched_ppass_all(bec_ctx *ctx, std::pair<cudaEvent_t, cudaEvent_t> *
 // One split step of every class, ending with its plane pass: kick fraction pre of dt before this step's half
 // kick (0.5 while the previous step's second half kick is pending), then any pending pulse. The classes of
 // the fused plan run as one launch of the fused step kernel, which advances the device step index; the
-// others launch their own passes, and without a fused plan the smallest plane launch advances it (or, when
-// no class can carry it, a one-thread launch). put_step writes
-// the host step index to the device first (eager steps); a captured step graph leaves it to the step before.
+// others launch their own passes. put_step writes the host step index to the device first (eager steps); the captured
+// steps of a fused plan leave it to the step before.
 bec_status batched_step(bec_ctx *ctx, float pre, bool put_step)
 {
     if (put_step) {
-        fp32_put_step(ctx->d_step, (uint32_t)ctx->step, ctx->stream);
+        fp32_put_step(ctx->d_step, 1, (uint32_t)ctx->step, ctx->stream);
         CKL();
     }
     const bool fused = ctx->plan.ready;
@@ -566,10 +551,8 @@ bec_status batched_step(bec_ctx *ctx, float pre, bool put_step)
     ctx->step_onchip = !fused && pre == 0.5f && !has_m;
     struct Clear { bool &f; ~Clear() { f = false; } } clear{ctx->step_onchip};
     if ((st = batched_zpass_all(ctx, pre + 0.5f, false, false, nullptr, fused))) return st;
-    bool advanced = false;
-    if ((st = batched_ppass_all(ctx, nullptr, false, fused, fused ? nullptr : &advanced))) return st;
+    if ((st = batched_ppass_all(ctx, nullptr, false, fused))) return st;
     if (fused) step_launch(ctx->plan, ctx->d_gparams, ctx->d_step, pre + 0.5f, has_m ? mf : nullptr, ctx->stream);
-    else if (!advanced) fp32_inc_step(ctx->d_step, ctx->stream);
     CKL();
     return BEC_OK;
 }
@@ -596,12 +579,33 @@ std::string candidate_name(int c)
     return std::string("fused ") + step_plan_name(c - kPerPassCandidates);
 }
 
+// A steady step (the previous step's second half-kick pending, no pulse, no observation) launches the
+// same kernels with the same arguments every time: the full kick in the pencil passes, and the plane passes.
+// kGraphSteps of them, and one, are captured once per context and replayed. A context of short steps (kSplitCells cells
+// at most) that is asked for kLongSteps of them also captures as many: what lies between two replays is 2 to 3 us
+// (a 32x128 slice: 5.38 us a step with 8 steps a graph, 5.00 with 32; four 16x16x128 trajectories 8.96 and 8.58; 64 of
+// them 40.9 and 40.7).
+//
+// Without a fused step kernel no class waits for another: each is a chain of launches with a step index of its own, which
+// its last plane launch advances by the stretch. A context of up to kForkCells cells captures the chains side by side, on
+// streams of their own, which fills the chip where one class does not (ten ensembles of five trajectories on five small
+// grids: 69 us a step one chain after another, 38 side by side; 64 trajectories each of 8x8x64, 16x16x128 and 32x32x256,
+// 19M cells: 388 and 380). Beyond it they run one after another: passes of different classes that share the SMs are
+// slower than in turn (twice as many trajectories: 760 us in turn, 798 side by side; the uneven batch of 1024: 2087, 2234).
+constexpr int kGraphSteps = 8, kLongSteps = 32;
+constexpr long long kForkCells = 1 << 24;
+constexpr int kSideStreams = 7;
+
+long long total_cells(const bec_ctx *ctx)
+{
+    long long n = 0;
+    for (auto &c : ctx->classes) n += (long long)c.geom.n_traj * c.geom.cells;
+    return n;
+}
+
+bec_status capture_steps(bec_ctx *ctx, int k, cudaGraphExec_t *out, long long *kernels);
 bec_status check_step_error(bec_ctx *ctx);
 
-// Per grid class, the faster of the two pencil kernels for the full-kick pass of a steady step: the register
-// kernel (16 pencils per CTA of nz threads, 16 warps per SM) or the persistent TMA kernel (three CTAs per SM,
-// the next tile's load in flight). Both compute the same bits; each is timed over three launches after one
-// warm-up on the current state (the caller restores it).
 // ms of what enqueue() launches, replayed from a captured graph; left alone (-1) when it cannot be captured
 template <class F>
 bec_status time_captured(bec_ctx *ctx, double *ms, F &&enqueue)
@@ -635,6 +639,10 @@ bec_status time_captured(bec_ctx *ctx, double *ms, F &&enqueue)
 // trajectories of 16x16x128: 42.2 us a step against 43.3; 32: 26.2 against 25.4).
 constexpr long long kSplitCells = 1 << 21;
 
+// Per grid class, the faster of the two pencil kernels for the full-kick pass of a steady step: the register
+// kernel (16 pencils per CTA of nz threads, 16 warps per SM) or the persistent TMA kernel (three CTAs per SM,
+// the next tile's load in flight). Both compute the same bits; each is timed over three launches after one
+// warm-up on the current state (the caller restores it).
 bec_status pick_pencil_kernels(bec_ctx *ctx)
 {
     for (auto &c : ctx->classes) {
@@ -693,10 +701,10 @@ bec_status pick_pencil_kernels(bec_ctx *ctx)
         const bool fast_plane = fp32_fast_plane_supported(c.geom), split_plane = fp32_plane_split_supported(c.geom);
         auto plane = [&](bool split) {
             if (split)
-                fp32_plane_split(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, ctx->d_step, nullptr, ctx->stream);
+                fp32_plane_split(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, StepRef{ctx->d_step}, ctx->stream);
             else if (fast_plane)
-                fp32_plane_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, ctx->d_step, ctx->plane_occupancy,
-                                nullptr, ctx->stream);
+                fp32_plane_fast(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, StepRef{ctx->d_step}, ctx->plane_occupancy,
+                                ctx->stream);
         };
         if (fast_plane && (st = time_launch(&c.plane_ms, [&] { plane(false); }))) return st;
         // a small class: the two launches of a step with four cells per thread in either, both or none, timed as a captured
@@ -715,8 +723,8 @@ bec_status pick_pencil_kernels(bec_ctx *ctx)
         // an 8x8x64 class: its steady step as one on-chip launch against its faster pencil launch plus its plane launch
         if (fp32_onchip_supported(c.geom)) {
             if ((st = time_launch(&c.onchip_ms, [&] {
-                     fp32_onchip_step(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, twf, c.kin_tab[1], ctx->d_step,
-                                      nullptr, ctx->stream);
+                     fp32_onchip_step(c.state, c.geom, ctx->d_gparams, c.d_tgroup, c.d_tlocal, twf, c.kin_tab[1],
+                                      StepRef{ctx->d_step}, ctx->stream);
                  })))
                 return st;
             c.onchip = c.onchip_ms < pencil_ms + c.plane_ms;
@@ -837,11 +845,25 @@ bec_status ensure_plan(bec_ctx *ctx)
                 double best = 1e30;
                 for (int k = 0; k < n_cand && st == BEC_OK; ++k) {
                     if ((st = apply(k))) break;
-                    const int reps = best < 0.2 ? 20 : 3;          // short steps need more of them
-                    for (int r = 0; r <= reps && st == BEC_OK; ++r) {
-                        if (r == 1) cudaEventRecord(ctx->ev0, ctx->stream);
-                        st = batched_step(ctx, 0.5f, true);
+                    // a context whose captured steps run side by side is timed on them
+                    cudaGraphExec_t exec = nullptr;
+                    long long kernels = 0;
+                    int reps = best < 0.2 ? 20 : 3;                // short steps need more of them
+                    const bool forked = total_cells(ctx) <= kForkCells;
+                    if (forked && (st = batched_step(ctx, 0.5f, true))) break;   // (its tables exist before a capture)
+                    if (forked && capture_steps(ctx, kGraphSteps, &exec, &kernels) == BEC_OK) {
+                        reps = 2 * kGraphSteps;
+                        for (int r = 0; r < 3; ++r) {
+                            if (r == 1) cudaEventRecord(ctx->ev0, ctx->stream);
+                            if (cudaGraphLaunch(exec, ctx->stream) != cudaSuccess) st = fail(ctx, BEC_ERR_CUDA, "step timing");
+                        }
+                    } else {
+                        for (int r = 0; r <= reps && st == BEC_OK; ++r) {
+                            if (r == 1) cudaEventRecord(ctx->ev0, ctx->stream);
+                            st = batched_step(ctx, 0.5f, true);
+                        }
                     }
+                    struct Drop { cudaGraphExec_t e; ~Drop() { if (e) cudaGraphExecDestroy(e); } } drop{exec};
                     if (st) break;
                     cudaEventRecord(ctx->ev1, ctx->stream);
                     if (cudaEventSynchronize(ctx->ev1) != cudaSuccess) {
@@ -984,25 +1006,55 @@ bec_status check_step_error(bec_ctx *ctx)
 }
 
 // ---------------------------------------------------------------- captured step loop
-// A steady step (the previous step's second half-kick pending, no pulse, no observation) launches the
-// same kernels with the same arguments every time: the full kick in the pencil passes, the plane passes
-// (the step scalar advanced by the last CTA of the smallest one, or of the fused kernel, or by a one-thread
-// launch). kGraphSteps of them, and one, are captured once per context and replayed; the device step
-// scalar is set once before a stretch of replays.
-constexpr int kGraphSteps = 8;
+// k steady steps of every class, on the context's stream and the side streams
+bec_status capture_chains(bec_ctx *ctx, int k)
+{
+    ctx->step_onchip = true;
+    struct Clear { bool &f; ~Clear() { f = false; } } clear{ctx->step_onchip};
+    const int lanes = 1 + (int)ctx->side.size();
+    CKC(cudaEventRecord(ctx->ev_chain, ctx->stream));
+    for (cudaStream_t s : ctx->side) CKC(cudaStreamWaitEvent(s, ctx->ev_chain, 0));
+    bec_status st = BEC_OK;
+    int chain = 0;
+    for (size_t ci = 0; ci < ctx->classes.size() && !st; ++ci) {
+        ClassRec &c = ctx->classes[ci];
+        if (c.geom.n_traj == 0) continue;
+        const int lane = chain++ % lanes;
+        cudaStream_t s = lane ? ctx->side[lane - 1] : ctx->stream;
+        for (int i = 0; i < k && !st; ++i) {
+            StepRef sr{ctx->d_step + ci, (uint32_t)i};
+            if (i == k - 1) { sr.done = ctx->d_done + ci; sr.inc = (uint32_t)k; }
+            if (!(st = zpass_class(ctx, c, 1.0f, false, false, nullptr, s))) st = ppass_class(ctx, c, sr, s);
+        }
+    }
+    for (cudaStream_t s : ctx->side) {
+        CKC(cudaEventRecord(ctx->ev_chain, s));
+        CKC(cudaStreamWaitEvent(ctx->stream, ctx->ev_chain, 0));
+    }
+    return st;
+}
 
 bec_status capture_steps(bec_ctx *ctx, int k, cudaGraphExec_t *out, long long *kernels)
 {
     const long long l0 = g_launches;
     cudaGraph_t graph = nullptr;
+    if (!ctx->plan.ready && total_cells(ctx) <= kForkCells) {
+        int chains = 0;
+        for (auto &c : ctx->classes) chains += c.geom.n_traj > 0;
+        while ((int)ctx->side.size() < std::min(kSideStreams, chains - 1)) {
+            cudaStream_t s;
+            CKC(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+            ctx->side.push_back(s);
+        }
+    }
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
         return BEC_ERR_CUDA;
     }
     bec_status st = BEC_OK;
-    for (int i = 0; i < k && st == BEC_OK; ++i) {
-        st = batched_step(ctx, 0.5f, false);
-    }
+    if (!ctx->plan.ready) st = capture_chains(ctx, k);
+    else
+        for (int i = 0; i < k && st == BEC_OK; ++i) st = batched_step(ctx, 0.5f, false);
     const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
     *kernels = g_launches - l0;
     g_launches = l0;                    // captured, not launched
@@ -1043,15 +1095,17 @@ bec_status run_steady(bec_ctx *ctx, long long m)
         }
         return BEC_OK;
     }
-    fp32_put_step(ctx->d_step, (uint32_t)ctx->step, ctx->stream);   // each replayed step advances it at its end
+    fp32_put_step(ctx->d_step, ctx->n_steps_dev, (uint32_t)ctx->step, ctx->stream);   // each replayed stretch advances them
     CKL();
-    for (long long i = 0; i < m / kGraphSteps; ++i) {
-        CKC(cudaGraphLaunch(ctx->step_graph[0], ctx->stream));
-        g_launches += ctx->graph_kernels[0];
-    }
-    for (long long i = 0; i < m % kGraphSteps; ++i) {
-        CKC(cudaGraphLaunch(ctx->step_graph[1], ctx->stream));
-        g_launches += ctx->graph_kernels[1];
+    if (m >= kLongSteps && !ctx->step_graph[2] && !ctx->long_failed && total_cells(ctx) <= kSplitCells)
+        ctx->long_failed = capture_steps(ctx, kLongSteps, &ctx->step_graph[2], &ctx->graph_kernels[2]) != BEC_OK;
+    long long left = m;
+    for (const int g : {2, 0, 1}) {
+        const int len = g == 2 ? kLongSteps : g == 0 ? kGraphSteps : 1;
+        for (; ctx->step_graph[g] && left >= len; left -= len) {
+            CKC(cudaGraphLaunch(ctx->step_graph[g], ctx->stream));
+            g_launches += ctx->graph_kernels[g];
+        }
     }
     ctx->step += m;
     ctx->evo_steps += m;
@@ -1281,7 +1335,8 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
     auto bail = [&](bec_status s) { bec_destroy(ctx); return s; };
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(BEC_ERR_CUDA);
     if (cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->ev_h2d, cudaEventDisableTiming) != cudaSuccess)
+        cudaEventCreateWithFlags(&ctx->ev_h2d, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_chain, cudaEventDisableTiming) != cudaSuccess)
         return bail(BEC_ERR_CUDA);
 
     // trajectory numbering: classes in first-appearance order, groups in order within a class
@@ -1383,7 +1438,10 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
         for (int g = 0; g < ng; ++g) gfs[g] = ctx->groups[g].gf;
         CKA(dalloc(ctx, &ctx->d_gparams, (size_t)ng));
         CKA(cudaMemcpyAsync(ctx->d_gparams, gfs.data(), sizeof(GroupParamsF) * ng, cudaMemcpyHostToDevice, ctx->stream));
-        CKA(dalloc(ctx, &ctx->d_step, (size_t)1));
+        ctx->n_steps_dev = (int)ctx->classes.size();
+        CKA(dalloc(ctx, &ctx->d_step, (size_t)ctx->n_steps_dev));
+        CKA(dalloc(ctx, &ctx->d_done, (size_t)ctx->n_steps_dev));
+        CKA(cudaMemsetAsync(ctx->d_done, 0, ctx->n_steps_dev * sizeof(int), ctx->stream));
         CKA(dalloc(ctx, &ctx->d_pflags, (size_t)4));
         CKA(cudaMemsetAsync(ctx->d_pflags, 0, 4 * sizeof(int), ctx->stream));
         {
@@ -1469,6 +1527,8 @@ void bec_destroy(bec_ctx *ctx)
         if (gr.gs_dev) { /* owned through allocs */ }
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev_h2d) cudaEventDestroy(ctx->ev_h2d);
+    if (ctx->ev_chain) cudaEventDestroy(ctx->ev_chain);
+    for (cudaStream_t s : ctx->side) cudaStreamDestroy(s);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -2867,7 +2927,7 @@ bec_status bec_profile_fused_step(bec_ctx *ctx, int32_t n_steps, double *ms_per_
     double tot = 0.0;
     long long l0 = g_launches;
     for (int i = 0; i < n_steps; ++i) {
-        fp32_put_step(ctx->d_step, (uint32_t)ctx->step, ctx->stream);
+        fp32_put_step(ctx->d_step, 1, (uint32_t)ctx->step, ctx->stream);
         if ((st = batched_zpass_all(ctx, 1.0f, false, false, nullptr, true))) return st;
         if ((st = batched_ppass_all(ctx, nullptr, false, true))) return st;
         CKC(cudaEventRecord(ctx->ev0, ctx->stream));

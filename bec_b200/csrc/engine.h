@@ -45,6 +45,15 @@ struct ClassGeom {
     int n_traj;
 };
 
+// The Philox step index of a plane launch: *step + off. A captured stretch of steps reads the index that the host wrote
+// before it and counts from there; the plane launch of its last step, given a counter (zero), adds the stretch's length.
+struct StepRef {
+    uint32_t *step = nullptr;
+    uint32_t off = 0;
+    int *done = nullptr;
+    uint32_t inc = 0;
+};
+
 // ----------------------------------------------------------------------------
 // plain_fp64.cu (one trajectory at a time; a, b point at that trajectory)
 void plain_kick(double2 *a, double2 *b, const GeomD &g, double scale, int apply_scale, cudaStream_t s);
@@ -164,15 +173,10 @@ void fp32_kick_table(float2 *tab, const ClassGeom &c, const GroupParamsF *gp, co
 void fp32_zpass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const float2 *tz,
                 const float2 *kick, const int *tindex, float frac, float scale, float out_scale, const float2 *m, double *obs,
                 cudaStream_t s);
-// inc_done as fp32_plane_fast; CTAs of the launch
 void fp32_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                const float2 *tx, const float2 *ty, uint32_t *d_step, int *inc_done, cudaStream_t s);
-int fp32_ppass_ctas(const ClassGeom &c);
-// the plane passes read the Philox step index from a device scalar, so a captured step graph can replay:
-// an eagerly launched step writes it (fp32_put_step); a step advances it at its end (fp32_inc_step, or the
-// last CTA of a plane launch given inc_done, or of the fused step kernel)
-void fp32_put_step(uint32_t *d_step, uint32_t v, cudaStream_t s);
-void fp32_inc_step(uint32_t *d_step, cudaStream_t s);
+                const float2 *tx, const float2 *ty, const StepRef &sr, cudaStream_t s);
+// fills n device step indexes
+void fp32_put_step(uint32_t *d_step, int n, uint32_t v, cudaStream_t s);
 int fp32_zpass_tiles(const ClassGeom &c);   // tiles per trajectory of an observing z pass (obs_partial layout)
 // obs_partial[traj][tile][z][4] -> traj_axial[traj][z][4] * traj_scale[traj] (1 if NULL),
 // traj_tot[traj][4] = sum over z; traj_axial may be NULL
@@ -244,9 +248,7 @@ bool fp32_fast_plane_supported(const ClassGeom &c);
 bool fp32_fast_pencil_supported(const ClassGeom &c);
 // occupancy: 0 = 16 warps per SM, no spill; 1 = 20 warps per SM at 96 registers (an autotuner choice)
 void fp32_plane_fast(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                     uint32_t *d_step, int occupancy, int *inc_done, cudaStream_t s);
-// CTAs of that launch; inc_done != NULL: its last CTA also advances *d_step (inc_done: a zero int counter)
-int fp32_plane_fast_ctas(const ClassGeom &c);
+                     const StepRef &sr, int occupancy, cudaStream_t s);
 // tw_full: nz entries W_nz^e; frac: kick in units of dt; scale: 1/cells times out_scale;
 // m: optional pulse matrix (row-major, 4 entries) or NULL; obs: when not NULL the pass
 // ends a step and writes per-z partial moments [traj][tile][z][4] (tiles = fp32_fast_pencil_tiles)
@@ -262,17 +264,16 @@ void fp32_kin_tables(float2 *tab, const ClassGeom &c, const GroupParamsF *gp, co
 // cells per thread, for classes with too few trajectories to fill the chip; the same bits as fp32_plane_fast and
 // fp32_pencil_fast
 bool fp32_plane_split_supported(const ClassGeom &c);
-int fp32_plane_split_ctas(const ClassGeom &c);
 void fp32_plane_split(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                      uint32_t *d_step, int *inc_done, cudaStream_t s);
+                      const StepRef &sr, cudaStream_t s);
 void fp32_pencil_split(float4 *state, const ClassGeom &c, const float2 *tw_full, float scale, const float2 *m,
                        const float2 *kin, cudaStream_t s);
 // onchip_step.cu: a steady step (full kick, no pulse, no observation) of an 8x8x64 class with each trajectory's
 // state in shared memory, one launch instead of its pencil and plane launches; kin_full: the class's full-kick
-// kinetic table; inc_done as fp32_plane_fast
+// kinetic table
 bool fp32_onchip_supported(const ClassGeom &c);
 void fp32_onchip_step(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                      const float2 *tw_full, const float2 *kin_full, uint32_t *d_step, int *inc_done, cudaStream_t s);
+                      const float2 *tw_full, const float2 *kin_full, const StepRef &sr, cudaStream_t s);
 // pencil_tma.cu: the non-observing pencil pass as a persistent kernel with TMA tile loads and stores
 // (bit-identical to fp32_pencil_fast); d_err: set to 1 when a wait gave up; d_never: a zero int
 bool fp32_pencil_tma_supported(const ClassGeom &c);

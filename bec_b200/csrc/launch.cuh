@@ -1,4 +1,5 @@
-// launch.cuh -- launches whose start overlaps the end of the kernel before them (programmatic dependent launch).
+// launch.cuh -- launches whose start overlaps the end of the kernel before them (programmatic dependent launch), and the
+// step index that a stretch of launches shares.
 //
 // A kernel launched by launch_after() may start while its predecessor in the stream still runs; it sets itself up, then
 // calls wait_predecessor(), which returns once the predecessor has completed and its writes are visible. It then calls
@@ -29,4 +30,19 @@ cudaError_t launch_after(void (*kernel)(Params...), int grid, int block, size_t 
     cfg.numAttrs = 1;
     g_launches++;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+// A plane launch that is given a counter advances its Philox step index once every CTA has read it: the CTA that finishes
+// last (the counter reaches the grid size) resets the counter and adds sr.inc.
+__device__ __forceinline__ void advance_step(const StepRef &sr)
+{
+    if (!sr.done) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(sr.done, 1) == (int)gridDim.x - 1) {
+            *sr.done = 0;
+            atomicAdd(sr.step, sr.inc);
+        }
+    }
 }

@@ -9,6 +9,7 @@
 // the two launches. Steady steps only (full kick, no pulse, no observation); the others take the two-pass
 // route.
 #include "engine.h"
+#include "launch.cuh"
 #include "step_bodies.cuh"
 
 namespace {
@@ -39,14 +40,13 @@ __device__ __forceinline__ void copy_async16(void *dst_smem, const void *src)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
-// done != NULL: the last CTA also advances the Philox step index (every CTA read it at its start)
 __global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(cpair *__restrict__ state,
                                                              const GroupParamsF *__restrict__ gp,
                                                              const int *__restrict__ tgroup,
                                                              const int *__restrict__ tlocal,
                                                              const float2 *__restrict__ tw_g,
                                                              const float2 *__restrict__ kin, float scale,
-                                                             uint32_t *stepp, int *done)
+                                                             const StepRef sr)
 {
     extern __shared__ cpair st[];
     float2 *tw = reinterpret_cast<float2 *>(st + CELLS);
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(cpair *__restrict
     float2 *kxyp = kzp + NZ;
     const int t = threadIdx.x, traj = blockIdx.x;
     cpair *__restrict__ g = state + (size_t)traj * CELLS;
-    const uint32_t step = *stepp;
+    const uint32_t step = *sr.step + sr.off;
 
     // W_64^e, this trajectory's kz and (kx, ky) kinetic factors (full kick), and the state, by asynchronous copies
     const float2 *kt = kin + (size_t)traj * (NZ + PLANE);
@@ -110,17 +110,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(cpair *__restrict
     }
     __syncthreads();
     for (int i = t; i < CELLS; i += kThreads) g[i] = st[i];
-
-    if (done) {
-        __syncthreads();
-        if (t == 0) {
-            __threadfence();
-            if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
-                *done = 0;
-                atomicAdd(stepp, 1u);
-            }
-        }
-    }
+    advance_step(sr);
 }
 
 } // namespace
@@ -128,11 +118,11 @@ __global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(cpair *__restrict
 bool fp32_onchip_supported(const ClassGeom &c) { return c.nx == 8 && c.ny == 8 && c.nz == 64 && c.n_traj > 0; }
 
 void fp32_onchip_step(float4 *cells, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                      const float2 *tw_full, const float2 *kin_full, uint32_t *d_step, int *inc_done, cudaStream_t s)
+                      const float2 *tw_full, const float2 *kin_full, const StepRef &sr, cudaStream_t s)
 {
     if (c.n_traj <= 0) return;
     ensure_smem_limit((const void *)k_onchip_8x8x64, (int)kSmem);
     k_onchip_8x8x64<<<c.n_traj, kThreads, kSmem, s>>>(reinterpret_cast<cpair *>(cells), gp, tgroup, tlocal, tw_full, kin_full,
-                                                       1.0f / (float)c.cells, d_step, inc_done);
+                                                       1.0f / (float)c.cells, sr);
     g_launches++;
 }

@@ -93,7 +93,7 @@ template <int N>
 __global__ void __launch_bounds__(32 * kSplit<N>) k_plane_split(cpair *__restrict__ state, int nz, int cells,
                                                                   const GroupParamsF *__restrict__ gp,
                                                                   const int *__restrict__ tgroup,
-                                                                  const int *__restrict__ tlocal, uint32_t *stepp, int *done)
+                                                                  const int *__restrict__ tlocal, const StepRef sr)
 {
     constexpr int S = kSplit<N>, E = 4, W = 32 / N, PLANE = N * N;
     __shared__ cpair tile[32 * N], ex[2][32 * N];
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(32 * kSplit<N>) k_plane_split(cpair *__restric
     const GroupParamsF P = gp[tgroup[traj]];
     wait_predecessor();
     allow_successor();
-    const uint32_t step = *stepp;
+    const uint32_t step = *sr.step + sr.off;
 
     cpair v[E];
 #pragma unroll
@@ -145,17 +145,7 @@ __global__ void __launch_bounds__(32 * kSplit<N>) k_plane_split(cpair *__restric
     line<N, true, S>(v, ex[1] + lane, 32, q, sync);
 #pragma unroll
     for (int j = 0; j < E; ++j) g[(q + S * j) * N + c] = v[j];
-    if (done) {
-        // the last CTA advances the Philox step index (fused_passes.cu, advance_step_if_last)
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
-                *done = 0;
-                atomicAdd(stepp, 1u);
-            }
-        }
-    }
+    advance_step(sr);
 }
 
 // ---------------------------------------------------------------- pencil pass
@@ -245,10 +235,10 @@ __global__ void __launch_bounds__(PencilSplit<NZ>::THREADS) k_pencil_split(cpair
 
 template <int N>
 void launch_plane(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                  uint32_t *step, int *done, cudaStream_t s)
+                  const StepRef &sr, cudaStream_t s)
 {
     launch_after(k_plane_split<N>, c.n_traj * c.nz / (32 / N), 32 * kSplit<N>, 0, s, reinterpret_cast<cpair *>(state), c.nz,
-                 c.cells, gp, tgroup, tlocal, step, done);
+                 c.cells, gp, tgroup, tlocal, sr);
 }
 
 template <int NZ>
@@ -265,14 +255,13 @@ bool fp32_plane_split_supported(const ClassGeom &c)
 {
     return c.nx == c.ny && (c.nx == 8 || c.nx == 16) && ((long long)c.n_traj * c.nz) % (32 / c.nx) == 0;
 }
-int fp32_plane_split_ctas(const ClassGeom &c) { return c.n_traj * c.nz / (32 / c.nx); }
 
 void fp32_plane_split(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
-                      uint32_t *d_step, int *inc_done, cudaStream_t s)
+                      const StepRef &sr, cudaStream_t s)
 {
     if (c.n_traj <= 0) return;
-    if (c.nx == 8) launch_plane<8>(state, c, gp, tgroup, tlocal, d_step, inc_done, s);
-    else launch_plane<16>(state, c, gp, tgroup, tlocal, d_step, inc_done, s);
+    if (c.nx == 8) launch_plane<8>(state, c, gp, tgroup, tlocal, sr, s);
+    else launch_plane<16>(state, c, gp, tgroup, tlocal, sr, s);
 }
 
 void fp32_pencil_split(float4 *state, const ClassGeom &c, const float2 *tw_full, float scale, const float2 *m,

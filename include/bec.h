@@ -357,7 +357,8 @@ bec_status bec_checkpoint_load(bec_ctx *ctx, const void *buf, int64_t bytes);
 
 /* Batched path: steady steps (no pulse or sample due) replay CUDA graphs captured once per context
  * (8 steps and 1 step; set BEC_CUDA_GRAPHS=0 in the environment before bec_create to launch them one by
- * one instead). Returns the number of step graphs captured and in use (0 or 2). */
+ * one instead); a context of few cells that is asked for 32 steady steps or more replays them 32 at a time.
+ * Returns the number of 8-step and 1-step graphs captured and in use (0 or 2). */
 int32_t bec_step_graphs(const bec_ctx *ctx);
 
 /* Batched path: the schedule of a split step, written to out as a JSON object (len bytes at most,
