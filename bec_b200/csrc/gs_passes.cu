@@ -24,62 +24,67 @@ struct GsArgs {
     float frac1, frac2;       // kick fractions of dt_steady before / after the measurement
     float scale;              // 1/cells (makes the inverse z transform the normalised k-space state)
     float out_scale;          // nx*ny when the pass ends a step, else 1
-    int measure;              // 1: accumulate sum |psi_k|^2 (and the kinetic sum) per trajectory
 };
 
-
 // ---------------------------------------------------------------- pencil pass
-// nz = 256: bounded to 3 CTAs (24 warps) per SM, 80 registers with a 60-byte spill; measured 4 % faster
-// over a batched ground-state loop than 2 CTAs at 99 registers
-template <int NZ>
-__global__ void __launch_bounds__(NZ, (NZ == 256 ? 3 : 1)) k_gs_pencil(float2 *__restrict__ state, int nx, int lx, int ny, int cells,
-                                                  int tiles, const GroupParamsF *__restrict__ gp,
+// 2^LP pencils a trajectory. STEADY: the pass between two steps (two equal kicks, the norm); otherwise the fractions differ
+// and norm and ekin may be null.
+//
+// Both passes are bound by latency at the few warps that a line of 16 or 32 complex values a thread leaves room for (DRAM
+// runs at 30 % of its rate). What counts is registers and instructions: with the shared lines padded by one element instead
+// of swizzled, and the grid's sizes known to the compiler, every shared and global access has an address and a constant
+// offset. The nz = 256 pencil pass then fits four CTAs an SM at 64 registers without a spill (three at 80 with one before),
+// the 32 x 32 plane pass five at 96 (four at 128). A step of 256 states of 32x32x256: 633 us before, 487 here; of 200 of
+// 16x16x128: 67.2 and 50.5; of 16 of 32x32x256: 49.3 and 40.7. (Two warps a plane with 16 values a thread: 532 us.)
+template <int NZ, int LP, bool STEADY>
+__global__ void __launch_bounds__(NZ, 4 * 256 / NZ) k_gs_pencil(float2 *__restrict__ state, const GroupParamsF *__restrict__ gp,
                                                   const GsParamsF *__restrict__ gs, const int *__restrict__ tgroup,
                                                   const float2 *__restrict__ tw_g, GsArgs a,
                                                   double *__restrict__ norm, double *__restrict__ ekin,
                                                   const int *__restrict__ active)
 {
-    constexpr int R = 16, G = NZ / 16;
+    constexpr int R = 16, G = NZ / 16, LX = LP / 2, NX = 1 << LX, PLANE = 1 << LP, TILES = PLANE / 16;
+    constexpr int LD = NZ + 1;                   // of a pencil in the buffer: its 16 first elements on different banks
     extern __shared__ float2 dyn2[];
-    float2 *buf = dyn2;                          // 16 pencils x NZ
-    float2 *tw = buf + 16 * NZ;                  // W_NZ^e
-    float *kz2 = reinterpret_cast<float *>(tw + NZ);   // kz^2/2 per kz
-    float *kxy2 = kz2 + NZ;                      // (kx^2 + ky^2)/2 per pencil
-    float *ez1 = kxy2 + 16, *ez2 = ez1 + NZ;     // exp(-dt frac1,2 kz^2/2) per kz
-    float *exy1 = ez2 + NZ, *exy2 = exy1 + 16;   // exp(-dt frac1,2 (kx^2 + ky^2)/2) x scale, out_scale
+    float2 *buf = dyn2;                          // 16 pencils
+    float2 *tw = buf + 16 * LD;                  // W_NZ^e
+    float *ez1 = reinterpret_cast<float *>(tw + NZ), *exy1 = ez1 + NZ;   // exp(-dt frac1 kz^2/2) per kz, per pencil x scale
+    float *ez2 = exy1 + 16, *exy2 = ez2 + NZ;    // the same for frac2, x out_scale
+    float *kz2 = exy2 + 16, *kxy2 = kz2 + NZ;    // kz^2/2 per kz, (kx^2 + ky^2)/2 per pencil
     __shared__ double red[2][NZ / 32];
 
     const int t = threadIdx.x;
-    const int lt = blockIdx.x / tiles;                   // position in the launch's trajectory list
+    const int lt = blockIdx.x / TILES;                   // position in the launch's trajectory list
     const int traj = active ? active[lt] : lt;
-    const int pen0 = (blockIdx.x - lt * tiles) * 16;
+    const int pen0 = (blockIdx.x - lt * TILES) * 16;
     const int gi = tgroup[traj];
-    const GroupParamsF P = gp[gi];
     const float dts = gs[gi].dt_steady;
-    const int plane = nx * ny;
-
-    for (int i = t; i < NZ; i += blockDim.x) {
-        tw[i] = tw_g[i];
-        const float kz = getk<float>(i, P.dkz, NZ);
-        kz2[i] = 0.5f * kz * kz;
-        ez1[i] = expf(-dts * a.frac1 * kz2[i]);
-        ez2[i] = expf(-dts * a.frac2 * kz2[i]);
-    }
-    if (t < 16) {
-        const int pen = pen0 + t;
-        const int x = pen & (nx - 1), y = pen >> lx;
-        const float kx = getk<float>(x, P.dkx, nx);
-        const float ky = (ny > 1) ? getk<float>(y, P.dky, ny) : 0.0f;
-        kxy2[t] = 0.5f * (kx * kx + ky * ky);
-        exy1[t] = expf(-dts * a.frac1 * kxy2[t]) * a.scale;
-        exy2[t] = expf(-dts * a.frac2 * kxy2[t]) * a.out_scale;
+    {
+        const GroupParamsF &P = gp[gi];
+        tw[t] = tw_g[t];
+        const float kz = getk<float>(t, P.dkz, NZ);
+        const float kz2t = 0.5f * kz * kz;
+        ez1[t] = expf(-dts * a.frac1 * kz2t);
+        if (!STEADY) {
+            kz2[t] = kz2t;
+            ez2[t] = expf(-dts * a.frac2 * kz2t);
+        }
+        if (t < 16) {
+            const int pen = pen0 + t;
+            const float kx = getk<float>(pen & (NX - 1), P.dkx, NX);
+            const float ky = getk<float>(pen >> LX, P.dky, NX);
+            const float kxyt = 0.5f * (kx * kx + ky * ky);
+            kxy2[t] = kxyt;
+            exy1[t] = expf(-dts * a.frac1 * kxyt) * a.scale;
+            exy2[t] = expf(-dts * a.frac2 * kxyt) * a.out_scale;
+        }
     }
 
     const int p = t & 15, j = t >> 4;
-    float2 *__restrict__ g = state + (size_t)traj * cells + pen0 + p;
+    float2 *__restrict__ g = state + ((size_t)traj * (NZ * PLANE) + (size_t)(pen0 + p + j * PLANE));
     float2 x[R];
 #pragma unroll
-    for (int m = 0; m < R; ++m) x[m] = g[(size_t)(j + G * m) * plane];
+    for (int m = 0; m < R; ++m) x[m] = g[G * m * PLANE];
     __syncthreads();
     dft<R, true, false>(x);
 #pragma unroll
@@ -87,44 +92,46 @@ __global__ void __launch_bounds__(NZ, (NZ == 256 ? 3 : 1)) k_gs_pencil(float2 *_
         const float2 w = tw[j * k1];
         x[k1] = fftreg::cmulw(x[k1], make_float2(w.x, -w.y));
     }
+    float2 *b1 = buf + p * LD + j * R;
 #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) buf[(p * G + j) * R + (k1 ^ (p & 15))] = x[k1];
+    for (int k1 = 0; k1 < R; ++k1) b1[k1] = x[k1];
     __syncthreads();
 
     const int q = t % G, p2 = t / G;
+    float2 *b2 = buf + p2 * LD + q;
     float2 y[R];
 #pragma unroll
     for (int r = 0; r < R / G; ++r)
 #pragma unroll
-        for (int jj = 0; jj < G; ++jj) y[r * G + jj] = buf[(p2 * G + jj) * R + ((q + G * r) ^ (p2 & 15))];
+        for (int jj = 0; jj < G; ++jj) y[r * G + jj] = b2[jj * R + G * r];
 #pragma unroll
     for (int r = 0; r < R / G; ++r) dft<G, true, false>(y + r * G);
 
     // propagateKSpaceImaginaryTime (wigner_kernel.cu:128-134): exp(-dt_steady frac k^2/2), real, as the
     // product of its (kx, ky) and kz factors
     double n_acc = 0.0, e_acc = 0.0;
-    const float kxy = kxy2[p2], fxy1 = exy1[p2], fxy2 = exy2[p2];
+    const float fxy1 = exy1[p2], fxy2 = exy2[p2];
 #pragma unroll
     for (int r = 0; r < R / G; ++r)
 #pragma unroll
         for (int k2 = 0; k2 < G; ++k2) {
             const int k = q + G * r + R * k2;
-            const float k2h = kxy + kz2[k];
             float2 v = y[r * G + k2];
-            const float e1 = fxy1 * ez1[k];
+            const float z1 = ez1[k];
+            const float e1 = fxy1 * z1;
             v = make_float2(v.x * e1, v.y * e1);
-            if (a.measure) {
+            if (STEADY || norm) {
                 const double nk = (double)v.x * v.x + (double)v.y * v.y;
                 n_acc += nk;
-                e_acc += nk * k2h;
+                if (!STEADY && ekin) e_acc += nk * (kxy2[p2] + kz2[k]);
             }
-            const float e2 = fxy2 * ez2[k];
+            const float e2 = fxy2 * (STEADY ? z1 : ez2[k]);
             y[r * G + k2] = make_float2(v.x * e2, v.y * e2);
         }
-    if (a.measure) {
+    if (STEADY || norm) {
         for (int off = 16; off > 0; off >>= 1) {
             n_acc += __shfl_down_sync(0xffffffffu, n_acc, off);
-            e_acc += __shfl_down_sync(0xffffffffu, e_acc, off);
+            if (!STEADY) e_acc += __shfl_down_sync(0xffffffffu, e_acc, off);
         }
         if ((t & 31) == 0) { red[0][t >> 5] = n_acc; red[1][t >> 5] = e_acc; }
     }
@@ -136,30 +143,48 @@ __global__ void __launch_bounds__(NZ, (NZ == 256 ? 3 : 1)) k_gs_pencil(float2 *_
 #pragma unroll
         for (int jj = 1; jj < G; ++jj) y[r * G + jj] = fftreg::cmulw(y[r * G + jj], tw[(q + G * r) * jj]);
     __syncthreads();
-    if (a.measure && t == 0) {
+    if ((STEADY || norm) && t == 0) {
         double sn = 0.0, se = 0.0;
         for (int w = 0; w < NZ / 32; ++w) { sn += red[0][w]; se += red[1][w]; }
         atomicAdd(norm + traj, sn);
-        if (ekin) atomicAdd(ekin + traj, se);
+        if (!STEADY && ekin) atomicAdd(ekin + traj, se);
     }
 #pragma unroll
     for (int r = 0; r < R / G; ++r)
 #pragma unroll
-        for (int jj = 0; jj < G; ++jj) buf[(p2 * G + jj) * R + ((q + G * r) ^ (p2 & 15))] = y[r * G + jj];
+        for (int jj = 0; jj < G; ++jj) b2[jj * R + G * r] = y[r * G + jj];
     __syncthreads();
 #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) x[k1] = buf[(p * G + j) * R + (k1 ^ (p & 15))];
+    for (int k1 = 0; k1 < R; ++k1) x[k1] = b1[k1];
     dft<R, false, false>(x);
 #pragma unroll
-    for (int m = 0; m < R; ++m) g[(size_t)(j + G * m) * plane] = x[m];
+    for (int m = 0; m < R; ++m) g[G * m * PLANE] = x[m];
 }
 
 // ---------------------------------------------------------------- plane passes
+// propagateXSpaceOneComponent (wigner_kernel.cu:154-181) of a renormalised cell; one midpoint iteration, every workload
+// here, runs without its loop
+__device__ __forceinline__ float2 nonlinear_gs(float2 a0, float V, float g11, float hdt, int itmax)
+{
+    float2 xa = a0;
+    float da = 0.0f;
+    if (itmax == 1) {
+        da = expf(hdt * fmaf(-g11, fmaf(a0.x, a0.x, a0.y * a0.y), -V));
+        xa = make_float2(a0.x * da, a0.y * da);
+    } else {
+        for (int it = 0; it < itmax; ++it) {
+            da = expf(hdt * fmaf(-g11, fmaf(xa.x, xa.x, xa.y * xa.y), -V));
+            xa = make_float2(a0.x * da, a0.y * da);
+        }
+    }
+    return make_float2(xa.x * da, xa.y * da);
+}
+
 // MODE 0: step (FFT_xy -> renormalise -> nonlinear -> IFFT_xy)
 // MODE 1: prep (x-space natural in -> IFFT_xy)
 // MODE 2: measure / output (FFT_xy, renormalise, write x-space rows to out, x-space sums)
 template <int N, int MODE>
-__global__ void __launch_bounds__(128, 4) k_gs_plane(float2 *__restrict__ state, int nz, int cells,
+__global__ void __launch_bounds__(128, N == 32 && MODE == 0 ? 5 : 4) k_gs_plane(float2 *__restrict__ state, int nz, int cells,
                                                   const GroupParamsF *__restrict__ gp,
                                                   const GsParamsF *__restrict__ gs, const int *__restrict__ tgroup,
                                                   const double *__restrict__ norm_in, double *__restrict__ norm_clear,
@@ -167,8 +192,7 @@ __global__ void __launch_bounds__(128, 4) k_gs_plane(float2 *__restrict__ state,
                                                   const int *__restrict__ active)
 {
     constexpr int W = 32 / N;
-    constexpr int PLANE = N * N;
-    constexpr int SW = N >= 16 ? 15 : 7;
+    constexpr int PLANE = N * N, LD = N + 1;
     extern __shared__ float2 tile2[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wp = lane / N, c = lane % N;
@@ -176,7 +200,7 @@ __global__ void __launch_bounds__(128, 4) k_gs_plane(float2 *__restrict__ state,
     const int lt = plane_id / nz, z = plane_id - lt * nz;
     const int traj = active ? active[lt] : lt;
     float2 *__restrict__ g = state + (size_t)traj * cells + (size_t)z * PLANE;
-    float2 *s = tile2 + (warp * W + wp) * PLANE;
+    float2 *s = tile2 + (warp * W + wp) * (N * LD);
     const int gi = tgroup[traj];
     const GroupParamsF P = gp[gi];
     const GsParamsF Q = gs[gi];
@@ -196,16 +220,15 @@ __global__ void __launch_bounds__(128, 4) k_gs_plane(float2 *__restrict__ state,
         else dft<N, false, false>(v);
         if (pass == 0) {
 #pragma unroll
-            for (int y = 0; y < N; ++y) s[y * N + (c ^ (y & SW))] = v[y];
+            for (int y = 0; y < N; ++y) s[y * LD + c] = v[y];
             __syncwarp();
 #pragma unroll
-            for (int x = 0; x < N; ++x) v[x] = s[c * N + (x ^ (c & SW))];
+            for (int x = 0; x < N; ++x) v[x] = s[c * LD + x];
         } else if (pass == 1 && MODE == 0) {
-            // propagateXSpaceOneComponent (wigner_kernel.cu:154-181) on the renormalised row
 #pragma unroll
-            for (int x = 0; x < N; ++x) s[c * N + (x ^ (c & SW))] = v[x];
+            for (int x = 0; x < N; ++x) s[c * LD + x] = v[x];
             // coordinates and potential with the fused multiply-adds written out; four cells per iteration, their
-            // exponentials independent (one midpoint iteration, every workload here, runs without its loop)
+            // exponentials independent
             const float Y = fmaf(P.dy, (float)c, -P.ymax);
             const float Z = fmaf(P.dz, (float)z, -P.zmax);
             const float base = fmaf(Y, Y, (Z * Z) * P.inv_lambda2);
@@ -217,32 +240,20 @@ __global__ void __launch_bounds__(128, 4) k_gs_plane(float2 *__restrict__ state,
                 for (int k = 0; k < 4; ++k) {
                     const float X = fmaf(P.dx, (float)(x + k), -P.xmax);
                     const float V = 0.5f * fmaf(X, X, base);
-                    const float2 w = s[c * N + ((x + k) ^ (c & SW))];
-                    const float2 a0 = make_float2(w.x * scale, w.y * scale);
-                    float2 xa = a0;
-                    float da = 0.0f;
-                    if (P.itmax == 1) {
-                        da = expf(hdt * fmaf(-P.g11, fmaf(a0.x, a0.x, a0.y * a0.y), -V));
-                        xa = make_float2(a0.x * da, a0.y * da);
-                    } else {
-                        for (int it = 0; it < P.itmax; ++it) {
-                            da = expf(hdt * fmaf(-P.g11, fmaf(xa.x, xa.x, xa.y * xa.y), -V));
-                            xa = make_float2(a0.x * da, a0.y * da);
-                        }
-                    }
-                    o[k] = make_float2(xa.x * da, xa.y * da);
+                    const float2 w = s[c * LD + x + k];
+                    o[k] = nonlinear_gs(make_float2(w.x * scale, w.y * scale), V, P.g11, hdt, P.itmax);
                 }
 #pragma unroll
-                for (int k = 0; k < 4; ++k) s[c * N + ((x + k) ^ (c & SW))] = o[k];
+                for (int k = 0; k < 4; ++k) s[c * LD + x + k] = o[k];
             }
 #pragma unroll
-            for (int x = 0; x < N; ++x) v[x] = s[c * N + (x ^ (c & SW))];
+            for (int x = 0; x < N; ++x) v[x] = s[c * LD + x];
         } else if (pass == 2) {
 #pragma unroll
-            for (int x = 0; x < N; ++x) s[c * N + (x ^ (c & SW))] = v[x];
+            for (int x = 0; x < N; ++x) s[c * LD + x] = v[x];
             __syncwarp();
 #pragma unroll
-            for (int y = 0; y < N; ++y) v[y] = s[y * N + (c ^ (y & SW))];
+            for (int y = 0; y < N; ++y) v[y] = s[y * LD + c];
         }
     }
     if (MODE == 2) {
@@ -311,24 +322,35 @@ void launch_gs_plane(float2 *state, const ClassGeom &c, const GroupParamsF *gp, 
                      float in_scale, const int *active, cudaStream_t s)
 {
     constexpr int W = 32 / N;
-    const size_t smem = sizeof(float2) * 4 * W * N * N;
+    const size_t smem = sizeof(float2) * 4 * W * N * (N + 1);
     ensure_smem_limit((const void *)k_gs_plane<N, MODE>, (int)smem);
     k_gs_plane<N, MODE><<<c.n_traj * c.nz / (4 * W), 128, smem, s>>>(state, c.nz, c.cells, gp, gs, tgroup, norm_in,
                                                                       norm_clear, out, xsums, in_scale, active);
     g_launches++;
 }
 
-template <int NZ>
+template <int NZ, int LP>
 void launch_gs_pencil(float2 *state, const ClassGeom &c, const GroupParamsF *gp, const GsParamsF *gs,
                       const int *tgroup, const float2 *tw, const GsArgs &a, double *norm, double *ekin,
                       const int *active, cudaStream_t s)
 {
-    const int tiles = c.nx * c.ny / 16;
-    const size_t smem = sizeof(float2) * (16 * NZ + NZ) + sizeof(float) * (3 * NZ + 3 * 16);
-    ensure_smem_limit((const void *)k_gs_pencil<NZ>, (int)smem);
-    k_gs_pencil<NZ><<<c.n_traj * tiles, NZ, smem, s>>>(state, c.nx, c.lx, c.ny, c.cells, tiles, gp, gs, tgroup, tw,
-                                                       a, norm, ekin, active);
+    const bool steady = a.frac1 == a.frac2 && norm && !ekin;
+    const size_t smem = sizeof(float2) * (16 * (NZ + 1) + NZ) + sizeof(float) * (3 * NZ + 3 * 16);
+    auto kernel = steady ? k_gs_pencil<NZ, LP, true> : k_gs_pencil<NZ, LP, false>;
+    ensure_smem_limit((const void *)kernel, (int)smem);
+    kernel<<<c.n_traj << (LP - 4), NZ, smem, s>>>(state, gp, gs, tgroup, tw, a, norm, ekin, active);
     g_launches++;
+}
+template <int NZ>
+void dispatch_pencil(float2 *state, const ClassGeom &c, const GroupParamsF *gp, const GsParamsF *gs, const int *tgroup,
+                     const float2 *tw, const GsArgs &a, double *norm, double *ekin, const int *active, cudaStream_t s)
+{
+    switch (c.nx) {
+    case 8: launch_gs_pencil<NZ, 6>(state, c, gp, gs, tgroup, tw, a, norm, ekin, active, s); break;
+    case 16: launch_gs_pencil<NZ, 8>(state, c, gp, gs, tgroup, tw, a, norm, ekin, active, s); break;
+    case 32: launch_gs_pencil<NZ, 10>(state, c, gp, gs, tgroup, tw, a, norm, ekin, active, s); break;
+    default: break;
+    }
 }
 
 template <int MODE>
@@ -383,11 +405,11 @@ void gs_pencil(float2 *state, const ClassGeom &c, const GroupParamsF *gp, const 
                const float2 *tw_full, float frac1, float frac2, float scale, float out_scale, double *norm,
                double *ekin, cudaStream_t s, const int *active)
 {
-    GsArgs a{frac1, frac2, scale, out_scale, norm ? 1 : 0};
+    GsArgs a{frac1, frac2, scale, out_scale};
     switch (c.nz) {
-    case 64: launch_gs_pencil<64>(state, c, gp, gs, tgroup, tw_full, a, norm, ekin, active, s); break;
-    case 128: launch_gs_pencil<128>(state, c, gp, gs, tgroup, tw_full, a, norm, ekin, active, s); break;
-    case 256: launch_gs_pencil<256>(state, c, gp, gs, tgroup, tw_full, a, norm, ekin, active, s); break;
+    case 64: dispatch_pencil<64>(state, c, gp, gs, tgroup, tw_full, a, norm, ekin, active, s); break;
+    case 128: dispatch_pencil<128>(state, c, gp, gs, tgroup, tw_full, a, norm, ekin, active, s); break;
+    case 256: dispatch_pencil<256>(state, c, gp, gs, tgroup, tw_full, a, norm, ekin, active, s); break;
     default: break;
     }
 }
