@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(128, MINB) k_plane(cpair *__restrict__ state, 
                                                const GroupParamsF *__restrict__ gp, const int *__restrict__ tgroup,
                                                const int *__restrict__ tlocal, const StepRef sr)
 {
-    extern __shared__ cpair tile[];   // 4 warps x W planes x N^2
+    extern __shared__ cpair tile[];   // plane_tile_cells<N>
     stepk::plane_body<N>(VBlock{(int)threadIdx.x, (int)blockIdx.x, 0, 128}, state, nz, cells, gp, tgroup, tlocal,
                          *sr.step + sr.off, tile);
     advance_step(sr);
@@ -35,23 +35,30 @@ __global__ void __launch_bounds__(64, MINB) k_plane32s(cpair *__restrict__ state
                                                       const int *__restrict__ tgroup, const int *__restrict__ tlocal,
                                                       const StepRef sr)
 {
-    __shared__ cpair tile[1024];
-    __shared__ cpair xb[512];
+    __shared__ cpair tile[stepk::kPlane32Cells];
     stepk::plane32_body(VBlock{(int)threadIdx.x, (int)blockIdx.x, 0, 64}, state, nz, cells, gp, tgroup, tlocal,
-                        *sr.step + sr.off, tile, xb);
+                        *sr.step + sr.off, tile);
     advance_step(sr);
 }
 
 // ---------------------------------------------------------------- pencil pass
+// Pencils per CTA: 16 as the sums of an observing pass are laid out, else 128 threads' worth at nz = 256. Twenty warps an SM
+// (96 registers, no spill) come to 87 % of the measured HBM rate at nz = 256: 365 trajectories of 32x32x256 take 0.546 ms,
+// 0.596 with 16 pencils and 256 threads (of which only two CTAs fit), 0.614 with swizzled lines and a run-time plane size
+// besides; sixteen warps 0.550, twenty-four (80 registers, spilling) 0.652.
 template <int NZ, bool OBS>
-__global__ void __launch_bounds__(NZ, OBS ? 1 : 512 / NZ) k_pencil(cpair *__restrict__ state, int nx, int lx, int ny, int cells,
+constexpr int kPen = !OBS && NZ == 256 ? 8 : 16;
+
+template <int NZ, bool OBS, int LP>
+__global__ void __launch_bounds__(kPen<NZ, OBS> * NZ / 16, OBS ? 1 : 640 / (kPen<NZ, OBS> * NZ / 16)) k_pencil(cpair *__restrict__ state, int nx, int lx, int ny, int cells,
                                                int tiles, const GroupParamsF *__restrict__ gp,
                                                const int *__restrict__ tgroup, const float2 *__restrict__ tw_g,
                                                PencilArgs pa, double *__restrict__ obs, float inv_out_scale,
                                                const float2 *__restrict__ kin)
 {
     extern __shared__ cpair dyn[];
-    stepk::pencil_body<NZ, OBS>(VBlock{(int)threadIdx.x, (int)blockIdx.x, 0, NZ}, state, nx, lx, ny, cells, tiles,
+    constexpr int PEN = kPen<NZ, OBS>;
+    stepk::pencil_body<NZ, OBS, LP, PEN>(VBlock{(int)threadIdx.x, (int)blockIdx.x, 0, PEN * NZ / 16}, state, nx, lx, ny, cells, tiles,
                                 gp, tgroup, tw_g, pa, obs, inv_out_scale, kin, dyn);
 }
 
@@ -76,16 +83,30 @@ __global__ void k_kin_tables(float2 *__restrict__ tab, const GroupParamsF *__res
     }
 }
 
+template <int NZ, bool OBS, int LP>
+void launch_pencil_lp(cpair *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const float2 *tw,
+                   const PencilArgs &pa, double *obs, float inv_out_scale, const float2 *kin, cudaStream_t s)
+{
+    constexpr int PEN = kPen<NZ, OBS>;
+    const int tiles = c.nx * c.ny / PEN;
+    const size_t smem = stepk::pencil_smem_bytes<NZ, PEN>();
+    ensure_smem_limit((const void *)k_pencil<NZ, OBS, LP>, (int)smem);
+    k_pencil<NZ, OBS, LP><<<c.n_traj * tiles, PEN * NZ / 16, smem, s>>>(state, c.nx, c.lx, c.ny, c.cells, tiles, gp, tgroup, tw,
+                                                         pa, obs, inv_out_scale, kin);
+    g_launches++;
+}
+
+// square planes with their size known to the compiler
 template <int NZ, bool OBS>
 void launch_pencil(cpair *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const float2 *tw,
                    const PencilArgs &pa, double *obs, float inv_out_scale, const float2 *kin, cudaStream_t s)
 {
-    const int tiles = c.nx * c.ny / 16;
-    const size_t smem = stepk::pencil_smem_bytes<NZ>();
-    ensure_smem_limit((const void *)k_pencil<NZ, OBS>, (int)smem);
-    k_pencil<NZ, OBS><<<c.n_traj * tiles, NZ, smem, s>>>(state, c.nx, c.lx, c.ny, c.cells, tiles, gp, tgroup, tw,
-                                                         pa, obs, inv_out_scale, kin);
-    g_launches++;
+    switch (c.nx * c.ny) {
+    case 64: launch_pencil_lp<NZ, OBS, 6>(state, c, gp, tgroup, tw, pa, obs, inv_out_scale, kin, s); break;
+    case 256: launch_pencil_lp<NZ, OBS, 8>(state, c, gp, tgroup, tw, pa, obs, inv_out_scale, kin, s); break;
+    case 1024: launch_pencil_lp<NZ, OBS, 10>(state, c, gp, tgroup, tw, pa, obs, inv_out_scale, kin, s); break;
+    default: launch_pencil_lp<NZ, OBS, 0>(state, c, gp, tgroup, tw, pa, obs, inv_out_scale, kin, s); break;
+    }
 }
 
 template <int N, int MINB>
@@ -94,7 +115,7 @@ void launch_plane(cpair *state, const ClassGeom &c, const GroupParamsF *gp, cons
 {
     constexpr int W = 32 / N;
     const int planes = c.n_traj * c.nz;
-    const size_t smem = sizeof(cpair) * 4 * W * N * N;
+    const size_t smem = sizeof(cpair) * stepk::plane_tile_cells<N>;
     ensure_smem_limit((const void *)k_plane<N, MINB>, (int)smem);
     k_plane<N, MINB><<<planes / (4 * W), 128, smem, s>>>(state, c.nz, c.cells, gp, tgroup, tlocal, sr);
     g_launches++;

@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_onchip_8x8x64(cpair *__restrict
     __syncthreads();
 
     // pencil pass: 4 tiles of 16 pencils, two 64-thread groups, two rounds
-    using Z = ZTile<NZ, 16>;
+    using Z = ZTile<NZ, 16, false>;
     const int grp = t >> 6, u = t & 63;
     const int p = u & 15, j = u >> 4;            // stages 1 and 3 (G = 4)
     const int q = u & 3, p2 = u >> 2;            // stage 2

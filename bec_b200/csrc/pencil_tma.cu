@@ -36,13 +36,15 @@ using stepk::ZTile;
 
 constexpr int kThreads = 128;
 constexpr int kTileBytes = 32768;
+// a tile's buffer also holds ZTile's padded exchange: up to 32 pencils of one cell more; 128-byte aligned for the TMA copies
+constexpr int kBufBytes = kTileBytes + 512;
 
 template <int NZ>
 constexpr size_t tma_smem_bytes()
 {
     // two tiles, W_NZ^e and the kz factors (NZ float2 each), the pencil factors (PEN float2), two mbarriers,
     // the abort flag
-    return 2 * (size_t)kTileBytes + sizeof(float2) * (2 * NZ + 2048 / NZ) + 2 * sizeof(uint64_t) + 16;
+    return 2 * (size_t)kBufBytes + sizeof(float2) * (2 * NZ + 2048 / NZ) + 2 * sizeof(uint64_t) + 16;
 }
 
 __device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -134,11 +136,11 @@ template <int NZ>
 __global__ void __launch_bounds__(kThreads, 3) k_pencil_tma(const __grid_constant__ CUtensorMap map, TmaArgs A)
 {
     constexpr int PEN = 2048 / NZ, G = NZ / 16, R = 16;
-    static_assert(PEN * G == kThreads && PEN * NZ * 16 == kTileBytes, "tile shape");
+    static_assert(PEN * G == kThreads && PEN * NZ * 16 == kTileBytes && ZTile<NZ, PEN>::CELLS * 16 <= kBufBytes, "tile shape");
     using Z = ZTile<NZ, PEN>;
     extern __shared__ __align__(1024) unsigned char smem[];
     cpair *bufs = reinterpret_cast<cpair *>(smem);
-    float2 *tw = reinterpret_cast<float2 *>(smem + 2 * kTileBytes);
+    float2 *tw = reinterpret_cast<float2 *>(smem + 2 * kBufBytes);
     float2 *kzp = tw + NZ;
     float2 *kxyp = kzp + NZ;
     uint64_t *full = reinterpret_cast<uint64_t *>(kxyp + PEN);
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_pencil_tma(const __grid_constan
     for (int i = first; i < last; ++i) {
         const int b = (i - first) & 1;
         const uint32_t parity = (uint32_t)((i - first) >> 1) & 1u;
-        cpair *B = bufs + b * (kTileBytes / 16);
+        cpair *B = bufs + b * (kBufBytes / 16);
         const int traj = i / A.tiles_per_traj;
         const int pen0 = (i - traj * A.tiles_per_traj) * PEN;
         // this tile's kinetic factors: the kz table when the trajectory changes, the pencils' every tile
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_pencil_tma(const __grid_constan
             const int tn = (i + 1) / A.tiles_per_traj;
             bulk_wait_read0();                             // tile i - 1's store has read buffer b ^ 1
             mbar_expect_tx(&full[b ^ 1], kTileBytes);
-            tma_load_2d(bufs + (b ^ 1) * (kTileBytes / 16), &map, 4 * PEN * (i + 1 - tn * A.tiles_per_traj), tn * NZ,
+            tma_load_2d(bufs + (b ^ 1) * (kBufBytes / 16), &map, 4 * PEN * (i + 1 - tn * A.tiles_per_traj), tn * NZ,
                         &full[b ^ 1]);
         }
 

@@ -6,7 +6,7 @@
 // kblk(s, h) (h = 0: k = 0..7, 16..23; h = 1: k = 8..15, 24..31). Inverse transforms use decimation in
 // frequency with the conjugate twiddles: block layout in, x[2m + h] out, which is the layout the next
 // forward step expects. (Written as conj(FFT(conj v)) instead, the sign flips cost the real-time plane
-// pass a 52-byte register spill and 4 % of its time.) tix() is the XOR swizzle of a 32 x 32 shared tile.
+// pass a 52-byte register spill and 4 % of its time.)
 // Elements are cpair (the two components of a cell, real-time passes) or float2 (one component).
 #pragma once
 
@@ -17,7 +17,6 @@
 namespace split32 {
 
 __device__ __forceinline__ int kblk(int s, int h) { return s < 8 ? s + 8 * h : s + 8 + 8 * h; }
-__device__ __forceinline__ int tix(int row, int col) { return row * 32 + (col ^ (row & 7)); }
 
 // (x - y) e^{+2 pi i K / 32}
 template <int K, typename T>

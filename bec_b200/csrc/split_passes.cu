@@ -96,13 +96,14 @@ __global__ void __launch_bounds__(32 * kSplit<N>) k_plane_split(cpair *__restric
                                                                   const int *__restrict__ tlocal, const StepRef sr)
 {
     constexpr int S = kSplit<N>, E = 4, W = 32 / N, PLANE = N * N;
-    __shared__ cpair tile[32 * N], ex[2][32 * N];
+    constexpr int LD = N + 1;
+    __shared__ cpair tile[32 * LD], ex[2][32 * N];
     const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wp = lane / N, c = lane % N;
     const int plane_id = blockIdx.x * W + wp;
     const int traj = plane_id / nz, z = plane_id - traj * nz;
     cpair *__restrict__ g = state + (size_t)traj * cells + (size_t)z * PLANE;
-    cpair *s = tile + wp * PLANE;
+    cpair *s = tile + wp * (N * LD);
     auto sync = []() { __syncthreads(); };
     const GroupParamsF P = gp[tgroup[traj]];
     wait_predecessor();
@@ -114,10 +115,10 @@ __global__ void __launch_bounds__(32 * kSplit<N>) k_plane_split(cpair *__restric
     for (int j = 0; j < E; ++j) v[j] = ld_cg(g + (q + S * j) * N + c);
     line<N, false, S>(v, ex[0] + lane, 32, q, sync);
 #pragma unroll
-    for (int j = 0; j < E; ++j) s[(q + S * j) * N + (c ^ ((q + S * j) & 7))] = v[j];
+    for (int j = 0; j < E; ++j) s[(q + S * j) * LD + c] = v[j];
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < E; ++j) v[j] = s[c * N + ((q + S * j) ^ (c & 7))];
+    for (int j = 0; j < E; ++j) v[j] = s[c * LD + q + S * j];
     line<N, false, S>(v, ex[1] + lane, 32, q, sync);
     {
         // this thread's cells x = q + S j of row y = c (plane_body's arithmetic)
@@ -138,10 +139,10 @@ __global__ void __launch_bounds__(32 * kSplit<N>) k_plane_split(cpair *__restric
     }
     line<N, true, S>(v, ex[0] + lane, 32, q, sync);
 #pragma unroll
-    for (int j = 0; j < E; ++j) s[c * N + ((q + S * j) ^ (c & 7))] = v[j];
+    for (int j = 0; j < E; ++j) s[c * LD + q + S * j] = v[j];
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < E; ++j) v[j] = s[(q + S * j) * N + (c ^ ((q + S * j) & 7))];
+    for (int j = 0; j < E; ++j) v[j] = s[(q + S * j) * LD + c];
     line<N, true, S>(v, ex[1] + lane, 32, q, sync);
 #pragma unroll
     for (int j = 0; j < E; ++j) g[(q + S * j) * N + c] = v[j];
@@ -165,12 +166,12 @@ __global__ void __launch_bounds__(PencilSplit<NZ>::THREADS) k_pencil_split(cpair
     using C = PencilSplit<NZ>;
     constexpr int G = C::G, PEN = C::PEN, LANES = C::LANES, R = 16;
     constexpr int SG = G == 16 ? 4 : G == 8 ? 2 : 1;      // threads per G-point line
-    __shared__ cpair buf[PEN * NZ], ex[PEN * NZ];
+    __shared__ cpair buf[PEN * (NZ + 1)], ex[PEN * NZ];
     __shared__ float2 tw[NZ], kzp[NZ];
     const int t = threadIdx.x, q = t / LANES, u = t % LANES;
     const int traj = blockIdx.x / tiles, pen0 = (blockIdx.x - traj * tiles) * PEN;
     auto sync = []() { __syncthreads(); };
-    auto bix = [](int p, int j, int k1) { return (p * G + j) * R + (k1 ^ (p & 7)); };
+    auto bix = [](int p, int j, int k1) { return p * (NZ + 1) + j * R + k1; };
     const float2 *kt = kin ? kin + (size_t)traj * (NZ + plane) : nullptr;
     for (int e = t; e < NZ; e += C::THREADS) {
         tw[e] = tw_g[e];

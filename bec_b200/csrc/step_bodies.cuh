@@ -26,8 +26,12 @@
 //   product of a per-pencil (kx, ky) factor and a per-kz factor; the forward transform retraces the
 //   same steps.
 //
-// Shared tiles are swizzled on the 16-byte unit index (col ^ (row & 7)) so that both the row-wise
-// and the column-wise access of a quarter warp touch eight different bank groups.
+// Shared lines are padded by one 16-byte cell, so that both the row-wise and the column-wise access of a quarter warp touch
+// eight different bank groups and every access has an address and a constant offset. (A tile that must stay dense, the
+// state held in shared memory, is swizzled on the cell index instead, col ^ (row & 7), at an instruction or two an access:
+// with every tile swizzled the 32 x 32 plane pass took 303.5 thread-instructions a cell, 280 padded, and a step of 256
+// trajectories of 32x32x256 1.309 ms, 1.247; with eight pencils a CTA besides, and the line exchange in the plane's tile,
+// 1.215 to 1.231.)
 //
 // The plane bodies read the state with ld.global.cg (L2 only): inside the fused step kernel another
 // SM's pencil item wrote those lines during the same launch, and L1 is not coherent across SMs.
@@ -65,9 +69,11 @@ struct VBlock {
 };
 
 // ---------------------------------------------------------------- plane pass, N = 8, 16
-// 4 warps (128 threads); tile: 4 warps x (32 / N) planes x N^2 cells
+// 4 warps (128 threads); tile: plane_tile_cells<N> cells, 4 warps x (32 / N) planes of N rows
 // SMEM: `state` is a trajectory held in shared memory and `tile` is the same memory (the transposes run in
 // place): plain loads instead of L2-only ones, and the warp's loads all done before its first store.
+template <int N>
+constexpr int plane_tile_cells = 4 * (32 / N) * N * (N + 1);
 template <int N, bool SMEM = false>
 __device__ __forceinline__ void plane_body(const VBlock &vb, cpair *__restrict__ state, int nz, int cells,
                                            const GroupParamsF *__restrict__ gp, const int *__restrict__ tgroup,
@@ -80,7 +86,12 @@ __device__ __forceinline__ void plane_body(const VBlock &vb, cpair *__restrict__
     const int plane_id = (vb.bid * 4 + warp) * W + wp;
     const int traj = plane_id / nz, z = plane_id - traj * nz;
     cpair *__restrict__ g = state + (size_t)traj * cells + (size_t)z * PLANE;
-    cpair *s = tile + (warp * W + wp) * PLANE;
+    // row and column c of the plane in shared memory: padded rows, or swizzled ones where the state lies there
+    constexpr int LD = SMEM ? N : N + 1;
+    cpair *s = tile + (warp * W + wp) * (N * LD);
+    cpair *row = s + c * LD;
+    auto in_row = [&](int x) -> cpair & { return row[SMEM ? x ^ (c & 7) : x]; };
+    auto in_col = [&](int y) -> cpair & { return s[y * LD + (SMEM ? c ^ (y & 7) : c)]; };
 
     const GroupParamsF P = gp[tgroup[traj]];
 
@@ -99,15 +110,15 @@ __device__ __forceinline__ void plane_body(const VBlock &vb, cpair *__restrict__
         if (pass == 0) {
             // column c -> row c
 #pragma unroll
-            for (int y = 0; y < N; ++y) s[y * N + (c ^ (y & 7))] = v[y];
+            for (int y = 0; y < N; ++y) in_col(y) = v[y];
             __syncwarp();
 #pragma unroll
-            for (int x = 0; x < N; ++x) v[x] = s[c * N + (x ^ (c & 7))];
+            for (int x = 0; x < N; ++x) v[x] = in_row(x);
         } else if (pass == 1) {
             // lane c owns row y = c: the cells go through the physics one at a time
             // from its own shared row (a rolled loop keeps the kernel small)
 #pragma unroll
-            for (int x = 0; x < N; ++x) s[c * N + (x ^ (c & 7))] = v[x];
+            for (int x = 0; x < N; ++x) in_row(x) = v[x];
             // coordinates and trap potential with every fused multiply-add written out (same bits in every kernel)
             const float Y = fmaf(P.dy, (float)c, -P.ymax);
             const float Z = fmaf(P.dz, (float)z, -P.zmax);
@@ -123,22 +134,22 @@ __device__ __forceinline__ void plane_body(const VBlock &vb, cpair *__restrict__
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float X = fmaf(P.dx, (float)(x + q), -P.xmax);
-                    v0[q] = s[c * N + ((x + q) ^ (c & 7))];
+                    v0[q] = in_row(x + q);
                     o[q] = nonlinear_cell(v0[q], 0.5f * fmaf(X, X, base), K);
                 }
                 if (P.noise) loss_noise_cell4(o, v0, K, keys, tl, step, cell0 + x);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) s[c * N + ((x + q) ^ (c & 7))] = o[q];
+                for (int q = 0; q < 4; ++q) in_row(x + q) = o[q];
             }
 #pragma unroll
-            for (int x = 0; x < N; ++x) v[x] = s[c * N + (x ^ (c & 7))];
+            for (int x = 0; x < N; ++x) v[x] = in_row(x);
         } else if (pass == 2) {
             // row c -> column c
 #pragma unroll
-            for (int x = 0; x < N; ++x) s[c * N + (x ^ (c & 7))] = v[x];
+            for (int x = 0; x < N; ++x) in_row(x) = v[x];
             __syncwarp();
 #pragma unroll
-            for (int y = 0; y < N; ++y) v[y] = s[y * N + (c ^ (y & 7))];
+            for (int y = 0; y < N; ++y) v[y] = in_col(y);
         }
     }
     if (SMEM) __syncwarp();
@@ -148,11 +159,13 @@ __device__ __forceinline__ void plane_body(const VBlock &vb, cpair *__restrict__
 
 // ---------------------------------------------------------------- plane pass, 32 x 32, two warps a plane
 // 64 threads; every 32-point line is shared by lane L of warp 0 and lane L of warp 1, 16 elements
-// each, half the registers of a one-lane line, so more warps fit on an SM. tile: 1024 cells (the
-// plane, swizzled like plane_body's), xb: 512 cells (the line exchange slots).
+// each, half the registers of a one-lane line, so more warps fit on an SM. tile: kPlane32Cells cells, the
+// plane and, between its transposes, the line exchange slots (slots of their own would take a third of the shared memory
+// from L1: 365 trajectories of 32x32x256 1.171 ms with them, 1.158 without, for five barriers more).
+constexpr int kPlane32Cells = 32 * 33;
 __device__ __forceinline__ void plane32_body(const VBlock &vb, cpair *__restrict__ state, int nz, int cells,
                                              const GroupParamsF *__restrict__ gp, const int *__restrict__ tgroup,
-                                             const int *__restrict__ tlocal, uint32_t step, cpair *tile, cpair *xb)
+                                             const int *__restrict__ tlocal, uint32_t step, cpair *tile)
 {
     using namespace split32;
     const int h = vb.tid >> 5, lane = vb.tid & 31;
@@ -161,6 +174,7 @@ __device__ __forceinline__ void plane32_body(const VBlock &vb, cpair *__restrict
     cpair *__restrict__ g = state + (size_t)traj * cells + (size_t)z * 1024;
     const GroupParamsF P = gp[tgroup[traj]];
     auto bar = [&vb]() { vb.sync(); };
+    cpair *row = tile + lane * 33, *col = tile + lane;
 
     cpair v[16];
     // forward along y (lane = column), then along x (lane = row); shared code body
@@ -171,27 +185,28 @@ __device__ __forceinline__ void plane32_body(const VBlock &vb, cpair *__restrict
             for (int j = 0; j < 16; ++j) v[j] = ld_cg(g + (2 * j + h) * 32 + lane);
         } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = tile[tix(lane, 2 * j + h)];
+            for (int j = 0; j < 16; ++j) v[j] = row[2 * j + h];
+            vb.sync();
         }
-        fwd_line(v, xb, h, lane, bar);
+        fwd_line(v, tile, h, lane, bar);
+        vb.sync();
         if (pass == 0) {
 #pragma unroll
-            for (int s = 0; s < 16; ++s) tile[tix(kblk(s, h), lane)] = v[s];
+            for (int s = 0; s < 16; ++s) col[kblk(s, h) * 33] = v[s];
             vb.sync();
         }
     }
     // x-space: lane owns row y = lane, cells x = kblk(s, h); the physics runs as a rolled loop
     // over those cells in the tile
     {
-        const int r = lane;
 #pragma unroll
-        for (int s = 0; s < 16; ++s) tile[tix(r, kblk(s, h))] = v[s];
-        const float Y = fmaf(P.dy, (float)r, -P.ymax);
+        for (int s = 0; s < 16; ++s) row[kblk(s, h)] = v[s];
+        const float Y = fmaf(P.dy, (float)lane, -P.ymax);
         const float Z = fmaf(P.dz, (float)z, -P.zmax);
         const float base = fmaf(Y, Y, (Z * Z) * P.inv_lambda2);
         const uint32_t tl = (uint32_t)tlocal[traj];
         const CellConsts K = cell_consts(P);
-        const uint32_t cell0 = (uint32_t)(z * 1024 + r * 32);
+        const uint32_t cell0 = (uint32_t)(z * 1024 + lane * 32);
         const PhiloxKeys keys = philox_keys(P.seed_lo, P.seed_hi);
         // cells in pairs (x, x + 1; kblk keeps pairs of even s adjacent): the two Philox draws interleave.
         // (Fours measured slower here: the larger loop body misses in the instruction cache.)
@@ -199,7 +214,7 @@ __device__ __forceinline__ void plane32_body(const VBlock &vb, cpair *__restrict
         for (int s = 0; s < 16; s += 2) {
             const int x = kblk(s, h);
             const float X0 = fmaf(P.dx, (float)x, -P.xmax), X1 = fmaf(P.dx, (float)(x + 1), -P.xmax);
-            cpair *s0 = tile + tix(r, x), *s1 = tile + tix(r, x + 1);
+            cpair *s0 = row + x, *s1 = row + x + 1;
             const cpair v0 = *s0, v1 = *s1;
             cpair o0 = nonlinear_cell(v0, 0.5f * fmaf(X0, X0, base), K);
             cpair o1 = nonlinear_cell(v1, 0.5f * fmaf(X1, X1, base), K);
@@ -209,20 +224,22 @@ __device__ __forceinline__ void plane32_body(const VBlock &vb, cpair *__restrict
             *s1 = o1;
         }
 #pragma unroll
-        for (int s = 0; s < 16; ++s) v[s] = tile[tix(r, kblk(s, h))];
+        for (int s = 0; s < 16; ++s) v[s] = row[kblk(s, h)];
     }
-    vb.sync();    // the partner's physics is done with the row, and its last exchange reads too
+    vb.sync();    // every row is read
     // inverse along x (lane = row), then along y (lane = column); shared code body
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
         if (pass == 1) {
 #pragma unroll
-            for (int s = 0; s < 16; ++s) v[s] = tile[tix(kblk(s, h), lane)];
+            for (int s = 0; s < 16; ++s) v[s] = col[kblk(s, h) * 33];
+            vb.sync();
         }
-        inv_line(v, xb, h, lane, bar);
+        inv_line(v, tile, h, lane, bar);
         if (pass == 0) {
+            vb.sync();
 #pragma unroll
-            for (int m = 0; m < 16; ++m) tile[tix(lane, 2 * m + h)] = v[m];
+            for (int m = 0; m < 16; ++m) row[2 * m + h] = v[m];
             vb.sync();
         }
     }
@@ -260,12 +277,17 @@ __device__ __forceinline__ cpair &zat(cpair *b, int i) { return b[i]; }
 template <class F>
 __device__ __forceinline__ cpair &zat(const F &f, int i) { return f(i); }
 
-template <int NZ, int PEN>
+// PAD: a pencil takes NZ + 1 cells of buf, so that every access has a base and a constant offset; otherwise NZ, its rows of
+// 16 swizzled.
+template <int NZ, int PEN, bool PAD = true>
 struct ZTile {
-    static constexpr int R = 16, G = NZ / 16;
+    static constexpr int R = 16, G = NZ / 16, CELLS = PEN * (PAD ? NZ + 1 : NZ);
     static_assert(NZ % 16 == 0 && G <= 16, "nz = 16 G with G <= 16");
 
-    __device__ static __forceinline__ int bix(int p, int jj, int k1) { return (p * G + jj) * R + (k1 ^ (p & 7)); }
+    __device__ static __forceinline__ int bix(int p, int jj, int k1)
+    {
+        return PAD ? p * (NZ + 1) + jj * R + k1 : (p * G + jj) * R + (k1 ^ (p & 7));
+    }
 
     template <class Buf>
     __device__ static __forceinline__ void inv1(cpair (&x)[R], Buf buf, const float2 *tw, int p, int j)
@@ -334,57 +356,60 @@ struct ZTile {
     }
 };
 
-// shared memory of one pencil body: 16 pencils x NZ cells, then W_NZ^e, the kz phase and the
+// shared memory of one pencil body: PEN pencils of NZ + 1 cells, then W_NZ^e, the kz phase and the
 // per-pencil (kx, ky) phase (float2 each)
-template <int NZ>
-__host__ __device__ constexpr size_t pencil_smem_bytes() { return sizeof(cpair) * 16 * NZ + sizeof(float2) * (2 * NZ + 16); }
+template <int NZ, int PEN = 16>
+__host__ __device__ constexpr size_t pencil_smem_bytes() { return sizeof(cpair) * PEN * (NZ + 1) + sizeof(float2) * (2 * NZ + PEN); }
 
 // OBS: the pass ends a step (no plane pass follows) and also writes, per z, the
 // FP64 sums over the tile's 16 pencils of |a|^2, |b|^2 and conj(a) b of the
 // z-transformed boundary state: obs[((traj * tiles + tile) * NZ + z) * 4 + k].
-// NZ threads; dyn: pencil_smem_bytes<NZ>() of shared memory.
-template <int NZ, bool OBS>
+// PEN G threads; dyn: pencil_smem_bytes<NZ, PEN>() of shared memory. LP: log2 of nx ny, or 0 where only run time tells.
+template <int NZ, bool OBS, int LP = 0, int PEN = 16>
 __device__ __forceinline__ void pencil_body(const VBlock &vb, cpair *__restrict__ state, int nx, int lx, int ny,
                                             int cells, int tiles, const GroupParamsF *__restrict__ gp,
                                             const int *__restrict__ tgroup, const float2 *__restrict__ tw_g,
                                             const PencilArgs &pa, double *__restrict__ obs, float inv_out_scale,
                                             const float2 *__restrict__ kin, cpair *dyn)
 {
-    using Z = ZTile<NZ, 16>;
+    using Z = ZTile<NZ, PEN>;
     constexpr int R = 16, G = NZ / 16;
+    static_assert(!OBS || PEN == 16, "the layout of obs");
     (void)gp; (void)tgroup; (void)lx;
-    cpair *buf = dyn;                                           // 16 pencils x NZ
-    float2 *tw = reinterpret_cast<float2 *>(dyn + 16 * NZ);     // W_NZ^e, e < NZ
+    cpair *buf = dyn;                                           // PEN pencils x NZ
+    float2 *tw = reinterpret_cast<float2 *>(dyn + Z::CELLS);    // W_NZ^e, e < NZ
     float2 *kzp = tw + NZ;                                       // kz phase
     float2 *kxyp = kzp + NZ;                                    // (kx, ky) phase x scale, per pencil
 
     const int t = vb.tid;
     const int traj = vb.bid / tiles;
-    const int pen0 = (vb.bid - traj * tiles) * 16;
-    const int plane = nx * ny;
+    const int pen0 = (vb.bid - traj * tiles) * PEN;
+    const int plane = LP ? 1 << LP : nx * ny;
 
     // kinetic phase e^{+i k^2/2 dt frac} (wigner_kernel.cu:137-151) as the product of the per-kz and the
     // per-pencil factors, from the class's table for this kick fraction (fp32_kin_tables); kin == NULL
-    // means frac == 0, no kick. Thread t fills entry t of the twiddle and kz tables (NZ threads).
+    // means frac == 0, no kick.
     // The table entries go to shared memory by asynchronous copies, so the state loads below issue at once
     // and no register holds a table value in between.
     const float2 *kt = kin ? kin + (size_t)traj * (NZ + plane) : nullptr;
-    copy_async8(tw + t, tw_g + t);
-    if (kt) {
-        copy_async8(kzp + t, kt + t);
-        if (t < 16) copy_async8(kxyp + t, kt + NZ + pen0 + t);
-    } else {
-        kzp[t] = make_float2(1.f, 0.f);
-        if (t < 16) kxyp[t] = make_float2(1.f, 0.f);
+#pragma unroll
+    for (int e = 0; e < NZ; e += PEN * G) {
+        copy_async8(tw + e + t, tw_g + e + t);
+        if (kt) copy_async8(kzp + e + t, kt + e + t);
+        else kzp[e + t] = make_float2(1.f, 0.f);
+    }
+    if (t < PEN) {
+        if (kt) copy_async8(kxyp + t, kt + NZ + pen0 + t);
+        else kxyp[t] = make_float2(1.f, 0.f);
     }
 
-    const int p = t & 15, j = t >> 4;
-    cpair *__restrict__ g = state + (size_t)traj * cells + pen0 + p;
+    const int p = t % PEN, j = t / PEN;
+    cpair *__restrict__ g = state + (size_t)traj * cells + pen0 + p + j * plane;
     cpair x[R];
 #pragma unroll
-    for (int m = 0; m < R; ++m) x[m] = g[(size_t)(j + G * m) * plane];
+    for (int m = 0; m < R; ++m) x[m] = g[G * m * plane];
     copy_async_wait();
-    if (t < 16) kxyp[t] = make_float2(pa.scale * kxyp[t].x, pa.scale * kxyp[t].y);
+    if (t < PEN) kxyp[t] = make_float2(pa.scale * kxyp[t].x, pa.scale * kxyp[t].y);
     vb.sync();                                                  // tables ready
     Z::inv1(x, buf, tw, p, j);
     vb.sync();
@@ -424,7 +449,7 @@ __device__ __forceinline__ void pencil_body(const VBlock &vb, cpair *__restrict_
         }
     }
 #pragma unroll
-    for (int m = 0; m < R; ++m) g[(size_t)(j + G * m) * plane] = x[m];
+    for (int m = 0; m < R; ++m) g[G * m * plane] = x[m];
 }
 
 } // namespace stepk

@@ -51,8 +51,11 @@ using stepk::VBlock;
 
 constexpr int kThreads = 256;
 constexpr int kPlane32PerItem = 4;                              // 64-thread virtual blocks
-constexpr size_t kSmemPlane32 = sizeof(cpair) * 1536;          // tile + exchange slots of one plane
-constexpr size_t kSmemBytes = kSmemPlane32 * kPlane32PerItem;   // 96 KiB: the largest item's need
+// shared memory of the largest item: its virtual blocks' share each (69.5 KiB)
+constexpr size_t kSmemBytes = std::max({sizeof(cpair) * stepk::kPlane32Cells * kPlane32PerItem,
+                                        2 * sizeof(cpair) * stepk::plane_tile_cells<8>, 2 * sizeof(cpair) * stepk::plane_tile_cells<16>,
+                                        4 * stepk::pencil_smem_bytes<64>(), 2 * stepk::pencil_smem_bytes<128>(),
+                                        stepk::pencil_smem_bytes<256>()});
 
 enum { ITEM_PENCIL = 0, ITEM_PLANE = 1 };
 
@@ -94,7 +97,7 @@ __device__ __forceinline__ void run_plane(const StepClassDev &c, const GroupPara
     const int planes_per_vb = 4 * W;
     const int bid = (traj * c.nz) / planes_per_vb + sub * 2 + v;
     const VBlock vb{(int)threadIdx.x % 128, bid, 0, 128};   // warp-synchronous: no block barrier used
-    stepk::plane_body<N>(vb, reinterpret_cast<cpair *>(c.state), c.nz, c.cells, gp, c.tgroup, c.tlocal, step, smem + v * 4 * W * N * N);
+    stepk::plane_body<N>(vb, reinterpret_cast<cpair *>(c.state), c.nz, c.cells, gp, c.tgroup, c.tlocal, step, smem + v * stepk::plane_tile_cells<N>);
 }
 
 __device__ __forceinline__ void run_plane32(const StepClassDev &c, const GroupParamsF *gp, int traj, int sub,
@@ -102,8 +105,8 @@ __device__ __forceinline__ void run_plane32(const StepClassDev &c, const GroupPa
 {
     const int v = threadIdx.x / 64;
     const VBlock vb{(int)threadIdx.x % 64, traj * c.nz + sub * kPlane32PerItem + v, 1 + v, 64};
-    cpair *tile = smem + v * 1536;
-    stepk::plane32_body(vb, reinterpret_cast<cpair *>(c.state), c.nz, c.cells, gp, c.tgroup, c.tlocal, step, tile, tile + 1024);
+    cpair *tile = smem + v * stepk::kPlane32Cells;
+    stepk::plane32_body(vb, reinterpret_cast<cpair *>(c.state), c.nz, c.cells, gp, c.tgroup, c.tlocal, step, tile);
 }
 
 __global__ void __launch_bounds__(kThreads, 2) k_step(StepLaunch L, PencilArgs pa)
