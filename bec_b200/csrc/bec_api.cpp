@@ -1910,6 +1910,8 @@ bec_status gs_batched(bec_ctx *ctx, int n, const int32_t *groups, const bec_gs_o
         CKC(talloc((void **)&d_gp, sizeof(GroupParamsF) * gfs.size()));
         CKC(cudaMemcpyAsync(d_gp, gfs.data(), sizeof(GroupParamsF) * gfs.size(), cudaMemcpyHostToDevice, s));
     }
+    bool blank = true;
+    for (const auto &gr : ctx->groups) blank = blank && !gr.initialised;
     // allocations and host-side staging first: the timed region holds the device work from the first copy on
     // (cudaMalloc of fresh memory can hold the host for tens of ms, which the device clock would count)
     std::vector<std::vector<float2>> warm_h(cls.size());
@@ -1919,8 +1921,15 @@ bec_status gs_batched(bec_ctx *ctx, int n, const int32_t *groups, const bec_gs_o
         GsClass &c = cls[k];
         const size_t nt = c.groups.size(), cells = c.geom.cells;
         c.geom.n_traj = (int)nt;
-        CKC(talloc((void **)&c.state, sizeof(float2) * nt * cells));
-        CKC(talloc((void **)&c.out, sizeof(float2) * nt * cells));
+        // before any group is initialised, the class's own state buffer (16 B a cell) has room for both
+        const ClassRec *home = ctx->path == BEC_PATH_FP32_BATCHED ? &ctx->classes[ctx->groups[c.groups[0]].cls] : nullptr;
+        if (blank && home && home->state && nt <= (size_t)home->geom.n_traj) {
+            c.state = reinterpret_cast<float2 *>(home->state);
+            c.out = c.state + nt * cells;
+        } else {
+            CKC(talloc((void **)&c.state, sizeof(float2) * nt * cells));
+            CKC(talloc((void **)&c.out, sizeof(float2) * nt * cells));
+        }
         CKC(talloc((void **)&c.d_tgroup, sizeof(int) * nt));
         CKC(talloc((void **)&c.d_active, sizeof(int) * nt));
         CKC(talloc((void **)&c.norm, sizeof(double) * 2 * nt));
@@ -1947,7 +1956,7 @@ bec_status gs_batched(bec_ctx *ctx, int n, const int32_t *groups, const bec_gs_o
                 dd[t] = ctx->groups[c.groups[t]].d;
                 for (int k2 = 0; k2 < nb; ++k2) cc[t * nb + k2] = coef_in[(size_t)c.batch[t] * nb + k2];
             }
-            CKC(talloc((void **)&c.warm, sizeof(float2) * nt * cells));
+            c.warm = c.state;                 // synthesised in place
         }
     }
     CKC(cudaEventRecord(ctx->ev0, s));      // the timed region includes the warm-start synthesis
@@ -1970,7 +1979,7 @@ bec_status gs_batched(bec_ctx *ctx, int n, const int32_t *groups, const bec_gs_o
     for (auto &c : cls) {
         float2 *tw;
         if ((st = tw_for(c.geom.nz, &tw))) return st;
-        gs_init(c.state, c.geom, d_gp, d_gs, c.d_tgroup, c.warm, s);
+        if (!c.warm || c.warm != c.state) gs_init(c.state, c.geom, d_gp, d_gs, c.d_tgroup, c.warm, s);
         gs_prep(c.state, c.geom, d_gp, d_gs, c.d_tgroup, s);
         gs_pencil(c.state, c.geom, d_gp, d_gs, c.d_tgroup, tw, 0.0f, 0.5f, 1.0f / c.geom.cells, 1.0f, c.norm,
                   nullptr, s);

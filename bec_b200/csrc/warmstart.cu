@@ -58,28 +58,17 @@ __device__ __forceinline__ void basis_at(int i, const WsGeom &g, float *b, float
     }
 }
 
-// Basis values at cell i: the analytic functions, or the rows of an installed table
-// (rows >= nb read as zero).
-template <bool TAB>
-__device__ __forceinline__ void basis_any(int i, const WsGeom &g, const float *tab, int nb, float *b, float &ftf)
+__device__ __forceinline__ float thomas_fermi(int i, const WsGeom &g)
 {
-    if (!TAB) {
-        basis_at(i, g, b, ftf);
-        return;
-    }
     const int x = i & (g.nx - 1), y = (i >> g.lx) & (g.ny - 1), z = i >> (g.lx + g.ly);
     const float X = -1.2f + g.dxs * x;
     const float Y = (g.ny > 1) ? -1.2f + g.dys * y : 0.0f;
     const float Z = -1.2f + g.dzs * z;
-    ftf = sqrtf(fmaxf(1.0f - (X * X + Y * Y + Z * Z), 0.0f));
-#pragma unroll
-    for (int k = 0; k < kBasis; ++k) b[k] = (k < nb) ? tab[(size_t)k * g.cells + i] : 0.0f;
+    return sqrtf(fmaxf(1.0f - (X * X + Y * Y + Z * Z), 0.0f));
 }
 
 // rhs[t][k] = sum_cells B_k d_t,  d_t = |psi_t| / A_t - f_TF  (written to profile when not NULL)
-template <bool TAB>
-__global__ void k_ws_project(const float2 *psi, int n_traj, WsGeom g, const float *amp, const float *tab, int nb,
-                             double *rhs, float *profile)
+__global__ void k_ws_project(const float2 *psi, int n_traj, WsGeom g, const float *amp, double *rhs, float *profile)
 {
     const int t = blockIdx.y;
     __shared__ double acc[kBasis];
@@ -91,7 +80,7 @@ __global__ void k_ws_project(const float2 *psi, int n_traj, WsGeom g, const floa
     const float inv_a = 1.0f / amp[t];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.cells; i += gridDim.x * blockDim.x) {
         float b[kBasis], ftf;
-        basis_any<TAB>(i, g, tab, nb, b, ftf);
+        basis_at(i, g, b, ftf);
         const float2 v = psi[(size_t)t * g.cells + i];
         const float d = sqrtf(v.x * v.x + v.y * v.y) * inv_a - ftf;
         if (profile) profile[(size_t)t * g.cells + i] = d;
@@ -108,23 +97,87 @@ __global__ void k_ws_project(const float2 *psi, int n_traj, WsGeom g, const floa
     for (int k = threadIdx.x; k < kBasis; k += blockDim.x) atomicAdd(rhs + (size_t)t * kBasis + k, acc[k]);
 }
 
+// The same with an installed table, kProjTraj trajectories a CTA, so that a row's cells are read once for all of them: read
+// for every trajectory they made up 13 GB for 256 states of 32x32x256 and 50 rows. A thread keeps its cells' d_t (the cells
+// that k_ws_project gives it, CELLS at most, in the same order) and goes through the rows; the sums round alike. With
+// k_ws_synth_rows and the buffers of a fresh context, 96 warm-started states and 60 steps take 15.4 ms, 19.4 before; the
+// projection of 256 states took 4.9 ms.
+constexpr int kProjTraj = 4;
+template <int CELLS>
+__global__ void __launch_bounds__(256) k_ws_project_rows(const float2 *psi, int n_traj, WsGeom g, const float *amp, const float *tab,
+                                                         int nb, double *rhs, float *profile)
+{
+    const int t0 = blockIdx.y * kProjTraj, T = min(kProjTraj, n_traj - t0);
+    __shared__ double acc[kProjTraj][kBasis];
+    for (int k = threadIdx.x; k < kProjTraj * kBasis; k += blockDim.x) acc[0][k] = 0.0;
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    float d[kProjTraj][CELLS];
+#pragma unroll
+    for (int q = 0; q < kProjTraj; ++q) {
+        const float inv_a = q < T ? 1.0f / amp[t0 + q] : 0.0f;
+#pragma unroll
+        for (int m = 0; m < CELLS; ++m) {
+            const int i = i0 + m * stride;
+            d[q][m] = 0.0f;
+            if (q < T && i < g.cells) {
+                const float2 v = psi[(size_t)(t0 + q) * g.cells + i];
+                d[q][m] = sqrtf(v.x * v.x + v.y * v.y) * inv_a - thomas_fermi(i, g);
+                if (profile) profile[(size_t)(t0 + q) * g.cells + i] = d[q][m];
+            }
+        }
+    }
+    __syncthreads();
+    // (the rows past the table's are zero: one of them is summed, which a d_t that is not finite makes NaN)
+    const int rows = min(nb + 1, kBasis);
+    for (int k = 0; k < rows; ++k) {
+        const float *row = tab + (size_t)k * g.cells + i0;
+        float v[kProjTraj] = {};
+#pragma unroll
+        for (int m = 0; m < CELLS; ++m) {
+            const float b = k < nb && i0 + m * stride < g.cells ? row[m * stride] : 0.0f;
+#pragma unroll
+            for (int q = 0; q < kProjTraj; ++q) v[q] += b * d[q][m];
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (int q = 0; q < kProjTraj; ++q) v[q] += __shfl_down_sync(0xffffffffu, v[q], off);
+        if ((threadIdx.x & 31) == 0)
+#pragma unroll
+            for (int q = 0; q < kProjTraj; ++q) atomicAdd(&acc[q][k], (double)v[q]);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < T * kBasis; e += blockDim.x) {
+        const int q = e / kBasis, k = e % kBasis;
+        atomicAdd(rhs + (size_t)t0 * kBasis + e, acc[q][min(k, rows - 1)]);
+    }
+}
+
 // gram[k][l] = sum_cells B_k B_l: 256 threads, each owns 16 of the 64 x 64 entries; the basis
 // rows of 32 cells at a time are staged in shared memory.
 template <bool TAB>
 __global__ void __launch_bounds__(256) k_ws_gram(WsGeom g, const float *tab, int nb, double *gram)
 {
-    __shared__ float rows[32][kBasis];
+    __shared__ float rows[32][kBasis + 1];
     double acc[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = 0.0;
     const int t = threadIdx.x;
     const int k = t >> 2, l0 = (t & 3) * 16;   // row k, columns l0 .. l0 + 15
     for (int base = blockIdx.x * 32; base < g.cells; base += gridDim.x * 32) {
-        if (t < 32) {
+        if (TAB) {
+            // a warp reads eight rows of the 32 cells
+            const int cell = t & 31, i = base + cell;
+#pragma unroll
+            for (int r = 0; r < kBasis / 8; ++r) {
+                const int row = (t >> 5) + 8 * r;
+                rows[cell][row] = row < nb && i < g.cells ? tab[(size_t)row * g.cells + i] : 0.0f;
+            }
+        } else if (t < 32) {
             float b[kBasis], ftf;
             const int i = base + t;
             if (i < g.cells) {
-                basis_any<TAB>(i, g, tab, nb, b, ftf);
+                basis_at(i, g, b, ftf);
 #pragma unroll
                 for (int q = 0; q < kBasis; ++q) rows[t][q] = b[q];
             } else {
@@ -150,9 +203,7 @@ __global__ void __launch_bounds__(256) k_ws_gram(WsGeom g, const float *tab, int
 }
 
 // psi_t = A_t max(f_TF + sum c_k B_k, 0) (real, x-space)
-template <bool TAB>
-__global__ void k_ws_synth(float2 *psi, int n_traj, WsGeom g, const float *amp, const float *coef, const float *tab,
-                           int nb)
+__global__ void k_ws_synth(float2 *psi, int n_traj, WsGeom g, const float *amp, const float *coef)
 {
     const int t = blockIdx.y;
     __shared__ float c[kBasis];
@@ -160,11 +211,45 @@ __global__ void k_ws_synth(float2 *psi, int n_traj, WsGeom g, const float *amp, 
     __syncthreads();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.cells; i += gridDim.x * blockDim.x) {
         float b[kBasis], ftf;
-        basis_any<TAB>(i, g, tab, nb, b, ftf);
+        basis_at(i, g, b, ftf);
         float f = ftf;
 #pragma unroll
         for (int k = 0; k < kBasis; ++k) f += c[k] * b[k];
         psi[(size_t)t * g.cells + i] = make_float2(amp[t] * fmaxf(f, 0.0f), 0.0f);
+    }
+}
+
+// The same with an installed table: a row's cell is read once for kSynthTraj trajectories.
+constexpr int kSynthTraj = 8;
+__global__ void __launch_bounds__(256) k_ws_synth_rows(float2 *psi, int n_traj, WsGeom g, const float *amp, const float *coef,
+                                                       const float *tab, int nb)
+{
+    const int t0 = blockIdx.y * kSynthTraj, T = min(kSynthTraj, n_traj - t0);
+    __shared__ float c[kBasis][kSynthTraj], rest[kSynthTraj];
+    if (threadIdx.x < kSynthTraj) {      // the rows past the table's are zero
+        float r = 0.0f;
+        for (int k = nb; k < kBasis && (int)threadIdx.x < T; ++k) r += coef[(size_t)(t0 + threadIdx.x) * kBasis + k] * 0.0f;
+        rest[threadIdx.x] = r;
+    }
+    for (int e = threadIdx.x; e < kBasis * kSynthTraj; e += blockDim.x) {
+        const int q = e % kSynthTraj, k = e / kSynthTraj;
+        c[k][q] = q < T ? coef[(size_t)(t0 + q) * kBasis + k] : 0.0f;
+    }
+    __syncthreads();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.cells; i += gridDim.x * blockDim.x) {
+        const float ftf = thomas_fermi(i, g);
+        float f[kSynthTraj];
+#pragma unroll
+        for (int q = 0; q < kSynthTraj; ++q) f[q] = ftf;
+#pragma unroll 8
+        for (int k = 0; k < nb; ++k) {
+            const float b = tab[(size_t)k * g.cells + i];
+#pragma unroll
+            for (int q = 0; q < kSynthTraj; ++q) f[q] += c[k][q] * b;
+        }
+#pragma unroll
+        for (int q = 0; q < kSynthTraj; ++q)
+            if (q < T) psi[(size_t)(t0 + q) * g.cells + i] = make_float2(amp[t0 + q] * fmaxf(f[q] + rest[q], 0.0f), 0.0f);
     }
 }
 
@@ -286,6 +371,7 @@ cudaError_t warmstart_project(const float2 *psi, int n, const bec_derived *d, co
     cudaError_t e = set_consts(s);
     if (e) return e;
     const WsGeom g = geom_dims(d[0].nvx, d[0].nvy, d[0].nvz);
+    if (tab && g.cells > 16 * 64 * 256) return cudaErrorInvalidValue;   // (the batched ground states' grids end there)
     std::vector<float> amp(n);
     for (int t = 0; t < n; ++t) amp[t] = (float)std::sqrt(d[t].mu / d[t].g11);
     float *damp = nullptr, *dprof = nullptr;
@@ -299,8 +385,12 @@ cudaError_t warmstart_project(const float2 *psi, int n, const bec_derived *d, co
     cudaMemcpyAsync(damp, amp.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(rhs, 0, sizeof(double) * n * kBasis, s);
     dim3 grid(64, n);
-    if (tab) k_ws_project<true><<<grid, 256, 0, s>>>(psi, n, g, damp, tab->d_basis, tab->nb, rhs, dprof);
-    else k_ws_project<false><<<grid, 256, 0, s>>>(psi, n, g, damp, nullptr, kBasis, rhs, dprof);
+    const dim3 shared(64, (n + kProjTraj - 1) / kProjTraj);
+    if (tab && g.cells <= 4 * 64 * 256)
+        k_ws_project_rows<4><<<shared, 256, 0, s>>>(psi, n, g, damp, tab->d_basis, tab->nb, rhs, dprof);
+    else if (tab)
+        k_ws_project_rows<16><<<shared, 256, 0, s>>>(psi, n, g, damp, tab->d_basis, tab->nb, rhs, dprof);
+    else k_ws_project<<<grid, 256, 0, s>>>(psi, n, g, damp, rhs, dprof);
     g_launches++;
     if ((e = cudaGetLastError())) {           // nothing solved from a projection that did not run
         cudaStreamSynchronize(s);
@@ -343,9 +433,9 @@ cudaError_t warmstart_synth(const double *coef, int n, const bec_derived *d, con
     if ((e = cudaMalloc(&dc, sizeof(float) * c.size()))) { cudaFree(damp); return e; }
     cudaMemcpyAsync(damp, amp.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dc, c.data(), sizeof(float) * c.size(), cudaMemcpyHostToDevice, s);
-    dim3 grid(64, n);
-    if (tab) k_ws_synth<true><<<grid, 256, 0, s>>>(psi_out, n, g, damp, dc, tab->d_basis, tab->nb);
-    else k_ws_synth<false><<<grid, 256, 0, s>>>(psi_out, n, g, damp, dc, nullptr, kBasis);
+    if (tab)
+        k_ws_synth_rows<<<dim3(64, (n + kSynthTraj - 1) / kSynthTraj), 256, 0, s>>>(psi_out, n, g, damp, dc, tab->d_basis, tab->nb);
+    else k_ws_synth<<<dim3(64, n), 256, 0, s>>>(psi_out, n, g, damp, dc);
     g_launches++;
     const cudaError_t el = cudaGetLastError();
     e = cudaStreamSynchronize(s);
