@@ -73,7 +73,9 @@ __device__ __forceinline__ void split_bf16(float v, bf16 &hi, bf16 &lo)
 // tiles onto an mbarrier, and, as each stage lands, per 16-wide K step the three tcgen05.mma (M 128, N tn, K 16, BF16
 // in, FP32 accumulate) lo*hi, hi*lo, hi*hi; tcgen05.commit arrives on the stage's second mbarrier when they are done.
 // Every wait is bounded. Rows of a last 64-row tile (M = 64 mod 128) are not loaded and not stored. The epilogue reads
-// the accumulator with tcgen05.ld (warp w owns lanes 32w..32w+31).
+// the accumulator with tcgen05.ld: warps w and w + 4 own lanes 32w..32w+31, and take turns at EC columns (with four warps and
+// 16 columns a thread the arithmetic of an epilogue, tanh or Adam, is a chain twice as long).
+constexpr int kThreads = 256;
 constexpr int GM = 128, GK = 64, GSTAGES = 4;
 constexpr int kTileA = GM * GK * 2;                           // 16 KiB each of hi and lo
 __host__ __device__ constexpr int stage_bytes(int tn) { return 2 * (kTileA + tn * GK * 2); }
@@ -207,24 +209,22 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
                  : "memory");
 }
 
-// 16 consecutive columns of one row, as operands: two 16-byte chunks of the plain matrix, and of the transposed one
+// EC consecutive columns of one row, as operands: a 16-byte chunk of the plain matrix, and of the transposed one
 // a 2-byte value per column (8 rows of consecutive lanes make a chunk)
-__device__ __forceinline__ void store_operands(const GemmJob &J, int row, int col, const float (&o)[16])
+constexpr int EC = 8;
+__device__ __forceinline__ void store_operands(const GemmJob &J, int row, int col, const float (&o)[EC])
 {
-    __align__(16) bf16 hi[16], lo[16];
+    __align__(16) bf16 hi[EC], lo[EC];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) split_bf16(o[q], hi[q], lo[q]);
+    for (int q = 0; q < EC; ++q) split_bf16(o[q], hi[q], lo[q]);
     if (J.out.hi) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const size_t at = blk(J.M, row, col + 8 * h);
-            *reinterpret_cast<uint4 *>(J.out.hi + at) = reinterpret_cast<const uint4 *>(hi)[h];
-            *reinterpret_cast<uint4 *>(J.out.lo + at) = reinterpret_cast<const uint4 *>(lo)[h];
-        }
+        const size_t at = blk(J.M, row, col);
+        *reinterpret_cast<uint4 *>(J.out.hi + at) = *reinterpret_cast<const uint4 *>(hi);
+        *reinterpret_cast<uint4 *>(J.out.lo + at) = *reinterpret_cast<const uint4 *>(lo);
     }
     if (J.outT.hi) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
+        for (int q = 0; q < EC; ++q) {
             const size_t at = blk(J.N, col + q, row);
             J.outT.hi[at] = hi[q];
             J.outT.lo[at] = lo[q];
@@ -232,74 +232,74 @@ __device__ __forceinline__ void store_operands(const GemmJob &J, int row, int co
     }
 }
 
-__device__ __forceinline__ void load16(float (&o)[16], const float *p)
+__device__ __forceinline__ void load_cols(float (&o)[EC], const float *p)
 {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < EC / 4; ++q) {
         const float4 v = reinterpret_cast<const float4 *>(p)[q];
         o[4 * q] = v.x; o[4 * q + 1] = v.y; o[4 * q + 2] = v.z; o[4 * q + 3] = v.w;
     }
 }
-__device__ __forceinline__ void store16(float *p, const float (&o)[16])
+__device__ __forceinline__ void store_cols(float *p, const float (&o)[EC])
 {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) reinterpret_cast<float4 *>(p)[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+    for (int q = 0; q < EC / 4; ++q) reinterpret_cast<float4 *>(p)[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
 }
 
-// what the epilogue reads beside the accumulator: the tile's first 16 columns are fetched while its operands load
+// what the epilogue reads beside the accumulator: the thread's first EC columns are fetched while the tile's operands load
 struct Aux {
-    float a[16], b[16], c[16];
+    float a[EC], b[EC], c[EC];
 };
 __device__ __forceinline__ void load_aux(const GemmJob &J, Aux &x, int row, int col)
 {
     const size_t at = (size_t)row * J.N + col;
-    if (J.epi <= EPI_LOSS) load16(x.a, J.bias + col);
-    if (J.epi == EPI_LOSS) load16(x.b, J.tgt + at);
-    if (J.epi == EPI_DX) load16(x.a, J.y + at);
+    if (J.epi <= EPI_LOSS) load_cols(x.a, J.bias + col);
+    if (J.epi == EPI_LOSS) load_cols(x.b, J.tgt + at);
+    if (J.epi == EPI_DX) load_cols(x.a, J.y + at);
     if (J.epi == EPI_ADAM) {
-        load16(x.a, J.w + at);
-        load16(x.b, J.m + at);
-        load16(x.c, J.v + at);
+        load_cols(x.a, J.w + at);
+        load_cols(x.b, J.m + at);
+        load_cols(x.c, J.v + at);
     }
 }
 
-// row's 16 accumulator columns from col on; returns the row's share of the loss (EPI_LOSS)
-__device__ __forceinline__ float epilogue(const GemmJob &J, int row, int col, float (&o)[16], Aux &x)
+// row's EC accumulator columns from col on; returns the row's share of the loss (EPI_LOSS)
+__device__ __forceinline__ float epilogue(const GemmJob &J, int row, int col, float (&o)[EC], Aux &x)
 {
     float l = 0.0f;
     const size_t at = (size_t)row * J.N + col;
     if (J.epi <= EPI_LOSS) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) o[q] += x.a[q];
+        for (int q = 0; q < EC; ++q) o[q] += x.a[q];
     }
     if (J.epi == EPI_TANH) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) o[q] = tanhf(o[q]);
+        for (int q = 0; q < EC; ++q) o[q] = tanhf(o[q]);
     } else if (J.epi == EPI_LOSS) {
         // the padding columns of y and t are zero, padding rows get no gradient
         const float s = 2.0f / ((float)J.valid * J.real_cols);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
+        for (int q = 0; q < EC; ++q) {
             const float d = row < J.valid ? o[q] - x.b[q] : 0.0f;
             l += d * d;
             o[q] = s * d;
         }
     } else if (J.epi == EPI_DX) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) o[q] *= 1.0f - x.a[q] * x.a[q];
+        for (int q = 0; q < EC; ++q) o[q] *= 1.0f - x.a[q] * x.a[q];
     } else if (J.epi == EPI_ADAM) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) o[q] = adam_update(x.a[q], x.b[q], x.c[q], o[q], J.adam);
-        store16(J.w + at, x.a);
-        store16(J.m + at, x.b);
-        store16(J.v + at, x.c);
+        for (int q = 0; q < EC; ++q) o[q] = adam_update(x.a[q], x.b[q], x.c[q], o[q], J.adam);
+        store_cols(J.w + at, x.a);
+        store_cols(J.m + at, x.b);
+        store_cols(J.v + at, x.c);
     }
     if (J.f32 && row < J.f32_rows) {
         float *dst = J.f32 + (size_t)row * J.f32_ld + col;
-        if (col + 16 <= J.f32_cols && (J.f32_ld & 3) == 0) {
-            store16(dst, o);
+        if (col + EC <= J.f32_cols && (J.f32_ld & 3) == 0) {
+            store_cols(dst, o);
         } else {
-            for (int q = 0; q < 16; ++q)
+            for (int q = 0; q < EC; ++q)
                 if (col + q < J.f32_cols) dst[q] = o[q];
         }
     }
@@ -333,9 +333,9 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
 
     wait_predecessor();
     allow_successor();
-    const int lr = warp * 32 + (t & 31);
+    const int lr = (warp & 3) * 32 + (t & 31), c0 = (warp >> 2) * EC;    // this thread's row, and its first columns
     Aux x;
-    if (lr < rows) load_aux(J, x, m0 + lr, n0);
+    if (lr < rows) load_aux(J, x, m0 + lr, n0 + c0);
     bool ok = true;
     if (t == 0) {
         // instruction descriptor, kind::f16: D F32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1), both K-major,
@@ -393,20 +393,17 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!failed) {
         float l = 0.0f;
-        for (int cb = 0; cb < tn; cb += 16) {
-            uint32_t r[16];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                         "%13, %14, %15}, [%16];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                           "=r"(r[15])
-                         : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)cb));
+        for (int cb = c0; cb < tn; cb += 2 * EC) {
+            uint32_t r[EC];
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                         : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cb));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (lr < rows) {
-                float o[16];
+                float o[EC];
 #pragma unroll
-                for (int q = 0; q < 16; ++q) o[q] = __uint_as_float(r[q]);
-                if (cb > 0) load_aux(J, x, m0 + lr, n0 + cb);
+                for (int q = 0; q < EC; ++q) o[q] = __uint_as_float(r[q]);
+                if (cb > c0) load_aux(J, x, m0 + lr, n0 + cb);
                 l += epilogue(J, m0 + lr, n0 + cb, o, x);
             }
         }
@@ -428,15 +425,15 @@ __device__ __forceinline__ void bias_columns(const BiasJob &J, int cta, float *s
     float s = 0.0f;
     for (int r0 = 0; r0 < J.rows; r0 += kBiasRows) {
         const int n = min(kBiasRows, J.rows - r0);
-        float v[kBiasRows / 4];
+        float v[kBiasRows / 8];
 #pragma unroll
-        for (int i = 0; i < kBiasRows / 4; ++i) {
-            const int r = i * 4 + (t >> 5);
+        for (int i = 0; i < kBiasRows / 8; ++i) {
+            const int r = i * 8 + (t >> 5);
             v[i] = r < n ? J.dz[(size_t)(r0 + r) * J.cols + c] : 0.0f;
         }
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < kBiasRows / 4; ++i) sm[(i * 4 + (t >> 5)) * 32 + (t & 31)] = v[i];
+        for (int i = 0; i < kBiasRows / 8; ++i) sm[(i * 8 + (t >> 5)) * 32 + (t & 31)] = v[i];
         __syncthreads();
         if (t < 32)
 #pragma unroll 16
@@ -447,32 +444,51 @@ __device__ __forceinline__ void bias_columns(const BiasJob &J, int cta, float *s
     else adam_update(J.w[c], J.m[c], J.v[c], s, J.adam);
 }
 
-// a row group (8 rows) of a minibatch per CTA
+// a row group (8 rows) of a minibatch per CTA; every thread finds its row once and has several loads in flight (a loop of
+// one load an iteration made the last link of a training step 19 us long)
 __device__ __forceinline__ void gather_rows(const GatherJob &J, int cta)
 {
-    for (int e = threadIdx.x; e < 8 * J.in; e += 128) {
-        const int r = cta * 8 + (e & 7), c = e >> 3;
-        float x = 0.0f;
-        if (r < J.valid && c < J.in_real) x = J.x[(size_t)(J.idx ? J.idx[r] : r) * J.in_real + c];
-        bf16 hi, lo;
-        split_bf16(x, hi, lo);
-        J.X.hi[blk(J.rows, r, c)] = hi;
-        J.X.lo[blk(J.rows, r, c)] = lo;
-        if (J.XT.hi) {
-            J.XT.hi[blk(J.in, c, r)] = hi;
-            J.XT.lo[blk(J.in, c, r)] = lo;
+    constexpr int U = 4;
+    const int t = threadIdx.x;
+    auto source = [&](int r) { return r < J.valid ? (J.idx ? J.idx[r] : r) : -1; };
+    const int r = cta * 8 + (t & 7), from = source(r);            // inputs: a thread's row, 32 columns a round
+    const int rt = cta * 8 + (t >> 5), from_t = J.tgt ? source(rt) : -1;   // targets: a warp's row
+    for (int c0 = t >> 3; c0 < J.in; c0 += 32 * U) {
+        float x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + 32 * u;
+            x[u] = from >= 0 && c < J.in_real ? J.x[(size_t)from * J.in_real + c] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + 32 * u;
+            if (c >= J.in) break;
+            bf16 hi, lo;
+            split_bf16(x[u], hi, lo);
+            J.X.hi[blk(J.rows, r, c)] = hi;
+            J.X.lo[blk(J.rows, r, c)] = lo;
+            if (J.XT.hi) {
+                J.XT.hi[blk(J.in, c, r)] = hi;
+                J.XT.lo[blk(J.in, c, r)] = lo;
+            }
         }
     }
-    if (J.tgt)
-        for (int e = threadIdx.x; e < 8 * J.out; e += 128) {
-            const int r = cta * 8 + e / J.out, c = e % J.out;
-            J.tgt[(size_t)r * J.out + c] =
-                r < J.valid && c < J.out_real ? J.t[(size_t)(J.idx ? J.idx[r] : r) * J.out_real + c] : 0.0f;
+    for (int c0 = t & 31; J.tgt && c0 < J.out; c0 += 32 * U) {
+        float y[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + 32 * u;
+            y[u] = from_t >= 0 && c < J.out_real ? J.t[(size_t)from_t * J.out_real + c] : 0.0f;
         }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (c0 + 32 * u < J.out) J.tgt[(size_t)rt * J.out + c0 + 32 * u] = y[u];
+    }
 }
 
 // one link of the chain: the tiles of up to two GEMMs, a bias gradient, the gathering of a minibatch
-__global__ void __launch_bounds__(128) k_mlp(const __grid_constant__ Jobs jobs)
+__global__ void __launch_bounds__(kThreads) k_mlp(const __grid_constant__ Jobs jobs)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     int b = blockIdx.x;
@@ -692,7 +708,7 @@ void launch(bec_mlp *m, Jobs &J)
     }
     const bool gemm = J.gemm[0].Ahi != nullptr;
     if (gemm) ensure_smem_limit((const void *)k_mlp, gemm_smem(64));
-    launch_after(k_mlp, total, 128, gemm ? gemm_smem(tn) : 0, m->s, J);
+    launch_after(k_mlp, total, kThreads, gemm ? gemm_smem(tn) : 0, m->s, J);
 }
 
 GatherJob gather_job(bec_mlp *m, int k, const float *x, const float *t, const int *idx, int rows, int valid, bool train)
