@@ -26,7 +26,7 @@
 // next minibatch is gathered beside the first layer's. A launch sets itself up (barriers, tensor memory) while the one
 // before it finishes (launch.cuh), and an epilogue fetches what it reads while the tile's operands load. Weights' operands alternate
 // between two buffers, so that a launch can update a layer that another tile of it
-// still reads. 78 us a step (batch 256, 400 steps with the set-up) against 314 us with one kernel per
+// still reads. 58 us a step (batch 256, 400 steps with the set-up) against 314 us with one kernel per
 // operation.
 #include <algorithm>
 #include <cstdlib>
@@ -66,18 +66,24 @@ __device__ __forceinline__ void split_bf16(float v, bf16 &hi, bf16 &lo)
 }
 
 // ---------------------------------------------------------------- GEMM on the 5th-generation tensor cores
-// C[M x N] = A[M x K] * B[N x K]^T with A = A_hi + A_lo, B = B_hi + B_lo; M, N, K multiples of 64. One CTA of 128
-// threads per 128 x tn tile of C (tn = 16, 32 or 64: the narrowest that keeps a launch within one CTA per SM, so that
-// a 256 x 256 product spreads over 32 SMs instead of 8). The FP32 accumulator lives in tensor memory (lane i = row i
-// of the tile). K runs in 64-wide stages through a ring of four: one thread issues the bulk copies of a stage's four
-// tiles onto an mbarrier, and, as each stage lands, per 16-wide K step the three tcgen05.mma (M 128, N tn, K 16, BF16
+// C[M x N] = A[M x K] * B[N x K]^T with A = A_hi + A_lo, B = B_hi + B_lo; M, N, K multiples of 64. One CTA of 256
+// threads per 64 x tn tile of C (tn = 16, 32, 64 or 128: the narrowest that keeps a launch within one CTA per SM, so that
+// a 256 x 256 product spreads over 64 SMs). The FP32 accumulator lives in tensor memory (row i of the tile in lane
+// 32 (i / 16) + i % 16). K runs in 64-wide stages through a ring of four: one thread issues the bulk copies of a stage's
+// four tiles onto an mbarrier, and, as each stage lands, per 16-wide K step the three tcgen05.mma (M 64, N tn, K 16, BF16
 // in, FP32 accumulate) lo*hi, hi*lo, hi*hi; tcgen05.commit arrives on the stage's second mbarrier when they are done.
-// Every wait is bounded. Rows of a last 64-row tile (M = 64 mod 128) are not loaded and not stored. The epilogue reads
-// the accumulator with tcgen05.ld: warps w and w + 4 own lanes 32w..32w+31, and take turns at EC columns (with four warps and
-// 16 columns a thread the arithmetic of an epilogue, tanh or Adam, is a chain twice as long).
+// Every wait is bounded. What a link reads besides the operand that the one before it has just written (the weights, the
+// epilogue's inputs) it fetches before it waits for that one (GemmJob::early).
+//
+// A link of the 256-wide chain at batch 256 is the arrival of its operands, then the last MMAs, then the epilogue. With
+// 128 x 16 tiles (144 KB of operands a CTA, 3.4 us to arrive; 0.6 us of MMAs; 1.9 us of tanh or 3.6 us of Adam in sixteen
+// columns a thread) a training step took 65 us of launches; with 64 x 16 tiles, four columns a thread and early fetches 45.
+//
+// The epilogue reads the accumulator with tcgen05.ld: warps w and w + 4 own the 16 rows of lanes 32 w, eight columns each
+// in turn, of which the idle upper lanes take half: EC columns a thread.
 constexpr int kThreads = 256;
-constexpr int GM = 128, GK = 64, GSTAGES = 4;
-constexpr int kTileA = GM * GK * 2;                           // 16 KiB each of hi and lo
+constexpr int GM = 64, GK = 64, GSTAGES = 4;
+constexpr int kTileA = GM * GK * 2;                           // 8 KiB each of hi and lo
 __host__ __device__ constexpr int stage_bytes(int tn) { return 2 * (kTileA + tn * GK * 2); }
 __host__ __device__ constexpr int gemm_smem(int tn) { return GSTAGES * stage_bytes(tn) + 128; }   // + mbarriers and TMEM slot
 
@@ -98,6 +104,7 @@ struct GemmJob {
     int Ra, Rb;                 // rows of the operand matrices
     int M, N, K, tn, ctas;
     int epi;
+    bool early;                 // B and the epilogue's inputs are older than the launch before this one
     const float *bias;          // [N]
     float *f32;                 // row-major [M x N] result (y, dz, gradient), may be NULL
     int f32_ld, f32_rows, f32_cols;      // ... stored for rows and columns below these
@@ -140,6 +147,9 @@ __device__ __forceinline__ float adam_update(float &w, float &m, float &v, float
     const float vi = b2 * v + (1.0f - b2) * gi * gi;
     m = mi;
     v = vi;
+    // (a zero moment changes nothing, and zeros, the padding's, would take the slow paths of division and square root:
+    // they made the epilogue of a layer of six inputs, padded to 64, 6.2 us long)
+    if (mi == 0.0f) return w;
     w -= a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + eps);
     return w;
 }
@@ -209,18 +219,18 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
                  : "memory");
 }
 
-// EC consecutive columns of one row, as operands: a 16-byte chunk of the plain matrix, and of the transposed one
+// EC consecutive columns of one row, as operands: half a chunk of the plain matrix, and of the transposed one
 // a 2-byte value per column (8 rows of consecutive lanes make a chunk)
-constexpr int EC = 8;
+constexpr int EC = 4;
 __device__ __forceinline__ void store_operands(const GemmJob &J, int row, int col, const float (&o)[EC])
 {
-    __align__(16) bf16 hi[EC], lo[EC];
+    __align__(8) bf16 hi[EC], lo[EC];
 #pragma unroll
     for (int q = 0; q < EC; ++q) split_bf16(o[q], hi[q], lo[q]);
     if (J.out.hi) {
         const size_t at = blk(J.M, row, col);
-        *reinterpret_cast<uint4 *>(J.out.hi + at) = *reinterpret_cast<const uint4 *>(hi);
-        *reinterpret_cast<uint4 *>(J.out.lo + at) = *reinterpret_cast<const uint4 *>(lo);
+        *reinterpret_cast<uint2 *>(J.out.hi + at) = *reinterpret_cast<const uint2 *>(hi);
+        *reinterpret_cast<uint2 *>(J.out.lo + at) = *reinterpret_cast<const uint2 *>(lo);
     }
     if (J.outT.hi) {
 #pragma unroll
@@ -312,13 +322,13 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
     const int tn = J.tn, tiles_n = J.N / tn, sbytes = stage_bytes(tn);
     const int t = threadIdx.x, warp = t >> 5;
     const int m0 = tile / tiles_n * GM, n0 = tile % tiles_n * tn;
-    const int rows = min(GM, J.M - m0), nk = J.K / GK;
-    // stage g at g * sbytes: A_hi (128 rows x 64 K), A_lo, B_hi (tn rows x 64 K), B_lo; then full and done barriers
+    const int nk = J.K / GK;
+    // stage g at g * sbytes: A_hi (64 rows x 64 K), A_lo, B_hi (tn rows x 64 K), B_lo; then full and done barriers
     const uint32_t full = saddr(sm + GSTAGES * sbytes), done = full + 8 * GSTAGES;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + GSTAGES * sbytes + 16 * GSTAGES);
 
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(saddr(tslot)) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(saddr(tslot)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (t == 0) {
@@ -331,31 +341,45 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
 
+    // this thread's row and first columns in the tile
+    const int lr = (warp & 3) * 16 + (t & 15), c0 = (warp >> 2) * 2 * EC + ((t >> 4) & 1) * EC;
+    const uint32_t ab = GM * GK * 2, bb = tn * GK * 2;
+    auto load_b = [&](int kb) {
+        const uint32_t dst = saddr(sm + (kb % GSTAGES) * sbytes) + 2 * kTileA, bar = full + 8 * (kb % GSTAGES);
+        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(2 * bb) : "memory");
+        const size_t b0 = blk(J.Rb, n0, kb * GK);
+        bulk_load(dst, J.Bhi + b0, bb, bar);
+        bulk_load(dst + bb, J.Blo + b0, bb, bar);
+    };
+    auto load_a = [&](int kb) {       // the stage's one arrival
+        const uint32_t dst = saddr(sm + (kb % GSTAGES) * sbytes), bar = full + 8 * (kb % GSTAGES);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * ab) : "memory");
+        const size_t a0 = blk(J.Ra, m0, kb * GK);
+        bulk_load(dst, J.Ahi + a0, ab, bar);
+        bulk_load(dst + kTileA, J.Alo + a0, ab, bar);
+    };
+    const int first = min(GSTAGES, nk);
+    Aux x;
+    if (J.early) {
+        if (t == 0)
+            for (int kb = 0; kb < first; ++kb) load_b(kb);
+        load_aux(J, x, m0 + lr, n0 + c0);
+    }
     wait_predecessor();
     allow_successor();
-    const int lr = (warp & 3) * 32 + (t & 31), c0 = (warp >> 2) * EC;    // this thread's row, and its first columns
-    Aux x;
-    if (lr < rows) load_aux(J, x, m0 + lr, n0 + c0);
+    if (!J.early) load_aux(J, x, m0 + lr, n0 + c0);
     bool ok = true;
     if (t == 0) {
         // instruction descriptor, kind::f16: D F32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1), both K-major,
         // N >> 3 at bits 17-22, M >> 4 at bits 24-28
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(GM >> 4) << 24);
-        auto load = [&](int kb) {
-            const int g = kb % GSTAGES;
-            const uint32_t dst = saddr(sm + g * sbytes), bar = full + 8 * g;
-            const uint32_t ab = rows * GK * 2, bb = tn * GK * 2;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * (ab + bb)) : "memory");
-            const size_t a0 = blk(J.Ra, m0, kb * GK), b0 = blk(J.Rb, n0, kb * GK);
-            bulk_load(dst, J.Ahi + a0, ab, bar);
-            bulk_load(dst + kTileA, J.Alo + a0, ab, bar);
-            bulk_load(dst + 2 * kTileA, J.Bhi + b0, bb, bar);
-            bulk_load(dst + 2 * kTileA + bb, J.Blo + b0, bb, bar);
-        };
+        for (int kb = 0; kb < first; ++kb) {
+            if (!J.early) load_b(kb);
+            load_a(kb);
+        }
         auto landed = [&](int kb) { return mbar_wait_bounded(full + 8 * (kb % GSTAGES), (kb / GSTAGES) & 1, all.limit_ns); };
         auto multiplied = [&](int kb) { return mbar_wait_bounded(done + 8 * (kb % GSTAGES), (kb / GSTAGES) & 1, all.limit_ns); };
-        int loaded = 0, waited = 0, issued = 0;
-        while (loaded < min(GSTAGES, nk)) load(loaded++);
+        int loaded = first, waited = 0, issued = 0;
         for (int kb = 0; kb < nk && ok; ++kb) {
             ok = landed(kb);
             // stall (fault injection): the first stage also waits for a flag that nothing sets
@@ -378,7 +402,10 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
             // refill the stage before this one once its MMAs have read it
             if (kb >= 1 && loaded < nk) {
                 ok = multiplied(kb - 1);
-                if (ok) load(loaded++);
+                if (ok) {
+                    load_b(loaded);
+                    load_a(loaded++);
+                }
             }
         }
         if (ok) ok = multiplied(nk - 1);
@@ -393,19 +420,20 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!failed) {
         float l = 0.0f;
-        for (int cb = c0; cb < tn; cb += 2 * EC) {
-            uint32_t r[EC];
+        for (int cb = 0; cb < tn; cb += 4 * EC) {
+            uint32_t r[2 * EC];
             asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                         : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cb));
+                         : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(cb + (warp >> 2) * 2 * EC)));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (lr < rows) {
-                float o[EC];
+            float o[EC];
 #pragma unroll
-                for (int q = 0; q < EC; ++q) o[q] = __uint_as_float(r[q]);
-                if (cb > c0) load_aux(J, x, m0 + lr, n0 + cb);
-                l += epilogue(J, m0 + lr, n0 + cb, o, x);
+            for (int q = 0; q < EC; ++q) {
+                const uint32_t upper = __shfl_sync(0xffffffffu, r[EC + q], t & 15);
+                o[q] = __uint_as_float(t & 16 ? upper : r[q]);
             }
+            if (cb > 0) load_aux(J, x, m0 + lr, n0 + cb + c0);
+            l += epilogue(J, m0 + lr, n0 + cb + c0, o, x);
         }
         if (J.epi == EPI_LOSS) {
             for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
@@ -414,7 +442,7 @@ __device__ void gemm_tile(const GemmJob &J, const Jobs &all, int tile, unsigned 
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem) : "memory");
 }
 
 // 32 columns per CTA, 128 rows at a time through shared memory, so that the loads overlap while the sum keeps its order
@@ -700,14 +728,14 @@ void launch(bec_mlp *m, Jobs &J)
     for (;; tn *= 2) {
         total = J.bias.ctas + J.gather.ctas;
         for (auto &g : J.gemm) {
-            g.tn = tn;
-            g.ctas = g.Ahi ? (g.M + GM - 1) / GM * (g.N / tn) : 0;
+            g.tn = std::min(tn, g.N % 128 ? 64 : 128);
+            g.ctas = g.Ahi ? g.M / GM * (g.N / tn) : 0;
             total += g.ctas;
         }
-        if (total <= m->sms || tn == 64) break;
+        if (total <= m->sms || tn == 128) break;
     }
     const bool gemm = J.gemm[0].Ahi != nullptr;
-    if (gemm) ensure_smem_limit((const void *)k_mlp, gemm_smem(64));
+    if (gemm) ensure_smem_limit((const void *)k_mlp, gemm_smem(128));
     launch_after(k_mlp, total, kThreads, gemm ? gemm_smem(tn) : 0, m->s, J);
 }
 
@@ -737,6 +765,8 @@ void forward_chain(bec_mlp *m, int k, int rows, int valid, bool train, float *ou
         Jobs J{};
         GemmJob &g = J.gemm[0];
         g = make_job(l ? m->X[l] : m->X0[k], rows, m->W[m->cur][l], ow, rows, ow, in, !last ? EPI_TANH : train ? EPI_LOSS : EPI_LINEAR);
+        // (the launch before the first layer's gathered its inputs and may have updated its weights)
+        g.early = l > 0;
         g.bias = m->p + m->boff[l];
         if (!last) {
             g.out = m->X[l + 1];
@@ -772,6 +802,7 @@ void backward_chain(bec_mlp *m, int k, int rows, const AdamArgs *adam, const Gat
         // dW [out x in] = dZ^T [out x rows] * (X^T [in x rows])^T
         GemmJob &g = J.gemm[0];
         g = make_job(m->DT[l + 1], ow, l ? m->XT[l] : m->XT0[k], in, ow, in, rows, adam ? EPI_ADAM : EPI_GRAD);
+        g.early = true;
         if (adam) {
             g.w = m->p + m->woff[l];
             g.m = m->m + m->woff[l];
@@ -789,6 +820,7 @@ void backward_chain(bec_mlp *m, int k, int rows, const AdamArgs *adam, const Gat
             // dX [rows x in] = dZ [rows x out] * (W^T [in x out])^T, times the tanh derivative: the next layer's dZ
             GemmJob &d = J.gemm[1];
             d = make_job(m->D[l + 1], rows, m->WT[m->cur][l], in, rows, in, ow, EPI_DX);
+            d.early = true;
             d.y = m->y[l];
             d.f32 = m->dz[l];
             d.f32_ld = in;
