@@ -264,8 +264,23 @@ __global__ void __launch_bounds__(256) k_prep(Cell *__restrict__ state, PlaneTil
     for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) state[first + i] = smw[T.reversed(i)];
 }
 
-// stored representation -> FFT_xy -> x-space cells (a.re, a.im, b.re, b.im) to out
-__global__ void __launch_bounds__(256) k_unprep(const Cell *__restrict__ state, PlaneTile T, float4 *__restrict__ out)
+// where x-space cells go: (a.re, a.im, b.re, b.im), or one component times scale in FP64, as the caller of a state wants it
+struct ToCells {
+    float4 *out;
+    __device__ void operator()(size_t i, const Cell &v) const { out[i] = make_float4(v.ar, v.ai, v.br, v.bi); }
+};
+struct ToComponent {
+    double2 *out;
+    double scale;
+    int second;
+    __device__ void operator()(size_t i, const Cell &v) const
+    {
+        out[i] = second ? make_double2(v.br * scale, v.bi * scale) : make_double2(v.ar * scale, v.ai * scale);
+    }
+};
+// stored representation -> FFT_xy -> x-space cells
+template <class Out>
+__global__ void __launch_bounds__(256) k_unprep(const Cell *__restrict__ state, PlaneTile T, Out out)
 {
     extern __shared__ Cell smw[];
     const int lchunk = T.lppc + T.lx + T.ly;
@@ -276,8 +291,7 @@ __global__ void __launch_bounds__(256) k_unprep(const Cell *__restrict__ state, 
     __syncthreads();
     T.forward(smw);
     for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) {
-        const Cell v = smw[T.natural(i)];
-        out[first + i] = make_float4(v.ar, v.ai, v.br, v.bi);
+        out(first + i, smw[T.natural(i)]);
     }
 }
 
@@ -591,13 +605,24 @@ void fp32_prep(float4 *state, const ClassGeom &c, const float4 *x, const float2 
     launch_prep(state, c, tx, ty, FromState{x}, s);
 }
 
-void fp32_unprep(const float4 *state, const ClassGeom &c, float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s)
+template <class Out>
+static void unprep(const float4 *state, const ClassGeom &c, const Out &out, const float2 *tx, const float2 *ty, cudaStream_t s)
 {
     if (c.n_traj <= 0) return;
     const PlaneTile T = plane_tile(c, tx, ty);
-    ensure_smem_limit((const void *)k_unprep, kMaxPlaneBytes);
-    k_unprep<<<plane_ctas(c, T), tile_threads(T.lppc + c.lx + c.ly), plane_bytes(T), s>>>(reinterpret_cast<const Cell *>(state), T, x);
+    ensure_smem_limit((const void *)k_unprep<Out>, kMaxPlaneBytes);
+    k_unprep<Out><<<plane_ctas(c, T), tile_threads(T.lppc + c.lx + c.ly), plane_bytes(T), s>>>(reinterpret_cast<const Cell *>(state),
+                                                                                              T, out);
     g_launches++;
+}
+void fp32_unprep(const float4 *state, const ClassGeom &c, float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s)
+{
+    unprep(state, c, ToCells{x}, tx, ty, s);
+}
+void fp32_unprep_component(const float4 *state, const ClassGeom &c, int second, double scale, double2 *x, const float2 *tx,
+                           const float2 *ty, cudaStream_t s)
+{
+    unprep(state, c, ToComponent{x, scale, second}, tx, ty, s);
 }
 
 void fp32_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,
@@ -692,5 +717,28 @@ void group_reduce(const double *traj_tot, const int *group_first, const int *gro
 {
     if (n_groups <= 0) return;
     k_group_reduce<<<n_groups, 256, 0, s>>>(traj_tot, group_first, group_count, out);
+    g_launches++;
+}
+
+namespace {
+// the profile of an ensemble: the compensated sum over its trajectories, in order
+__global__ void k_group_axial(const double *__restrict__ traj_axial, int row, const int *__restrict__ groups,
+                              const int *__restrict__ first, const int *__restrict__ count, int base,
+                              const int *__restrict__ off, double *__restrict__ out)
+{
+    const int g = groups ? groups[blockIdx.x] : blockIdx.x, i = blockIdx.y * blockDim.x + threadIdx.x;
+    if (i >= off[g + 1] - off[g]) return;
+    const double *src = traj_axial + (size_t)(first[g] - base) * row * 4 + i;
+    KSum acc;
+    for (int t = 0; t < count[g]; ++t) acc.add(src[(size_t)t * row * 4]);
+    out[off[g] + i] = acc.value();
+}
+} // namespace
+
+void group_axial(const double *traj_axial, int row, const int *groups, int n, const int *first, const int *count, int base,
+                 const int *off, double *out, cudaStream_t s)
+{
+    if (n <= 0) return;
+    k_group_axial<<<dim3(n, (4 * row + 127) / 128), 128, 0, s>>>(traj_axial, row, groups, first, count, base, off, out);
     g_launches++;
 }

@@ -164,6 +164,9 @@ void fp32_init_batched(float4 *state, const ClassGeom &c, const int *tgroup, con
 // x-space cells (a.re, a.im, b.re, b.im) -> stored representation (inverse transform over x and y), and back
 void fp32_prep(float4 *state, const ClassGeom &c, const float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s);
 void fp32_unprep(const float4 *state, const ClassGeom &c, float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s);
+// one component in FP64, times scale
+void fp32_unprep_component(const float4 *state, const ClassGeom &c, int second, double scale, double2 *x, const float2 *tx,
+                           const float2 *ty, cudaStream_t s);
 // kinetic phases of every cell of n_groups ensembles of a class (groups: their indices, device) for kick fraction frac
 void fp32_kick_table(float2 *tab, const ClassGeom &c, const GroupParamsF *gp, const int *groups, int n_groups, float frac,
                      cudaStream_t s);
@@ -178,6 +181,10 @@ void fp32_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const
 // fills n device step indexes
 void fp32_put_step(uint32_t *d_step, int n, uint32_t v, cudaStream_t s);
 int fp32_zpass_tiles(const ClassGeom &c);   // tiles per trajectory of an observing z pass (obs_partial layout)
+// for each of n groups g (groups[i], or i when NULL): traj_axial[traj][row][4] -> out + off[g], off[g + 1] - off[g] sums over
+// the count[g] trajectories from first[g] - base on
+void group_axial(const double *traj_axial, int row, const int *groups, int n, const int *first, const int *count, int base,
+                 const int *off, double *out, cudaStream_t s);
 // obs_partial[traj][tile][z][4] -> traj_axial[traj][z][4] * traj_scale[traj] (1 if NULL),
 // traj_tot[traj][4] = sum over z; traj_axial may be NULL
 void obs_reduce(const double *obs_partial, int n_traj, int tiles, int nz, const double *traj_scale,
