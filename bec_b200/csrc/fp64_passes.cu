@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(256) k64_evo_plane(double2 *A, double2 *B, con
         if (ly > 0) fft_freq<true>(sm64, cols, twy);
         fft_freq<true>(sm64, rows, twx);
     }
-    if (MODE == E_OBSERVE) {
+    if constexpr (MODE == E_OBSERVE) {
         const int plane = 1 << lplane;
         auto sums = [&](int pl, int i0, int di) {
             KVec<4> acc;
@@ -544,10 +544,10 @@ __global__ void __launch_bounds__(256) k64_evo_plane(double2 *A, double2 *B, con
                     for (int k = 0; k < 4; ++k) o[4 * pl + k] = r.v[k].value() * g.dV;
             }
         }
-        return;
+    } else {
+        for (int i = threadIdx.x; i < 2 * chunk; i += blockDim.x)
+            (i < chunk ? gA + i : gB + (i - chunk))[0] = sm64[MODE == E_TO_X ? natural(i) : reversed(i)];
     }
-    for (int i = threadIdx.x; i < 2 * chunk; i += blockDim.x)
-        (i < chunk ? gA + i : gB + (i - chunk))[0] = sm64[MODE == E_TO_X ? natural(i) : reversed(i)];
 }
 
 // A CTA holds 2^lp adjacent pencils of one component: [IFFT_z ->] scale -> `kicks` half kicks [-> FFT_z], from (sA, sB) to

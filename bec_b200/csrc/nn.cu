@@ -563,7 +563,7 @@ struct bec_mlp {
     size_t n_params = 0;
     // device memory, one slab per use: parameters and their operands; Adam moments and the second set of operands; the
     // buffers of a batch for inference, for its gradients, and for training. The first and, for kFirstBatch rows, the third
-    // exist from the start, the others from the first call that needs them.
+    // and fourth exist from the start, in one allocation, the others from the first call that needs them.
     char *slab[5] = {};
     int cap[5] = {};                 // 1, or the batch capacity of slabs 2 to 4
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;   // FP32 params, grads, Adam moments
@@ -904,7 +904,16 @@ bec_status bec_mlp_create(const int32_t *widths, int32_t n_layers, uint64_t seed
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking) != cudaSuccess)
         return bail(BEC_ERR_CUDA);
-    if ((st = reserve(m, SLAB_PARAMS, 1)) || (st = reserve(m, SLAB_FORWARD, kFirstBatch))) return bail(st);
+    // the parameters, and the buffers of a first batch, in one allocation (a later, larger batch gets slabs of its own)
+    const Slab at_once[3] = {SLAB_PARAMS, SLAB_FORWARD, SLAB_BACKWARD};
+    size_t used = 0;
+    for (Slab k : at_once) used += carve(m, k, nullptr, kFirstBatch);
+    if ((st = slab_alloc(&m->slab[SLAB_PARAMS], used))) return bail(st);
+    used = 0;
+    for (Slab k : at_once) {
+        used += carve(m, k, m->slab[SLAB_PARAMS] + used, kFirstBatch);
+        m->cap[k] = kFirstBatch;
+    }
     if (cudaMemsetAsync(m->d_err, 0, 2 * sizeof(int), m->s) != cudaSuccess) return bail(BEC_ERR_CUDA);
     // Glorot-uniform weights on the real block, zero padding and biases
     std::vector<float> h(m->n_params, 0.0f);

@@ -29,12 +29,12 @@ sys.path.insert(0, ROOT)
 # ncu: DRAM bytes (read + write) per cell of one launch of a pass kernel, from a capture of 64 x 32x32x256
 # trajectories (268 MB of state, larger than L2; dram__bytes_read.sum + dram__bytes_write.sum over the launch's
 # cells); traffic scales with the cells a launch processes (algorithmic: 32 B per cell).
-NCU_TRAFFIC_PER_CELL = {"plane_32x32x256": 28.44, "pencil_32x32x256": 28.47}
+NCU_TRAFFIC_PER_CELL = {"plane_32x32x256": 28.43, "pencil_32x32x256": 28.51}
 
 # ncu: thread-instructions per cell of one launch (smsp__inst_executed.sum x 32 / cells), from the same
 # capture. With the launch time they give the kernel's instruction issue rate, whose ceiling is one
 # warp-instruction per scheduler per clock: SMs x 4 x 32 thread-instructions per clock.
-NCU_INSTR_PER_CELL = {"plane_32x32x256": 354.9, "pencil_32x32x256": 131.8}
+NCU_INSTR_PER_CELL = {"plane_32x32x256": 282.9, "pencil_32x32x256": 96.6}
 
 N_TRAJ = 1024
 # stopping rules of the ground-state leg: |d mu|/mu between checks below 1e-7 stops every held-out set
@@ -534,7 +534,8 @@ def main():
             pk = sms * 4 * 32 * mhz * 1e6
             issue_roof = {"kernel": dom["kernel"], "thread_instructions_per_cell": NCU_INSTR_PER_CELL[dom["kernel"]],
                           "achieved": ach, "peak": pk, "unit": "thread-instr/s", "frac": ach / pk,
-                          "note": "instruction issue, the bound of this kernel: one warp-instruction per scheduler "
+                          "note": "instruction issue (a third of the instructions are packed FMAs, which take the FMA pipe "
+                                  "twice as long: that pipe is the nearer bound): one warp-instruction per scheduler "
                                   "per clock at the sampled SM clock; instructions per cell from ncu"}
     # the transforms' FLOPs (5 n log2 n per complex transform of n points; two components, one inverse and
     # one forward 3D transform per step) against the FP32 FMA pipes: the compute bound beside the HBM bound
