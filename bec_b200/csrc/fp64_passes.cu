@@ -13,13 +13,14 @@
 // What bounds it: latency. A 16x16x128 state is 512 KiB; at HBM rate the two passes would take 0.3 us. A pass is a
 // launch, one trip to L2 and back, and two to three radix-8 stages per axis in shared memory. Tiles are therefore
 // small (a plane, or two to eight pencils), so that one trajectory fills the chip. Measured on one 16x16x128 ground
-// state of 500 steps: 83.4 ms with one kernel per operation (30 launches a step), 5.33 ms here (8.43 ms before the
+// state of 500 steps: 83.4 ms with one kernel per operation (30 launches a step), 5.1 ms here (8.43 ms before the
 // twiddles and kick factors lay in shared memory at the pass's start and a launch overlapped the end of the one before). The measures of a
 // batch (mu, energy, norm, residual) took twenty launches and two synchronisations a state; here they take eight
 // launches for half the batch (96 states of 32x32x256 with 60 steps: the whole call 42.6 -> 23.2 ms).
 //
 // Real time (wigner.cu:178-199): the passes of k64_evo_plane and k64_evo_pencil below, over every trajectory of an ensemble.
 #include <algorithm>
+#include <climits>
 
 #include "engine.h"
 #include "launch.cuh"
@@ -627,7 +628,11 @@ size_t pencil_smem(int lz, int lp) { return sizeof(double2) * (((size_t)1 << (lz
 constexpr size_t kMaxSmem = 200 * 1024;
 
 int ilog(int n) { int r = 0; while ((1 << r) < n) ++r; return r; }
-int threads_for(int log_elems) { return log_elems >= 11 ? 256 : 128; }
+// A tile of 2048 elements or more takes 256 threads; so does one of 256 or more where the launch has no more than four CTAs an
+// SM, which then wait for one another's latency less (a step of one ground state of 32x32x256 29.8 -> 20.4 us, of 16x16x128
+// 10.3 -> 9.8; the pencil passes of four FP64 trajectories of 16x16x128, 256 CTAs: 27.4 -> 22.7 us a step; of 64, 4096 CTAs: 199
+// -> 208). The real-time plane pass, bound by arithmetic, keeps 128 (four trajectories 27.4 -> 26.3 us, 64: 199 -> 248).
+int threads_for(int log_elems, long long ctas) { return log_elems >= 11 || (log_elems >= 8 && ctas <= 4 * 148) ? 256 : 128; }
 
 template <int MODE, typename S>
 cudaError_t plane_launch(const Gs64Dims &d, const Gs64Tab &t, double2 *state, const Gs64Par *par, const double *norm_part,
@@ -636,7 +641,7 @@ cudaError_t plane_launch(const Gs64Dims &d, const Gs64Tab &t, double2 *state, co
     const size_t smem = plane_smem(d.lx, d.ly, d.lppc);
     cudaError_t e = ensure_smem_limit((const void *)k64_plane<MODE, S>, (int)kMaxSmem);
     if (e) return e;
-    return launch_after(k64_plane<MODE, S>, d.n * d.plane_ctas(), threads_for(d.lppc + d.lx + d.ly), smem, s, state, par, d.lx,
+    return launch_after(k64_plane<MODE, S>, d.n * d.plane_ctas(), threads_for(d.lppc + d.lx + d.ly, (long long)d.n * d.plane_ctas()), smem, s, state, par, d.lx,
                         d.ly, d.lz, d.lppc, t.x, t.y, norm_part, d.pencil_ctas(), src, out, kout, sums4, part);
 }
 
@@ -645,7 +650,7 @@ cudaError_t pencil_launch(const Gs64Dims &d, const Gs64Tab &t, double2 *state, c
 {
     cudaError_t e = ensure_smem_limit((const void *)k64_pencil, (int)kMaxSmem);
     if (e) return e;
-    return launch_after(k64_pencil, d.n * d.pencil_ctas(), threads_for(d.lz + d.lp), pencil_smem(d.lz, d.lp), s, state, par, d.lx,
+    return launch_after(k64_pencil, d.n * d.pencil_ctas(), threads_for(d.lz + d.lp, (long long)d.n * d.pencil_ctas()), pencil_smem(d.lz, d.lp), s, state, par, d.lx,
                         d.ly, d.lz, d.lp, t.z, t.kick, scale, what, part, kout);
 }
 
@@ -662,7 +667,7 @@ cudaError_t evo_pencil(const Evo64 &e, const double2 *sA, const double2 *sB, dou
     cudaError_t err = ensure_smem_limit((const void *)k64_evo_pencil<FROM_Z, TO_Z>, (int)kMaxSmem);
     if (err) return err;
     const GeomD &g = e.g;
-    return launch_after(k64_evo_pencil<FROM_Z, TO_Z>, 2 * n << (g.lx + g.ly - e.lp), threads_for(g.lz + e.lp),
+    return launch_after(k64_evo_pencil<FROM_Z, TO_Z>, 2 * n << (g.lx + g.ly - e.lp), threads_for(g.lz + e.lp, (long long)2 * n << (g.lx + g.ly - e.lp)),
                         evo_pencil_smem(g.lz, e.lp), s, sA, sB, dA, dB, g.lx, g.ly, g.lz, e.lp, n, e.z, (const double2 *)e.kick, scale,
                         kicks);
 }
@@ -674,7 +679,7 @@ cudaError_t evo_plane(const Evo64 &e, double2 *A, double2 *B, int n, uint32_t tr
     cudaError_t err = ensure_smem_limit((const void *)k64_evo_plane<MODE>, (int)kMaxSmem);
     if (err) return err;
     const GeomD &g = e.g;
-    return launch_after(k64_evo_plane<MODE>, n << (g.lz - e.lppc), threads_for(e.lppc + g.lx + g.ly),
+    return launch_after(k64_evo_plane<MODE>, n << (g.lz - e.lppc), threads_for(e.lppc + g.lx + g.ly, LLONG_MAX),
                         evo_plane_smem(g.lx, g.ly, e.lppc), s, A, B, g, e.lppc, e.x, e.y, traj0, step, obs, row);
 }
 
