@@ -669,7 +669,7 @@ bec_status time_captured(bec_ctx *ctx, double *ms, F &&enqueue)
 constexpr long long kSplitCells = 1 << 21;
 
 // Per grid class, the faster of the two pencil kernels for the full-kick pass of a steady step: the register
-// kernel (16 pencils per CTA of nz threads, 16 warps per SM) or the persistent TMA kernel (three CTAs per SM,
+// kernel (16 pencils per CTA of nz threads, 8 and 128 threads at nz = 256, 20 warps per SM) or the persistent TMA kernel (three CTAs per SM,
 // the next tile's load in flight). Both compute the same bits; each is timed over three launches after one
 // warm-up on the current state (the caller restores it).
 bec_status pick_pencil_kernels(bec_ctx *ctx)

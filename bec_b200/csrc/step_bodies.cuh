@@ -14,13 +14,13 @@
 //
 // plane pass (square planes N x N, N = 8, 16): one warp per 32/N planes. Lane c loads column c of its
 //   plane from HBM (each load instruction of the warp reads consecutive 16-byte cells), transforms it
-//   along y, writes it to an XOR-swizzled shared tile, reads back row c, transforms along x, applies
+//   along y, writes it to a padded shared tile, reads back row c, transforms along x, applies
 //   the nonlinear / loss / loss-noise step to its N cells, and returns the same way. Both components of
 //   a cell are one 16-byte cpair (fft_reg.cuh).
 // plane pass, 32 x 32 planes: two warps per plane, a 32-point line shared by lane L of each warp
 //   (split32.cuh).
-// pencil pass (nz = 64, 128, 256 = 16 G): 16 adjacent pencils of a trajectory per virtual block of
-//   nz threads. A four-step decomposition nz = 16 x G: each thread holds 16 elements (z = j + G m)
+// pencil pass (nz = 64, 128, 256 = 16 G): 16 (or 8) adjacent pencils of a trajectory per virtual block of
+//   nz (or nz / 2) threads. A four-step decomposition nz = 16 x G: each thread holds 16 elements (z = j + G m)
 //   and does a 16-point DFT, twiddles, and after one shared-memory transpose a G-point DFT across j;
 //   the kinetic phase e^{i k^2/2 dt} (wigner_kernel.cu:137-151) is applied in full k-space as the
 //   product of a per-pencil (kx, ky) factor and a per-kz factor; the forward transform retraces the
@@ -29,7 +29,7 @@
 // Shared lines are padded by one 16-byte cell, so that both the row-wise and the column-wise access of a quarter warp touch
 // eight different bank groups and every access has an address and a constant offset. (A tile that must stay dense, the
 // state held in shared memory, is swizzled on the cell index instead, col ^ (row & 7), at an instruction or two an access:
-// with every tile swizzled the 32 x 32 plane pass took 303.5 thread-instructions a cell, 280 padded, and a step of 256
+// with every tile swizzled the 32 x 32 plane pass took 303.5 thread-instructions a cell, 283 padded, and a step of 256
 // trajectories of 32x32x256 1.309 ms, 1.247; with eight pencils a CTA besides, and the line exchange in the plane's tile,
 // 1.215 to 1.231.)
 //
@@ -264,7 +264,7 @@ struct PencilArgs {
 };
 
 // The four-step z transform of a tile of PEN adjacent pencils (nz = 16 G; PEN * G threads), in three
-// stages separated by barriers of the tile's threads. buf holds PEN x NZ cells (swizzled rows of 16).
+// stages separated by barriers of the tile's threads. buf holds CELLS cells.
 //   inv1:  thread (p, j) = (t % PEN, t / PEN) holds z = j + G m, m < 16: inverse 16-point DFT over
 //          m -> k1, twiddle W^{-j k1}, to buf
 //   mid:   thread (q, p2) = (t % G, t / G) gathers k1 = q + G r (r < 16 / G) for all j: inverse G-point
