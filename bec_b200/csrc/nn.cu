@@ -40,6 +40,7 @@
 
 #include "engine.h"
 #include "launch.cuh"
+#include "mlp_tiles.h"
 
 namespace {
 
@@ -82,7 +83,7 @@ __device__ __forceinline__ void split_bf16(float v, bf16 &hi, bf16 &lo)
 // The epilogue reads the accumulator with tcgen05.ld: warps w and w + 4 own the 16 rows of lanes 32 w, eight columns each
 // in turn, of which the idle upper lanes take half: EC columns a thread.
 constexpr int kThreads = 256;
-constexpr int GM = 64, GK = 64, GSTAGES = 4;
+constexpr int GM = kTileRows, GK = 64, GSTAGES = 4;
 constexpr int kTileA = GM * GK * 2;                           // 8 KiB each of hi and lo
 __host__ __device__ constexpr int stage_bytes(int tn) { return 2 * (kTileA + tn * GK * 2); }
 __host__ __device__ constexpr int gemm_smem(int tn) { return GSTAGES * stage_bytes(tn) + 128; }   // + mbarriers and TMEM slot
@@ -581,6 +582,7 @@ struct bec_mlp {
     long long adam_t = 0;
     cudaStream_t s = nullptr;
     std::string err;
+    cudaError_t launched = cudaSuccess;      // the first launch since the last check that was refused
     // waits of the device side (read from the environment at every call): limit, fault injection
     int stall = 0;
     unsigned long long limit_ns = 2000000000ull;
@@ -717,7 +719,7 @@ GemmJob make_job(const Split &A, int Ra, const Split &B, int Rb, int M, int N, i
     return j;
 }
 
-// launches the jobs: column tiles as narrow as one CTA per SM allows
+// launches the jobs: column tiles as narrow as one CTA per SM allows. A launch that is refused is reported by check_gemm.
 void launch(bec_mlp *m, Jobs &J)
 {
     J.err = m->d_err;
@@ -728,15 +730,16 @@ void launch(bec_mlp *m, Jobs &J)
     for (;; tn *= 2) {
         total = J.bias.ctas + J.gather.ctas;
         for (auto &g : J.gemm) {
-            g.tn = std::min(tn, g.N % 128 ? 64 : 128);
-            g.ctas = g.Ahi ? g.M / GM * (g.N / tn) : 0;
+            g.tn = tile_cols(g.N, tn);
+            g.ctas = g.Ahi ? tile_ctas(g.M, g.N, tn) : 0;
             total += g.ctas;
         }
-        if (total <= m->sms || tn == 128) break;
+        if (total <= m->sms || tn == kWidestTile) break;
     }
     const bool gemm = J.gemm[0].Ahi != nullptr;
-    if (gemm) ensure_smem_limit((const void *)k_mlp, gemm_smem(128));
-    launch_after(k_mlp, total, kThreads, gemm ? gemm_smem(tn) : 0, m->s, J);
+    cudaError_t e = gemm ? ensure_smem_limit((const void *)k_mlp, gemm_smem(kWidestTile)) : cudaSuccess;
+    if (!e) e = launch_after(k_mlp, total, kThreads, gemm ? gemm_smem(tn) : 0, m->s, J);
+    if (!m->launched) m->launched = e;
 }
 
 GatherJob gather_job(bec_mlp *m, int k, const float *x, const float *t, const int *idx, int rows, int valid, bool train)
@@ -857,10 +860,12 @@ void split_weights(bec_mlp *m)
     }
 }
 
-// BEC_ERR_CUDA when a GEMM since the last check gave up a wait (synchronises the stream)
+// BEC_ERR_CUDA when a launch since the last check was refused, or a GEMM gave up a wait (synchronises the stream)
 bec_status check_gemm(bec_mlp *m)
 {
     int e = 0;
+    const cudaError_t launched = m->launched;
+    m->launched = cudaSuccess;
     if (cudaMemcpyAsync(&e, m->d_err, sizeof(int), cudaMemcpyDeviceToHost, m->s) != cudaSuccess ||
         cudaStreamSynchronize(m->s) != cudaSuccess) {
         m->err = cudaGetErrorString(cudaGetLastError());
@@ -869,6 +874,11 @@ bec_status check_gemm(bec_mlp *m)
     if (e) {
         cudaMemsetAsync(m->d_err, 0, sizeof(int), m->s);
         m->err = "MLP GEMM: a tensor-core wait gave up";
+        return BEC_ERR_CUDA;
+    }
+    if (launched != cudaSuccess) {
+        m->err = cudaGetErrorString(launched);
+        cudaGetLastError();
         return BEC_ERR_CUDA;
     }
     return BEC_OK;
