@@ -565,8 +565,11 @@ struct bec_mlp {
     // device memory, one slab per use: parameters and their operands; Adam moments and the second set of operands; the
     // buffers of a batch for inference, for its gradients, and for training. The first and, for kFirstBatch rows, the third
     // and fourth exist from the start, in one allocation, the others from the first call that needs them.
-    char *slab[5] = {};
+    char *slab[5] = {};              // the allocations, and
+    size_t size[5] = {};             // ... their bytes
+    char *base[5] = {};              // where each use's buffers lie
     int cap[5] = {};                 // 1, or the batch capacity of slabs 2 to 4
+    size_t bytes = 0, limit = 0;     // device bytes in use; BEC_DEVICE_BYTES_LIMIT at creation (0: none)
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;   // FP32 params, grads, Adam moments
     std::vector<Split> W[2], WT[2];  // per layer the weights' operands, plain and transposed: the current set and the
     int cur = 0;                     // one that a training step writes
@@ -673,29 +676,47 @@ size_t carve(bec_mlp *m, Slab which, char *base, int cap)
     return c.used;
 }
 
-bec_status slab_alloc(char **p, size_t bytes)
+// With a byte limit set, an allocation that would take the network past it fails without reaching the device.
+bec_status slab_alloc(bec_mlp *m, char **p, size_t bytes)
 {
+    *p = nullptr;
+    if (m->limit && m->bytes + bytes > m->limit) return BEC_ERR_OUT_OF_MEMORY;
     if (cudaMalloc((void **)p, bytes) != cudaSuccess) { cudaGetLastError(); *p = nullptr; return BEC_ERR_OUT_OF_MEMORY; }
+    m->bytes += bytes;
     return BEC_OK;
 }
 
-// makes a slab hold at least cap rows (batch slabs; 1 for the others)
+void slab_free(bec_mlp *m, char *p, size_t bytes)
+{
+    if (!p) return;
+    cudaStreamSynchronize(m->s);
+    cudaFree(p);
+    m->bytes -= bytes;
+}
+
+// makes a slab hold at least cap rows (batch slabs; 1 for the others). When the memory is not to be had the first batch's
+// buffers, which lie in the parameters' slab, stay as they are; others are given back to make room, and cap says so.
 bec_status reserve(bec_mlp *m, Slab which, int cap)
 {
     if (cap <= m->cap[which]) return BEC_OK;
+    slab_free(m, m->slab[which], m->size[which]);
     if (m->slab[which]) {
-        cudaStreamSynchronize(m->s);
-        cudaFree(m->slab[which]);
-        m->slab[which] = nullptr;
+        m->slab[which] = m->base[which] = nullptr;
         m->cap[which] = 0;
     }
-    bec_status st = slab_alloc(&m->slab[which], carve(m, which, nullptr, cap));
-    if (st) return st;
+    const size_t bytes = carve(m, which, nullptr, cap);     // (leaves the slab's pointers null)
+    const bec_status st = slab_alloc(m, &m->slab[which], bytes);
+    if (st) {
+        if (m->base[which]) carve(m, which, m->base[which], m->cap[which]);
+        return st;
+    }
+    m->size[which] = bytes;
+    m->base[which] = m->slab[which];
     carve(m, which, m->slab[which], cap);
-    m->cap[which] = cap;
     if (which == SLAB_ADAM && (cudaMemsetAsync(m->m, 0, sizeof(float) * m->n_params, m->s) != cudaSuccess ||
                                cudaMemsetAsync(m->v, 0, sizeof(float) * m->n_params, m->s) != cudaSuccess))
         return BEC_ERR_CUDA;
+    m->cap[which] = cap;
     return BEC_OK;
 }
 
@@ -898,6 +919,7 @@ bec_status bec_mlp_create(const int32_t *widths, int32_t n_layers, uint64_t seed
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { cudaGetLastError(); return BEC_ERR_NO_DEVICE; }
     bec_mlp *m = new bec_mlp();
+    if (const char *lim = std::getenv("BEC_DEVICE_BYTES_LIMIT")) m->limit = (size_t)std::strtoull(lim, nullptr, 10);
     m->L = n_layers;
     m->w_real.assign(widths, widths + n_layers + 1);
     m->w.resize(n_layers + 1);
@@ -918,10 +940,12 @@ bec_status bec_mlp_create(const int32_t *widths, int32_t n_layers, uint64_t seed
     const Slab at_once[3] = {SLAB_PARAMS, SLAB_FORWARD, SLAB_BACKWARD};
     size_t used = 0;
     for (Slab k : at_once) used += carve(m, k, nullptr, kFirstBatch);
-    if ((st = slab_alloc(&m->slab[SLAB_PARAMS], used))) return bail(st);
+    if ((st = slab_alloc(m, &m->slab[SLAB_PARAMS], used))) return bail(st);
+    m->size[SLAB_PARAMS] = used;
     used = 0;
     for (Slab k : at_once) {
-        used += carve(m, k, m->slab[SLAB_PARAMS] + used, kFirstBatch);
+        m->base[k] = m->slab[SLAB_PARAMS] + used;
+        used += carve(m, k, m->base[k], kFirstBatch);
         m->cap[k] = kFirstBatch;
     }
     if (cudaMemsetAsync(m->d_err, 0, 2 * sizeof(int), m->s) != cudaSuccess) return bail(BEC_ERR_CUDA);
@@ -1074,8 +1098,9 @@ bec_status bec_mlp_train(bec_mlp *m, const float *x, const float *target, int32_
         return c.used;
     };
     char *slab = nullptr;
-    if ((st = slab_alloc(&slab, samples(nullptr)))) return st;
-    struct F { char *p; cudaStream_t s; ~F() { cudaStreamSynchronize(s); cudaFree(p); } } f{slab, m->s};
+    const size_t slab_bytes = samples(nullptr);
+    if ((st = slab_alloc(m, &slab, slab_bytes))) return st;
+    struct F { bec_mlp *m; char *p; size_t n; ~F() { slab_free(m, p, n); } } f{m, slab, slab_bytes};
     samples(slab);
     if (cudaMemcpyAsync(dx, x, sizeof(float) * (size_t)n * in_r, cudaMemcpyHostToDevice, m->s) != cudaSuccess ||
         cudaMemcpyAsync(dt, target, sizeof(float) * (size_t)n * out_r, cudaMemcpyHostToDevice, m->s) != cudaSuccess ||

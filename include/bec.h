@@ -416,6 +416,8 @@ bec_status bec_profile_steps(bec_ctx *ctx, int32_t n_steps, int32_t max_classes,
  * seeds bec_ground_state_batch (warm_start), which alone decides convergence.
  * widths has n_layers + 1 entries (inputs, hidden..., outputs). Host parameter
  * layout: for each layer W [out x in] row-major, then b [out].
+ * BEC_DEVICE_BYTES_LIMIT at creation bounds a network's device buffers as it does a context's: the call that
+ * would pass it fails with BEC_ERR_OUT_OF_MEMORY, and smaller ones go on.
  */
 typedef struct bec_mlp bec_mlp;
 bec_status bec_mlp_create(const int32_t *widths, int32_t n_layers, uint64_t seed, bec_mlp **out);
