@@ -1146,7 +1146,12 @@ bec_status bec_mlp_train(bec_mlp *m, const float *x, const float *target, int32_
     }
     std::vector<float> hist(steps, 0.0f);
     cudaMemcpyAsync(hist.data(), dhist, sizeof(float) * steps, cudaMemcpyDeviceToHost, m->s);
-    if ((st = check_gemm(m))) return st;
+    if ((st = check_gemm(m))) {
+        // a tile that gave up has written neither its weights nor their operands in the set that is current now
+        split_weights(m);
+        cudaStreamSynchronize(m->s);
+        return st;
+    }
     if (loss_history)
         for (int s = 0; s < steps; ++s) loss_history[s] = hist[s];
     return cudaGetLastError() == cudaSuccess ? BEC_OK : BEC_ERR_CUDA;

@@ -46,3 +46,22 @@ def test_refused_batch_leaves_small_ones_as_they_were(call, grown, monkeypatch):
     np.testing.assert_array_equal(bounded.get_params(), free.get_params())
     bounded.close()
     free.close()
+
+
+@pytest.mark.parametrize("steps", [1, 2, 3])
+def test_training_that_gave_up_leaves_operands_of_its_weights(steps, monkeypatch):
+    x, t = samples(100)
+    net, fresh = MLP(WIDTHS, seed=3), MLP(WIDTHS, seed=4)
+    monkeypatch.setenv("BEC_GEMM_INJECT_STALL", "1")
+    monkeypatch.setenv("BEC_STEP_WAIT_LIMIT_MS", "20")
+    with pytest.raises(BecError):
+        net.train(x, t, steps, batch=64)
+    monkeypatch.delenv("BEC_GEMM_INJECT_STALL")
+    monkeypatch.delenv("BEC_STEP_WAIT_LIMIT_MS")
+    fresh.set_params(net.get_params())
+    np.testing.assert_array_equal(net.forward(x), fresh.forward(x))
+    got, want = net.gradients(x, t), fresh.gradients(x, t)
+    np.testing.assert_allclose(got[0], want[0], rtol=LOSS)
+    np.testing.assert_array_equal(got[1], want[1])
+    net.close()
+    fresh.close()
