@@ -2369,8 +2369,8 @@ bec_status bec_init_group(bec_ctx *ctx, int32_t group, const double *psi_gs, con
         CKL();
     } else {
         // bring the other groups to a clean step boundary first (without others, the state is overwritten as it is)
-        if (ctx->groups.size() == 1) ctx->pending = ctx->has_pulse = false;
-        else if ((st = batched_resolve(ctx))) return st;
+        const bool alone = ctx->groups.size() == 1;
+        if (!alone && (st = batched_resolve(ctx))) return st;
         if ((st = gs_stage_ready(ctx))) return st;
         size_t off = 0;
         for (int g = 0; g < group; ++g) off += sizeof(double2) * (size_t)ctx->groups[g].gd.cells;
@@ -2399,6 +2399,7 @@ bec_status bec_init_group(bec_ctx *ctx, int32_t group, const double *psi_gs, con
         fp32_init_group(base, sub, gr.gf, gr.gs_dev, nz, tx, ty, s);
         if (nz) { cudaStreamSynchronize(s); cudaFree(nz); }
         CKL();
+        if (alone) ctx->pending = ctx->has_pulse = false;     // (a call that failed before this has changed nothing)
     }
     gr.initialised = true;
     ctx->last_launches = g_launches - l0;
@@ -2443,8 +2444,8 @@ bec_status bec_init_groups(bec_ctx *ctx, int32_t n, const int32_t *groups, const
         ctx->last_launches = g_launches - l0;
         return BEC_OK;
     }
-    if (n == ng) ctx->pending = ctx->has_pulse = false;      // every group listed: the whole state is overwritten
-    else if ((st = batched_resolve(ctx))) return st;
+    // with every group listed the whole state is overwritten: what is pending goes once nothing can fail before that
+    if (n < ng && (st = batched_resolve(ctx))) return st;
     const long long l0 = g_launches;
     cudaStream_t s = ctx->stream;
     if (!ctx->d_gs_ptrs) CKC(dalloc(ctx, &ctx->d_gs_ptrs, (size_t)ng));
@@ -2472,6 +2473,11 @@ bec_status bec_init_groups(bec_ctx *ctx, int32_t n, const int32_t *groups, const
         ctx->gs_ptrs_host = tab;
     }
     CKC(cudaEventRecord(ctx->ev_h2d, s));
+    for (auto &c : ctx->classes) {
+        float2 *tx, *ty;
+        if ((st = get_tw32_full(ctx, c.geom.nx, &tx)) || (st = get_tw32_full(ctx, c.geom.ny, &ty))) return st;
+    }
+    if (n == ng) ctx->pending = ctx->has_pulse = false;
     // one initialisation pass per run of consecutive listed trajectories
     for (auto &c : ctx->classes) {
         std::vector<std::pair<int, int>> runs;    // (first local trajectory, count)
