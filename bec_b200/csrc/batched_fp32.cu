@@ -390,15 +390,17 @@ __device__ __forceinline__ float2 kick_phase(const GroupParamsF &P, int x, int y
     return kin_phase(k2h * (double)frac);
 }
 
-// the phases of every cell of each of the class's ensembles (ensemble e: parameters gp[groups[e]])
-__global__ void k_kick_table(float2 *__restrict__ tab, const GroupParamsF *__restrict__ gp, const int *__restrict__ groups,
+// the phases of every cell of each of the class's n ensembles (ensemble e: parameters gp[groups[e]])
+__global__ void k_kick_table(float2 *__restrict__ tab, const GroupParamsF *__restrict__ gp, const int *__restrict__ groups, int n,
                              int lx, int ly, int lz, float frac)
 {
-    const GroupParamsF &P = gp[groups[blockIdx.y]];
-    const int cells = 1 << (lx + ly + lz);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += gridDim.x * blockDim.x)
-        tab[(size_t)blockIdx.y * cells + i] = kick_phase(P, i & ((1 << lx) - 1), (i >> lx) & ((1 << ly) - 1), i >> (lx + ly),
-                                                         1 << lx, 1 << ly, 1 << lz, frac);
+    const int lcells = lx + ly + lz;
+    const size_t total = (size_t)n << lcells;
+    for (size_t at = blockIdx.x * (size_t)blockDim.x + threadIdx.x; at < total; at += (size_t)gridDim.x * blockDim.x) {
+        const int i = (int)(at & ((1u << lcells) - 1));
+        tab[at] = kick_phase(gp[groups[at >> lcells]], i & ((1 << lx) - 1), (i >> lx) & ((1 << ly) - 1), i >> (lx + ly), 1 << lx,
+                             1 << ly, 1 << lz, frac);
+    }
 }
 
 struct ZArgs {
@@ -654,8 +656,8 @@ void fp32_kick_table(float2 *tab, const ClassGeom &c, const GroupParamsF *gp, co
                      cudaStream_t s)
 {
     if (n_groups <= 0) return;
-    k_kick_table<<<dim3((unsigned)std::min((c.cells + 127) / 128, 1024), (unsigned)n_groups), 128, 0, s>>>(tab, gp, groups, c.lx,
-                                                                                                          c.ly, c.lz, frac);
+    const size_t blocks = ((size_t)n_groups * c.cells + 127) / 128;
+    k_kick_table<<<(int)std::min<size_t>(blocks, 148 * 128), 128, 0, s>>>(tab, gp, groups, n_groups, c.lx, c.ly, c.lz, frac);
     g_launches++;
 }
 

@@ -1562,12 +1562,12 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
                     dalloc(ctx, &d_groups, n) == cudaSuccess && dalloc(ctx, &c.d_tindex, nt) == cudaSuccess) {
                     CKA(cudaMemcpyAsync(c.d_tindex, ti.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream));
                     CKA(cudaMemcpyAsync(d_groups, c.groups.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
-                    for (int k = 0; k < 2; ++k) {
+                    for (int k = 0; k < 2; ++k)
                         fp32_kick_table(tab[k], c.geom, ctx->d_gparams, d_groups, (int)n, k ? 1.0f : 0.5f, ctx->stream);
-                        c.kick_tab[k] = tab[k];
-                    }
+                    if (cudaGetLastError() == cudaSuccess)
+                        for (int k = 0; k < 2; ++k) c.kick_tab[k] = tab[k];
                 }
-                if (cudaGetLastError() != cudaSuccess && c.kick_tab[0]) return bail(BEC_ERR_CUDA);
+                cudaGetLastError();
             }
         }
     }
