@@ -177,6 +177,50 @@ cudaError_t dalloc(bec_ctx *ctx, T **p, size_t n)
     return e;
 }
 
+template <typename T>
+void dfree(bec_ctx *ctx, T *p, size_t n)
+{
+    if (!p) return;
+    cudaFree(p);
+    ctx->allocs.erase(std::find(ctx->allocs.begin(), ctx->allocs.end(), (void *)p));
+    ctx->alloc_bytes -= n * sizeof(T);
+}
+
+// Gives back the phase tables of the general z pass, which evaluates the phases without them, and the captured steps that
+// read them; false when there are none.
+bool drop_kick_tables(bec_ctx *ctx)
+{
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
+    bool any = false;
+    for (auto &c : ctx->classes) any = any || c.kick_tab[0];
+    if (!any) return false;
+    cudaStreamSynchronize(ctx->stream);
+    for (auto &c : ctx->classes)
+        for (float2 *&t : c.kick_tab) {
+            dfree(ctx, t, c.groups.size() * c.geom.cells);
+            t = nullptr;
+        }
+    for (cudaGraphExec_t &g : ctx->step_graph)
+        if (g) {
+            cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+    return true;
+}
+
+// a buffer that a call cannot do without
+template <typename T>
+cudaError_t dalloc_needed(bec_ctx *ctx, T **p, size_t n)
+{
+    cudaError_t e = dalloc(ctx, p, n);
+    if (e == cudaErrorMemoryAllocation && drop_kick_tables(ctx)) {
+        cudaGetLastError();
+        e = dalloc(ctx, p, n);
+    }
+    return e;
+}
+
 double2 cd(double re, double im) { return make_double2(re, im); }
 
 // report.tex rotation matrix: [[cos t/2, -i e^{-i phi} sin t/2], [-i e^{i phi} sin t/2, cos t/2]]
@@ -320,7 +364,7 @@ bec_status get_tw32_full(bec_ctx *ctx, int n, float2 **out)
     std::vector<float2> f(n);
     for (int k = 0; k < n; ++k) f[k] = tw32_unit(k, n);
     float2 *d = nullptr;
-    CKC(dalloc(ctx, &d, f.size()));
+    CKC(dalloc_needed(ctx, &d, f.size()));
     CKC(cudaMemcpyAsync(d, f.data(), f.size() * sizeof(float2), cudaMemcpyHostToDevice, ctx->stream));
     ctx->tw32_full[n] = d;
     *out = d;
@@ -1545,8 +1589,8 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
             }
         }
         CKA(dalloc(ctx, &ctx->scratch4, (size_t)ctx->max_cells));
-        // the general z pass evaluates its phases in FP64: a table per ensemble where it stays small, after all that a
-        // context cannot do without
+        // the general z pass evaluates its phases in FP64: a table per ensemble where it stays small, given back when a later
+        // buffer needs the room
         for (auto &c : ctx->classes) {
             if (fp32_fast_pencil_supported(c.geom)) continue;
             const size_t nt = (size_t)c.geom.n_traj;
@@ -1568,6 +1612,8 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
                         for (int k = 0; k < 2; ++k) c.kick_tab[k] = tab[k];
                 }
                 cudaGetLastError();
+                if (!c.kick_tab[0])
+                    for (int k = 0; k < 2; ++k) dfree(ctx, tab[k], n * c.geom.cells);
             }
         }
     }
@@ -2334,7 +2380,7 @@ bec_status gs_stage_ready(bec_ctx *ctx)
     if (ctx->gs_stage) return BEC_OK;
     size_t total = 0;
     for (auto &gr : ctx->groups) total += sizeof(double2) * (size_t)gr.gd.cells;
-    CKC(dalloc(ctx, &ctx->gs_stage, total));
+    CKC(dalloc_needed(ctx, &ctx->gs_stage, total));
     return BEC_OK;
 }
 } // namespace
@@ -2448,7 +2494,7 @@ bec_status bec_init_groups(bec_ctx *ctx, int32_t n, const int32_t *groups, const
     if (n < ng && (st = batched_resolve(ctx))) return st;
     const long long l0 = g_launches;
     cudaStream_t s = ctx->stream;
-    if (!ctx->d_gs_ptrs) CKC(dalloc(ctx, &ctx->d_gs_ptrs, (size_t)ng));
+    if (!ctx->d_gs_ptrs) CKC(dalloc_needed(ctx, &ctx->d_gs_ptrs, (size_t)ng));
     // the staging area holds the listed ground states in group order at the call's element size, so that
     // consecutive groups whose host buffers are adjacent arrive in one copy
     const size_t esz = host_type == BEC_HOST_R32 ? sizeof(float) : c64 ? sizeof(float2) : sizeof(double2);
