@@ -636,7 +636,8 @@ bec_status batched_step(bec_ctx *ctx, float pre, bool put_step)
 //   2, 3  as 0, 1 with each class's non-observing pencil pass on the faster pencil kernel (pick_pencil_kernels)
 //   4 + k  the fused step kernel on work list k (two-phase, interleaved at 0.5, 1, 2, 4 waves)
 // BEC_STEP_PLAN in the environment forces one ("unfused" = 0, "unfused-20" = 1, "unfused-tma" = 2 and
-// "unfused-20-tma" = 3 with every class on the TMA pencil kernel, "0".."4" = fused k); otherwise a choice
+// "unfused-20-tma" = 3 with every class on the TMA pencil kernel, "unfused-onchip" and "unfused-split", "-pencil", "-plane" = 2
+// with those passes wherever they exist, "0".."4" = fused k); otherwise a choice
 // cached for the same class mix on this device is reused, or every candidate is timed on a copy of the state
 // (BEC_AUTOTUNE=0 skips the timing and takes candidate 0).
 constexpr int kPerPassCandidates = 4;
@@ -876,6 +877,15 @@ bec_status ensure_plan(bec_ctx *ctx)
             c.pencil_kind = kPencilRegister;
             c.onchip = fp32_onchip_supported(c.geom);
             c.split_pencil = c.split_plane = false;
+        }
+        how = "forced";
+    } else if (fs == "unfused-split" || fs == "unfused-split-pencil" || fs == "unfused-split-plane") {
+        cand = 2;                                      // four cells a thread in both passes, or one, of the classes they cover
+        for (auto &c : ctx->classes) {
+            c.pencil_kind = kPencilRegister;
+            c.onchip = false;
+            c.split_pencil = fs != "unfused-split-plane" && fp32_fast_pencil_supported(c.geom);
+            c.split_plane = fs != "unfused-split-pencil" && fp32_plane_split_supported(c.geom);
         }
         how = "forced";
     } else if (!fs.empty()) {

@@ -5,7 +5,9 @@
 // calls wait_predecessor(), which returns once the predecessor has completed and its writes are visible. It then calls
 // allow_successor(), so that the kernel after it may start in turn: because every kernel waits before it lets the next one
 // start, a kernel that has started knows that everything before its direct predecessor is complete. Nothing that the
-// direct predecessor writes may be touched before the wait.
+// direct predecessor writes may be touched before the wait. An ordinary load through a __restrict__ pointer could be moved
+// above it by the compiler, which sees no write to that memory: what a predecessor writes is read by volatile loads (copies
+// to shared memory, ld_cg) or through pointers that may alias.
 #pragma once
 
 #include <cuda_runtime.h>

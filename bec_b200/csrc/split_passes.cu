@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(PencilSplit<NZ>::THREADS) k_pencil_split(cpair
 
     cpair x[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = g[(size_t)(j + G * (q + 4 * i)) * plane];
+    for (int i = 0; i < 4; ++i) x[i] = ld_cg(g + (size_t)(j + G * (q + 4 * i)) * plane);
     line<16, true, 4>(x, ex + u, LANES, q, sync);         // over m -> k1 = q + 4 i
 #pragma unroll
     for (int i = 0; i < 4; ++i) {

@@ -48,7 +48,7 @@ using fftreg::cpair;
 using fftreg::dft;
 using fftreg::f32x2;
 
-// a cell from L2 (ld.global.cg)
+// a cell from L2 (ld.global.cg; a volatile load, which keeps its place among waits and barriers)
 __device__ __forceinline__ cpair ld_cg(const cpair *p)
 {
     const ulonglong2 u = __ldcg(reinterpret_cast<const ulonglong2 *>(p));

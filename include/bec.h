@@ -375,7 +375,8 @@ int32_t bec_step_graphs(const bec_ctx *ctx);
  * fastest for this class mix and device (cached per process). BEC_STEP_PLAN in the environment
  * forces one (unfused, unfused-20, unfused-tma and unfused-20-tma with every class on the TMA
  * pencil kernel, unfused-onchip with every 8x8x64 class's steady steps as one launch holding each
- * trajectory in shared memory, or 0..4 for the work lists), BEC_AUTOTUNE=0 takes the per-pass launches
+ * trajectory in shared memory, unfused-split with four cells per thread in every pass that has such a
+ * kernel, unfused-split-pencil and unfused-split-plane in the one, or 0..4 for the work lists), BEC_AUTOTUNE=0 takes the per-pass launches
  * untimed; every schedule computes the same bits. The reference has one fixed schedule of eight
  * launches per ensemble and step (wigner.cu:178-199) with cuFFT plans built by batchfftPlan3d
  * (batchfft.cu:22-100). */
