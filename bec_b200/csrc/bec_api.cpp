@@ -95,7 +95,8 @@ struct bec_ctx {
     bool pencil_tuned = false;           // per-pass pencil launches: each class's own pencil kernel (pencil_kind)
     bool step_onchip = false;            // the step being launched is steady: classes with `onchip` take one launch
     int *d_pflags = nullptr;             // batched: [0] error flag of the TMA pencil pass, [1] a flag nothing sets
-    std::string plan_desc;               // the chosen plan and the autotuner's timings (JSON)
+    std::string plan_desc;               // the chosen plan and the autotuner's timings (JSON), and
+    std::string plan_short;              // ... without those of the passes with four cells per thread
     cudaGraphExec_t step_graph[3] = {nullptr, nullptr, nullptr};   // kGraphSteps steps, 1 step, kLongSteps
     long long graph_kernels[3] = {0, 0, 0};               // kernels per replay of each
     bool long_failed = false;            // the kLongSteps graph could not be captured
@@ -995,6 +996,7 @@ bec_status ensure_plan(bec_ctx *ctx)
                                          : 2 * n_classes);
     if (fused) j += ", \"grid\": " + std::to_string(ctx->plan.grid) + ", \"items\": " + std::to_string(ctx->plan.n_items);
     j += ", \"pencil_kernels\": [";
+    std::string shorter = j;
     bool firstc = true;
     for (auto &c : ctx->classes) {
         if (c.geom.n_traj == 0) continue;
@@ -1003,22 +1005,25 @@ bec_status ensure_plan(bec_ctx *ctx)
         const int sp = ctx->pencil_tuned ? (c.split_pencil ? 1 : 0) | (c.split_plane ? 2 : 0) : 0;
         std::snprintf(buf, sizeof buf,
                       "%s{\"grid\": [%d, %d, %d], \"kernel\": \"%s\", \"register_ms\": %.4f, \"tma_ms\": %.4f, "
-                      "\"onchip\": %s, \"plane_ms\": %.4f, \"onchip_ms\": %.4f, \"split_pencil\": %s, "
-                      "\"split_plane\": %s, \"pair_ms\": [%.4f, %.4f, %.4f, %.4f]}",
+                      "\"onchip\": %s, \"plane_ms\": %.4f, \"onchip_ms\": %.4f",
                       firstc ? "" : ", ", c.geom.nx, c.geom.ny, c.geom.nz, kPencilNames[kind], c.pencil_ms[0],
-                      c.pencil_ms[1], oc ? "true" : "false", c.plane_ms, c.onchip_ms, sp & 1 ? "true" : "false",
-                      sp & 2 ? "true" : "false", c.pair_ms[0], c.pair_ms[1], c.pair_ms[2], c.pair_ms[3]);
+                      c.pencil_ms[1], oc ? "true" : "false", c.plane_ms, c.onchip_ms);
+        j += buf;
+        shorter += std::string(buf) + "}";
+        std::snprintf(buf, sizeof buf, ", \"split_pencil\": %s, \"split_plane\": %s, \"pair_ms\": [%.4f, %.4f, %.4f, %.4f]}",
+                      sp & 1 ? "true" : "false", sp & 2 ? "true" : "false", c.pair_ms[0], c.pair_ms[1], c.pair_ms[2], c.pair_ms[3]);
         j += buf;
         firstc = false;
     }
-    j += "], \"candidates\": [";
-    for (int k = 0; k < kAllCandidates; ++k) j += (k ? ", \"" : "\"") + candidate_name(k) + "\"";
-    j += "], \"candidate_ms_per_step\": [";
+    std::string end = "], \"candidates\": [";
+    for (int k = 0; k < kAllCandidates; ++k) end += (k ? ", \"" : "\"") + candidate_name(k) + "\"";
+    end += "], \"candidate_ms_per_step\": [";
     for (int k = 0; k < kAllCandidates; ++k) {
         std::snprintf(buf, sizeof buf, "%s%.4f", k ? ", " : "", tms[k]);
-        j += buf;
+        end += buf;
     }
-    ctx->plan_desc = j + "]}";
+    ctx->plan_short = shorter + end + "]}";
+    ctx->plan_desc = j + end + "]}";
     return BEC_OK;
 }
 
@@ -3055,9 +3060,10 @@ bec_status bec_step_plan(bec_ctx *ctx, char *out, int32_t len)
 {
     if (!ctx) return BEC_ERR_INVALID_ARG;
     if (!out || len < 1) return fail(ctx, BEC_ERR_INVALID_ARG, "null output");
-    const std::string d = ctx->path != BEC_PATH_FP32_BATCHED ? std::string("{\"plan\": \"plain path\"}")
+    std::string d = ctx->path != BEC_PATH_FP32_BATCHED ? std::string("{\"plan\": \"plain path\"}")
                           : ctx->plan_mode == -2 ? std::string("{\"plan\": \"not chosen (no step taken)\"}")
                                                  : ctx->plan_desc;
+    if ((int32_t)d.size() >= len && d == ctx->plan_desc) d = ctx->plan_short;
     if ((int32_t)d.size() >= len) return fail(ctx, BEC_ERR_INVALID_ARG, "output buffer too small");
     std::memcpy(out, d.c_str(), d.size() + 1);
     return BEC_OK;

@@ -193,7 +193,7 @@ class Engine:
     def step_plan(self):
         """The split-step schedule (bec_step_plan) as a dict."""
         import json
-        buf = C.create_string_buffer(4096)
+        buf = C.create_string_buffer(4096 + 512 * self.n_groups)
         self._check(lib().bec_step_plan(self._h, buf, len(buf)), "bec_step_plan")
         return json.loads(buf.value.decode())
 
