@@ -553,6 +553,7 @@ bec_status batched_zpass_all(bec_ctx *ctx, float frac, bool observe, bool ends_s
 }
 
 constexpr size_t kPlainScratch = (size_t)1 << 21;       // cells of each x-space copy of the FP64 path, at most
+constexpr size_t kPlainSpare = (size_t)1 << 30;
 constexpr size_t kKickTableBytes = (size_t)256 << 20;   // phase tables of a class of the general z pass, at most
 
 // the plane pass of one class; for a class whose steady step is one on-chip launch, that step
@@ -1524,33 +1525,38 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
         }
         CKA(dalloc(ctx, &ctx->d_plain_obs, (size_t)ctx->n_traj * ctx->max_nz * 4));
         CKA(dalloc(ctx, &ctx->d_plain_axial, (size_t)ctx->n_traj * ctx->max_nz * 4));
-        // the fused passes' tables, and x-space copies of as many trajectories as an observation takes at once; without
-        // room for them, one kernel per operation, and one trajectory
+        // the fused passes' tables (16 bytes a cell of each ensemble), and x-space copies of as many trajectories as an
+        // observation takes at once; without room for them, one kernel per operation, and one trajectory
         size_t elems = 0, wide = 0;
         for (auto &gr : ctx->groups)
             if (evo64_dims(gr.gd, gr.p.ne, gr.evo)) {
-                elems += (size_t)gr.evo.kick_elems();
+                elems += (size_t)gr.gd.cells;
                 wide = std::max(wide, std::min((size_t)gr.p.ne * gr.d.cells, kPlainScratch));
             }
         ctx->scratch_cells = std::max((size_t)ctx->max_cells, wide);
-        if (dalloc(ctx, &ctx->scratch_a, 2 * ctx->scratch_cells)) {
+        // (large tables are only taken where they leave a gigabyte to later calls)
+        const size_t bytes = sizeof(double2) * elems;
+        size_t left = 0, all = 0;
+        const bool fits = bytes < kPlainSpare || (cudaMemGetInfo(&left, &all) == cudaSuccess && left > bytes + kPlainSpare);
+        double2 *kick = nullptr;
+        if (fits && dalloc(ctx, &ctx->scratch_a, 2 * ctx->scratch_cells + elems) == cudaSuccess) {
+            kick = ctx->scratch_a + 2 * ctx->scratch_cells;
+        } else {
             cudaGetLastError();
             ctx->scratch_cells = (size_t)ctx->max_cells;
             CKA(dalloc(ctx, &ctx->scratch_a, 2 * ctx->scratch_cells));
         }
         ctx->scratch_b = ctx->scratch_a + ctx->scratch_cells;
-        double2 *kick = nullptr;
-        const bool room = dalloc(ctx, &kick, elems) == cudaSuccess;
         for (auto &gr : ctx->groups) {
             Evo64 &e = gr.evo;
             Gs64Tab t;
-            if (!e.ready || !room || get_gs64_tab(ctx, gr.gd, t)) {
+            if (!e.ready || !kick || get_gs64_tab(ctx, gr.gd, t)) {
                 e.ready = false;
                 continue;
             }
             e.x = t.x; e.y = t.y; e.z = t.z;
             e.kick = kick;
-            kick += e.kick_elems();
+            kick += gr.gd.cells;
             evo64_kick_table(e, ctx->stream);
         }
         cudaGetLastError();

@@ -136,8 +136,7 @@ struct Evo64 {
     int lppc = 0, lp = 0;                    // log2 of the planes and of the pencils per CTA
     bool ready = false;                      // false: one kernel per operation (plain_fp64.cu)
     const double2 *x = nullptr, *y = nullptr, *z = nullptr;   // all n twiddles W_n^k of each axis
-    double2 *kick = nullptr;                 // half-kick phases, kick_elems()
-    int kick_elems() const { return g.nz + g.nx * g.ny; }
+    double2 *kick = nullptr;                 // half-kick phases of every cell
 };
 // fills e.g and the tiles; false when a plane of both components or two pencils do not fit in shared memory
 bool evo64_dims(const GeomD &g, int n, Evo64 &e);

@@ -50,6 +50,10 @@ __device__ __forceinline__ void dft4(double2 &a, double2 &b, double2 &c, double2
     b = c;
     c = t;
 }
+// v / sqrt(2), rounded once. The double nearest to 1 / sqrt(2) is 4.8e-17 larger, which every radix-8 stage would put into a
+// quarter of its values: the population then grows by 1.3e-16 to 2.6e-16 a step (six transforms) on every grid, against a
+// few 1e-17 so or with radix-2 stages.
+__device__ __forceinline__ double over_root2(double v) { return fma(0x1.6a09e667f3bcdp-1, v, -0x1.bdd3413b26456p-55 * v); }
 // x[k] <- sum_n x[n] e^{-+2 pi i n k / R}, R = 2, 4, 8
 template <int R, bool INV>
 __device__ __forceinline__ void dft_small(double2 *x)
@@ -61,12 +65,11 @@ __device__ __forceinline__ void dft_small(double2 *x)
     } else {
         dft4<INV>(x[0], x[2], x[4], x[6]);      // even samples -> E0..E3 in x[0], x[2], x[4], x[6]
         dft4<INV>(x[1], x[3], x[5], x[7]);
-        const double h = 0.70710678118654752440;
         const double2 o0 = x[1], o1 = x[3], o2 = x[5], o3 = x[7];
         const double2 i1 = mul_i(o1, INV), i3 = mul_i(o3, INV);
-        const double2 t1 = make_double2(h * (o1.x + i1.x), h * (o1.y + i1.y));       // W o1
-        const double2 t2 = mul_i(o2, INV);                                           // W^2 o2
-        const double2 t3 = make_double2(h * (i3.x - o3.x), h * (i3.y - o3.y));       // W^3 o3
+        const double2 t1 = make_double2(over_root2(o1.x + i1.x), over_root2(o1.y + i1.y));       // W o1
+        const double2 t2 = mul_i(o2, INV);                                                       // W^2 o2
+        const double2 t3 = make_double2(over_root2(i3.x - o3.x), over_root2(i3.y - o3.y));       // W^3 o3
         const double2 e0 = x[0], e1 = x[2], e2 = x[4], e3 = x[6];
         x[0] = cadd(e0, o0); x[4] = csub(e0, o0);
         x[1] = cadd(e1, t1); x[5] = csub(e1, t1);
@@ -428,8 +431,10 @@ __global__ void k64_fold(const double *__restrict__ part, int n, int K, int firs
 // The two half kicks between steps are applied one after the other, so that a run has the same bits however it is cut
 // into calls. Where one kernel per operation and trajectory moved the state nine times a step, it moves twice. The plane
 // pass is bound by FP64 arithmetic (most of it exp, sincos and the normals): 15 us of a step of four 16x16x128
-// trajectories, whose pencil pass takes 7, near its latency. Measured, a step: 22.9 us for those four, 199 for 64, and 183
-// for eight of 32x32x256; with one kernel per operation and trajectory 565, 9154 and 1311.
+// trajectories, whose pencil pass takes 7, near its latency. Measured, a step: 22.7 us for those four, 201 for 64, and 184
+// for eight of 32x32x256; with one kernel per operation and trajectory 565, 9154 and 1311. Against an 80-bit reference the
+// states are as far off as with one kernel per operation (two 30-to-100-step runs of each of five grids: 5e-15 to 2.4e-14,
+// 8e-15 to 1.9e-14).
 
 // A CTA holds ppc planes of both components, the second's after the first's.
 //   E_STEP    state -> FFT_xy -> midpoint iteration (wigner_kernel.cu:184-229) and loss noise -> IFFT_xy -> state
@@ -551,8 +556,15 @@ __global__ void __launch_bounds__(256) k64_evo_plane(double2 *A, double2 *B, con
     }
 }
 
+// v times a kick's phase, with the fused multiply-adds written out: the same bits in every pass
+__device__ __forceinline__ double2 kicked(double2 v, double2 e)
+{
+    return make_double2(fma(v.x, e.x, -(v.y * e.y)), fma(v.x, e.y, v.y * e.x));
+}
+
 // A CTA holds 2^lp adjacent pencils of one component: [IFFT_z ->] scale -> `kicks` half kicks [-> FFT_z], from (sA, sB) to
-// (dA, dB), which may be the same. kick: e^{i k^2/2 dt/2}, nz of the kz, then nx ny of (kx, ky).
+// (dA, dB), which may be the same. kick: e^{i k^2/2 dt/2} of every cell (k64_evo_kick), copied beside the tile before the
+// predecessor ends.
 template <bool FROM_Z, bool TO_Z>
 __global__ void __launch_bounds__(256) k64_evo_pencil(const double2 *sA, const double2 *sB, double2 *dA, double2 *dB, int lx, int ly,
                                                       int lz, int lp, int n, const double2 *__restrict__ tz,
@@ -560,7 +572,7 @@ __global__ void __launch_bounds__(256) k64_evo_pencil(const double2 *sA, const d
 {
     extern __shared__ double2 sm64[];
     const int nz = 1 << lz, lplane = lx + ly, P = 1 << lp, chunk = nz << lp, ltiles = lplane - lp;
-    double2 *tw = sm64 + chunk, *ez = tw + nz, *exy = ez + nz;
+    double2 *tw = sm64 + chunk, *ek = tw + nz;
     const bool second = (int)blockIdx.x >= n << ltiles;
     const int blk = second ? blockIdx.x - (n << ltiles) : blockIdx.x;
     const int traj = blk >> ltiles, pen0 = (blk & ((1 << ltiles) - 1)) << lp;
@@ -568,10 +580,9 @@ __global__ void __launch_bounds__(256) k64_evo_pencil(const double2 *sA, const d
     const double2 *src = (second ? sB : sA) + off;
     double2 *dst = (second ? dB : dA) + off;
     for (int i = threadIdx.x; i < nz; i += blockDim.x) copy16(tw + i, tz + i);
-    if (kicks) {
-        for (int i = threadIdx.x; i < nz; i += blockDim.x) copy16(ez + i, kick + i);
-        if (threadIdx.x < P) copy16(exy + threadIdx.x, kick + nz + pen0 + threadIdx.x);
-    }
+    if (kicks)
+        for (int i = threadIdx.x; i < chunk; i += blockDim.x)
+            copy16(ek + i, kick + ((size_t)(i >> lp) << lplane) + pen0 + (i & (P - 1)));
     wait_predecessor();
     allow_successor();
     for (int i = threadIdx.x; i < chunk; i += blockDim.x)
@@ -583,9 +594,9 @@ __global__ void __launch_bounds__(256) k64_evo_pencil(const double2 *sA, const d
     for (int i = threadIdx.x; i < chunk; i += blockDim.x) {
         double2 u = cscale(sm64[i], scale);
         if (kicks) {
-            const double2 e = cmul(ez[i >> lp], exy[i & (P - 1)]);
-            u = cmul(u, e);
-            if (kicks > 1) u = cmul(u, e);
+            const double2 e = ek[i];
+            u = kicked(u, e);
+            if (kicks > 1) u = kicked(u, e);
         }
         if (TO_Z) sm64[i] = u;
         else dst[((size_t)(i >> lp) << lplane) + (i & (P - 1))] = u;
@@ -597,23 +608,18 @@ __global__ void __launch_bounds__(256) k64_evo_pencil(const double2 *sA, const d
         dst[((size_t)(i >> lp) << lplane) + (i & (P - 1))] = sm64[(digit_rev(i >> lp, lz) << lp) + (i & (P - 1))];
 }
 
-// e^{i k^2/2 dt/2} (propagateKSpaceRealTime, wigner_kernel.cu:137-151): nz of the kz, then nx ny of (kx, ky)
+// e^{i k^2/2 dt/2} of every cell (propagateKSpaceRealTime, wigner_kernel.cu:137-151), one sine and cosine each. As the product
+// of a (kx, ky) and a kz factor it had an error of the modulus that the many cells of a factor share, and with it the
+// population drifted by up to 1.3e-14 in 100 steps of 8x8x64; now by up to 5e-15, as with one kernel per operation. The pass
+// takes the same time, since a tile's phases are copied while the pass before it ends (a step of four 16x16x128 trajectories
+// 22.75 us with factors, 22.7).
 __global__ void k64_evo_kick(const GeomD g, double2 *__restrict__ kick)
 {
-    const int n = g.nz + g.nx * g.ny;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double k2;
-        if (i < g.nz) {
-            const double kz = getk<double>(i, g.dkz, g.nz);
-            k2 = kz * kz / 2.0;
-        } else {
-            const int pen = i - g.nz;
-            const double kx = getk<double>(pen & (g.nx - 1), g.dkx, g.nx);
-            const double ky = g.ly > 0 ? getk<double>(pen >> g.lx, g.dky, g.ny) : 0.0;
-            k2 = (kx * kx + ky * ky) / 2.0;
-        }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.cells; i += gridDim.x * blockDim.x) {
+        const double kx = getk<double>(i & (g.nx - 1), g.dkx, g.nx), kz = getk<double>(i >> (g.lx + g.ly), g.dkz, g.nz);
+        const double ky = g.ly > 0 ? getk<double>((i >> g.lx) & (g.ny - 1), g.dky, g.ny) : 0.0;
         double s, c;
-        sincos(k2 * g.dt_evo / 2.0, &s, &c);
+        sincos((kx * kx + ky * ky + kz * kz) / 2.0 * g.dt_evo / 2.0, &s, &c);
         kick[i] = make_double2(c, s);
     }
 }
@@ -623,7 +629,7 @@ size_t plane_smem(int lx, int ly, int lppc)
     return sizeof(double2) * ((((size_t)1 << (ly + lppc)) * ((1 << lx) + 1)) + ((size_t)1 << lx) + ((size_t)1 << ly));
 }
 size_t evo_plane_smem(int lx, int ly, int lppc) { return 2 * plane_smem(lx, ly, lppc); }    // (the twiddles' share is ample)
-size_t evo_pencil_smem(int lz, int lp) { return sizeof(double2) * (((size_t)1 << (lz + lp)) + ((size_t)2 << lz) + 8); }
+size_t evo_pencil_smem(int lz, int lp) { return sizeof(double2) * (((size_t)2 << (lz + lp)) + ((size_t)1 << lz)); }
 size_t pencil_smem(int lz, int lp) { return sizeof(double2) * (((size_t)1 << (lz + lp)) + ((size_t)2 << lz)); }
 constexpr size_t kMaxSmem = 200 * 1024;
 
@@ -691,7 +697,7 @@ bool evo64_dims(const GeomD &g, int n, Evo64 &e)
     e.g = g;
     e.lppc = std::max(0, std::min(8 - g.lx - g.ly, g.lz));
     e.lp = std::min(3, g.lx + g.ly);
-    while (e.lp > 1 && (((long long)2 * n << (g.lx + g.ly - e.lp)) < 148 || evo_pencil_smem(g.lz, e.lp) > 64 * 1024)) --e.lp;
+    while (e.lp > 1 && (((long long)2 * n << (g.lx + g.ly - e.lp)) < 148 || sizeof(double2) << (g.lz + e.lp) > 32 * 1024)) --e.lp;
     e.ready = g.lx >= 1 && g.lz >= 1 && g.lx <= 10 && g.ly <= 10 && g.lz <= 10 && evo_plane_smem(g.lx, g.ly, e.lppc) <= kMaxSmem &&
               evo_pencil_smem(g.lz, e.lp) <= kMaxSmem && ((long long)2 * n << (g.lx + g.ly - e.lp)) < (1ll << 31) &&
               ((long long)n << (g.lz - e.lppc)) < (1ll << 31);
@@ -700,7 +706,7 @@ bool evo64_dims(const GeomD &g, int n, Evo64 &e)
 
 void evo64_kick_table(const Evo64 &e, cudaStream_t s)
 {
-    k64_evo_kick<<<(e.kick_elems() + 127) / 128, 128, 0, s>>>(e.g, e.kick);
+    k64_evo_kick<<<std::min((e.g.cells + 127) / 128, 148 * 16), 128, 0, s>>>(e.g, e.kick);
     g_launches++;
 }
 
