@@ -680,7 +680,7 @@ long long total_cells(const bec_ctx *ctx)
 }
 
 bec_status capture_steps(bec_ctx *ctx, int k, cudaGraphExec_t *out, long long *kernels);
-bec_status check_step_error(bec_ctx *ctx);
+bec_status check_step_error(bec_ctx *ctx, bool tma = false);
 
 // ms of what enqueue() launches, replayed from a captured graph; left alone (-1) when it cannot be captured
 template <class F>
@@ -970,7 +970,7 @@ bec_status ensure_plan(bec_ctx *ctx)
                 cudaFree(save);
                 ctx->has_pulse = had_pulse;
                 if (st) return st;
-                if ((st = check_step_error(ctx))) return st;
+                if ((st = check_step_error(ctx, true))) return st;
                 how = "autotuned";
                 long long picks = 0;
                 for (size_t ci = 0; ci < ctx->classes.size() && ci < kPickClasses; ++ci) {
@@ -1089,12 +1089,15 @@ bec_status batched_resolve(bec_ctx *ctx)
 
 // Error flags of the fused step kernel (a dependency wait that gave up) and of the TMA pencil kernel (a tile
 // load wait that gave up); both kernels bound every wait.
-bec_status check_step_error(bec_ctx *ctx)
+bec_status check_step_error(bec_ctx *ctx, bool tma)
 {
     int err = 0;
     CKC(step_read_error(ctx->plan, &err, ctx->stream));
     if (err) return fail(ctx, BEC_ERR_CUDA, "fused step: a dependency wait gave up (state of that step is invalid)");
-    if (ctx->pencil_tuned && ctx->d_pflags) {
+    // (the flag is fetched where a class's steps run the TMA kernel: the copy and its wait take 12 us of every call)
+    for (auto &c : ctx->classes)
+        tma = tma || (ctx->pencil_tuned && c.pencil_kind == kPencilTma && !c.split_pencil && fp32_pencil_tma_supported(c.geom));
+    if (tma && ctx->d_pflags) {
         CKC(cudaMemcpyAsync(&err, ctx->d_pflags, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CKC(cudaStreamSynchronize(ctx->stream));
         if (err) {
