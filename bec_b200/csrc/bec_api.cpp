@@ -116,7 +116,7 @@ struct bec_ctx {
     double *d_plain_axial = nullptr;     // [n_traj][nzmax][4]
     double2 *scratch_a = nullptr, *scratch_b = nullptr;  // plain: x-space copies (scratch_cells each)
     size_t scratch_cells = 0;
-    float4 *scratch4 = nullptr;          // batched: one trajectory (max cells)
+    float4 *scratch4 = nullptr;          // batched: one trajectory (max cells), 32 bytes a cell
     int max_cells = 0, max_nz = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1612,7 +1612,7 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
                 if (cudaGetLastError() != cudaSuccess) return bail(BEC_ERR_CUDA);
             }
         }
-        CKA(dalloc(ctx, &ctx->scratch4, (size_t)ctx->max_cells));
+        CKA(dalloc(ctx, &ctx->scratch4, 2 * (size_t)ctx->max_cells));
         // the general z pass evaluates its phases in FP64: a table per ensemble where it stays small, given back when a later
         // buffer needs the room
         for (auto &c : ctx->classes) {
@@ -2896,15 +2896,13 @@ bec_status bec_get_state(bec_ctx *ctx, int32_t group, int32_t traj, double *ab)
     one.n_traj = 1;
     float2 *tx, *ty;
     if ((st = get_tw32_full(ctx, one.nx, &tx)) || (st = get_tw32_full(ctx, one.ny, &ty))) return st;
-    // one component after the other in FP64, straight to the caller: the scratch holds 16 bytes a cell. (A state of
-    // 16x16x128: 0.43 ms with the conversion on the host, 0.26 so.) The stored representation carries the unnormalised x-y
-    // inverse transform.
+    // both components in FP64 and one copy, straight to the caller. (A state of 2x2x512 takes 43 us and one of 16x16x128 225;
+    // with a pass and a copy per component 62 and 255 to 296, with the conversion on the host 50 and 250.) The stored
+    // representation carries the unnormalised x-y inverse transform.
     double2 *x = reinterpret_cast<double2 *>(ctx->scratch4);
-    for (int k = 0; k < 2; ++k) {
-        fp32_unprep_component(c.state + (size_t)(gr.local_first + traj) * cells, one, k, 1.0 / ((double)one.nx * one.ny), x, tx, ty, s);
-        CKL();
-        CKC(cudaMemcpyAsync(ab + (size_t)k * 2 * cells, x, sizeof(double2) * cells, cudaMemcpyDeviceToHost, s));
-    }
+    fp32_unprep_components(c.state + (size_t)(gr.local_first + traj) * cells, one, 1.0 / ((double)one.nx * one.ny), x, tx, ty, s);
+    CKL();
+    CKC(cudaMemcpyAsync(ab, x, sizeof(double2) * 2 * cells, cudaMemcpyDeviceToHost, s));
     CKC(cudaStreamSynchronize(s));
     return BEC_OK;
 }
