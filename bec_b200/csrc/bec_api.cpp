@@ -1296,15 +1296,17 @@ bec_status fetch_sample(bec_ctx *ctx, bec_moments *out, double *axial = nullptr,
     double *sums = ctx->d_group_mom + ng * 4;
     if (axial) {
         const int g0 = only < 0 ? 0 : only, g1 = only < 0 ? (int)ng : only + 1;
+        int longest = 0;
+        for (int g = g0; g < g1; ++g) longest = std::max(longest, ctx->groups[g].p.ne);
         if (ctx->path == BEC_PATH_FP64_PLAIN)
             // (the kernel counts groups from its arrays' start)
             group_axial(ctx->d_plain_axial, ctx->max_nz, nullptr, g1 - g0, ctx->d_group_first + g0, ctx->d_group_count + g0, 0,
-                        ctx->d_axial_off + g0, sums, ctx->stream);
+                        longest, ctx->d_axial_off + g0, sums, ctx->stream);
         for (auto &c : ctx->classes) {
             if (c.geom.n_traj == 0 || (only >= 0 && &c != &ctx->classes[ctx->groups[only].cls])) continue;
             const size_t i0 = only < 0 ? 0 : std::find(c.groups.begin(), c.groups.end(), only) - c.groups.begin();
             group_axial(c.traj_axial, c.geom.nz, c.d_groups + i0, only < 0 ? (int)c.groups.size() : 1, ctx->d_group_first,
-                        ctx->d_group_count, c.traj_offset, ctx->d_axial_off, sums, ctx->stream);
+                        ctx->d_group_count, c.traj_offset, longest, ctx->d_axial_off, sums, ctx->stream);
         }
         CKL();
     }

@@ -181,9 +181,9 @@ void fp32_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const
 void fp32_put_step(uint32_t *d_step, int n, uint32_t v, cudaStream_t s);
 int fp32_zpass_tiles(const ClassGeom &c);   // tiles per trajectory of an observing z pass (obs_partial layout)
 // for each of n groups g (groups[i], or i when NULL): traj_axial[traj][row][4] -> out + off[g], off[g + 1] - off[g] sums over
-// the count[g] trajectories from first[g] - base on
+// the count[g] <= longest trajectories from first[g] - base on
 void group_axial(const double *traj_axial, int row, const int *groups, int n, const int *first, const int *count, int base,
-                 const int *off, double *out, cudaStream_t s);
+                 int longest, const int *off, double *out, cudaStream_t s);
 // obs_partial[traj][tile][z][4] -> traj_axial[traj][z][4] * traj_scale[traj] (1 if NULL),
 // traj_tot[traj][4] = sum over z; traj_axial may be NULL
 void obs_reduce(const double *obs_partial, int n_traj, int tiles, int nz, const double *traj_scale,
