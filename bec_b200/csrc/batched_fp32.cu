@@ -264,20 +264,19 @@ __global__ void __launch_bounds__(256) k_prep(Cell *__restrict__ state, PlaneTil
     for (int i = threadIdx.x; i < 1 << lchunk; i += blockDim.x) state[first + i] = smw[T.reversed(i)];
 }
 
-// where x-space cells go: (a.re, a.im, b.re, b.im), or one component after the other, times scale, in FP64, as the caller of a
-// state wants it
+// where x-space cells go: (a.re, a.im, b.re, b.im), or the components times scale in FP64, as the caller of a state wants them
+// (NULL: not that one)
 struct ToCells {
     float4 *out;
     __device__ void operator()(size_t i, const Cell &v) const { out[i] = make_float4(v.ar, v.ai, v.br, v.bi); }
 };
 struct ToComponents {
-    double2 *out;
+    double2 *a, *b;
     double scale;
-    size_t cells;
     __device__ void operator()(size_t i, const Cell &v) const
     {
-        out[i] = make_double2(v.ar * scale, v.ai * scale);
-        out[cells + i] = make_double2(v.br * scale, v.bi * scale);
+        if (a) a[i] = make_double2(v.ar * scale, v.ai * scale);
+        if (b) b[i] = make_double2(v.br * scale, v.bi * scale);
     }
 };
 // stored representation -> FFT_xy -> x-space cells
@@ -623,10 +622,10 @@ void fp32_unprep(const float4 *state, const ClassGeom &c, float4 *x, const float
 {
     unprep(state, c, ToCells{x}, tx, ty, s);
 }
-void fp32_unprep_components(const float4 *state, const ClassGeom &c, double scale, double2 *x, const float2 *tx, const float2 *ty,
-                            cudaStream_t s)
+void fp32_unprep_components(const float4 *state, const ClassGeom &c, double scale, double2 *a, double2 *b, const float2 *tx,
+                            const float2 *ty, cudaStream_t s)
 {
-    unprep(state, c, ToComponents{x, scale, (size_t)c.cells * c.n_traj}, tx, ty, s);
+    unprep(state, c, ToComponents{a, b, scale}, tx, ty, s);
 }
 
 void fp32_ppass(float4 *state, const ClassGeom &c, const GroupParamsF *gp, const int *tgroup, const int *tlocal,

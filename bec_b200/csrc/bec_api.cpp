@@ -116,7 +116,8 @@ struct bec_ctx {
     double *d_plain_axial = nullptr;     // [n_traj][nzmax][4]
     double2 *scratch_a = nullptr, *scratch_b = nullptr;  // plain: x-space copies (scratch_cells each)
     size_t scratch_cells = 0;
-    float4 *scratch4 = nullptr;          // batched: one trajectory (max cells), 32 bytes a cell
+    float4 *scratch4 = nullptr;          // batched: one trajectory (max cells), and
+    size_t scratch4_cells = 0;           // ... twice a small one
     int max_cells = 0, max_nz = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -553,6 +554,7 @@ bec_status batched_zpass_all(bec_ctx *ctx, float frac, bool observe, bool ends_s
 }
 
 constexpr size_t kPlainScratch = (size_t)1 << 21;       // cells of each x-space copy of the FP64 path, at most
+constexpr size_t kBothComponents = (size_t)1 << 15;     // the FP32 path's scratch holds both components of states of up to half so many cells
 constexpr size_t kPlainSpare = (size_t)1 << 30;
 constexpr size_t kKickTableBytes = (size_t)256 << 20;   // phase tables of a class of the general z pass, at most
 
@@ -1507,7 +1509,8 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
     ctx->axial_off.assign(ng + 1, 0);
     for (int g = 0; g < ng; ++g) ctx->axial_off[g + 1] = ctx->axial_off[g] + (size_t)4 * ctx->groups[g].d.nvz;
     if (ctx->axial_off[ng] > (size_t)INT_MAX) return bail(BEC_ERR_OUT_OF_MEMORY);
-    CKA(dalloc(ctx, &ctx->d_group_mom, (size_t)ng * 4 + ctx->axial_off[ng]));
+    const size_t n_sample = (size_t)ng * 4 + ctx->axial_off[ng];
+    if (path == BEC_PATH_FP64_PLAIN) CKA(dalloc(ctx, &ctx->d_group_mom, n_sample));
     CKA(dalloc(ctx, &ctx->d_axial_off, (size_t)ng + 1));
     {
         const std::vector<int> off(ctx->axial_off.begin(), ctx->axial_off.end());
@@ -1583,7 +1586,18 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
         for (auto &c : ctx->classes) {
             const size_t nt = (size_t)c.geom.n_traj;
             c.tiles = fp32_zpass_tiles(c.geom);
-            CKA(dalloc(ctx, &c.state, nt * c.geom.cells));
+            // the scratch and the samples' buffer lie behind the first class's state: an allocation of a megabyte or more
+            // takes 0.3 ms of a context's 0.4 to 2
+            const bool first = &c == &ctx->classes[0];
+            const size_t cells = nt * c.geom.cells;
+            ctx->scratch4_cells = std::max((size_t)ctx->max_cells, std::min(2 * (size_t)ctx->max_cells, kBothComponents));
+            const size_t behind =
+                first ? ctx->scratch4_cells + (n_sample * sizeof(double) + sizeof(float4) - 1) / sizeof(float4) : 0;
+            CKA(dalloc(ctx, &c.state, cells + behind));
+            if (first) {
+                ctx->scratch4 = c.state + cells;
+                ctx->d_group_mom = reinterpret_cast<double *>(ctx->scratch4 + ctx->scratch4_cells);
+            }
             CKA(cudaMemsetAsync(c.state, 0, sizeof(float4) * nt * c.geom.cells, ctx->stream));
             CKA(dalloc(ctx, &c.d_tgroup, nt));
             CKA(dalloc(ctx, &c.d_tlocal, nt));
@@ -1614,7 +1628,6 @@ bec_status bec_create(const bec_params *groups, int32_t n_groups, int32_t path, 
                 if (cudaGetLastError() != cudaSuccess) return bail(BEC_ERR_CUDA);
             }
         }
-        CKA(dalloc(ctx, &ctx->scratch4, 2 * (size_t)ctx->max_cells));
         // the general z pass evaluates its phases in FP64: a table per ensemble where it stays small, given back when a later
         // buffer needs the room
         for (auto &c : ctx->classes) {
@@ -2898,13 +2911,18 @@ bec_status bec_get_state(bec_ctx *ctx, int32_t group, int32_t traj, double *ab)
     one.n_traj = 1;
     float2 *tx, *ty;
     if ((st = get_tw32_full(ctx, one.nx, &tx)) || (st = get_tw32_full(ctx, one.ny, &ty))) return st;
-    // both components in FP64 and one copy, straight to the caller. (A state of 2x2x512 takes 43 us and one of 16x16x128 225;
-    // with a pass and a copy per component 62 and 255 to 296, with the conversion on the host 50 and 250.) The stored
-    // representation carries the unnormalised x-y inverse transform.
+    // in FP64 straight to the caller: both components of a small state in one pass and one copy, those of a larger one in turn.
+    // (A state of 2x2x512 takes 43 us; with a pass and a copy per component 62, with the conversion on the host 50.) The
+    // stored representation carries the unnormalised x-y inverse transform.
     double2 *x = reinterpret_cast<double2 *>(ctx->scratch4);
-    fp32_unprep_components(c.state + (size_t)(gr.local_first + traj) * cells, one, 1.0 / ((double)one.nx * one.ny), x, tx, ty, s);
-    CKL();
-    CKC(cudaMemcpyAsync(ab, x, sizeof(double2) * 2 * cells, cudaMemcpyDeviceToHost, s));
+    const float4 *from = c.state + (size_t)(gr.local_first + traj) * cells;
+    const double scale = 1.0 / ((double)one.nx * one.ny);
+    const bool both = 2 * (size_t)cells <= ctx->scratch4_cells;
+    for (int k = 0; k < (both ? 1 : 2); ++k) {
+        fp32_unprep_components(from, one, scale, k ? nullptr : x, both ? x + cells : k ? x : nullptr, tx, ty, s);
+        CKL();
+        CKC(cudaMemcpyAsync(ab + (size_t)k * 2 * cells, x, sizeof(double2) * (both ? 2 : 1) * cells, cudaMemcpyDeviceToHost, s));
+    }
     CKC(cudaStreamSynchronize(s));
     return BEC_OK;
 }

@@ -163,9 +163,9 @@ void fp32_init_batched(float4 *state, const ClassGeom &c, const int *tgroup, con
 // x-space cells (a.re, a.im, b.re, b.im) -> stored representation (inverse transform over x and y), and back
 void fp32_prep(float4 *state, const ClassGeom &c, const float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s);
 void fp32_unprep(const float4 *state, const ClassGeom &c, float4 *x, const float2 *tx, const float2 *ty, cudaStream_t s);
-// every a, then every b, in FP64, times scale: 32 bytes a cell
-void fp32_unprep_components(const float4 *state, const ClassGeom &c, double scale, double2 *x, const float2 *tx, const float2 *ty,
-                            cudaStream_t s);
+// the components in FP64, times scale; a or b may be NULL
+void fp32_unprep_components(const float4 *state, const ClassGeom &c, double scale, double2 *a, double2 *b, const float2 *tx,
+                            const float2 *ty, cudaStream_t s);
 // kinetic phases of every cell of n_groups ensembles of a class (groups: their indices, device) for kick fraction frac
 void fp32_kick_table(float2 *tab, const ClassGeom &c, const GroupParamsF *gp, const int *groups, int n_groups, float frac,
                      cudaStream_t s);
