@@ -2042,7 +2042,18 @@ bec_status gs_batched(bec_ctx *ctx, int n, const int32_t *groups, const bec_gs_o
         hp[g].mu = (float)d.mu;
     }
     std::vector<void *> tmp_allocs;
-    struct Free { std::vector<void *> &v; cudaStream_t s; ~Free() { cudaStreamSynchronize(s); for (void *p : v) cudaFree(p); } } fr{tmp_allocs, s};
+    std::vector<std::pair<void *, size_t>> borrowed;      // of the evolution's state, which is zero until it is initialised
+    struct Free {
+        std::vector<void *> &v;
+        std::vector<std::pair<void *, size_t>> &borrowed;
+        cudaStream_t s;
+        ~Free()
+        {
+            cudaStreamSynchronize(s);
+            for (void *p : v) cudaFree(p);
+            for (auto &b : borrowed) cudaMemsetAsync(b.first, 0, b.second, s);
+        }
+    } fr{tmp_allocs, borrowed, s};
     auto talloc = [&](void **p, size_t bytes) -> cudaError_t {
         cudaError_t e = cudaMalloc(p, bytes > 0 ? bytes : 16);
         if (e == cudaSuccess) tmp_allocs.push_back(*p);
@@ -2075,6 +2086,7 @@ bec_status gs_batched(bec_ctx *ctx, int n, const int32_t *groups, const bec_gs_o
         if (blank && home && home->state && nt <= (size_t)home->geom.n_traj) {
             c.state = reinterpret_cast<float2 *>(home->state);
             c.out = c.state + nt * cells;
+            borrowed.push_back({c.state, 2 * sizeof(float2) * nt * cells});
         } else {
             CKC(talloc((void **)&c.state, sizeof(float2) * nt * cells));
             CKC(talloc((void **)&c.out, sizeof(float2) * nt * cells));
