@@ -23,8 +23,6 @@ namespace {
 const double kHbar = 1.054571628e-34;   // wigner.cpp:121
 const double kBohr = 5.2917720859e-11;  // wigner.cpp:122
 
-// Neumaier-compensated host accumulator
-
 bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 int ilog2(int n) { int r = 0; while ((1 << r) < n) ++r; return r; }
 

@@ -22,28 +22,6 @@ BEC_HD float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); 
 BEC_HD double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 BEC_HD float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 
-// float4 holds (a.re, a.im, b.re, b.im): both components of one cell (reordered from the stored order by
-// the kernels of batched_fp32.cu).
-BEC_HD float4 pmul(float4 v, float2 w)
-{
-    return make_float4(v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x,
-                       v.z * w.x - v.w * w.y, v.z * w.y + v.w * w.x);
-}
-BEC_HD float4 padd(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
-BEC_HD float4 psub(float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
-BEC_HD float4 pscale(float4 a, float s) { return make_float4(a.x * s, a.y * s, a.z * s, a.w * s); }
-
-// Twiddle multiply used by the FFT stages, overloaded on the element type.
-BEC_HD double2 tmul(double2 v, double2 w) { return cmul(v, w); }
-BEC_HD float2 tmul(float2 v, float2 w) { return cmul(v, w); }
-BEC_HD float4 tmul(float4 v, float2 w) { return pmul(v, w); }
-BEC_HD double2 vadd(double2 a, double2 b) { return cadd(a, b); }
-BEC_HD float2 vadd(float2 a, float2 b) { return cadd(a, b); }
-BEC_HD float4 vadd(float4 a, float4 b) { return padd(a, b); }
-BEC_HD double2 vsub(double2 a, double2 b) { return csub(a, b); }
-BEC_HD float2 vsub(float2 a, float2 b) { return csub(a, b); }
-BEC_HD float4 vsub(float4 a, float4 b) { return psub(a, b); }
-
 // ---------------------------------------------------------------- Philox4x32-10
 // Counter-based generator of Salmon, Moraes, Dror and Shaw (SC'11):
 // ten rounds of two 32x32->64 multiplies with Weyl-sequence key bumps.
