@@ -433,8 +433,8 @@ __global__ void k64_fold(const double *__restrict__ part, int n, int K, int firs
 // pass is bound by FP64 arithmetic (most of it exp, sincos and the normals): 15 us of a step of four 16x16x128
 // trajectories, whose pencil pass takes 7, near its latency. Measured, a step: 22.7 us for those four, 201 for 64, and 184
 // for eight of 32x32x256; with one kernel per operation and trajectory 565, 9154 and 1311. Against an 80-bit reference the
-// states are as far off as with one kernel per operation (two 30-to-100-step runs of each of five grids: 5e-15 to 2.4e-14,
-// 8e-15 to 1.9e-14).
+// states are as far off as with one kernel per operation (nine runs of 20 to 100 steps on five grids: median 8.1e-15 of
+// the state, 1.1e-14).
 
 // A CTA holds ppc planes of both components, the second's after the first's.
 //   E_STEP    state -> FFT_xy -> midpoint iteration (wigner_kernel.cu:184-229) and loss noise -> IFFT_xy -> state

@@ -30,8 +30,9 @@ struct GsArgs {
 // 2^LP pencils a trajectory. STEADY: the pass between two steps (two equal kicks, the norm); otherwise the fractions differ
 // and norm and ekin may be null.
 //
-// Both passes are bound by latency at the few warps that a line of 16 or 32 complex values a thread leaves room for (DRAM
-// runs at 30 % of its rate). What counts is registers and instructions: with the shared lines padded by one element instead
+// On 256 states of 32x32x256 the pencil pass moves 1.01 GB in 229 us, 69 % of the measured HBM copy rate, and the plane pass as
+// much in 260 us, 60 % (ncu, one launch each): what keeps them from the memory is the few warps that a line of 16 or 32
+// complex values a thread leaves room for. So registers and instructions count: with the shared lines padded by one element instead
 // of swizzled, and the grid's sizes known to the compiler, every shared and global access has an address and a constant
 // offset. The nz = 256 pencil pass then fits four CTAs an SM at 64 registers without a spill (three at 80 with one before),
 // the 32 x 32 plane pass five at 96 (four at 128). A step of 256 states of 32x32x256: 633 us before, 487 here; of 200 of

@@ -535,8 +535,8 @@ def main():
             issue_roof = {"kernel": dom["kernel"], "thread_instructions_per_cell": NCU_INSTR_PER_CELL[dom["kernel"]],
                           "achieved": ach, "peak": pk, "unit": "thread-instr/s", "frac": ach / pk,
                           "note": "instruction issue (a third of the instructions are packed FMAs, which take the FMA pipe "
-                                  "twice as long: that pipe is the nearer bound): one warp-instruction per scheduler "
-                                  "per clock at the sampled SM clock; instructions per cell from ncu"}
+                                  "twice as long: ncu has that pipe active 55 % of the cycles): one warp-instruction per "
+                                  "scheduler per clock at the sampled SM clock; instructions per cell from ncu"}
     # the transforms' FLOPs (5 n log2 n per complex transform of n points; two components, one inverse and
     # one forward 3D transform per step) against the FP32 FMA pipes: the compute bound beside the HBM bound
     flop_roof = None
